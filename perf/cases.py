@@ -107,16 +107,20 @@ def _denoiser(c, seed, p):
     return net
 
 
+def _attention_inputs(c, gen):
+    B, H, D, dt = c["B"], c["H"], c["D"], DTYPES[c["dtype"]]
+    mk = lambda L, s: _normal(gen, (B, L, H, D), s, dt)  # the denoiser's memory order
+    q, k, v = mk(c["Lq"], D ** -0.5), mk(c["Lk"], 1.0), mk(c["Lk"], 1.0)
+    tq, tk, tv = mk(c["Lq"], 0.1), mk(c["Lk"], 0.1), mk(c["Lk"], 0.1)
+    return q, k, v, tq, tk, tv, mk(c["Lq"], 1.0), mk(c["Lq"], 1.0)
+
+
 def prepare(c, seed):
     gen = torch.Generator(device="cuda").manual_seed(seed)
     kind = c["kind"]
     if kind in ("attention", "plan"):
-        dt = DTYPES[c["dtype"]]
-        B, H, D = c["B"], c["H"], c["D"]
-        mk = lambda L, s: _normal(gen, (B, L, H, D), s, dt)  # the denoiser's memory order
-        q, k, v = mk(c["Lq"], D ** -0.5), mk(c["Lk"], 1.0), mk(c["Lk"], 1.0)
-        tq, tk, tv = mk(c["Lq"], 0.1), mk(c["Lk"], 0.1), mk(c["Lk"], 0.1)
-        g_o, g_to = mk(c["Lq"], 1.0), mk(c["Lq"], 1.0)
+        q, k, v, tq, tk, tv, g_o, g_to = _attention_inputs(c, gen)
+        B, H = c["B"], c["H"]
         st = {"case": c}
         if kind == "attention":
             to = (lambda t: t) if c["entry"] == "safe" else (lambda t: t.transpose(1, 2))
@@ -300,3 +304,169 @@ def tolerance(c):
     if kind == "vocabulary":
         return {"rel": 0.01}
     return {"rel": 0.05}
+
+
+# ------------------------------------------------------------------------------------------------------------ in 64 bits
+def exact(c, seed):
+    """What ``run`` returns, from plain torch in 64 bits; ``None`` for what depends on generated dropout masks and for the
+    training step."""
+    kind = c["kind"]
+    if kind in ("attention", "plan"):
+        return _exact_attention(c, seed)
+    if kind == "block_ops":
+        return _exact_block(c, prepare(c, seed))
+    if kind == "vocabulary":
+        return _exact_vocabulary(c, prepare(c, seed))
+    return _exact_denoiser(c, prepare(c, seed)) if kind == "denoiser" else None
+
+
+def _exact_attention(c, seed):
+    gen = torch.Generator(device="cuda").manual_seed(seed)
+    x = [t.transpose(1, 2) for t in _attention_inputs(c, gen)]
+    B, H, Lq, Lk, D = c["B"], c["H"], c["Lq"], c["Lk"], c["D"]
+    r = D ** -0.5
+    outs = [torch.zeros(t.shape, dtype=torch.float64, device="cuda") for t in (x[0], x[0], *x[:6])]
+    y, ty, dq, dk, dv, dtq, dtk, dtv = outs
+    stats = torch.zeros(2, B, H, -(-Lq // 128) * 128, dtype=torch.float64, device="cuda")
+    T = lambda t: t.transpose(-1, -2)
+    for b in range(B):
+        step = max(1, int(2e8 // (Lq * Lk)))
+        for h in range(0, H, step):
+            i = (b, slice(h, h + step))
+            q, k, v, tq, tk, tv, g, G = (t[i].double() for t in x)
+            s = (q @ T(k)) * r
+            stats[0][i][:, :Lq] = lse = s.logsumexp(-1)
+            p = torch.exp(s.sub_(lse[..., None]))
+            n = (tq @ T(k) + q @ T(tk)) * r
+            mu = (p * n).sum(-1, keepdim=True)
+            stats[1][i][:, :Lq] = mu[..., 0]
+            n -= mu
+            y[i] = p @ v
+            ty[i] = (p * n) @ v + p @ tv
+            if c["cot"] == "primal":
+                dv[i] = T(p) @ g
+                w = p * (g @ T(v) - (g * y[i]).sum(-1, keepdim=True)) * r
+                dq[i], dk[i] = w @ k, T(w) @ q
+                continue
+            if c["cot"] == "tangent":
+                g = torch.zeros_like(g)
+            a = G @ T(v) - (G * y[i]).sum(-1, keepdim=True)
+            w = (a * n + G @ T(tv) + g @ T(v) - (G * ty[i] + g * y[i]).sum(-1, keepdim=True)) * p * r
+            dtv[i] = T(p) @ G
+            dv[i] = T(p * n) @ G + T(p) @ g
+            u = a.mul_(p).mul_(r)
+            dtq[i], dtk[i] = u @ k, T(u) @ q
+            dq[i], dk[i] = u @ tk + w @ k, T(u) @ tq + T(w) @ q
+    if c["kind"] == "plan":
+        return [y, ty, *stats, *outs[2:]]
+    if c["entry"] == "safe":
+        y, ty, *grads = [t.transpose(1, 2) for t in outs]
+    else:
+        grads = outs[2:]
+    return [y, *grads[:3]] if c["cot"] == "primal" else [y, ty, *grads]
+
+
+def _rotate(t, cos, sin):
+    t1, t2 = t.chunk(2, dim=-1)
+    cos, sin = cos[None, :, None], sin[None, :, None]
+    return torch.cat((t1 * cos - t2 * sin, t1 * sin + t2 * cos), dim=-1)
+
+
+def _exact_block(c, st):
+    F = torch.nn.functional
+    cos, sin = st["cos"].double(), st["sin"].double()
+    C = c["C"]
+
+    def chain(w, b, x, qkv, branch, mlp, mod):
+        shift, scale, gate = mod.chunk(3, dim=2)
+        q, k, v = qkv.unbind(2)
+        return (F.layer_norm(x, (C,), w, b, st["norm"].eps) * (1 + scale) + shift, _rotate(q, cos, sin), _rotate(k, cos, sin),
+                v.clone(), x + branch * gate, F.gelu(mlp, approximate="tanh"))
+
+    leaf = lambda t: t.detach().double().requires_grad_(True)
+    prim = [leaf(t) for t in st["prim"].values()]
+    wb = [leaf(st["norm"].weight), leaf(st["norm"].bias)]
+    g = [t.double() for t in st["g"]]
+    if c["dual"]:
+        tang = [leaf(t) for t in st["tang"].values()]
+        ys, tys = torch.func.jvp(lambda *a: chain(*wb, *a), tuple(prim), tuple(tang))
+        outs, wrt = [*ys, *tys], [*prim, *tang, *wb]
+        g += [t.double() for t in st["gt"]]
+    else:
+        outs, wrt = list(chain(*wb, *prim)), [*prim, *wb]
+    grads = list(torch.autograd.grad(outs, wrt, g))
+    outs = [t.detach() for t in outs]
+    if c["p"] > 0:  # the gated residual and the gradients of its branch and of the modulation depend on the masks
+        for i in range(0, len(outs), 6):
+            outs[i + 4] = None
+        for i in range(0, len(grads) - 2, 5):
+            grads[i + 2] = grads[i + 4] = None
+    return [*outs, *grads]
+
+
+def _exact_vocabulary(c, st):
+    sd, V = c["sd"], c["V"]
+    W = st["pred"].shape[-1]
+    pad = lambda t: torch.nn.functional.pad(t, (0, W - V))
+    col = lambda t: t.double().view(-1, 1, 1)
+
+    def mix(x0, ids, t):
+        x = x0.double() * (1 - col(t))
+        return x.scatter_add_(-1, ids[..., None], col(t).expand(*ids.shape, 1).contiguous())
+
+    def smooth(ids, logp):
+        return -((1 - c["eps"]) * logp.gather(-1, ids[..., None])[..., 0] + c["eps"] * logp.mean(-1)).mean()
+
+    ids, s, t = st["ids"], st["s"], st["t"][:sd]
+    xt = pad(mix(st["x0"][sd:], ids[sd:], st["t"][sd:]))
+    pred = st["pred"].detach().double().requires_grad_(True)
+    ce = smooth(ids[sd:], pred[..., :V].log_softmax(-1))
+    d_pred, = torch.autograd.grad(ce, [pred])
+    xs = mix(st["x0"][:sd], ids[:sd], s)
+    l, tl = (st[n].detach().double().requires_grad_(True) for n in ("l", "tl"))
+    p, u = l[..., :V].softmax(-1), tl[..., :V]
+    ddt = 1 / (1 - col(s) + 1e-8)
+    dt = (col(t) - col(s)) * ddt
+    xst = (xs + dt * (p - xs)).detach()
+    dv = ddt * (p - xs) + dt * p * (u - (p * u).sum(-1, keepdim=True))
+    lag = ((1 - col(t)) * dv - st["target"][..., :V].double().softmax(-1) + xst).square().sum(-1).mean()
+    d_l, d_tl = torch.autograd.grad(lag, [l, tl])
+    lse = l.detach()[..., :V].logsumexp(-1).flatten()
+    return [xt, ce.detach(), pad(xs), pad(xst), lse, lag.detach(), d_pred, d_l, d_tl]
+
+
+def _exact_denoiser(c, st):
+    F = torch.nn.functional
+    w = {n: t.double() for n, t in st["net"].state_dict().items()}
+    lin = lambda n, x: F.linear(x, w[n + ".weight"], w.get(n + ".bias"))
+    norm = lambda n, x: F.layer_norm(x, x.shape[-1:], w[n + ".weight"], w[n + ".bias"])
+    gelu = lambda x: F.gelu(x, approximate="tanh")
+    B, L, V = c["B"], c["L"], c["V"]
+    s, t = st["s"].double(), st["t"].double()
+
+    def clock(n, v):
+        a = v[:, None] * w[n + ".freqs"][None]
+        return lin(n + ".mlp.2", F.silu(lin(n + ".mlp.0", torch.cat((a.cos(), a.sin()), -1))))
+
+    x = st["noise"]["x0"].double() * (1 - s.view(-1, 1, 1))
+    x.scatter_add_(-1, st["x1"][..., None], s.view(-1, 1, 1).expand(B, L, 1).contiguous())
+    cond = F.silu(clock("s_map", s)) + F.silu(clock("t_map", t - s))
+    with torch.no_grad():
+        if V < 512:
+            h = lin("embed.proj", x * torch.rsqrt(s ** 2 + (1 - s) ** 2 * V + 1e-6).view(-1, 1, 1))
+            h = h + 0.1 * lin("embed.mlp.2", gelu(lin("embed.mlp.0", h)))
+            h = (1 + lin("embed.gamma", cond)[:, None]) * h + lin("embed.beta", cond)[:, None]
+            h = F.rms_norm(h, h.shape[-1:], w["embed.norm.weight"], 1e-8)
+        else:
+            h = lin("embed.seq", x * V ** -0.5)
+        for i in range(c["blocks"]):
+            n = "blocks.%d." % i
+            sh1, sc1, g1, sh2, sc2, g2 = lin(n + "ada", cond)[:, None].chunk(6, dim=2)
+            q, k, v = lin(n + "attn_qkv", norm(n + "norm1", h) * (1 + sc1) + sh1).view(B, L, 3, 12, 64).unbind(2)
+            q, k, v = (z.transpose(1, 2) for z in (_rotate(q, w["cos"], w["sin"]), _rotate(k, w["cos"], w["sin"]), v))
+            a = (torch.softmax(q @ k.transpose(-1, -2) / 8, -1) @ v).transpose(1, 2).reshape(B, L, 768)
+            h = h + lin(n + "attn_out", a) * g1
+            m = lin(n + "mlp.2", gelu(lin(n + "mlp.0", norm(n + "norm2", h) * (1 + sc2) + sh2)))
+            h = h + m * g2
+        shift, scale = lin("ada_out", cond)[:, None].chunk(2, dim=2)
+        return lin("head", norm("norm_out", h) * (1 + scale) + shift)
