@@ -30,6 +30,9 @@
 //               write-back over consumed score columns, epilogue.  Four threads per row where a tile has 64
 //               columns (18 warps): the algebra is a chain of tensor-memory reads, exponentials and tensor-memory
 //               writes, and with two warps per scheduler its latency, not its instruction count, set the tile time
+//
+// kPair = true serves head dimensions between the two tile widths (see sm100_head_dim_ok): the four operands go into
+// the output products as a 16-bit value plus the 16-bit rounding of what is left of it, two products per operand.
 #include <algorithm>
 
 #include "jvpattn_common.cuh"
@@ -94,6 +97,7 @@ struct BwdKernelArgs {
   const float *delta, *dsum;
   unsigned int *status;
   long long wait_cycles;           // budget of every bounded wait
+  int D;                           // channels of a head (the tiles may be wider)
   int B, H, Lx, Ly, Lq, stat_len;  // Lx rows on the owner side, Ly on the streamed side
   int xmask, ymask;             // which of the four X / Y tensors are loaded
   int has_t, has_o;
@@ -110,7 +114,7 @@ __global__ void __launch_bounds__(256) row_dots_kernel(BwdArgs a, float *delta, 
   const int64_t r = gid / kTpr;
   const int part = (int)(gid % kTpr);
   float d1 = 0.f, d2 = 0.f;
-  const bool live = r < nrows;
+  const bool live = r < nrows && part * 8 < a.D;  // heads narrower than the tile: the threads past the end add zero
   int b = 0, h = 0, i = 0;
   if (live) {
     i = (int)(r % a.Lq);
@@ -151,7 +155,7 @@ __global__ void __launch_bounds__(256) row_dots_kernel(BwdArgs a, float *delta, 
   }
 }
 
-template <int D, int TILE, bool kKV, bool kDoK, bool kDoV, typename T>
+template <int D, int TILE, bool kKV, bool kDoK, bool kDoV, typename T, bool kPair>
 __global__ void __launch_bounds__(bwd_threads(bwd_parts(TILE))) sm100_bwd_kernel(const __grid_constant__ BwdMaps maps, BwdKernelArgs a) {
   constexpr int kParts = bwd_parts(TILE);
   constexpr int kComputeThreads = 128 * kParts;
@@ -171,7 +175,8 @@ __global__ void __launch_bounds__(bwd_threads(bwd_parts(TILE))) sm100_bwd_kernel
   // instead of when the output products have consumed the operands written over it.
   constexpr bool kSplit = !kKV;
   constexpr uint32_t kColW = kAcc * D + 4 * TILE;
-  constexpr uint32_t kUsed = kColW + (kSplit ? 2 * TILE : 0);
+  constexpr uint32_t kWBuf = kPair ? 2 * TILE : TILE;  // columns of one buffer: W1, W2, each with its low parts where kPair
+  constexpr uint32_t kUsed = kColW + (kSplit ? 2 * kWBuf : 0);
   static_assert(kUsed <= 512, "TMEM budget");
   constexpr uint32_t kTmemCols = kUsed <= 256 ? 256 : 512;
   constexpr bool kBf16 = IsBf16<T>::value;
@@ -413,7 +418,8 @@ __global__ void __launch_bounds__(bwd_threads(bwd_parts(TILE))) sm100_bwd_kernel
       };
       // the thread that owned score columns [16 kk, 16 kk + 16) left its 8 packed operand columns at the start
       // of its own column range (see the score-algebra warps)
-      auto oa = [&](int kk) -> uint32_t { return ((16 * kk) / CH) * CH + ((16 * kk) % CH) / 2; };
+      // (kPair: every 16 score columns became 8 packed columns of high parts and 8 of low parts, in place)
+      auto oa = [&](int kk) -> uint32_t { return kPair ? 16 * kk : ((16 * kk) / CH) * CH + ((16 * kk) % CH) / 2; };
       if constexpr (kSplit) {
         // ---- query owner: two issuers and a chain-free schedule.
         // Measured per 64-key tile with one issuer: the score algebra needed ~1570 cycles, the tensor pipe ~1280, but a
@@ -489,8 +495,27 @@ __global__ void __launch_bounds__(bwd_threads(bwd_parts(TILE))) sm100_bwd_kernel
             }
             tc_fence_after();
             const uint32_t ylo_out = ybase(st);
-            const uint32_t w1 = tmem + kColW + (uint32_t)(g & 1) * TILE, w2 = w1 + TILE / 2;
-            if (acc_merge) {
+            const uint32_t w1 = tmem + kColW + (uint32_t)(g & 1) * kWBuf, w2 = w1 + kWBuf / 2;
+            if constexpr (kPair) {
+              constexpr uint32_t kLow = TILE / 2;  // low parts behind the high parts
+              bool init0 = j > 0;
+#pragma unroll
+              for (int kk = 0; kk < TILE / 16; ++kk) {
+#pragma unroll
+                for (uint32_t part = 0; part <= kLow; part += kLow) {
+                  if (acc_merge) {
+                    mma_ts_lo(tmem + kColKd, w1 + part + 8 * kk, yb(ylo_out, 0, kk), idesc_o2, init0);
+                    init0 = true;
+                  } else if (has_t) {
+                    mma_ts_lo(tmem + kColKd, w1 + part + 8 * kk, yb(ylo_out, 0, kk), idesc_o, init0);
+                    mma_ts_lo(tmem + kColK, w1 + part + 8 * kk, yb(ylo_out, 1, kk), idesc_o, init0);
+                    init0 = true;
+                  }
+                  mma_ts_lo(tmem + kColK, w2 + part + 8 * kk, yb(ylo_out, 0, kk), idesc_o, init0);
+                  init0 = true;
+                }
+              }
+            } else if (acc_merge) {
               const bool acc = j > 0;
 #pragma unroll
               for (int kk = 0; kk < TILE / 16; ++kk) {
@@ -560,7 +585,32 @@ __global__ void __launch_bounds__(bwd_threads(bwd_parts(TILE))) sm100_bwd_kernel
         const uint32_t ylo_out = ybase(st);
         // (the common case, both cotangents present, is issued as straight-line code: a run-time condition between
         //  two instructions of a group costs this thread tens of cycles per instruction)
-        if (kDoV && kMerge && has_t && has_o) {
+        if constexpr (kPair) {
+          if (kDoV) {
+#pragma unroll
+            for (int kk = 0; kk < TILE / 16; ++kk) {
+#pragma unroll
+              for (uint32_t part = 0; part <= 8; part += 8) {
+                const uint32_t p = tmem + kColS + oa(kk) + part, pn = tmem + kColSd + oa(kk) + part;
+                if (kMerge && has_t && has_o) {
+                  mma_ts_lo(tmem + kColVd, p, yb(ylo_out, 2, kk), idesc_o2, initvd);
+                  mma_ts_lo(tmem + kColV, pn, yb(ylo_out, 2, kk), idesc_o, true);
+                  initv = initvd = true;
+                } else {
+                  if (has_t) {
+                    mma_ts_lo(tmem + kColVd, p, yb(ylo_out, 2, kk), idesc_o, initvd);
+                    mma_ts_lo(tmem + kColV, pn, yb(ylo_out, 2, kk), idesc_o, initv);
+                    initv = initvd = true;
+                  }
+                  if (has_o) {
+                    mma_ts_lo(tmem + kColV, p, yb(ylo_out, 3, kk), idesc_o, initv);
+                    initv = true;
+                  }
+                }
+              }
+            }
+          }
+        } else if (kDoV && kMerge && has_t && has_o) {
           const bool acc = j > 0;
 #pragma unroll
           for (int kk = 0; kk < TILE / 16; ++kk) {
@@ -605,7 +655,25 @@ __global__ void __launch_bounds__(bwd_threads(bwd_parts(TILE))) sm100_bwd_kernel
             break;
           }
           tc_fence_after();
-          if (kMerge && has_t) {
+          if constexpr (kPair) {
+#pragma unroll
+            for (int kk = 0; kk < TILE / 16; ++kk) {
+#pragma unroll
+              for (uint32_t part = 0; part <= 8; part += 8) {
+                const uint32_t w1 = tmem + kColA + oa(kk) + part, w2 = tmem + kColC + oa(kk) + part;
+                if (kMerge && has_t) {
+                  mma_ts_lo(tmem + kColKd, w1, yb(ylo_out, 0, kk), idesc_o2, init1);
+                  init0 = init1 = true;
+                } else if (has_t) {
+                  mma_ts_lo(tmem + kColKd, w1, yb(ylo_out, 0, kk), idesc_o, init1);
+                  mma_ts_lo(tmem + kColK, w1, yb(ylo_out, 1, kk), idesc_o, init0);
+                  init0 = init1 = true;
+                }
+                mma_ts_lo(tmem + kColK, w2, yb(ylo_out, 0, kk), idesc_o, init0);
+                init0 = true;
+              }
+            }
+          } else if (kMerge && has_t) {
             const bool acc = j > 0;
 #pragma unroll
             for (int kk = 0; kk < TILE / 16; ++kk) {
@@ -714,6 +782,7 @@ __global__ void __launch_bounds__(bwd_threads(bwd_parts(TILE))) sm100_bwd_kernel
             if (cs + i >= nvalid) rs[i] = __float_as_uint(-INFINITY);  // key past the end: P = 0
         }
         uint32_t kp[8], kpn[8];
+        uint32_t kpl[kPair ? 8 : 1], kpnl[kPair ? 8 : 1];  // low parts
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
           const float4 s0 = kKV ? st[cs + 2 * i] : rstat, s1 = kKV ? st[cs + 2 * i + 1] : rstat;
@@ -728,17 +797,28 @@ __global__ void __launch_bounds__(bwd_threads(bwd_parts(TILE))) sm100_bwd_kernel
           nn[c / 2 + i] = n;
           if (kDoV) {
             kp[i] = pack2<T>(p.x, p.y);
+            if constexpr (kPair) kpl[i] = pack2_rest<T>(p.x, p.y, kp[i]);
             if (has_t) {
               const float2 pn = __fmul2_rn(p, n);
               kpn[i] = pack2<T>(pn.x, pn.y);
+              if constexpr (kPair) kpnl[i] = pack2_rest<T>(pn.x, pn.y, kpn[i]);
             }
           }
         }
         if (kDoV) {
           // 16 score columns become 8 packed operand columns, written at the start of this thread's own
           // column range, over columns it has already consumed
-          tmem_st8(tlane + kColS + col0 + c / 2, kp);
-          if (has_t) tmem_st8(tlane + kColSd + col0 + c / 2, kpn);
+          if constexpr (kPair) {
+            tmem_st8(tlane + kColS + cs, kp);
+            tmem_st8(tlane + kColS + cs + 8, kpl);
+            if (has_t) {
+              tmem_st8(tlane + kColSd + cs, kpn);
+              tmem_st8(tlane + kColSd + cs + 8, kpnl);
+            }
+          } else {
+            tmem_st8(tlane + kColS + col0 + c / 2, kp);
+            if (has_t) tmem_st8(tlane + kColSd + col0 + c / 2, kpn);
+          }
         }
       }
       if (kDoV) {
@@ -772,6 +852,7 @@ __global__ void __launch_bounds__(bwd_threads(bwd_parts(TILE))) sm100_bwd_kernel
           mbar_arrive(&s.r2_free);  // (A | C) read: the next tile's products may overwrite the region
         }
         uint32_t kw1[8], kw2[8];
+        uint32_t kw1l[kPair ? 8 : 1], kw2l[kPair ? 8 : 1];  // low parts
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
           const float4 s0 = kKV ? st[cs + 2 * i] : rstat, s1 = kKV ? st[cs + 2 * i + 1] : rstat;
@@ -782,16 +863,29 @@ __global__ void __launch_bounds__(bwd_threads(bwd_parts(TILE))) sm100_bwd_kernel
                                          make_float2(-s0.z, -s1.z));
             const float2 w1 = __fmul2_rn(sp[c / 2 + i], da);
             kw1[i] = pack2<T>(w1.x, w1.y);
+            if constexpr (kPair) kw1l[i] = pack2_rest<T>(w1.x, w1.y, kw1[i]);
             inner = __ffma2_rn(da, nn[c / 2 + i], inner);
           }
           const float2 w2 = __fmul2_rn(sp[c / 2 + i], inner);
           kw2[i] = pack2<T>(w2.x, w2.y);
+          if constexpr (kPair) kw2l[i] = pack2_rest<T>(w2.x, w2.y, kw2[i]);
         }
         if (kSplit) {
           // contiguous packing in the operands' own buffer: key column k of the tile sits in packed column k / 2
-          const uint32_t wbase = tlane + kColW + (uint32_t)(g & 1) * TILE + (col0 + c) / 2;
+          const uint32_t wbase = tlane + kColW + (uint32_t)(g & 1) * kWBuf + (col0 + c) / 2;
           if (has_t) tmem_st8(wbase, kw1);
-          tmem_st8(wbase + TILE / 2, kw2);
+          tmem_st8(wbase + kWBuf / 2, kw2);
+          if constexpr (kPair) {
+            if (has_t) tmem_st8(wbase + TILE / 2, kw1l);
+            tmem_st8(wbase + kWBuf / 2 + TILE / 2, kw2l);
+          }
+        } else if constexpr (kPair) {
+          if (has_t) {
+            tmem_st8(tlane + kColA + cs, kw1);
+            tmem_st8(tlane + kColA + cs + 8, kw1l);
+          }
+          tmem_st8(tlane + kColC + cs, kw2);
+          tmem_st8(tlane + kColC + cs + 8, kw2l);
         } else {
           if (has_t) tmem_st8(tlane + kColA + col0 + c / 2, kw1);
           tmem_st8(tlane + kColC + col0 + c / 2, kw2);
@@ -820,7 +914,8 @@ __global__ void __launch_bounds__(bwd_threads(bwd_parts(TILE))) sm100_bwd_kernel
           if (live) {
 #pragma unroll
             for (int i = 0; i < 4; ++i)
-              reinterpret_cast<uint4 *>(dst + c)[i] = make_uint4(pk[4 * i], pk[4 * i + 1], pk[4 * i + 2], pk[4 * i + 3]);
+              if (!kPair || cbase + c + 8 * i < a.D)  // heads narrower than the tile
+                reinterpret_cast<uint4 *>(dst + c)[i] = make_uint4(pk[4 * i], pk[4 * i + 1], pk[4 * i + 2], pk[4 * i + 3]);
           }
         }
       };
@@ -914,7 +1009,7 @@ __global__ void __launch_bounds__(bwd_threads(bwd_parts(TILE))) sm100_bwd_kernel
   if (warp == 1) tmem_dealloc(tmem, kTmemCols);
 }
 
-template <int D, int TILE, bool kKV, bool kDoK, bool kDoV, typename T>
+template <int D, int TILE, bool kKV, bool kDoK, bool kDoV, typename T, bool kPair>
 cudaError_t launch_side(const BwdArgs &a, const float *delta, const float *dsum, cudaStream_t stream) {
   const bool has_t = a.g_to.ptr != nullptr, has_o = a.g_o.ptr != nullptr;
   const View qside[4] = {a.q, a.tq, a.g_to, a.g_o};
@@ -931,10 +1026,10 @@ cudaError_t launch_side(const BwdArgs &a, const float *delta, const float *dsum,
   ka.ymask = kKV ? qmask : kmask;
   for (int t = 0; t < 4; ++t) {
     if ((ka.xmask >> t & 1) &&
-        !make_tensor_map(&maps.x[t], xs[t].ptr, a.dtype, a.B, a.H, Lx, D, xs[t].sb, xs[t].sh, xs[t].sl, kRows))
+        !make_tensor_map(&maps.x[t], xs[t].ptr, a.dtype, a.B, a.H, Lx, a.D, xs[t].sb, xs[t].sh, xs[t].sl, kRows))
       return cudaErrorInvalidValue;
     if ((ka.ymask >> t & 1) &&
-        !make_tensor_map(&maps.y[t], ys[t].ptr, a.dtype, a.B, a.H, Ly, D, ys[t].sb, ys[t].sh, ys[t].sl, TILE))
+        !make_tensor_map(&maps.y[t], ys[t].ptr, a.dtype, a.B, a.H, Ly, a.D, ys[t].sb, ys[t].sh, ys[t].sl, TILE))
       return cudaErrorInvalidValue;
   }
   if (kKV) {
@@ -945,13 +1040,14 @@ cudaError_t launch_side(const BwdArgs &a, const float *delta, const float *dsum,
   if (D == 64) {
     for (int t = 0; t < 4; ++t)
       if (ka.out[t].ptr &&
-          !make_tensor_map(&maps.out[t], ka.out[t].ptr, a.dtype, a.B, a.H, Lx, D, ka.out[t].sb, ka.out[t].sh, ka.out[t].sl, kRows))
+          !make_tensor_map(&maps.out[t], ka.out[t].ptr, a.dtype, a.B, a.H, Lx, a.D, ka.out[t].sb, ka.out[t].sh, ka.out[t].sl, kRows))
         return cudaErrorInvalidValue;
   }
   ka.lse = a.lse; ka.mu = a.mu; ka.delta = delta; ka.dsum = dsum; ka.status = a.status; ka.wait_cycles = a.wait_cycles;
+  ka.D = a.D;
   ka.B = a.B; ka.H = a.H; ka.Lx = Lx; ka.Ly = Ly; ka.Lq = a.Lq; ka.stat_len = a.stat_len;
   ka.has_t = has_t; ka.has_o = has_o; ka.scale = a.scale;
-  auto kernel = sm100_bwd_kernel<D, TILE, kKV, kDoK, kDoV, T>;
+  auto kernel = sm100_bwd_kernel<D, TILE, kKV, kDoK, kDoV, T, kPair>;
   const size_t smem = sizeof(BwdSmem<D, TILE>) + 1024;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
@@ -964,7 +1060,7 @@ cudaError_t launch_side(const BwdArgs &a, const float *delta, const float *dsum,
   return e != cudaSuccess ? e : cudaGetLastError();
 }
 
-template <int D, typename T>
+template <int D, typename T, bool kPair>
 cudaError_t launch_bwd(const BwdArgs &a, cudaStream_t stream) {
   float *delta = static_cast<float *>(a.workspace);
   float *dsum = delta + (size_t)a.B * a.H * a.stat_len;
@@ -980,17 +1076,18 @@ cudaError_t launch_bwd(const BwdArgs &a, cudaStream_t stream) {
   }
   cudaError_t e = cudaSuccess;
   if constexpr (D == 64) {
-    e = launch_side<D, 64, false, true, false, T>(a, delta, dsum, stream);
+    // (query owner with operand pairs: two accumulators, a 64-column score tile and both W buffers would take 640 columns)
+    e = launch_side<D, kPair ? 32 : 64, false, true, false, T, kPair>(a, delta, dsum, stream);
     if (e != cudaSuccess) return e;
-    return launch_side<D, 64, true, true, true, T>(a, delta, dsum, stream);
+    return launch_side<D, 64, true, true, true, T, kPair>(a, delta, dsum, stream);
   } else {
   // head_dim 128: four fp32 accumulators of 128 columns do not fit TMEM next to the score tiles, so the
   // key side runs as two passes (dK, dKd | dV, dVd) over 32-row query tiles
-  e = launch_side<D, 32, false, true, false, T>(a, delta, dsum, stream);
+  e = launch_side<D, 32, false, true, false, T, kPair>(a, delta, dsum, stream);
   if (e != cudaSuccess) return e;
-  e = launch_side<D, 32, true, true, false, T>(a, delta, dsum, stream);
+  e = launch_side<D, 32, true, true, false, T, kPair>(a, delta, dsum, stream);
   if (e != cudaSuccess) return e;
-  return launch_side<D, 32, true, false, true, T>(a, delta, dsum, stream);
+  return launch_side<D, 32, true, false, true, T, kPair>(a, delta, dsum, stream);
   }
 }
 
@@ -1003,7 +1100,7 @@ size_t sm100_bwd_workspace_bytes(int B, int H, int Lq, int Lk, int D, int stat_l
 }
 
 bool sm100_bwd_supported(const BwdArgs &a) {
-  if (a.D != 64 && a.D != 128) return false;
+  if (!sm100_head_dim_ok(a.D, a.dtype)) return false;
   if (a.Lq < 1 || a.Lk < 1 || a.H > 65535 || a.B > 65535) return false;
   const bool has_t = a.g_to.ptr != nullptr, has_o = a.g_o.ptr != nullptr;
   auto ok_q = [&](const View &v) { return tma_view_ok(v, a.B, a.H, a.Lq, a.D); };
@@ -1020,9 +1117,11 @@ bool sm100_bwd_supported(const BwdArgs &a) {
 }
 
 cudaError_t sm100_bwd(const BwdArgs &a, cudaStream_t stream) {
+  if (!sm100_native_head_dim(a.D))
+    return a.D < 64 ? launch_bwd<64, __nv_bfloat16, true>(a, stream) : launch_bwd<128, __nv_bfloat16, true>(a, stream);
   if (a.dtype == JVPATTN_BF16)
-    return a.D == 64 ? launch_bwd<64, __nv_bfloat16>(a, stream) : launch_bwd<128, __nv_bfloat16>(a, stream);
-  return a.D == 64 ? launch_bwd<64, __half>(a, stream) : launch_bwd<128, __half>(a, stream);
+    return a.D == 64 ? launch_bwd<64, __nv_bfloat16, false>(a, stream) : launch_bwd<128, __nv_bfloat16, false>(a, stream);
+  return a.D == 64 ? launch_bwd<64, __half, false>(a, stream) : launch_bwd<128, __half, false>(a, stream);
 }
 
 }  // namespace jvpattn

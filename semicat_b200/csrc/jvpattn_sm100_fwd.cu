@@ -16,6 +16,9 @@
 // kHasT = false is the primal-only instance (no tangents given): the same pipeline without Qd, Kd, Vd, Sd, U and Od,
 // i.e. plain flash attention that writes O and lse.  It serves the callers' non-JVP attention (the reference uses
 // F.scaled_dot_product_attention there, semicat/net/duo.py:143-152) so that one kernel family covers the whole step.
+//
+// kPair = true serves head dimensions between the two tile widths (see sm100_head_dim_ok): P and U go into the second
+// products as a 16-bit value plus the 16-bit rounding of what is left of it.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
@@ -54,7 +57,7 @@ struct FwdMaps {
   CUtensorMap o, to;  // outputs as 128-row x 64-channel store boxes
 };
 
-template <int D, typename T, bool kHasT>
+template <int D, typename T, bool kHasT, bool kPair>
 __global__ void __launch_bounds__(kThreads, D == 64 ? 2 : 1) sm100_fwd_kernel(const __grid_constant__ FwdMaps maps, FwdArgs a) {
   extern __shared__ unsigned char smem_raw[];
   using Smem = FwdSmem<D>;
@@ -190,7 +193,25 @@ __global__ void __launch_bounds__(kThreads, D == 64 ? 2 : 1) sm100_fwd_kernel(co
           const uint32_t dv = kvlo + (uint32_t)((2 * kBoxes * kKvTile + kk * 2048) >> 4) + desc_lo_mn_major(kKvTile);
           const uint32_t dtv = kvlo + (uint32_t)((3 * kBoxes * kKvTile + kk * 2048) >> 4) + desc_lo_mn_major(kKvTile);
           const bool acc = (j > 0) || (kk > 0);
-          if (!kHasT) {
+          if constexpr (kPair) {
+            // high parts at packed columns 16 kk, low parts 8 further: two products per operand and step
+            const uint32_t ph = tmem + kColS + 16 * kk, uh = tmem + kColSd + 16 * kk;
+            if (kHasT && kMerge) {
+              mma_ts_lo(tmem + kColO, ph, dv, idesc_o2, acc);
+              mma_ts_lo(tmem + kColO, ph + 8, dv, idesc_o2, true);
+            } else {
+              mma_ts_lo(tmem + kColO, ph, dv, idesc_o, acc);
+              mma_ts_lo(tmem + kColO, ph + 8, dv, idesc_o, true);
+              if (kHasT) {
+                mma_ts_lo(tmem + kColOd, ph, dtv, idesc_o, acc);
+                mma_ts_lo(tmem + kColOd, ph + 8, dtv, idesc_o, true);
+              }
+            }
+            if (kHasT) {
+              mma_ts_lo(tmem + kColOd, uh, dv, idesc_o, true);
+              mma_ts_lo(tmem + kColOd, uh + 8, dv, idesc_o, true);
+            }
+          } else if (!kHasT) {
             mma_ts_lo(tmem + kColO, tmem + kColS + kk * 8, dv, idesc_o, acc);     // O += P V
           } else if (kMerge) {
             mma_ts_lo(tmem + kColO, tmem + kColS + kk * 8, dv, idesc_o2, acc);    // [O | Od'] += P [V | Vd]
@@ -269,6 +290,7 @@ __global__ void __launch_bounds__(kThreads, D == 64 ? 2 : 1) sm100_fwd_kernel(co
 #pragma unroll
       for (int c0 = 0; c0 < 64; c0 += 32) {
         uint32_t pk[16], uk[16];
+        uint32_t pl[kPair ? 16 : 1], ul[kPair ? 16 : 1];  // low parts
         if (kHasT && c0 > 0) {
           tmem_ld32(tlane + kColSd + c0, sd);
           tc_wait_ld();
@@ -279,16 +301,31 @@ __global__ void __launch_bounds__(kThreads, D == 64 ? 2 : 1) sm100_fwd_kernel(co
           const float2 p = make_float2(fast_exp2(t.x), fast_exp2(t.y));
           psum[i & 1] = __fadd2_rn(psum[i & 1], p);
           pk[i] = pack2<T>(p.x, p.y);
+          if constexpr (kPair) pl[i] = pack2_rest<T>(p.x, p.y, pk[i]);
           if (kHasT) {
             const float2 u = __fmul2_rn(__fmul2_rn(p, scx2),
                                         make_float2(__uint_as_float(sd[2 * i]), __uint_as_float(sd[2 * i + 1])));
             usum[i & 1] = __fadd2_rn(usum[i & 1], u);
             uk[i] = pack2<T>(u.x, u.y);
+            if constexpr (kPair) ul[i] = pack2_rest<T>(u.x, u.y, uk[i]);
           }
         }
-        // 32 score columns become 16 packed operand columns, written over columns already consumed
-        tmem_st16(tlane + kColS + c0 / 2, pk);
-        if (kHasT) tmem_st16(tlane + kColSd + c0 / 2, uk);
+        if constexpr (kPair) {
+          // 16 score columns become 8 packed columns of high parts and 8 of low parts, in place
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            tmem_st8(tlane + kColS + c0 + 16 * h, *reinterpret_cast<uint32_t(*)[8]>(&pk[8 * h]));
+            tmem_st8(tlane + kColS + c0 + 16 * h + 8, *reinterpret_cast<uint32_t(*)[8]>(&pl[8 * h]));
+            if (kHasT) {
+              tmem_st8(tlane + kColSd + c0 + 16 * h, *reinterpret_cast<uint32_t(*)[8]>(&uk[8 * h]));
+              tmem_st8(tlane + kColSd + c0 + 16 * h + 8, *reinterpret_cast<uint32_t(*)[8]>(&ul[8 * h]));
+            }
+          }
+        } else {
+          // 32 score columns become 16 packed operand columns, written over columns already consumed
+          tmem_st16(tlane + kColS + c0 / 2, pk);
+          if (kHasT) tmem_st16(tlane + kColSd + c0 / 2, uk);
+        }
       }
       l = l * alpha + ((psum[0].x + psum[0].y) + (psum[1].x + psum[1].y));
       mu = mu * alpha + ((usum[0].x + usum[0].y) + (usum[1].x + usum[1].y));
@@ -357,7 +394,7 @@ __global__ void __launch_bounds__(kThreads, D == 64 ? 2 : 1) sm100_fwd_kernel(co
   if (warp == 1) tmem_dealloc(tmem, kTmemCols);
 }
 
-template <int D, typename T, bool kHasT>
+template <int D, typename T, bool kHasT, bool kPair>
 cudaError_t launch_fwd(const FwdArgs &a, cudaStream_t stream) {
   FwdMaps maps;
   const View *views[8] = {&a.q, &a.tq, &a.k, &a.tk, &a.v, &a.tv, &a.o, &a.to};
@@ -365,11 +402,11 @@ cudaError_t launch_fwd(const FwdArgs &a, cudaStream_t stream) {
   for (int i = 0; i < 8; ++i) {
     if (!kHasT && (i & 1)) continue;  // the tangent-side tensors are absent
     const bool is_q = i < 2 || i >= 6;
-    if (!make_tensor_map(dst[i], views[i]->ptr, a.dtype, a.B, a.H, is_q ? a.Lq : a.Lk, D, views[i]->sb, views[i]->sh,
+    if (!make_tensor_map(dst[i], views[i]->ptr, a.dtype, a.B, a.H, is_q ? a.Lq : a.Lk, a.D, views[i]->sb, views[i]->sh,
                          views[i]->sl, is_q ? kBM : kBN))
       return cudaErrorInvalidValue;
   }
-  auto kernel = sm100_fwd_kernel<D, T, kHasT>;
+  auto kernel = sm100_fwd_kernel<D, T, kHasT, kPair>;
   const size_t smem = sizeof(FwdSmem<D>) + 1024;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
@@ -384,7 +421,7 @@ cudaError_t launch_fwd(const FwdArgs &a, cudaStream_t stream) {
 }  // namespace
 
 bool sm100_fwd_supported(const FwdArgs &a) {
-  if (a.D != 64 && a.D != 128) return false;
+  if (!sm100_head_dim_ok(a.D, a.dtype)) return false;
   if (a.Lq < 1 || a.Lk < 1 || a.H > 65535 || a.B > 65535) return false;
   const View *qside[4] = {&a.q, &a.o, &a.tq, &a.to}, *kside[4] = {&a.k, &a.v, &a.tk, &a.tv};
   const int n = a.has_t ? 4 : 2;  // the tangent-side views exist only with tangents
@@ -393,14 +430,15 @@ bool sm100_fwd_supported(const FwdArgs &a) {
   return true;
 }
 
-template <typename T>
+template <typename T, bool kPair>
 cudaError_t dispatch_fwd(const FwdArgs &a, cudaStream_t stream) {
-  if (a.has_t) return a.D == 64 ? launch_fwd<64, T, true>(a, stream) : launch_fwd<128, T, true>(a, stream);
-  return a.D == 64 ? launch_fwd<64, T, false>(a, stream) : launch_fwd<128, T, false>(a, stream);
+  if (a.has_t) return a.D <= 64 ? launch_fwd<64, T, true, kPair>(a, stream) : launch_fwd<128, T, true, kPair>(a, stream);
+  return a.D <= 64 ? launch_fwd<64, T, false, kPair>(a, stream) : launch_fwd<128, T, false, kPair>(a, stream);
 }
 
 cudaError_t sm100_fwd(const FwdArgs &a, cudaStream_t stream) {
-  return a.dtype == JVPATTN_BF16 ? dispatch_fwd<__nv_bfloat16>(a, stream) : dispatch_fwd<__half>(a, stream);
+  if (!sm100_native_head_dim(a.D)) return dispatch_fwd<__nv_bfloat16, true>(a, stream);
+  return a.dtype == JVPATTN_BF16 ? dispatch_fwd<__nv_bfloat16, false>(a, stream) : dispatch_fwd<__half, false>(a, stream);
 }
 
 }  // namespace jvpattn

@@ -30,8 +30,30 @@ __device__ __forceinline__ uint32_t pack2<__half>(float a, float b) {
   return *reinterpret_cast<uint32_t *>(&h);
 }
 
+// What the pair (a, b) is above its 16-bit rounding `hi` = pack2(a, b), rounded to 16 bits itself: hi + rest carries 16
+// significant bits where bf16 carries 8.
+template <typename T>
+__device__ __forceinline__ uint32_t pack2_rest(float a, float b, uint32_t hi);
+template <>
+__device__ __forceinline__ uint32_t pack2_rest<__nv_bfloat16>(float a, float b, uint32_t hi) {
+  return pack2<__nv_bfloat16>(a - __uint_as_float(hi << 16), b - __uint_as_float(hi & 0xffff0000u));
+}
+
 template <typename T> struct IsBf16 { static constexpr bool value = false; };
 template <> struct IsBf16<__nv_bfloat16> { static constexpr bool value = true; };
+
+// Head dimensions of the tcgen05 kernels.  Their tiles are 64 or 128 channels wide.  A bf16 head of another width (a
+// multiple of 8, so that rows stay 16-byte aligned) runs on the next wider tile: the tensor maps carry the true width, a
+// load fills the channels past it with zeros (no memory is read for them), which add nothing to any product, and a
+// store drops them.  The portable kernels that these widths had before keep P, U and the backward's weights in
+// fp32, so here each such operand goes into its product as two bf16 parts (16 significant bits, below the rounding of
+// the bf16 result by 2^-8) instead of one.  fp16 heads of other widths stay on the portable kernels: fp16 parts do not have
+// the exponent range of the fp32 values.  Forward and backward of 32 x 8 heads of 32 channels at length 256: 5.0 ms on the
+// portable kernels, 0.16 ms of device time here.
+inline bool sm100_native_head_dim(int D) { return D == 64 || D == 128; }
+inline bool sm100_head_dim_ok(int D, int dtype) {
+  return sm100_native_head_dim(D) || (D >= 16 && D < 128 && D % 8 == 0 && dtype == JVPATTN_BF16);
+}
 
 // A view the TMA / vector-store paths can take: 16-byte aligned base, strides that keep every row 16-byte
 // aligned, rows that do not overlap, and a positive stride below 2^40 bytes on every axis that has more than one

@@ -28,7 +28,7 @@ bool make_tensor_map(CUtensorMap *out, const void *ptr, int dtype, int B, int H,
   std::call_once(g_encode_once, resolve_encode);
   if (!g_encode) return false;
   if (reinterpret_cast<uintptr_t>(ptr) % 16 != 0) return false;
-  if (D % 64 != 0 || box_rows < 1 || box_rows > 256) return false;
+  if (D % 8 != 0 || box_rows < 1 || box_rows > 256) return false;
   const cuuint64_t dims[4] = {(cuuint64_t)D, (cuuint64_t)L, (cuuint64_t)H, (cuuint64_t)B};
   // a size-1 axis may carry a meaningless stride; any multiple of 16 bytes will do for it
   auto fix = [&](int64_t s, int n) -> int64_t { return n == 1 ? (int64_t)D : s; };
