@@ -27,9 +27,7 @@
 //   warp 1      MMA issuer (query owner: the score products)
 //   last warp   query owner only: second MMA issuer (the output products)
 //   warps 2..   kParts threads per owned row (each on 1/kParts of the tile's columns): score algebra, operand
-//               write-back over consumed score columns, epilogue.  Four threads per row where a tile has 64
-//               columns (18 warps): the algebra is a chain of tensor-memory reads, exponentials and tensor-memory
-//               writes, and with two warps per scheduler its latency, not its instruction count, set the tile time
+//               write-back over consumed score columns, epilogue
 //
 // kPair = true serves head dimensions between the two tile widths (see sm100_head_dim_ok): the four operands go into
 // the output products as a 16-bit value plus the 16-bit rounding of what is left of it, two products per operand.
@@ -45,30 +43,45 @@ namespace {
 using namespace ptx;
 
 constexpr int kRows = 128;
-// threads of a CTA: TMA warp, MMA warp, 4 * parts score-algebra warps, and the second MMA warp of the query owner
-__host__ __device__ constexpr int bwd_threads(int parts) { return 64 + 128 * parts + 32; }
+// threads of a CTA: TMA warp, MMA warp, 4 * parts score-algebra warps, and the second MMA warp of the head_dim 64 query owner
+__host__ __device__ constexpr int bwd_threads(int parts, bool two_issuers) { return 64 + 128 * parts + (two_issuers ? 32 : 0); }
 // score-algebra threads per owned row: each handles at least 16 columns of a streamed tile
 #ifndef JVPATTN_BWD_PARTS_WIDE
 #define JVPATTN_BWD_PARTS_WIDE 2
 #endif
 __host__ __device__ constexpr int bwd_parts(int tile) { return tile >= 64 ? JVPATTN_BWD_PARTS_WIDE : 2; }
 
-template <int D, int TILE>
+// head_dim 128 streams 64-row tiles as two pairs with barriers of their own, (Y0, Y1) and (Y2, Y3).  Shared memory holds the
+// owned rows (128 KB with dK, 64 KB without) and three or four pairs of 32 KB, not two stages of all four tensors; but
+// (Y2, Y3) of a tile are last read by its A / C products, long before (Y0, Y1) by dK / dQ, so one stage of the former
+// and two of the latter keep the tensor core fed.  64-row tiles rather than two whole stages of 32-row ones, because a product
+// whose A operand comes from shared memory re-reads all of A for every N: at 128 B / clk a 16-channel step of N = 64 takes
+// 48 cycles for 32 cycles of arithmetic and N = 32 takes 40 for 16, while N = 128 ([S | Sd], [A | C] of a 64-row tile)
+// reads as long as it multiplies.  Forward and backward of 128 heads at length 2048: 5.42 ms with 32-row tiles, 4.30 ms so.
+__host__ __device__ constexpr bool bwd_pair_ring(int D) { return D == 128; }
+__host__ __device__ constexpr bool bwd_two_issuers(int D, bool kv) { return !kv && !bwd_pair_ring(D); }
+
+template <int D, int TILE, bool kKV, bool kDoK>
 struct BwdSmem {
   static constexpr int kBoxes = D / 64;
   static constexpr int kXBuf = D == 64 ? 2 : 1;  // owned-row tiles are double buffered where shared memory allows
   static constexpr int kStages = 2;
-  alignas(1024) uint16_t x[kXBuf][4][kBoxes][kRows * 64];
-  // streamed tiles, 64-channel box outermost: within a box the four tensors are adjacent, so that [Y0 ; Y1] and
-  // [Y2 ; Y3] are each one K-major B operand of 2 TILE rows (merged score products) at any head dimension
-  alignas(1024) uint16_t y[kStages][kBoxes][4][TILE * 64];
-  float4 stats[2][TILE];  // key owner only: per query column {lse*log2e, mu, delta, dsum} (double buffered)
+  static constexpr bool kRing = bwd_pair_ring(D);
+  static constexpr int kStages2 = kRing && kDoK ? 1 : 2;  // stages of (Y2, Y3)
+  static constexpr int kXTensors = kDoK ? 4 : 2;          // the dV / dVd pass reads X0 and X1 only
+  alignas(1024) uint16_t x[kXBuf][kXTensors][kBoxes][kRows * 64];
+  // Streamed tiles.  Within a stage the 64-channel box is outermost and the four tensors of a box (kRing: the two of a pair)
+  // are adjacent, so that [Y0 ; Y1] and [Y2 ; Y3] are each one K-major B operand of 2 TILE rows (merged score products) at
+  // any head dimension.  kRing: the stages of (Y0, Y1), then those of (Y2, Y3).
+  alignas(1024) uint16_t y[(kRing ? 2 * (kStages + kStages2) : 4 * kStages) * kBoxes][TILE * 64];
+  float4 stats[kKV ? 2 : 1][kKV ? TILE : 1];  // key owner only: per query column {lse*log2e, mu, delta, dsum} (double buffered)
   // Query owner: the owned rows' statistics {lse, mu, delta, dsum} as four float arrays, brought in by bulk copies
   // that complete on the same barrier as the rows.  Its compute warps then issue no global loads at all: a load in
   // flight holds a scoreboard slot that the tensor-memory reads of the score algebra also wait on, which exposed
   // the memory latency once per item even with nothing depending on the load.
-  alignas(16) float xstat[kXBuf][4][kRows];
-  uint64_t x_full[kXBuf], x_empty[kXBuf], acc_free, y_full[kStages], y_empty[kStages], s1_full, s2_full, c1_done, c2_done[2], r2_free, done, vdone;
+  alignas(16) float xstat[kKV ? 1 : kXBuf][4][kKV ? 4 : kRows];
+  uint64_t x_full[kXBuf], x_empty[kXBuf], acc_free, y_full[kStages], y_empty[kStages], y2_full[kStages], y2_empty[kStages], s1_full[2],
+      s2_full, c1_done[2], c2_done[2], r2_free, done, vdone;
   uint32_t tmem_base;
 };
 
@@ -156,24 +169,41 @@ __global__ void __launch_bounds__(256) row_dots_kernel(BwdArgs a, float *delta, 
 }
 
 template <int D, int TILE, bool kKV, bool kDoK, bool kDoV, typename T, bool kPair>
-__global__ void __launch_bounds__(bwd_threads(bwd_parts(TILE))) sm100_bwd_kernel(const __grid_constant__ BwdMaps maps, BwdKernelArgs a) {
+__global__ void __launch_bounds__(bwd_threads(bwd_parts(TILE), bwd_two_issuers(D, kKV)), 1) sm100_bwd_kernel(const __grid_constant__ BwdMaps maps, BwdKernelArgs a) {
   constexpr int kParts = bwd_parts(TILE);
   constexpr int kComputeThreads = 128 * kParts;
-  extern __shared__ unsigned char smem_raw[];
-  using Smem = BwdSmem<D, TILE>;
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  using Smem = BwdSmem<D, TILE, kKV, kDoK>;
   Smem &s = *reinterpret_cast<Smem *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  if constexpr (Smem::kRing && kDoK) {  // no room was left to round up: the base must have been aligned
+    if (reinterpret_cast<uintptr_t>(smem_raw) % 1024 != 0) {
+      if (threadIdx.x == 0) atomicCAS(a.status, 0u, 220u);
+      return;
+    }
+  }
   constexpr int kBoxes = D / 64;
   constexpr int kStages = Smem::kStages;
+  constexpr bool kRing = Smem::kRing;
+  constexpr int kStages2 = Smem::kStages2;
   constexpr int kAcc = (kDoK ? 2 : 0) + (kDoV ? 2 : 0);
   // accumulators; the tangent-gradient tile sits below its partner so that one N = 2D instruction can update both
   constexpr uint32_t kColKd = 0, kColK = D;                          // dX1, dX0
   constexpr uint32_t kColVd = kDoK ? 2 * D : 0, kColV = kColVd + D;  // dVd, dV
   // two score regions that are in different phases of the pipeline: (S | Sd) and (A | C)
-  constexpr uint32_t kColS = kAcc * D, kColSd = kColS + TILE, kColA = kColS + 2 * TILE, kColC = kColS + 3 * TILE;
+  constexpr uint32_t kColS = kAcc * D, kColA = kColS + 2 * TILE, kColC = kColS + 3 * TILE;
   // Query owner: its two accumulators leave room for a separate, double-buffered home of the W1 / W2 operands
   // (TILE / 2 packed columns each), so that the (A | C) region is free again as soon as the score algebra has read it
   // instead of when the output products have consumed the operands written over it.
-  constexpr bool kSplit = !kKV;
+  // (Not at head_dim 128: accumulators and score regions of 64 columns fill tensor memory.)
+  constexpr bool kSplit = bwd_two_issuers(D, kKV);
+  // The dV / dVd pass at head_dim 128 has no (A | C): (S | Sd) takes both regions in turn, so that the tensor core forms the next
+  // tile's scores while the compute warps work on this one's.
+  // Scores and score algebra then run up to two tiles ahead of each other's waits, which a parity wait on one barrier would
+  // mistake for none: their barriers alternate with the region.  (Tile g + 2 cannot complete either before tile g has been
+  // waited for: its products are issued behind the wait for the algebra of tile g.)
+  constexpr bool kAlternate = kRing && !kDoK;
+  auto alt = [](int g) { return kAlternate ? g & 1 : 0; };
+  auto alt_parity = [](int g) { return (kAlternate ? g >> 1 : g) & 1; };
   constexpr uint32_t kColW = kAcc * D + 4 * TILE;
   constexpr uint32_t kWBuf = kPair ? 2 * TILE : TILE;  // columns of one buffer: W1, W2, each with its low parts where kPair
   constexpr uint32_t kUsed = kColW + (kSplit ? 2 * kWBuf : 0);
@@ -217,10 +247,14 @@ __global__ void __launch_bounds__(bwd_threads(bwd_parts(TILE))) sm100_bwd_kernel
     for (int i = 0; i < kStages; ++i) {
       mbar_init(&s.y_full[i], 1);
       mbar_init(&s.y_empty[i], 1);
+      mbar_init(&s.y2_full[i], 1);
+      mbar_init(&s.y2_empty[i], 1);
     }
-    mbar_init(&s.s1_full, 1);
+    mbar_init(&s.s1_full[0], 1);
+    mbar_init(&s.s1_full[1], 1);
     mbar_init(&s.s2_full, 1);
-    mbar_init(&s.c1_done, kComputeThreads);
+    mbar_init(&s.c1_done[0], kComputeThreads);
+    mbar_init(&s.c1_done[1], kComputeThreads);
     mbar_init(&s.c2_done[0], kComputeThreads);
     mbar_init(&s.c2_done[1], kComputeThreads);
     mbar_init(&s.r2_free, kComputeThreads);
@@ -263,7 +297,7 @@ __global__ void __launch_bounds__(bwd_threads(bwd_parts(TILE))) sm100_bwd_kernel
           return false;
         }
         mbar_expect_tx(&s.x_full[xb], __popc(a.xmask) * kRows * D * 2 + (kKV ? 0 : (has_t ? 4 : 3) * kRows * 4));
-        for (int t = 0; t < 4; ++t)
+        for (int t = 0; t < Smem::kXTensors; ++t)
           if (a.xmask >> t & 1)
             for (int x = 0; x < kBoxes; ++x) tma_load_4d(s.x[xb][t][x], &maps.x[t], &s.x_full[xb], 64 * x, x0, h, b);
         if (!kKV) {
@@ -312,10 +346,25 @@ __global__ void __launch_bounds__(bwd_threads(bwd_parts(TILE))) sm100_bwd_kernel
             ok = false;
             break;
           }
-          mbar_expect_tx(&s.y_full[st], __popc(a.ymask) * kTileBytes);
-          for (int t = 0; t < 4; ++t)
+          constexpr int kPer = kRing ? 2 : 4;  // tensors that complete on one barrier
+          mbar_expect_tx(&s.y_full[st], __popc(a.ymask & ((1 << kPer) - 1)) * kTileBytes);
+          for (int t = 0; t < kPer; ++t)
             if (a.ymask >> t & 1)
-              for (int x = 0; x < kBoxes; ++x) tma_load_4d(s.y[st][x][t], &maps.y[t], &s.y_full[st], 64 * x, j * TILE, h, b);
+              for (int x = 0; x < kBoxes; ++x)
+                tma_load_4d(s.y[(st * kBoxes + x) * kPer + t], &maps.y[t], &s.y_full[st], 64 * x, j * TILE, h, b);
+          if constexpr (kRing) {
+            const int st2 = g % kStages2;
+            if (!mbar_wait_for(a.wait_cycles, &s.y2_empty[st2], ((g / kStages2) & 1) ^ 1)) {
+              atomicCAS(a.status, 0u, 217u);
+              ok = false;
+              break;
+            }
+            mbar_expect_tx(&s.y2_full[st2], __popc(a.ymask >> 2) * kTileBytes);
+            for (int t = 2; t < 4; ++t)
+              if (a.ymask >> t & 1)
+                for (int x = 0; x < kBoxes; ++x)
+                  tma_load_4d(s.y[((kStages + st2) * kBoxes + x) * 2 + t - 2], &maps.y[t], &s.y2_full[st2], 64 * x, j * TILE, h, b);
+          }
           prefetch_y(n, j);
           if (j == jx && it + (int)gridDim.x < items && !(ok = load_x(it + gridDim.x, n + 1))) break;
         }
@@ -346,13 +395,16 @@ __global__ void __launch_bounds__(bwd_threads(bwd_parts(TILE))) sm100_bwd_kernel
       // that issuing an MMA costs a handful of instructions (the issue rate of this one thread bounds the kernel).
       const uint32_t base16 = smem_u32(&s) >> 4;
       constexpr uint32_t kXTile = kRows * 128, kYTile = TILE * 128;  // bytes of one 64-channel box
-      auto xbase = [&](int xb) { return base16 + (uint32_t)((offsetof(Smem, x) + (size_t)xb * 4 * kBoxes * kXTile) >> 4); };
-      auto ybase = [&](int st) { return base16 + (uint32_t)((offsetof(Smem, y) + (size_t)st * 4 * kBoxes * kYTile) >> 4); };
+      constexpr int kPer = kRing ? 2 : 4;  // adjacent tensors of a box
+      auto xbase = [&](int xb) { return base16 + (uint32_t)((offsetof(Smem, x) + (size_t)xb * Smem::kXTensors * kBoxes * kXTile) >> 4); };
+      auto ybase = [&](int st) { return base16 + (uint32_t)((offsetof(Smem, y) + (size_t)st * kPer * kBoxes * kYTile) >> 4); };
+      // base for tensors 2 and 3 of tile g (their place follows from their index as in a stage of four)
+      auto ybase2 = [&](int g) { return kRing ? ybase(kStages + g % kStages2) - (2 * kYTile >> 4) : ybase(g % kStages); };
       auto xd = [&](uint32_t xlo, int t, int kk) {
         return xlo + (uint32_t)(((t * kBoxes + (kk >> 2)) * kXTile + (kk & 3) * 32) >> 4) + kDescLoKMajor;
       };
       auto yd = [&](uint32_t ylo, int t, int kk) {
-        return ylo + (uint32_t)((((kk >> 2) * 4 + t) * kYTile + (kk & 3) * 32) >> 4) + kDescLoKMajor;
+        return ylo + (uint32_t)((((kk >> 2) * kPer + t) * kYTile + (kk & 3) * 32) >> 4) + kDescLoKMajor;
       };
       // one accumulator at a time, 16 channels per instruction.  g = tile counter (stage / parity), xb = X buffer,
       // last = this is the item's last tile (its X tiles are released once no later score MMA needs them)
@@ -361,31 +413,37 @@ __global__ void __launch_bounds__(bwd_threads(bwd_parts(TILE))) sm100_bwd_kernel
         if (!mbar_wait_for(a.wait_cycles, &s.y_full[st], (g / kStages) & 1)) return false;
         tc_fence_after();
         const uint32_t xlo = xbase(xb), ylo = ybase(st);
+        const uint32_t sc = kColS + (kAlternate ? (uint32_t)(g & 1) * 2 * TILE : 0);
         if (kMergeS && has_t) {
           // [S | Sd] = X0 [Y0 ; Y1]^T in one N = 2 TILE instruction per step, then Sd += X1 Y0^T
 #pragma unroll
-          for (int kk = 0; kk < D / 16; ++kk) mma_ss_lo(tmem + kColS, xd(xlo, 0, kk), yd(ylo, 0, kk), idesc_s2, kk > 0);
+          for (int kk = 0; kk < D / 16; ++kk) mma_ss_lo(tmem + sc, xd(xlo, 0, kk), yd(ylo, 0, kk), idesc_s2, kk > 0);
 #pragma unroll
-          for (int kk = 0; kk < D / 16; ++kk) mma_ss_lo(tmem + kColSd, xd(xlo, 1, kk), yd(ylo, 0, kk), idesc_s, true);
+          for (int kk = 0; kk < D / 16; ++kk) mma_ss_lo(tmem + sc + TILE, xd(xlo, 1, kk), yd(ylo, 0, kk), idesc_s, true);
         } else {
 #pragma unroll
-          for (int kk = 0; kk < D / 16; ++kk) mma_ss_lo(tmem + kColS, xd(xlo, 0, kk), yd(ylo, 0, kk), idesc_s, kk > 0);
+          for (int kk = 0; kk < D / 16; ++kk) mma_ss_lo(tmem + sc, xd(xlo, 0, kk), yd(ylo, 0, kk), idesc_s, kk > 0);
           if (has_t) {
 #pragma unroll
             for (int kk = 0; kk < D / 16; ++kk) {
-              mma_ss_lo(tmem + kColSd, xd(xlo, 1, kk), yd(ylo, 0, kk), idesc_s, kk > 0);
-              mma_ss_lo(tmem + kColSd, xd(xlo, 0, kk), yd(ylo, 1, kk), idesc_s, true);
+              mma_ss_lo(tmem + sc + TILE, xd(xlo, 1, kk), yd(ylo, 0, kk), idesc_s, kk > 0);
+              mma_ss_lo(tmem + sc + TILE, xd(xlo, 0, kk), yd(ylo, 1, kk), idesc_s, true);
             }
           }
         }
-        tc_commit(&s.s1_full);
+        tc_commit(&s.s1_full[alt(g)]);
+        if (kRing && !kDoK) tc_commit(&s.y_empty[st]);  // the dV / dVd products read (Y2, Y3) only
         if (!kDoK && last) tc_commit(&s.x_empty[xb]);
         return true;
       };
-      auto scores2 = [&](int g, int xb, bool last) {
-        if (!kDoK) return;
-        const int st = g % kStages;  // already resident: scores1 waited for it
-        const uint32_t xlo = xbase(xb), ylo = ybase(st);
+      auto scores2 = [&](int g, int xb, bool last) -> bool {
+        if (!kDoK) return true;
+        if constexpr (kRing) {
+          if (!mbar_wait_for(a.wait_cycles, &s.y2_full[g % kStages2], (g / kStages2) & 1)) return false;
+          tc_fence_after();
+        }
+        // (not kRing: already resident, scores1 waited for the whole stage)
+        const uint32_t xlo = xbase(xb), ylo = ybase2(g);
         bool c_started = false;
         if (kMergeS && has_t && term23) {
           // [A | C] = X2 [Y2 ; Y3]^T in one N = 2 TILE instruction per step
@@ -408,11 +466,13 @@ __global__ void __launch_bounds__(bwd_threads(bwd_parts(TILE))) sm100_bwd_kernel
             mma_ss_lo(tmem + kColC, xd(xlo, 3, kk), yd(ylo, 2, kk), idesc_s, c_started || kk > 0);
         }
         tc_commit(&s.s2_full);
+        if (kRing) tc_commit(&s.y2_empty[g % kStages2]);
         if (last) tc_commit(&s.x_empty[xb]);
+        return true;
       };
       // Y tiles as MN-major B operands of the output products: consecutive 64-channel blocks are the two boxes of
-      // one tensor (d = 128: four tiles apart) or, for the merged d = 64 products, two adjacent tensors
-      constexpr uint32_t lbo = (kBoxes == 1 ? 1 : 4) * TILE * 128;
+      // one tensor (d = 128: kPer tiles apart) or, for the merged d = 64 products, two adjacent tensors
+      constexpr uint32_t lbo = (kBoxes == 1 ? 1 : kPer) * TILE * 128;
       auto yb = [&](uint32_t ylo, int t, int kk) {
         return ylo + (uint32_t)((t * kYTile + kk * 2048) >> 4) + desc_lo_mn_major(lbo);
       };
@@ -456,7 +516,7 @@ __global__ void __launch_bounds__(bwd_threads(bwd_parts(TILE))) sm100_bwd_kernel
               n2 = n + 1;
             }
             if (it2 >= items) break;
-            if (!mbar_wait_for(a.wait_cycles, &s.c1_done, g & 1)) {  // (S | Sd) of tile g has been read
+            if (!mbar_wait_for(a.wait_cycles, &s.c1_done[alt(g)], alt_parity(g))) {  // (S | Sd) of tile g has been read
               atomicCAS(a.status, 0u, 204u);
               break;
             }
@@ -554,11 +614,9 @@ __global__ void __launch_bounds__(bwd_threads(bwd_parts(TILE))) sm100_bwd_kernel
         ok = false;
       }
       if (ok) {
-        if (!scores1(0, 0, ntiles == 1)) {
+        if (!scores1(0, 0, ntiles == 1) || !scores2(0, 0, ntiles == 1)) {
           atomicCAS(a.status, 0u, 203u);
           ok = false;
-        } else {
-          scores2(0, 0, ntiles == 1);
         }
       }
       bool init0 = false, init1 = false, initv = false, initvd = false;  // accumulators written in this item
@@ -573,7 +631,20 @@ __global__ void __launch_bounds__(bwd_threads(bwd_parts(TILE))) sm100_bwd_kernel
         }
         const bool has_next = it2 < items;
         if (j == 0) init0 = init1 = initv = initvd = false;
-        if (!mbar_wait_for(a.wait_cycles, &s.c1_done, g & 1)) {
+        auto next_scores1 = [&]() -> bool {
+          if (j2 == 0 && !mbar_wait_for(a.wait_cycles, &s.x_full[n2 % kXBuf], (n2 / kXBuf) & 1)) {
+            atomicCAS(a.status, 0u, 202u);
+            return false;
+          }
+          if (!scores1(g + 1, n2 % kXBuf, j2 == ntiles - 1)) {
+            atomicCAS(a.status, 0u, 203u);
+            return false;
+          }
+          return true;
+        };
+        // kAlternate: the other region's operands were read by the products of tile g - 1, which are ahead in the queue
+        if (kAlternate && has_next && !next_scores1()) break;
+        if (!mbar_wait_for(a.wait_cycles, &s.c1_done[alt(g)], alt_parity(g))) {
           atomicCAS(a.status, 0u, 204u);
           break;
         }
@@ -581,8 +652,13 @@ __global__ void __launch_bounds__(bwd_threads(bwd_parts(TILE))) sm100_bwd_kernel
           atomicCAS(a.status, 0u, 210u);
           break;
         }
+        if (kAlternate && !mbar_wait_for(a.wait_cycles, &s.y2_full[g % kStages2], (g / kStages2) & 1)) {
+          atomicCAS(a.status, 0u, 218u);
+          break;
+        }
         tc_fence_after();
-        const uint32_t ylo_out = ybase(st);
+        const uint32_t ylo_out = ybase(st), ylo_v = ybase2(g);
+        const uint32_t sp_ = tmem + kColS + (kAlternate ? (uint32_t)(g & 1) * 2 * TILE : 0), spn_ = sp_ + TILE;
         // (the common case, both cotangents present, is issued as straight-line code: a run-time condition between
         //  two instructions of a group costs this thread tens of cycles per instruction)
         if constexpr (kPair) {
@@ -591,19 +667,19 @@ __global__ void __launch_bounds__(bwd_threads(bwd_parts(TILE))) sm100_bwd_kernel
             for (int kk = 0; kk < TILE / 16; ++kk) {
 #pragma unroll
               for (uint32_t part = 0; part <= 8; part += 8) {
-                const uint32_t p = tmem + kColS + oa(kk) + part, pn = tmem + kColSd + oa(kk) + part;
+                const uint32_t p = sp_ + oa(kk) + part, pn = spn_ + oa(kk) + part;
                 if (kMerge && has_t && has_o) {
-                  mma_ts_lo(tmem + kColVd, p, yb(ylo_out, 2, kk), idesc_o2, initvd);
-                  mma_ts_lo(tmem + kColV, pn, yb(ylo_out, 2, kk), idesc_o, true);
+                  mma_ts_lo(tmem + kColVd, p, yb(ylo_v, 2, kk), idesc_o2, initvd);
+                  mma_ts_lo(tmem + kColV, pn, yb(ylo_v, 2, kk), idesc_o, true);
                   initv = initvd = true;
                 } else {
                   if (has_t) {
-                    mma_ts_lo(tmem + kColVd, p, yb(ylo_out, 2, kk), idesc_o, initvd);
-                    mma_ts_lo(tmem + kColV, pn, yb(ylo_out, 2, kk), idesc_o, initv);
+                    mma_ts_lo(tmem + kColVd, p, yb(ylo_v, 2, kk), idesc_o, initvd);
+                    mma_ts_lo(tmem + kColV, pn, yb(ylo_v, 2, kk), idesc_o, initv);
                     initv = initvd = true;
                   }
                   if (has_o) {
-                    mma_ts_lo(tmem + kColV, p, yb(ylo_out, 3, kk), idesc_o, initv);
+                    mma_ts_lo(tmem + kColV, p, yb(ylo_v, 3, kk), idesc_o, initv);
                     initv = true;
                   }
                 }
@@ -614,41 +690,32 @@ __global__ void __launch_bounds__(bwd_threads(bwd_parts(TILE))) sm100_bwd_kernel
           const bool acc = j > 0;
 #pragma unroll
           for (int kk = 0; kk < TILE / 16; ++kk) {
-            mma_ts_lo(tmem + kColVd, tmem + kColS + oa(kk), yb(ylo_out, 2, kk), idesc_o2, acc || kk > 0);  // [dVd | dV] += P [G | gO]
-            mma_ts_lo(tmem + kColV, tmem + kColSd + oa(kk), yb(ylo_out, 2, kk), idesc_o, true);          // dV += (P o N) G
+            mma_ts_lo(tmem + kColVd, sp_ + oa(kk), yb(ylo_v, 2, kk), idesc_o2, acc || kk > 0);  // [dVd | dV] += P [G | gO]
+            mma_ts_lo(tmem + kColV, spn_ + oa(kk), yb(ylo_v, 2, kk), idesc_o, true);          // dV += (P o N) G
           }
           initv = initvd = true;
         } else if (kDoV) {
 #pragma unroll
           for (int kk = 0; kk < TILE / 16; ++kk) {
             if (kMerge && has_t && has_o) {
-              mma_ts_lo(tmem + kColVd, tmem + kColS + oa(kk), yb(ylo_out, 2, kk), idesc_o2, initvd);  // [dVd | dV] += P [G | gO]
-              mma_ts_lo(tmem + kColV, tmem + kColSd + oa(kk), yb(ylo_out, 2, kk), idesc_o, true);     // dV += (P o N) G
+              mma_ts_lo(tmem + kColVd, sp_ + oa(kk), yb(ylo_v, 2, kk), idesc_o2, initvd);  // [dVd | dV] += P [G | gO]
+              mma_ts_lo(tmem + kColV, spn_ + oa(kk), yb(ylo_v, 2, kk), idesc_o, true);     // dV += (P o N) G
               initv = initvd = true;
             } else {
               if (has_t) {
-                mma_ts_lo(tmem + kColVd, tmem + kColS + oa(kk), yb(ylo_out, 2, kk), idesc_o, initvd);  // dVd += P G
-                mma_ts_lo(tmem + kColV, tmem + kColSd + oa(kk), yb(ylo_out, 2, kk), idesc_o, initv);   // dV  += (P o N) G
+                mma_ts_lo(tmem + kColVd, sp_ + oa(kk), yb(ylo_v, 2, kk), idesc_o, initvd);  // dVd += P G
+                mma_ts_lo(tmem + kColV, spn_ + oa(kk), yb(ylo_v, 2, kk), idesc_o, initv);   // dV  += (P o N) G
                 initv = initvd = true;
               }
               if (has_o) {
-                mma_ts_lo(tmem + kColV, tmem + kColS + oa(kk), yb(ylo_out, 3, kk), idesc_o, initv);    // dV  += P gO
+                mma_ts_lo(tmem + kColV, sp_ + oa(kk), yb(ylo_v, 3, kk), idesc_o, initv);    // dV  += P gO
                 initv = true;
               }
             }
           }
         }
         if (kEarlyV && j == ntiles - 1) tc_commit(&s.vdone);  // dV / dVd of this item are final
-        if (has_next) {
-          if (j2 == 0 && !mbar_wait_for(a.wait_cycles, &s.x_full[n2 % kXBuf], (n2 / kXBuf) & 1)) {
-            atomicCAS(a.status, 0u, 202u);
-            break;
-          }
-          if (!scores1(g + 1, n2 % kXBuf, j2 == ntiles - 1)) {
-            atomicCAS(a.status, 0u, 203u);
-            break;
-          }
-        }
+        if (!kAlternate && has_next && !next_scores1()) break;
         if (kDoK) {
           if (!mbar_wait_for(a.wait_cycles, &s.c2_done[0], g & 1)) {
             atomicCAS(a.status, 0u, 207u);
@@ -696,10 +763,13 @@ __global__ void __launch_bounds__(bwd_threads(bwd_parts(TILE))) sm100_bwd_kernel
             init0 = true;
           }
         }
-        tc_commit(&s.y_empty[st]);
+        tc_commit(kAlternate ? &s.y2_empty[g % kStages2] : &s.y_empty[st]);
         if (j == ntiles - 1) tc_commit(&s.done);
         if (!has_next) break;
-        scores2(g + 1, n2 % kXBuf, j2 == ntiles - 1);
+        if (!scores2(g + 1, n2 % kXBuf, j2 == ntiles - 1)) {
+          atomicCAS(a.status, 0u, 219u);
+          break;
+        }
         it = it2; j = j2; n = n2; ++g;
       }
       }  // single issuer
@@ -754,7 +824,7 @@ __global__ void __launch_bounds__(bwd_threads(bwd_parts(TILE))) sm100_bwd_kernel
         asm volatile("bar.sync 1, %0;" ::"n"(kComputeThreads) : "memory");
       }
       // a warp whose wait ran out keeps walking the loops without touching TMEM so that the barrier above still matches
-      if (ok && !__all_sync(0xffffffffu, mbar_wait_for(a.wait_cycles, &s.s1_full, g & 1))) {
+      if (ok && !__all_sync(0xffffffffu, mbar_wait_for(a.wait_cycles, &s.s1_full[alt(g)], alt_parity(g)))) {
         atomicCAS(a.status, 0u, 205u);
         ok = false;
       }
@@ -762,19 +832,20 @@ __global__ void __launch_bounds__(bwd_threads(bwd_parts(TILE))) sm100_bwd_kernel
       tc_fence_after();
       const float4 *st = s.stats[g & 1];
       const int nvalid = a.Ly - j * TILE;  // streamed rows in this tile (masking for the query owner)
+      const uint32_t tS = tlane + kColS + (kAlternate ? (uint32_t)(g & 1) * 2 * TILE : 0), tSd = tS + TILE;
       // ---- first half: P = exp2(s*scale*log2e - lse*log2e), N = scale*sd - mu
       float2 sp[CH / 2], nn[CH / 2];  // scale * P and N, carried into the second half
 #pragma unroll
       for (int c = 0; c < CH; c += 16) {
         const int cs = col0 + c;  // first score column of this chunk
         uint32_t rs[16], rd[16];
-        tmem_ld16(tlane + kColS + cs, rs);
-        if (has_t) tmem_ld16(tlane + kColSd + cs, rd);
+        tmem_ld16(tS + cs, rs);
+        if (has_t) tmem_ld16(tSd + cs, rd);
         tc_wait_ld();
         if (!kDoV && c + 16 >= CH) {
           // nothing is written back over the scores: the region is free once this thread's last read has landed
           tc_fence_before();
-          mbar_arrive(&s.c1_done);
+          mbar_arrive(&s.c1_done[alt(g)]);
         }
         if (!kKV && nvalid < TILE) {
 #pragma unroll
@@ -809,22 +880,22 @@ __global__ void __launch_bounds__(bwd_threads(bwd_parts(TILE))) sm100_bwd_kernel
           // 16 score columns become 8 packed operand columns, written at the start of this thread's own
           // column range, over columns it has already consumed
           if constexpr (kPair) {
-            tmem_st8(tlane + kColS + cs, kp);
-            tmem_st8(tlane + kColS + cs + 8, kpl);
+            tmem_st8(tS + cs, kp);
+            tmem_st8(tS + cs + 8, kpl);
             if (has_t) {
-              tmem_st8(tlane + kColSd + cs, kpn);
-              tmem_st8(tlane + kColSd + cs + 8, kpnl);
+              tmem_st8(tSd + cs, kpn);
+              tmem_st8(tSd + cs + 8, kpnl);
             }
           } else {
-            tmem_st8(tlane + kColS + col0 + c / 2, kp);
-            if (has_t) tmem_st8(tlane + kColSd + col0 + c / 2, kpn);
+            tmem_st8(tS + col0 + c / 2, kp);
+            if (has_t) tmem_st8(tSd + col0 + c / 2, kpn);
           }
         }
       }
       if (kDoV) {
         tc_wait_st();
         tc_fence_before();
-        mbar_arrive(&s.c1_done);  // S / Sd consumed (the region may be refilled) and P / PoN in place
+        mbar_arrive(&s.c1_done[alt(g)]);  // S / Sd consumed (the region may be refilled) and P / PoN in place
       }
       if (pending_xb >= 0) {
         // the previous item's output stores have long finished reading its X buffer: hand it back to the producer
@@ -1048,14 +1119,17 @@ cudaError_t launch_side(const BwdArgs &a, const float *delta, const float *dsum,
   ka.B = a.B; ka.H = a.H; ka.Lx = Lx; ka.Ly = Ly; ka.Lq = a.Lq; ka.stat_len = a.stat_len;
   ka.has_t = has_t; ka.has_o = has_o; ka.scale = a.scale;
   auto kernel = sm100_bwd_kernel<D, TILE, kKV, kDoK, kDoV, T, kPair>;
-  const size_t smem = sizeof(BwdSmem<D, TILE>) + 1024;
+  using Smem = BwdSmem<D, TILE, kKV, kDoK>;
+  // room to round the base up to 1 KB, as far as the SM has it (the kernel checks that it fits)
+  const size_t smem = std::min<size_t>(sizeof(Smem) + 1024, 227 * 1024);
+  static_assert(sizeof(Smem) <= 227 * 1024, "shared memory of one SM");
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   const int64_t items = (int64_t)a.B * a.H * ((Lx + kRows - 1) / kRows);
   dim3 grid((unsigned)std::min<int64_t>(items, sm_count()));  // persistent: one CTA per SM walks the items
   {
     LaunchScope scope(kKV ? kIdBwdKeyTc : kIdBwdQueryTc, stream);
-    e = launch_overlapped(kernel, grid, dim3(bwd_threads(bwd_parts(TILE))), smem, stream, maps, ka);
+    e = launch_overlapped(kernel, grid, dim3(bwd_threads(bwd_parts(TILE), bwd_two_issuers(D, kKV))), smem, stream, maps, ka);
   }
   return e != cudaSuccess ? e : cudaGetLastError();
 }
@@ -1082,12 +1156,12 @@ cudaError_t launch_bwd(const BwdArgs &a, cudaStream_t stream) {
     return launch_side<D, 64, true, true, true, T, kPair>(a, delta, dsum, stream);
   } else {
   // head_dim 128: four fp32 accumulators of 128 columns do not fit TMEM next to the score tiles, so the
-  // key side runs as two passes (dK, dKd | dV, dVd) over 32-row query tiles
-  e = launch_side<D, 32, false, true, false, T, kPair>(a, delta, dsum, stream);
+  // key side runs as two passes (dK, dKd | dV, dVd)
+  e = launch_side<D, 64, false, true, false, T, kPair>(a, delta, dsum, stream);
   if (e != cudaSuccess) return e;
-  e = launch_side<D, 32, true, true, false, T, kPair>(a, delta, dsum, stream);
+  e = launch_side<D, 64, true, true, false, T, kPair>(a, delta, dsum, stream);
   if (e != cudaSuccess) return e;
-  return launch_side<D, 32, true, false, true, T, kPair>(a, delta, dsum, stream);
+  return launch_side<D, 64, true, false, true, T, kPair>(a, delta, dsum, stream);
   }
 }
 
