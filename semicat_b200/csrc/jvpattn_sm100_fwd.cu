@@ -2,7 +2,7 @@
 // tcgen05 MMAs accumulating in TMEM, TMA-staged operand tiles, online softmax.
 //
 // One CTA owns 128 query rows of one (batch, head) and walks the key axis in tiles of 64.
-//   warp 0      TMA producer: Q, Qd once; K, Kd, V, Vd per key tile through a 2-stage ring
+//   warp 0      TMA producer: Q, Qd once; (K, Kd) and (V, Vd) per key tile through 2-stage rings
 //   warp 1      MMA issuer (one elected thread): S = Q K^T, Sd = Qd K^T + Q Kd^T into TMEM, then
 //               O += P V and Od' += U V + P Vd with P, U read back from TMEM as the A operand
 //   warps 2..5  softmax: one thread per query row; reads S, Sd from TMEM, keeps the running max, sum and
@@ -11,7 +11,8 @@
 // algebra as the reference kernel (semicat/jvp_utils/ryu_triton.py:198-291).
 //
 // TMEM columns: [0,D) O, [D,2D) Od', [2D,2D+64) S / P, [2D+64,2D+128) Sd / U.  For D = 64 that is 256 columns
-// and under 100 KB of shared memory, so two CTAs share an SM and one's MMAs overlap the other's softmax.
+// and under 100 KB of shared memory, so two CTAs share an SM and one's MMAs overlap the other's softmax.  For D = 128 there is
+// one CTA per SM and a second (S | Sd) region behind the first, for the same overlap within the CTA.
 //
 // kHasT = false is the primal-only instance (no tangents given): the same pipeline without Qd, Kd, Vd, Sd, U and Od,
 // i.e. plain flash attention that writes O and lse.  It serves the callers' non-JVP attention (the reference uses
@@ -47,8 +48,11 @@ struct FwdSmem {
   static constexpr int kBoxes = D / 64;
   alignas(1024) uint16_t q[kBoxes][kBM * 64];
   alignas(1024) uint16_t tq[kBoxes][kBM * 64];
-  alignas(1024) uint16_t kv[kStages][4][kBoxes][kBN * 64];  // per stage: K, Kd, V, Vd (adjacent so pairs can be one operand)
-  uint64_t q_full, kv_full[kStages], kv_empty[kStages], s_full, p_full, o_done;
+  // Per stage the pairs (K, Kd) and (V, Vd), each with barriers of its own: the score products are done with K long before
+  // the value products with V.  [K ; Kd] is one K-major operand of 128 rows (64-channel box outermost), [V | Vd] one MN-major
+  // operand of 2 D columns (tensor outermost).
+  alignas(1024) uint16_t kv[kStages][2][2 * kBoxes][kBN * 64];
+  uint64_t q_full, k_full[kStages], k_empty[kStages], v_full[kStages], v_empty[kStages], s_full[2], p_full[2], o_done;
   uint32_t tmem_base;
 };
 
@@ -64,28 +68,57 @@ __global__ void __launch_bounds__(kThreads, D == 64 ? 2 : 1) sm100_fwd_kernel(co
   Smem &s = *reinterpret_cast<Smem *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   constexpr int kBoxes = D / 64;
   constexpr uint32_t kTmemCols = (2 * D + 128) <= 256 ? 256 : 512;
-  constexpr uint32_t kColO = 0, kColOd = D, kColS = 2 * D, kColSd = 2 * D + 64;
+  constexpr uint32_t kColO = 0, kColOd = D, kColS = 2 * D;  // Sd / U 64 columns behind S / P
+  // D = 128 leaves one CTA per SM, with nothing to run beside its softmax: (S | Sd) alternates between two regions and the
+  // scores of tile j + 1 are issued ahead of the value products of tile j.  Scores and softmax then run up to two tiles ahead of
+  // each other's waits, which a parity wait on one barrier would mistake for none: their barriers alternate too.
+  // 128 heads at length 2048: 934 -> 614 us.
+  constexpr bool kAlternate = D == 128;
+  static_assert(2 * D + (kAlternate ? 256 : 128) <= kTmemCols, "TMEM budget");
+  auto alt = [](int j) { return kAlternate ? j & 1 : 0; };
+  auto alt_parity = [](int j) { return (kAlternate ? j >> 1 : j) & 1; };
   constexpr bool kBf16 = IsBf16<T>::value;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int b = blockIdx.z, h = blockIdx.y, q0 = blockIdx.x * kBM;
   const int ntiles = (a.Lk + kBN - 1) / kBN;
 
+  constexpr uint32_t kPairBytes = (kHasT ? 2 : 1) * kBN * D * 2;
+  auto load_k = [&](int j, uint32_t extra) {
+    const int st = j % kStages;
+    mbar_expect_tx(&s.k_full[st], kPairBytes + extra);
+    for (int x = 0; x < kBoxes; ++x) {
+      tma_load_4d(s.kv[st][0][2 * x], &maps.k, &s.k_full[st], 64 * x, j * kBN, h, b);
+      if (kHasT) tma_load_4d(s.kv[st][0][2 * x + 1], &maps.tk, &s.k_full[st], 64 * x, j * kBN, h, b);
+    }
+  };
+  auto load_v = [&](int j) {
+    const int st = j % kStages;
+    mbar_expect_tx(&s.v_full[st], kPairBytes);
+    for (int x = 0; x < kBoxes; ++x) {
+      tma_load_4d(s.kv[st][1][x], &maps.v, &s.v_full[st], 64 * x, j * kBN, h, b);
+      if (kHasT) tma_load_4d(s.kv[st][1][kBoxes + x], &maps.tv, &s.v_full[st], 64 * x, j * kBN, h, b);
+    }
+  };
+
   if (threadIdx.x == 0) {
     mbar_init(&s.q_full, 1);
     for (int i = 0; i < kStages; ++i) {
-      mbar_init(&s.kv_full[i], 1);
-      mbar_init(&s.kv_empty[i], 1);
+      mbar_init(&s.k_full[i], 1);
+      mbar_init(&s.k_empty[i], 1);
+      mbar_init(&s.v_full[i], 1);
+      mbar_init(&s.v_empty[i], 1);
     }
-    mbar_init(&s.s_full, 1);
-    mbar_init(&s.p_full, 128);
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&s.s_full[i], 1);
+      mbar_init(&s.p_full[i], 128);
+    }
     mbar_init(&s.o_done, 1);
     fence_barrier_init();
     // The barriers this thread just initialised are all the first requests need: the query rows and the first
     // key tiles are on their way while the other warps allocate tensor memory and meet at the barrier below.
     prefetch_tensormap(&maps.q);
     prefetch_tensormap(&maps.k);
-    constexpr uint32_t kKvBytes = (kHasT ? 4 : 2) * kBN * D * 2;
     mbar_expect_tx(&s.q_full, (kHasT ? 2 : 1) * kBM * D * 2);
     for (int x = 0; x < kBoxes; ++x) {
       tma_load_4d(s.q[x], &maps.q, &s.q_full, 64 * x, q0, h, b);
@@ -94,13 +127,8 @@ __global__ void __launch_bounds__(kThreads, D == 64 ? 2 : 1) sm100_fwd_kernel(co
     for (int j = 0; j < ntiles && j < kStages; ++j) {
       // (test hook: with `inject` the first tile's barrier expects 16 bytes that never arrive, so every role's wait
       //  on it, or on what follows from it, runs out and the CTA leaves through the normal teardown)
-      mbar_expect_tx(&s.kv_full[j], kKvBytes + ((a.inject == 1 && j == 0) ? 16 : 0));
-      for (int x = 0; x < kBoxes; ++x) {
-        tma_load_4d(s.kv[j][0][x], &maps.k, &s.kv_full[j], 64 * x, j * kBN, h, b);
-        if (kHasT) tma_load_4d(s.kv[j][1][x], &maps.tk, &s.kv_full[j], 64 * x, j * kBN, h, b);
-        tma_load_4d(s.kv[j][2][x], &maps.v, &s.kv_full[j], 64 * x, j * kBN, h, b);
-        if (kHasT) tma_load_4d(s.kv[j][3][x], &maps.tv, &s.kv_full[j], 64 * x, j * kBN, h, b);
-      }
+      load_k(j, (a.inject == 1 && j == 0) ? 16 : 0);
+      load_v(j);
     }
   }
   if (warp == 1) {
@@ -117,17 +145,16 @@ __global__ void __launch_bounds__(kThreads, D == 64 ? 2 : 1) sm100_fwd_kernel(co
     if (lane == 0) {
       for (int j = kStages; j < ntiles; ++j) {  // the first kStages tiles were requested before the set-up barrier
         const int st = j % kStages;
-        if (!mbar_wait_for(a.wait_cycles, &s.kv_empty[st], ((j / kStages) & 1) ^ 1)) {
+        if (!mbar_wait_for(a.wait_cycles, &s.k_empty[st], ((j / kStages) & 1) ^ 1)) {
           atomicCAS(a.status, 0u, 101u);
           break;
         }
-        mbar_expect_tx(&s.kv_full[st], (kHasT ? 4 : 2) * kBN * D * 2);
-        for (int x = 0; x < kBoxes; ++x) {
-          tma_load_4d(s.kv[st][0][x], &maps.k, &s.kv_full[st], 64 * x, j * kBN, h, b);
-          if (kHasT) tma_load_4d(s.kv[st][1][x], &maps.tk, &s.kv_full[st], 64 * x, j * kBN, h, b);
-          tma_load_4d(s.kv[st][2][x], &maps.v, &s.kv_full[st], 64 * x, j * kBN, h, b);
-          if (kHasT) tma_load_4d(s.kv[st][3][x], &maps.tv, &s.kv_full[st], 64 * x, j * kBN, h, b);
+        load_k(j, 0);
+        if (!mbar_wait_for(a.wait_cycles, &s.v_empty[st], ((j / kStages) & 1) ^ 1)) {
+          atomicCAS(a.status, 0u, 101u);
+          break;
         }
+        load_v(j);
       }
     }
   } else if (warp == 1) {
@@ -137,92 +164,75 @@ __global__ void __launch_bounds__(kThreads, D == 64 ? 2 : 1) sm100_fwd_kernel(co
       constexpr uint32_t idesc_o = make_idesc(kBM, D, kBf16, false, true);
       // products that share their A operand and have adjacent B tiles / accumulators go out as one instruction of
       // twice the width (fewer instructions for the one issuing thread; N = 128 runs at the full tensor rate)
-      constexpr bool kMerge = kBoxes == 1;
       constexpr uint32_t idesc_s2 = make_idesc(kBM, 2 * kBN, kBf16, false, false);
-      constexpr uint32_t idesc_o2 = make_idesc(kBM, 2 * D <= 256 ? 2 * D : D, kBf16, false, true);
+      constexpr uint32_t idesc_o2 = make_idesc(kBM, 2 * D, kBf16, false, true);
       const uint32_t base16 = smem_u32(&s) >> 4;
       constexpr uint32_t kQTile = kBM * 128, kKvTile = kBN * 128;  // bytes of one 64-channel box
-      bool ok = mbar_wait_for(a.wait_cycles, &s.q_full, 0);
-      if (!ok) atomicCAS(a.status, 0u, 102u);
-      for (int j = 0; ok && j < ntiles; ++j) {
+      // Descriptors are one runtime base word plus compile-time offsets: this one thread issues every MMA of the CTA, so
+      // instructions per MMA bound the tensor throughput.
+      auto pair_base = [&](int st, int pair) {
+        return base16 + (uint32_t)((offsetof(Smem, kv) + (size_t)(st * 2 + pair) * 2 * kBoxes * kKvTile) >> 4);
+      };
+      // S = Q K^T ; Sd = Qd K^T + Q Kd^T      (K-major operands, 16 channels per instruction)
+      auto scores = [&](int j) -> bool {
         const int st = j % kStages;
-        if (!mbar_wait_for(a.wait_cycles, &s.kv_full[st], (j / kStages) & 1)) {
+        if (!mbar_wait_for(a.wait_cycles, &s.k_full[st], (j / kStages) & 1)) {
           atomicCAS(a.status, 0u, 103u);
-          break;
+          return false;
         }
         tc_fence_after();
-        // S = Q K^T ; Sd = Qd K^T + Q Kd^T      (K-major operands, 16 channels per instruction; one
-        // accumulator at a time).  Descriptors are one runtime base word plus compile-time offsets: this one
-        // thread issues every MMA of the CTA, so instructions per MMA bound the tensor throughput.
-        const uint32_t kvlo = base16 + (uint32_t)((offsetof(Smem, kv) + (size_t)st * 4 * kBoxes * kKvTile) >> 4);
+        const uint32_t klo = pair_base(st, 0), sc = tmem + kColS + alt(j) * 128;
         auto qd = [&](size_t member, int kk) {
           return base16 + (uint32_t)((member + (kk >> 2) * kQTile + (kk & 3) * 32) >> 4) + kDescLoKMajor;
         };
-        auto kd = [&](int t, int kk) {
-          return kvlo + (uint32_t)(((t * kBoxes + (kk >> 2)) * kKvTile + (kk & 3) * 32) >> 4) + kDescLoKMajor;
-        };
-        if (!kHasT) {
+        auto kd = [&](int kk) { return klo + (uint32_t)(((kk >> 2) * 2 * kKvTile + (kk & 3) * 32) >> 4) + kDescLoKMajor; };
+        // [S | Sd] = Q [K ; Kd]^T in one N = 128 instruction per step, then Sd += Qd K^T
 #pragma unroll
-          for (int kk = 0; kk < D / 16; ++kk) mma_ss_lo(tmem + kColS, qd(offsetof(Smem, q), kk), kd(0, kk), idesc_s, kk > 0);
-        } else if (kMerge) {
-          // [S | Sd] = Q [K ; Kd]^T in one N = 128 instruction per step, then Sd += Qd K^T
+        for (int kk = 0; kk < D / 16; ++kk) mma_ss_lo(sc, qd(offsetof(Smem, q), kk), kd(kk), kHasT ? idesc_s2 : idesc_s, kk > 0);
+        if (kHasT) {
 #pragma unroll
-          for (int kk = 0; kk < D / 16; ++kk) mma_ss_lo(tmem + kColS, qd(offsetof(Smem, q), kk), kd(0, kk), idesc_s2, kk > 0);
-#pragma unroll
-          for (int kk = 0; kk < D / 16; ++kk) mma_ss_lo(tmem + kColSd, qd(offsetof(Smem, tq), kk), kd(0, kk), idesc_s, true);
-        } else {
-#pragma unroll
-          for (int kk = 0; kk < D / 16; ++kk) mma_ss_lo(tmem + kColS, qd(offsetof(Smem, q), kk), kd(0, kk), idesc_s, kk > 0);
-#pragma unroll
-          for (int kk = 0; kk < D / 16; ++kk) {
-            mma_ss_lo(tmem + kColSd, qd(offsetof(Smem, tq), kk), kd(0, kk), idesc_s, kk > 0);
-            mma_ss_lo(tmem + kColSd, qd(offsetof(Smem, q), kk), kd(1, kk), idesc_s, true);
-          }
+          for (int kk = 0; kk < D / 16; ++kk) mma_ss_lo(sc + 64, qd(offsetof(Smem, tq), kk), kd(kk), idesc_s, true);
         }
-        tc_commit(&s.s_full);
-        if (!mbar_wait_for(a.wait_cycles, &s.p_full, j & 1)) {
+        tc_commit(&s.s_full[alt(j)]);
+        tc_commit(&s.k_empty[st]);
+        return true;
+      };
+      bool ok = mbar_wait_for(a.wait_cycles, &s.q_full, 0);
+      if (!ok) atomicCAS(a.status, 0u, 102u);
+      if (ok && kAlternate) ok = scores(0);
+      for (int j = 0; ok && j < ntiles; ++j) {
+        const int st = j % kStages;
+        // (the region of tile j + 1 was the operand of the value products of tile j - 1, which are ahead in the queue)
+        if (kAlternate ? (j + 1 < ntiles && !scores(j + 1)) : !scores(j)) break;
+        if (!mbar_wait_for(a.wait_cycles, &s.p_full[alt(j)], alt_parity(j)) ||
+            !mbar_wait_for(a.wait_cycles, &s.v_full[st], (j / kStages) & 1)) {
           atomicCAS(a.status, 0u, 104u);
           break;
         }
         tc_fence_after();
+        const uint32_t vlo = pair_base(st, 1), pcol = tmem + kColS + alt(j) * 128, ucol = pcol + 64;
         // O += P V ; Od' += U V + P Vd          (A from TMEM, B = value tile read MN-major, 16 keys per instruction)
 #pragma unroll
         for (int kk = 0; kk < kBN / 16; ++kk) {
-          // value tiles read MN-major: 16 keys = 2 KiB per step; consecutive 64-channel column blocks (and, for
-          // D = 64, V followed by Vd) are kBN * 128 bytes apart
-          const uint32_t dv = kvlo + (uint32_t)((2 * kBoxes * kKvTile + kk * 2048) >> 4) + desc_lo_mn_major(kKvTile);
-          const uint32_t dtv = kvlo + (uint32_t)((3 * kBoxes * kKvTile + kk * 2048) >> 4) + desc_lo_mn_major(kKvTile);
+          // value tiles read MN-major: 16 keys = 2 KiB per step; consecutive 64-channel column blocks of V and then
+          // Vd are kBN * 128 bytes apart
+          const uint32_t dv = vlo + (uint32_t)((kk * 2048) >> 4) + desc_lo_mn_major(kKvTile);
           const bool acc = (j > 0) || (kk > 0);
+          constexpr uint32_t idesc_p = kHasT ? idesc_o2 : idesc_o;
           if constexpr (kPair) {
             // high parts at packed columns 16 kk, low parts 8 further: two products per operand and step
-            const uint32_t ph = tmem + kColS + 16 * kk, uh = tmem + kColSd + 16 * kk;
-            if (kHasT && kMerge) {
-              mma_ts_lo(tmem + kColO, ph, dv, idesc_o2, acc);
-              mma_ts_lo(tmem + kColO, ph + 8, dv, idesc_o2, true);
-            } else {
-              mma_ts_lo(tmem + kColO, ph, dv, idesc_o, acc);
-              mma_ts_lo(tmem + kColO, ph + 8, dv, idesc_o, true);
-              if (kHasT) {
-                mma_ts_lo(tmem + kColOd, ph, dtv, idesc_o, acc);
-                mma_ts_lo(tmem + kColOd, ph + 8, dtv, idesc_o, true);
-              }
-            }
+            mma_ts_lo(tmem + kColO, pcol + 16 * kk, dv, idesc_p, acc);
+            mma_ts_lo(tmem + kColO, pcol + 16 * kk + 8, dv, idesc_p, true);
             if (kHasT) {
-              mma_ts_lo(tmem + kColOd, uh, dv, idesc_o, true);
-              mma_ts_lo(tmem + kColOd, uh + 8, dv, idesc_o, true);
+              mma_ts_lo(tmem + kColOd, ucol + 16 * kk, dv, idesc_o, true);
+              mma_ts_lo(tmem + kColOd, ucol + 16 * kk + 8, dv, idesc_o, true);
             }
-          } else if (!kHasT) {
-            mma_ts_lo(tmem + kColO, tmem + kColS + kk * 8, dv, idesc_o, acc);     // O += P V
-          } else if (kMerge) {
-            mma_ts_lo(tmem + kColO, tmem + kColS + kk * 8, dv, idesc_o2, acc);    // [O | Od'] += P [V | Vd]
-            mma_ts_lo(tmem + kColOd, tmem + kColSd + kk * 8, dv, idesc_o, true);  // Od' += U V
           } else {
-            mma_ts_lo(tmem + kColO, tmem + kColS + kk * 8, dv, idesc_o, acc);
-            mma_ts_lo(tmem + kColOd, tmem + kColSd + kk * 8, dv, idesc_o, acc);
-            mma_ts_lo(tmem + kColOd, tmem + kColS + kk * 8, dtv, idesc_o, true);
+            mma_ts_lo(tmem + kColO, pcol + 8 * kk, dv, idesc_p, acc);              // [O | Od'] += P [V | Vd]
+            if (kHasT) mma_ts_lo(tmem + kColOd, ucol + 8 * kk, dv, idesc_o, true);  // Od' += U V
           }
         }
-        tc_commit(&s.kv_empty[st]);
+        tc_commit(&s.v_empty[st]);
         tc_commit(&s.o_done);
       }
     }
@@ -236,20 +246,21 @@ __global__ void __launch_bounds__(kThreads, D == 64 ? 2 : 1) sm100_fwd_kernel(co
     bool ok = true;
     for (int j = 0; j < ntiles; ++j) {
       // tcgen05.ld / st are warp-collective: keep every decision that guards them warp-uniform
-      if (!__all_sync(0xffffffffu, mbar_wait_for(a.wait_cycles, &s.s_full, j & 1))) {
+      if (!__all_sync(0xffffffffu, mbar_wait_for(a.wait_cycles, &s.s_full[alt(j)], alt_parity(j)))) {
         atomicCAS(a.status, 0u, 105u);
         ok = false;
         break;
       }
       tc_fence_after();
+      const uint32_t tS = tlane + kColS + alt(j) * 128, tSd = tS + 64;
       // the 64 scores of this row and the first half of Sd in flight at once, one wait
       uint32_t sv[64], sd[32];
       {
         uint32_t(&lo)[32] = *reinterpret_cast<uint32_t(*)[32]>(&sv[0]);
         uint32_t(&hi)[32] = *reinterpret_cast<uint32_t(*)[32]>(&sv[32]);
-        tmem_ld32(tlane + kColS, lo);
-        tmem_ld32(tlane + kColS + 32, hi);
-        if (kHasT) tmem_ld32(tlane + kColSd, sd);
+        tmem_ld32(tS, lo);
+        tmem_ld32(tS + 32, hi);
+        if (kHasT) tmem_ld32(tSd, sd);
         tc_wait_ld();
       }
       const int nvalid = a.Lk - j * kBN;  // >= 1; < 64 only on the last tile
@@ -271,7 +282,16 @@ __global__ void __launch_bounds__(kThreads, D == 64 ? 2 : 1) sm100_fwd_kernel(co
       if (j == 0) m_new = mx;
       const float alpha = fast_exp2(m - m_new);  // 1 when unchanged, 0 on the first tile
       if (j > 0 && __any_sync(0xffffffffu, m_new != m)) {
-        // S of this tile is complete, so every earlier O / Od' update has retired: safe to rescale in place.
+        // S of this tile is complete, so every earlier O / Od' update has retired (kAlternate: all but the last one, which
+        // was issued behind S of this tile): safe to rescale in place.
+        if (kAlternate) {
+          if (!__all_sync(0xffffffffu, mbar_wait_for(a.wait_cycles, &s.o_done, (j - 1) & 1))) {
+            atomicCAS(a.status, 0u, 107u);
+            ok = false;
+            break;
+          }
+          tc_fence_after();
+        }
 #pragma unroll
         for (int c = 0; c < (kHasT ? 2 : 1) * D; c += 32) {
           uint32_t r[32];
@@ -292,7 +312,7 @@ __global__ void __launch_bounds__(kThreads, D == 64 ? 2 : 1) sm100_fwd_kernel(co
         uint32_t pk[16], uk[16];
         uint32_t pl[kPair ? 16 : 1], ul[kPair ? 16 : 1];  // low parts
         if (kHasT && c0 > 0) {
-          tmem_ld32(tlane + kColSd + c0, sd);
+          tmem_ld32(tSd + c0, sd);
           tc_wait_ld();
         }
 #pragma unroll
@@ -314,27 +334,29 @@ __global__ void __launch_bounds__(kThreads, D == 64 ? 2 : 1) sm100_fwd_kernel(co
           // 16 score columns become 8 packed columns of high parts and 8 of low parts, in place
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
-            tmem_st8(tlane + kColS + c0 + 16 * h, *reinterpret_cast<uint32_t(*)[8]>(&pk[8 * h]));
-            tmem_st8(tlane + kColS + c0 + 16 * h + 8, *reinterpret_cast<uint32_t(*)[8]>(&pl[8 * h]));
+            tmem_st8(tS + c0 + 16 * h, *reinterpret_cast<uint32_t(*)[8]>(&pk[8 * h]));
+            tmem_st8(tS + c0 + 16 * h + 8, *reinterpret_cast<uint32_t(*)[8]>(&pl[8 * h]));
             if (kHasT) {
-              tmem_st8(tlane + kColSd + c0 + 16 * h, *reinterpret_cast<uint32_t(*)[8]>(&uk[8 * h]));
-              tmem_st8(tlane + kColSd + c0 + 16 * h + 8, *reinterpret_cast<uint32_t(*)[8]>(&ul[8 * h]));
+              tmem_st8(tSd + c0 + 16 * h, *reinterpret_cast<uint32_t(*)[8]>(&uk[8 * h]));
+              tmem_st8(tSd + c0 + 16 * h + 8, *reinterpret_cast<uint32_t(*)[8]>(&ul[8 * h]));
             }
           }
         } else {
           // 32 score columns become 16 packed operand columns, written over columns already consumed
-          tmem_st16(tlane + kColS + c0 / 2, pk);
-          if (kHasT) tmem_st16(tlane + kColSd + c0 / 2, uk);
+          tmem_st16(tS + c0 / 2, pk);
+          if (kHasT) tmem_st16(tSd + c0 / 2, uk);
         }
       }
       l = l * alpha + ((psum[0].x + psum[0].y) + (psum[1].x + psum[1].y));
       mu = mu * alpha + ((usum[0].x + usum[0].y) + (usum[1].x + usum[1].y));
       tc_wait_st();
       tc_fence_before();
-      mbar_arrive(&s.p_full);
+      mbar_arrive(&s.p_full[alt(j)]);
     }
     // ---- epilogue: O = acc / l ; Od = Od'/l - (mu/l) O ; statistics
-    if (ok && !__all_sync(0xffffffffu, mbar_wait_for(a.wait_cycles, &s.o_done, (ntiles - 1) & 1))) {
+    // (kAlternate: the last two value products may both be outstanding, and a parity wait tells adjacent phases apart only)
+    if (ok && ((kAlternate && ntiles > 1 && !__all_sync(0xffffffffu, mbar_wait_for(a.wait_cycles, &s.o_done, ntiles & 1))) ||
+               !__all_sync(0xffffffffu, mbar_wait_for(a.wait_cycles, &s.o_done, (ntiles - 1) & 1)))) {
       atomicCAS(a.status, 0u, 106u);
       ok = false;
     }
