@@ -117,22 +117,20 @@ struct BwdKernelArgs {
   float scale;
 };
 
-// rows of (G o O), (G o Od) + (gO o O): D/8 threads per row, 16-byte loads
+// rows of (G o O), (G o Od) + (gO o O): D/8 threads per row, 16-byte loads.  Bound by memory; a grid over (rows, heads,
+// batch), because taking a linear row index apart with 64-bit divisions cost more instructions than everything else here
+// (64 x 12 heads of 128 rows: 14.4 -> 10.5 us; 192 x 12 without tangents: 28.3 -> 19.0 us).
 template <int D, typename T>
 __global__ void __launch_bounds__(256) row_dots_kernel(BwdArgs a, float *delta, float *dsum) {
   constexpr int kTpr = D / 8;
   ptx::griddep_launch_dependents();  // the query-owner launch may set up while this kernel drains
-  const int64_t nrows = (int64_t)a.B * a.H * a.Lq;
-  const int64_t gid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t r = gid / kTpr;
-  const int part = (int)(gid % kTpr);
+  const int part = threadIdx.x % kTpr;
+  const int b = blockIdx.z, h = blockIdx.y;
+  const int64_t row = (int64_t)blockIdx.x * (256 / kTpr) + threadIdx.x / kTpr;
+  const int i = (int)row;
   float d1 = 0.f, d2 = 0.f;
-  const bool live = r < nrows && part * 8 < a.D;  // heads narrower than the tile: the threads past the end add zero
-  int b = 0, h = 0, i = 0;
+  const bool live = row < a.Lq && part * 8 < a.D;  // heads narrower than the tile: the threads past the end add zero
   if (live) {
-    i = (int)(r % a.Lq);
-    h = (int)((r / a.Lq) % a.H);
-    b = (int)(r / ((int64_t)a.Lq * a.H));
     auto load8 = [&](const View &v, float (&f)[8]) {
       const uint4 u = *reinterpret_cast<const uint4 *>(static_cast<const T *>(v.ptr) + v.offset(b, h, i) + part * 8);
       const T *e = reinterpret_cast<const T *>(&u);
@@ -1140,10 +1138,10 @@ cudaError_t launch_bwd(const BwdArgs &a, cudaStream_t stream) {
   float *dsum = delta + (size_t)a.B * a.H * a.stat_len;
   {
     constexpr int kTpr = D / 8;
-    const int64_t threads = (int64_t)a.B * a.H * a.Lq * kTpr;
+    const dim3 grid((unsigned)((a.Lq + 256 / kTpr - 1) / (256 / kTpr)), a.H, a.B);
     {
       LaunchScope scope(kIdRowDots, stream);
-      row_dots_kernel<D, T><<<(unsigned)((threads + 255) / 256), 256, 0, stream>>>(a, delta, dsum);
+      row_dots_kernel<D, T><<<grid, 256, 0, stream>>>(a, delta, dsum);
     }
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
