@@ -239,6 +239,21 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32
       : "memory");
 }
 
+// Fragment forms over 16 lanes (`taddr` at the warp's base lane or 16 lanes further) and 16 columns: thread t holds lanes
+// t / 4 and t / 4 + 8 at columns 8 k + 2 (t % 4) and the next, k = 0, 1, as r[4 k .. 4 k + 1] and r[4 k + 2 .. 4 k + 3].
+__device__ __forceinline__ void tmem_ld16_frag(uint32_t taddr, uint32_t *r) {
+  asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(taddr)
+               : "memory");
+}
+// The same elements after each column pair became one packed column: 8 columns, r[2 k] and r[2 k + 1] at column
+// 4 k + t % 4 of lanes t / 4 and t / 4 + 8.
+__device__ __forceinline__ void tmem_st8_frag(uint32_t taddr, const uint32_t *r) {
+  asm volatile("tcgen05.st.sync.aligned.16x128b.x2.b32 [%0], {%1,%2,%3,%4};" ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3])
+               : "memory");
+}
+
 __device__ __forceinline__ bool elect_one() {
   uint32_t pred;
   asm volatile(
