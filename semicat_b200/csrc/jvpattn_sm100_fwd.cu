@@ -159,7 +159,7 @@ __global__ void __launch_bounds__(kThreads, D == 64 ? 2 : 1) sm100_fwd_kernel(co
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    if (elect_one()) {  // not `lane == 0`: a branch that is known to be uniform keeps the descriptors in uniform registers
       constexpr uint32_t idesc_s = make_idesc(kBM, kBN, kBf16, false, false);
       constexpr uint32_t idesc_o = make_idesc(kBM, D, kBf16, false, true);
       // products that share their A operand and have adjacent B tiles / accumulators go out as one instruction of
