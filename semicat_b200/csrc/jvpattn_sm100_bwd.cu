@@ -113,7 +113,7 @@ struct BwdKernelArgs {
   int D;                           // channels of a head (the tiles may be wider)
   int B, H, Lx, Ly, Lq, stat_len;  // Lx rows on the owner side, Ly on the streamed side
   int xmask, ymask;             // which of the four X / Y tensors are loaded
-  int has_t, has_o;
+  int has_o;
   float scale;
 };
 
@@ -166,7 +166,7 @@ __global__ void __launch_bounds__(256) row_dots_kernel(BwdArgs a, float *delta, 
   }
 }
 
-template <int D, int TILE, bool kKV, bool kDoK, bool kDoV, typename T, bool kPair>
+template <int D, int TILE, bool kKV, bool kDoK, bool kDoV, typename T, bool kPair, bool kHasT>
 __global__ void __launch_bounds__(bwd_threads(bwd_parts(TILE), bwd_two_issuers(D, kKV)), 1) sm100_bwd_kernel(const __grid_constant__ BwdMaps maps, BwdKernelArgs a) {
   constexpr int kParts = bwd_parts(TILE);
   constexpr int kComputeThreads = 128 * kParts;
@@ -219,7 +219,10 @@ __global__ void __launch_bounds__(bwd_threads(bwd_parts(TILE), bwd_two_issuers(D
   constexpr int kWarpB = 2 + 4 * kParts;  // the second MMA issuer sits behind the score-algebra warps
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int ntiles = (a.Ly + TILE - 1) / TILE;
-  const bool has_t = a.has_t != 0, has_o = a.has_o != 0;
+  // (compile-time: as a kernel argument it left a branch at every use in the score algebra, and those showed in its stalls:
+  // 128 heads of 64 channels at length 2048: key owner 772 -> 693 us, query owner 622 -> 568 us)
+  constexpr bool has_t = kHasT;
+  const bool has_o = a.has_o != 0;
   // Persistent CTA: work item = 128 owned rows of one (batch, head); items blockIdx.x, + gridDim.x, ...
   // Counters shared by all roles: n = items done by this CTA, g = streamed tiles done (across items).
   const int nx = (a.Lx + kRows - 1) / kRows;
@@ -783,6 +786,8 @@ __global__ void __launch_bounds__(bwd_threads(bwd_parts(TILE), bwd_two_issuers(D
     const int ctid = threadIdx.x - 64;  // 0..255 among the compute threads
     const uint32_t tlane = tmem + ((uint32_t)(quad * 32) << 16);
     const float sl2 = a.scale * kLog2e;
+    // without dV only scale * P is needed: the scale goes into the exponent
+    const float lscale = kDoV ? 0.f : __log2f(a.scale);
     const float2 sl2x2 = make_float2(sl2, sl2), scx2 = make_float2(a.scale, a.scale);
     // Score columns [c, c + 16) of this warp's 32 rows in 16 registers, and 16-bit operands back as 8 packed columns.
     // Query owner: a thread has its own row.  Key owner: two fragments of 16 rows, so that a thread meets 4 of the 16
@@ -837,12 +842,12 @@ __global__ void __launch_bounds__(bwd_threads(bwd_parts(TILE), bwd_two_issuers(D
         ok = false;
       }
       if (ok && x0 + row < a.Lx)
-        rstat = make_float4(s.xstat[xb_][0][row] * kLog2e, has_t ? s.xstat[xb_][1][row] : 0.f, s.xstat[xb_][2][row],
+        rstat = make_float4(s.xstat[xb_][0][row] * kLog2e - lscale, has_t ? s.xstat[xb_][1][row] : 0.f, s.xstat[xb_][2][row],
                             s.xstat[xb_][3][row]);
     }
     for (int j = 0; j < ntiles; ++j, ++g) {
       if (kKV) {
-        if (ctid < TILE) s.stats[g & 1][ctid] = make_float4(pre.x * kLog2e, pre.y, pre.z, pre.w);
+        if (ctid < TILE) s.stats[g & 1][ctid] = make_float4(pre.x * kLog2e - lscale, pre.y, pre.z, pre.w);
         if (j + 1 < ntiles) pre = fetch_stat(it, j + 1);
         else if (it + (int)gridDim.x < items) pre = fetch_stat(it + gridDim.x, 0);
         asm volatile("bar.sync 1, %0;" ::"n"(kComputeThreads) : "memory");
@@ -889,7 +894,7 @@ __global__ void __launch_bounds__(bwd_threads(bwd_parts(TILE), bwd_two_issuers(D
           if (has_t)
             n = __ffma2_rn(make_float2(__uint_as_float(rd[2 * i]), __uint_as_float(rd[2 * i + 1])), scx2,
                            make_float2(-s0.y, -s1.y));
-          sp[c / 2 + i] = __fmul2_rn(p, scx2);
+          sp[c / 2 + i] = kDoV ? __fmul2_rn(p, scx2) : p;
           nn[c / 2 + i] = n;
           if (kDoV) {
             kp[i] = pack2<T>(p.x, p.y);
@@ -1106,9 +1111,10 @@ __global__ void __launch_bounds__(bwd_threads(bwd_parts(TILE), bwd_two_issuers(D
   if (warp == 1) tmem_dealloc(tmem, kTmemCols);
 }
 
-template <int D, int TILE, bool kKV, bool kDoK, bool kDoV, typename T, bool kPair>
+template <int D, int TILE, bool kKV, bool kDoK, bool kDoV, typename T, bool kPair, bool kHasT>
 cudaError_t launch_side(const BwdArgs &a, const float *delta, const float *dsum, cudaStream_t stream) {
-  const bool has_t = a.g_to.ptr != nullptr, has_o = a.g_o.ptr != nullptr;
+  constexpr bool has_t = kHasT;
+  const bool has_o = a.g_o.ptr != nullptr;
   const View qside[4] = {a.q, a.tq, a.g_to, a.g_o};
   const View kside[4] = {a.k, a.tk, a.v, a.tv};
   const View *xs = kKV ? kside : qside, *ys = kKV ? qside : kside;
@@ -1143,8 +1149,8 @@ cudaError_t launch_side(const BwdArgs &a, const float *delta, const float *dsum,
   ka.lse = a.lse; ka.mu = a.mu; ka.delta = delta; ka.dsum = dsum; ka.status = a.status; ka.wait_cycles = a.wait_cycles;
   ka.D = a.D;
   ka.B = a.B; ka.H = a.H; ka.Lx = Lx; ka.Ly = Ly; ka.Lq = a.Lq; ka.stat_len = a.stat_len;
-  ka.has_t = has_t; ka.has_o = has_o; ka.scale = a.scale;
-  auto kernel = sm100_bwd_kernel<D, TILE, kKV, kDoK, kDoV, T, kPair>;
+  ka.has_o = has_o; ka.scale = a.scale;
+  auto kernel = sm100_bwd_kernel<D, TILE, kKV, kDoK, kDoV, T, kPair, kHasT>;
   using Smem = BwdSmem<D, TILE, kKV, kDoK>;
   // room to round the base up to 1 KB, as far as the SM has it (the kernel checks that it fits)
   const size_t smem = std::min<size_t>(sizeof(Smem) + 1024, 227 * 1024);
@@ -1160,7 +1166,7 @@ cudaError_t launch_side(const BwdArgs &a, const float *delta, const float *dsum,
   return e != cudaSuccess ? e : cudaGetLastError();
 }
 
-template <int D, typename T, bool kPair>
+template <int D, typename T, bool kPair, bool kHasT>
 cudaError_t launch_bwd(const BwdArgs &a, cudaStream_t stream) {
   float *delta = static_cast<float *>(a.workspace);
   float *dsum = delta + (size_t)a.B * a.H * a.stat_len;
@@ -1177,17 +1183,17 @@ cudaError_t launch_bwd(const BwdArgs &a, cudaStream_t stream) {
   cudaError_t e = cudaSuccess;
   if constexpr (D == 64) {
     // (query owner with operand pairs: two accumulators, a 64-column score tile and both W buffers would take 640 columns)
-    e = launch_side<D, kPair ? 32 : 64, false, true, false, T, kPair>(a, delta, dsum, stream);
+    e = launch_side<D, kPair ? 32 : 64, false, true, false, T, kPair, kHasT>(a, delta, dsum, stream);
     if (e != cudaSuccess) return e;
-    return launch_side<D, 64, true, true, true, T, kPair>(a, delta, dsum, stream);
+    return launch_side<D, 64, true, true, true, T, kPair, kHasT>(a, delta, dsum, stream);
   } else {
   // head_dim 128: four fp32 accumulators of 128 columns do not fit TMEM next to the score tiles, so the
   // key side runs as two passes (dK, dKd | dV, dVd)
-  e = launch_side<D, 64, false, true, false, T, kPair>(a, delta, dsum, stream);
+  e = launch_side<D, 64, false, true, false, T, kPair, kHasT>(a, delta, dsum, stream);
   if (e != cudaSuccess) return e;
-  e = launch_side<D, 64, true, true, false, T, kPair>(a, delta, dsum, stream);
+  e = launch_side<D, 64, true, true, false, T, kPair, kHasT>(a, delta, dsum, stream);
   if (e != cudaSuccess) return e;
-  return launch_side<D, 64, true, false, true, T, kPair>(a, delta, dsum, stream);
+  return launch_side<D, 64, true, false, true, T, kPair, kHasT>(a, delta, dsum, stream);
   }
 }
 
@@ -1216,12 +1222,17 @@ bool sm100_bwd_supported(const BwdArgs &a) {
   return true;
 }
 
-cudaError_t sm100_bwd(const BwdArgs &a, cudaStream_t stream) {
+template <bool kHasT>
+cudaError_t dispatch_bwd(const BwdArgs &a, cudaStream_t stream) {
   if (!sm100_native_head_dim(a.D))
-    return a.D < 64 ? launch_bwd<64, __nv_bfloat16, true>(a, stream) : launch_bwd<128, __nv_bfloat16, true>(a, stream);
+    return a.D < 64 ? launch_bwd<64, __nv_bfloat16, true, kHasT>(a, stream) : launch_bwd<128, __nv_bfloat16, true, kHasT>(a, stream);
   if (a.dtype == JVPATTN_BF16)
-    return a.D == 64 ? launch_bwd<64, __nv_bfloat16, false>(a, stream) : launch_bwd<128, __nv_bfloat16, false>(a, stream);
-  return a.D == 64 ? launch_bwd<64, __half, false>(a, stream) : launch_bwd<128, __half, false>(a, stream);
+    return a.D == 64 ? launch_bwd<64, __nv_bfloat16, false, kHasT>(a, stream) : launch_bwd<128, __nv_bfloat16, false, kHasT>(a, stream);
+  return a.D == 64 ? launch_bwd<64, __half, false, kHasT>(a, stream) : launch_bwd<128, __half, false, kHasT>(a, stream);
+}
+
+cudaError_t sm100_bwd(const BwdArgs &a, cudaStream_t stream) {
+  return a.g_to.ptr ? dispatch_bwd<true>(a, stream) : dispatch_bwd<false>(a, stream);
 }
 
 }  // namespace jvpattn
