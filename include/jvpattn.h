@@ -155,6 +155,16 @@ int jvpattn_ln_modulate(int which, const void *x, const void *tx, const float *g
                         const void *scale, const void *tshift, const void *tscale, int64_t mod_stride, int64_t tmod_stride,
                         float *mean, float *rstd, void *out, const void *g, void *dx, void *dtx, float *sums, int batch, int len,
                         int channels, float eps, int exact, int dtype, void *stream);
+/* The same on a (primal, tangent) pair in one pass each way, with the results of which = 0 then 1, and of 2 then 3:
+ * which 0: y and ty from x and tx (also writes mean / rstd); which 1: from cotangents g on y and gt on ty, both present: dx
+ * and dtx.  tx, tshift, tscale may be NULL (zero).  The VJP adds into `sums`, fp32 (5, batch, channels) zeroed by the caller,
+ * what jvpattn_ln_finalize takes as sums_y (the first two) and sums_ty (the last three); sum_s gt nd is added to sum_s g n,
+ * which enters the gradients with the same factors, and the fifth stays zero.  JVPATTN_BF16 only.  Every pointer 16-byte aligned (else
+ * JVPATTN_EALIGN). */
+int jvpattn_ln_modulate_dual(int which, const void *x, const void *tx, const float *gamma, const float *beta, const void *shift,
+                             const void *scale, const void *tshift, const void *tscale, int64_t mod_stride, int64_t tmod_stride,
+                             float *mean, float *rstd, void *y, void *ty, const void *g, const void *gt, void *dx, void *dtx,
+                             float *sums, int batch, int len, int channels, float eps, int exact, int dtype, void *stream);
 /* Dropout keep mask generated inside the gated-residual kernels instead of read from `mask` (used when `mask` is NULL):
  * element e of the call is kept with probability 1 - p and scaled by 1 / (1 - p); the decision is a counter-based hash
  * (Philox-4x32-10) of (*seed, call, e / 8), so every kernel given the same three values sees the same mask - forward,

@@ -30,7 +30,7 @@ EXPORTS = (
     "jvpattn_launch_count", "jvpattn_device_status", "jvpattn_strerror", "jvpattn_last_cuda_error",
     "jvpattn_abi_version", "jvpattn_profile_begin", "jvpattn_profile_end", "jvpattn_kernel_name",
     "jvpattn_bwd_static", "jvpattn_rotary_cast", "jvpattn_stream_check", "jvpattn_debug_set",
-    "jvpattn_ln_modulate", "jvpattn_gated_residual", "jvpattn_flow_map_head", "jvpattn_gelu_dual", "jvpattn_vocab_op",
+    "jvpattn_ln_modulate", "jvpattn_ln_modulate_dual", "jvpattn_gated_residual", "jvpattn_flow_map_head", "jvpattn_gelu_dual", "jvpattn_vocab_op",
     "jvpattn_gated_residual_dual", "jvpattn_ln_finalize", "jvpattn_rotary_qkv",
 )
 DEBUG_WAIT_CYCLES, DEBUG_STALL_NEXT_FWD = 0, 1
@@ -133,6 +133,8 @@ def load() -> ctypes.CDLL:
         V, I64, I = ctypes.c_void_p, ctypes.c_int64, ctypes.c_int
         lib.jvpattn_ln_modulate.argtypes = [I] + [V] * 8 + [I64, I64] + [V] * 7 + [I, I, I, ctypes.c_float, I, I, V]
         lib.jvpattn_ln_modulate.restype = ctypes.c_int
+        lib.jvpattn_ln_modulate_dual.argtypes = [I] + [V] * 8 + [I64, I64] + [V] * 9 + [I, I, I, ctypes.c_float, I, I, V]
+        lib.jvpattn_ln_modulate_dual.restype = ctypes.c_int
         lib.jvpattn_gated_residual.argtypes = [V] * 4 + [I64, V, I, I, I, I, ctypes.POINTER(Dropout), V]
         lib.jvpattn_gated_residual.restype = ctypes.c_int
         lib.jvpattn_flow_map_head.argtypes = [I, V, V, I64, I64] + [V] * 8 + [I, I, I, I, V]

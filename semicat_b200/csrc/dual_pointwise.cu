@@ -33,9 +33,9 @@ __device__ __forceinline__ void load8<float>(const float *p, float (&f)[8]) {
   const float4 a = reinterpret_cast<const float4 *>(p)[0], b = reinterpret_cast<const float4 *>(p)[1];
   f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w; f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
 }
-template <>
-__device__ __forceinline__ void load8<__nv_bfloat16>(const __nv_bfloat16 *p, float (&f)[8]) {
-  const uint4 u = *reinterpret_cast<const uint4 *>(p);
+// 8 elements as loaded
+template <typename T> struct alignas(16) Raw8 { uint32_t w[2 * sizeof(T)]; };
+__device__ __forceinline__ void unpack8(const Raw8<__nv_bfloat16> &u, float (&f)[8]) {
   const __nv_bfloat162 *h = reinterpret_cast<const __nv_bfloat162 *>(&u);
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
@@ -43,6 +43,10 @@ __device__ __forceinline__ void load8<__nv_bfloat16>(const __nv_bfloat16 *p, flo
     f[2 * i] = v.x;
     f[2 * i + 1] = v.y;
   }
+}
+template <>
+__device__ __forceinline__ void load8<__nv_bfloat16>(const __nv_bfloat16 *p, float (&f)[8]) {
+  unpack8(*reinterpret_cast<const Raw8<__nv_bfloat16> *>(p), f);
 }
 template <typename T> __device__ __forceinline__ float ldf(const T *p);
 template <> __device__ __forceinline__ float ldf<float>(const float *p) { return *p; }
@@ -82,8 +86,8 @@ struct LnArgs {
   const void *tshift, *tscale;   // tangents of shift / scale (null = zero)
   int64_t mod_stride, tmod_stride;
   float *mean, *rstd;            // [rows]
-  void *y;                       // output of the forward kernels
-  const void *g;                 // cotangent (backward kernels)
+  void *y, *ty;                  // outputs of the forward kernels (ty: the one-pass kernel only)
+  const void *g, *gt;            // cotangents (backward kernels; gt, on ty, in the one-pass kernel only)
   void *dx, *dtx;                // gradients with respect to x / tx
   float *sums;                   // [3, B, C] fp32 column sums (zeroed by the caller)
   int B, S, C;
@@ -187,6 +191,72 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) ln_modulate_fwd_kernel(LnAr
       }
       store8<T>(y + c0, out);
     }
+  }
+}
+
+// y and ty of the kernel above in one pass: x is read once instead of twice (4 row-sized transfers instead of 5) and the
+// statistics need not travel through memory.  Bound by memory; 128 x 128 rows of 768: 42.5 us in two kernels, 35.6 us so.
+template <typename T, int NV>
+__global__ void __launch_bounds__(kWarpsPerCta * 32) ln_modulate_dual_fwd_kernel(LnArgs a) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int64_t row = (int64_t)blockIdx.x * kWarpsPerCta + warp;
+  if (row >= (int64_t)a.B * a.S) return;
+  const int b = (int)(row / a.S);
+  constexpr int C = NV * 256;
+  float xv[NV][8], tv[NV][8];
+#pragma unroll
+  for (int v = 0; v < NV; ++v) {
+    load8<T>(static_cast<const T *>(a.x) + row * C + chan(v, lane), xv[v]);
+    if (a.tx) load8<T>(static_cast<const T *>(a.tx) + row * C + chan(v, lane), tv[v]);
+    else
+#pragma unroll
+      for (int i = 0; i < 8; ++i) tv[v][i] = 0.f;
+  }
+  float s = 0.f, s1 = 0.f;
+#pragma unroll
+  for (int v = 0; v < NV; ++v)
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      s += xv[v][i];
+      s1 += tv[v][i];
+    }
+  const float mean = warp_sum(s) / C, m1 = warp_sum(s1) / C;
+  float q = 0.f, s2 = 0.f;
+#pragma unroll
+  for (int v = 0; v < NV; ++v)
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      xv[v][i] -= mean;
+      q += xv[v][i] * xv[v][i];
+      s2 += xv[v][i] * tv[v][i];
+    }
+  const float rstd = rsqrtf(warp_sum(q) / C + a.eps), m2 = warp_sum(s2) * rstd / C;
+  if (lane == 0) {
+    a.mean[row] = mean;
+    a.rstd[row] = rstd;
+  }
+  const T *sc = static_cast<const T *>(a.scale) + (int64_t)b * a.mod_stride;
+  const T *sh = static_cast<const T *>(a.shift) + (int64_t)b * a.mod_stride;
+  const T *tsc = a.tscale ? static_cast<const T *>(a.tscale) + (int64_t)b * a.tmod_stride : nullptr;
+  const T *tsh = a.tshift ? static_cast<const T *>(a.tshift) + (int64_t)b * a.tmod_stride : nullptr;
+#pragma unroll
+  for (int v = 0; v < NV; ++v) {
+    const int c0 = chan(v, lane);
+    float g[8], be[8], scv[8], shv[8], tscv[8], tshv[8], o[8], to[8];
+    load8<float>(a.gamma + c0, g);
+    if (a.beta) load8<float>(a.beta + c0, be);
+    load8<T>(sc + c0, scv);
+    load8<T>(sh + c0, shv);
+    if (tsc) load8<T>(tsc + c0, tscv);
+    if (tsh) load8<T>(tsh + c0, tshv);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const float n = xv[v][i] * rstd, ln = n * g[i] + (a.beta ? be[i] : 0.f);
+      o[i] = ln * (1.f + scv[i]) + shv[i];
+      to[i] = rstd * (tv[v][i] - m1 - n * m2) * g[i] * (1.f + scv[i]) + (tsc ? ln * tscv[i] : 0.f) + (tsh ? tshv[i] : 0.f);
+    }
+    store8<T>(static_cast<T *>(a.y) + row * C + c0, o);
+    store8<T>(static_cast<T *>(a.ty) + row * C + c0, to);
   }
 }
 
@@ -361,6 +431,119 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) ln_modulate_bwd_tangent_ker
   }
   float *const dst[3] = {a.sums + (int64_t)b * C, a.sums + ((int64_t)a.B + b) * C, a.sums + ((int64_t)2 * a.B + b) * C};
   flush_column_sums<3, NV>(smem_raw, part, lane, dst);
+}
+
+// Both backward kernels in one pass, for the cotangents g on y and gt on ty: x is read once and dx written once, 6 row-sized
+// transfers instead of 9, and dx is rounded once.  With u1 = g gamma (1 + scale) and w, u of the kernel above, dx follows
+// from u1 + w in the place of w.  gamma (1 + scale) multiplies sum(g n) and sum(gt nd) alike, so those share one column
+// sum: sums[0] += g n + gt nd, sums[1] += g, sums[2] += gt n, sums[3] += gt.
+// Bound by memory.  A thread owns 8 channels of every row of its CTA (C / 8 threads), not a lane 8 NV of one row in four: the
+// four column sums and the next row's four operands then fit the registers with room for several CTAs per SM (a warp per
+// row took all 255 at C = 768 and spilled; fp32 rows would not fit here either and keep the kernels above), the per-sample factors are loaded once, and the column sums need no pass through
+// shared memory.  The price is a block-wide reduction of the row's sums: one barrier per row (its buffer alternates).
+// 128 x 128 rows of 768: 99 us in two kernels, 60 us so.
+template <typename T, int NV>
+__global__ void __launch_bounds__(NV * 32, 16 / NV) ln_modulate_dual_bwd_kernel(LnArgs a, int rows_per_cta) {
+  constexpr int C = NV * 256;
+  __shared__ float scratch[2][8][NV];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, c0 = threadIdx.x * 8;
+  const int ctas_per_sample = (a.S + rows_per_cta - 1) / rows_per_cta;
+  const int b = blockIdx.x / ctas_per_sample;
+  const int s0 = (blockIdx.x % ctas_per_sample) * rows_per_cta, s1 = min(a.S, s0 + rows_per_cta);
+  const bool exact = a.exact & 1;
+  float gs[8], gw[8];  // gamma (1 + scale), gamma tscale
+  {
+    float gam[8], scv[8];
+    load8<float>(a.gamma + c0, gam);
+    load8<T>(static_cast<const T *>(a.scale) + (int64_t)b * a.mod_stride + c0, scv);
+    if (a.tscale) load8<T>(static_cast<const T *>(a.tscale) + (int64_t)b * a.tmod_stride + c0, gw);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      gs[i] = gam[i] * (1.f + scv[i]);
+      gw[i] = a.tscale ? gam[i] * gw[i] : 0.f;
+    }
+  }
+  struct Row {
+    Raw8<T> x, t, g, gt;
+    float mean, rstd;
+  };
+  auto load_row = [&](int s, Row &r) {
+    const int64_t row = (int64_t)b * a.S + s, e = row * C + c0;
+    r.x = *reinterpret_cast<const Raw8<T> *>(static_cast<const T *>(a.x) + e);
+    r.t = a.tx ? *reinterpret_cast<const Raw8<T> *>(static_cast<const T *>(a.tx) + e) : Raw8<T>{};
+    r.g = *reinterpret_cast<const Raw8<T> *>(static_cast<const T *>(a.g) + e);
+    r.gt = *reinterpret_cast<const Raw8<T> *>(static_cast<const T *>(a.gt) + e);
+    r.mean = a.mean[row];
+    r.rstd = a.rstd[row];
+  };
+  float part[4][8] = {};
+  Row cur;
+  load_row(s0, cur);
+  for (int s = s0; s < s1; ++s) {
+    const float mean = cur.mean, rstd = cur.rstd;
+    float n[8], t[8], g[8], gt[8];
+    unpack8(cur.x, n), unpack8(cur.t, t), unpack8(cur.g, g), unpack8(cur.gt, gt);
+    if (s + 1 < s1) load_row(s + 1, cur);  // in flight across the barrier below
+    float v[7] = {};  // t, n t, u, u n, w, w n, u t
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      n[i] = (n[i] - mean) * rstd;
+      const float u = gt[i] * gs[i], w = g[i] * gs[i] + gt[i] * gw[i];
+      v[0] += t[i];
+      v[1] += n[i] * t[i];
+      v[2] += u;
+      v[3] += u * n[i];
+      v[4] += w;
+      v[5] += w * n[i];
+      v[6] += u * t[i];
+    }
+#pragma unroll
+    for (int q = 0; q < 7; ++q) {
+      if (q == 6 && !exact) break;
+      v[q] = warp_sum(v[q]);
+      if (NV > 1 && lane == 0) scratch[s & 1][q][warp] = v[q];
+    }
+    if (NV > 1) {
+      __syncthreads();
+#pragma unroll
+      for (int q = 0; q < 7; ++q) {
+        if (q == 6 && !exact) break;
+        v[q] = scratch[s & 1][q][0];
+#pragma unroll
+        for (int k = 1; k < NV; ++k) v[q] += scratch[s & 1][q][k];
+      }
+    }
+    constexpr float inv = 1.f / C;
+    const float m_t = v[0] * inv, m_nt = v[1] * inv, m_u = v[2] * inv, m_un = v[3] * inv, m_w = v[4] * inv, m_wn = v[5] * inv;
+    const float m_und = exact ? rstd * (v[6] * inv - m_u * m_t - m_un * m_nt) : 0.f;
+    const float m_gn = -rstd * (m_u * m_nt + m_t * m_un), m_gnn = -2.f * rstd * m_un * m_nt;
+    float o1[8], o2[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const float u = gt[i] * gs[i], w = g[i] * gs[i] + gt[i] * gw[i];
+      const float nd = rstd * (t[i] - m_t - n[i] * m_nt);
+      o2[i] = rstd * (u - m_u - n[i] * m_un);
+      if (exact) {
+        const float gn = -rstd * (u * m_nt + t[i] * m_un);
+        o1[i] = rstd * ((w + gn) - (m_w + m_gn) - n[i] * (m_wn + m_gnn)) - rstd * n[i] * m_und;
+      } else {
+        o1[i] = rstd * ((w - m_w - n[i] * m_wn) - rstd * (u * m_nt + (t[i] - m_t) * m_un));
+      }
+      part[0][i] += g[i] * n[i] + gt[i] * nd;
+      part[1][i] += g[i];
+      part[2][i] += gt[i] * n[i];
+      part[3][i] += gt[i];
+    }
+    const int64_t e = ((int64_t)b * a.S + s) * C + c0;
+    store8<T>(static_cast<T *>(a.dx) + e, o1);
+    store8<T>(static_cast<T *>(a.dtx) + e, o2);
+  }
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    float *dst = a.sums + ((int64_t)q * a.B + b) * C + c0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) atomicAdd(dst + i, part[q][i]);
+  }
 }
 
 // ---- dropout keep mask computed in the kernel instead of read from memory.  Philox-4x32-10 (Salmon et al., "Parallel
@@ -663,7 +846,8 @@ cudaError_t ln_modulate(int which, const void *x, const void *tx, const float *g
                         const void *scale, const void *tshift, const void *tscale, int64_t mod_stride, int64_t tmod_stride,
                         float *mean, float *rstd, void *out, const void *g, void *dx, void *dtx, float *sums, int B, int S, int C,
                         float eps, int exact, int dtype, cudaStream_t stream) {
-  LnArgs a{x, tx, gamma, beta, shift, scale, tshift, tscale, mod_stride, tmod_stride, mean, rstd, out, g, dx, dtx, sums, B, S, C, eps, exact};
+  LnArgs a{x, tx, gamma, beta, shift, scale, tshift, tscale, mod_stride, tmod_stride, mean, rstd, out, nullptr, g, nullptr, dx, dtx, sums,
+           B, S, C, eps, exact};
   const int64_t rows = (int64_t)B * S;
   if (rows == 0) return cudaSuccess;
   LaunchScope scope(kIdDual, stream);
@@ -685,6 +869,30 @@ cudaError_t ln_modulate(int which, const void *x, const void *tx, const float *g
         if (smem > 48 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         k<<<grid, kWarpsPerCta * 32, smem, stream>>>(a, rows_cta);
       }
+    }
+    return cudaGetLastError();
+  });
+}
+
+cudaError_t ln_modulate_dual(int which, const void *x, const void *tx, const float *gamma, const float *beta, const void *shift,
+                             const void *scale, const void *tshift, const void *tscale, int64_t mod_stride, int64_t tmod_stride,
+                             float *mean, float *rstd, void *y, void *ty, const void *g, const void *gt, void *dx, void *dtx,
+                             float *sums, int B, int S, int C, float eps, int exact, int dtype, cudaStream_t stream) {
+  LnArgs a{x, tx, gamma, beta, shift, scale, tshift, tscale, mod_stride, tmod_stride, mean, rstd, y, ty, g, gt, dx, dtx, sums,
+           B, S, C, eps, exact};
+  const int64_t rows = (int64_t)B * S;
+  if (rows == 0) return cudaSuccess;
+  LaunchScope scope(kIdDual, stream);
+  return dispatch(dtype, C, [&](auto t, auto nv) -> cudaError_t {
+    using T = decltype(t);
+    constexpr int NV = decltype(nv)::value;
+    if constexpr (!std::is_same<T, __nv_bfloat16>::value) {
+      return cudaErrorInvalidValue;
+    } else if (which == 0) {
+      ln_modulate_dual_fwd_kernel<T, NV><<<(unsigned)((rows + kWarpsPerCta - 1) / kWarpsPerCta), kWarpsPerCta * 32, 0, stream>>>(a);
+    } else {
+      const int rows_cta = rows_per_cta(B, S, 16);
+      ln_modulate_dual_bwd_kernel<T, NV><<<(unsigned)(B * ((S + rows_cta - 1) / rows_cta)), NV * 32, 0, stream>>>(a, rows_cta);
     }
     return cudaGetLastError();
   });

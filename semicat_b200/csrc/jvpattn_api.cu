@@ -271,6 +271,24 @@ int jvpattn_ln_modulate(int which, const void *x, const void *tx, const float *g
                                dx, dtx, sums, batch, len, channels, eps, exact, dtype, static_cast<cudaStream_t>(stream)));
 }
 
+int jvpattn_ln_modulate_dual(int which, const void *x, const void *tx, const float *gamma, const float *beta, const void *shift,
+                             const void *scale, const void *tshift, const void *tscale, int64_t mod_stride, int64_t tmod_stride,
+                             float *mean, float *rstd, void *y, void *ty, const void *g, const void *gt, void *dx, void *dtx,
+                             float *sums, int batch, int len, int channels, float eps, int exact, int dtype, void *stream) {
+  if (which < 0 || which > 1 || dtype != JVPATTN_BF16 || !dual_shape_ok(batch, len, channels)) return JVPATTN_EINVAL;
+  DeviceInfo *d = nullptr;
+  if (int rc = current_device(&d)) return rc;
+  if ((int64_t)batch * len == 0) return JVPATTN_OK;
+  if (!x || !gamma || !scale || !mean || !rstd) return JVPATTN_EINVAL;
+  if ((which == 0 && (!shift || !y || !ty)) || (which == 1 && (!g || !gt || !dx || !dtx || !sums))) return JVPATTN_EINVAL;
+  for (const void *p : {x, tx, (const void *)gamma, (const void *)beta, shift, scale, tshift, tscale, (const void *)y, (const void *)ty, g, gt,
+                        (const void *)dx, (const void *)dtx})
+    if (p && reinterpret_cast<uintptr_t>(p) % 16) return JVPATTN_EALIGN;
+  if (mod_stride % 8 || tmod_stride % 8) return JVPATTN_EALIGN;
+  return note_cuda(ln_modulate_dual(which, x, tx, gamma, beta, shift, scale, tshift, tscale, mod_stride, tmod_stride, mean, rstd, y, ty, g,
+                                    gt, dx, dtx, sums, batch, len, channels, eps, exact, dtype, static_cast<cudaStream_t>(stream)));
+}
+
 int jvpattn_gated_residual(const void *x, const void *y, const void *gate, const void *mask, int64_t gate_stride, void *z,
                            int batch, int len, int channels, int dtype, const jvpattn_dropout *drop, void *stream) {
   if (batch < 0 || len < 0 || channels < 8 || channels % 8) return JVPATTN_EINVAL;

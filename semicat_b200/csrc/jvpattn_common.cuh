@@ -69,6 +69,10 @@ cudaError_t ln_modulate(int which, const void *x, const void *tx, const float *g
                         const void *scale, const void *tshift, const void *tscale, int64_t mod_stride, int64_t tmod_stride,
                         float *mean, float *rstd, void *out, const void *g, void *dx, void *dtx, float *sums, int B, int S, int C,
                         float eps, int exact, int dtype, cudaStream_t stream);
+cudaError_t ln_modulate_dual(int which, const void *x, const void *tx, const float *gamma, const float *beta, const void *shift,
+                             const void *scale, const void *tshift, const void *tscale, int64_t mod_stride, int64_t tmod_stride,
+                             float *mean, float *rstd, void *y, void *ty, const void *g, const void *gt, void *dx, void *dtx,
+                             float *sums, int B, int S, int C, float eps, int exact, int dtype, cudaStream_t stream);
 cudaError_t gated_residual(const void *x, const void *y, const void *gate, const void *mask, int64_t gate_stride, void *z, int B,
                            int S, int C, int dtype, const unsigned long long *drop_seed, unsigned drop_call, float drop_p,
                            cudaStream_t stream);

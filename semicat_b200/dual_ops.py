@@ -66,8 +66,8 @@ def _stream(t):
     return torch.cuda.current_stream(t.device).cuda_stream
 
 
-def _ln_launch(which, x, tx, gamma, beta, shift, scale, tshift, tscale, mean, rstd, out, g, dx, dtx, sums, eps, exact):
-    B, S, C = x.shape
+def _modulation_rows(shift, scale, tshift, tscale, B, C):
+    """((shift, scale, their row stride), (tshift, tscale, theirs)) as the kernels take them: rows of a pair equally spaced."""
     sc, sc_stride = _rows(scale, B, C)
     sh, sh_stride = _rows(shift, B, C)
     tsc, tsc_stride = _rows(tscale, B, C)
@@ -79,13 +79,30 @@ def _ln_launch(which, x, tx, gamma, beta, shift, scale, tshift, tscale, mean, rs
     if tsc is not None and tsh is not None and tsc_stride != tsh_stride:
         tsc, tsh = tsc.contiguous(), tsh.contiguous()
         tsc_stride = C
-    tstride = tsc_stride if tsc is not None else tsh_stride
+    return (sh, sc, sc_stride), (tsh, tsc, tsc_stride if tsc is not None else tsh_stride)
+
+
+def _ln_launch(which, x, tx, gamma, beta, shift, scale, tshift, tscale, mean, rstd, out, g, dx, dtx, sums, eps, exact):
+    B, S, C = x.shape
+    (sh, sc, sc_stride), (tsh, tsc, tstride) = _modulation_rows(shift, scale, tshift, tscale, B, C)
     lib = _lib.load()
     with torch.cuda.device(x.device):
         rc = lib.jvpattn_ln_modulate(which, _ptr(x), _ptr(tx), _ptr(gamma), _ptr(beta), _ptr(sh), _ptr(sc), _ptr(tsh), _ptr(tsc),
                                      sc_stride, tstride, _ptr(mean), _ptr(rstd), _ptr(out), _ptr(g), _ptr(dx), _ptr(dtx), _ptr(sums),
                                      B, S, C, float(eps), int(exact), _CODES[x.dtype], _stream(x))
     _lib.check(rc, "jvpattn_ln_modulate")
+
+
+def _ln_dual_launch(which, x, tx, gamma, beta, shift, scale, tshift, tscale, mean, rstd, y, ty, g, gt, dx, dtx, sums, eps, exact):
+    """bf16 primal and tangent in one pass (``which`` 0), or the cotangents of both outputs (1)."""
+    B, S, C = x.shape
+    (sh, sc, sc_stride), (tsh, tsc, tstride) = _modulation_rows(shift, scale, tshift, tscale, B, C)
+    lib = _lib.load()
+    with torch.cuda.device(x.device):
+        rc = lib.jvpattn_ln_modulate_dual(which, _ptr(x), _ptr(tx), _ptr(gamma), _ptr(beta), _ptr(sh), _ptr(sc), _ptr(tsh), _ptr(tsc),
+                                          sc_stride, tstride, _ptr(mean), _ptr(rstd), _ptr(y), _ptr(ty), _ptr(g), _ptr(gt), _ptr(dx),
+                                          _ptr(dtx), _ptr(sums), B, S, C, float(eps), int(exact), _CODES[x.dtype], _stream(x))
+    _lib.check(rc, "jvpattn_ln_modulate_dual")
 
 
 def _ln_finalize(sums_y, sums_ty, gamma, beta, scale, tscale, want_tangent_grads, B, C, param_grads):
@@ -112,8 +129,8 @@ def _ln_finalize(sums_y, sums_ty, gamma, beta, scale, tscale, want_tangent_grads
 
 class _LnModulateDual(torch.autograd.Function):
     """(x, gamma, beta, shift, scale, tx, tshift, tscale) -> (y, ty) as one autograd node: a reverse pass brings the
-    cotangents of both outputs at once, the two backward kernels leave their sum in dx, and one more launch turns
-    their column sums into the gradients of the modulation tensors and of the LayerNorm weight and bias."""
+    cotangents of both outputs at once (bf16: to one backward kernel; fp32: to one each, which leave their sum in dx), and
+    one more launch turns the column sums into the gradients of the modulation tensors and of the LayerNorm weight and bias."""
 
     @staticmethod
     def forward(x, gamma, beta, shift, scale, tx, tshift, tscale, eps, exact):
@@ -121,9 +138,13 @@ class _LnModulateDual(torch.autograd.Function):
         y, ty = torch.empty_like(x), torch.empty_like(x)
         mean = torch.empty(B * S, dtype=torch.float32, device=x.device)
         rstd = torch.empty_like(mean)
-        _ln_launch(0, x, None, gamma, beta, shift, scale, None, None, mean, rstd, y, None, None, None, None, eps, exact)
-        tx_ = torch.zeros_like(x) if tx is None else tx.contiguous()
-        _ln_launch(1, x, tx_, gamma, beta, None, scale, tshift, tscale, mean, rstd, ty, None, None, None, None, eps, exact)
+        tx_ = None if tx is None else tx.contiguous()
+        if x.dtype != torch.bfloat16:
+            _ln_launch(0, x, None, gamma, beta, shift, scale, None, None, mean, rstd, y, None, None, None, None, eps, exact)
+            tx_ = torch.zeros_like(x) if tx_ is None else tx_
+            _ln_launch(1, x, tx_, gamma, beta, None, scale, tshift, tscale, mean, rstd, ty, None, None, None, None, eps, exact)
+            return y, ty, mean, rstd
+        _ln_dual_launch(0, x, tx_, gamma, beta, shift, scale, tshift, tscale, mean, rstd, y, ty, None, None, None, None, None, eps, exact)
         return y, ty, mean, rstd
 
     @staticmethod
@@ -148,13 +169,19 @@ class _LnModulateDual(torch.autograd.Function):
         sums, param_grads = zeros[:5 * B * C].view(5, B, C), zeros[5 * B * C:].view(2, C)
         sums_y = sums[:2] if gy is not None else None
         sums_ty = sums[2:] if gty is not None else None
-        if gy is not None:
-            _ln_launch(2, x, None, gamma, None, None, scale, None, None, mean, rstd, None, gy.contiguous(), dx, None, sums_y, ctx.eps, ctx.exact)
         if gty is not None:
-            tx_ = torch.zeros_like(x) if tx is None else tx.contiguous()
+            tx_ = None if tx is None else tx.contiguous()
             dtx = torch.empty_like(x)
-            flags = int(ctx.exact) | (2 if gy is not None else 0)
-            _ln_launch(3, x, tx_, gamma, None, None, scale, None, tscale, mean, rstd, None, gty.contiguous(), dx, dtx, sums_ty, ctx.eps, flags)
+        if gy is not None and gty is not None and x.dtype == torch.bfloat16:
+            _ln_dual_launch(1, x, tx_, gamma, None, None, scale, None, tscale, mean, rstd, None, None, gy.contiguous(), gty.contiguous(),
+                            dx, dtx, sums, ctx.eps, ctx.exact)
+        else:
+            if gy is not None:
+                _ln_launch(2, x, None, gamma, None, None, scale, None, None, mean, rstd, None, gy.contiguous(), dx, None, sums_y, ctx.eps, ctx.exact)
+            if gty is not None:
+                tx_ = torch.zeros_like(x) if tx is None else tx_
+                flags = int(ctx.exact) | (2 if gy is not None else 0)
+                _ln_launch(3, x, tx_, gamma, None, None, scale, None, tscale, mean, rstd, None, gty.contiguous(), dx, dtx, sums_ty, ctx.eps, flags)
         d_shift, d_scale, d_tshift, d_tscale, d_gamma, d_beta = _ln_finalize(
             sums_y, sums_ty, gamma, beta, scale, tscale, (tshift is not None, tscale is not None), B, C, param_grads)
         shaped = lambda v, ref: None if v is None or ref is None else v.reshape(ref.shape)

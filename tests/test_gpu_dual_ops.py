@@ -223,3 +223,41 @@ def test_generated_dropout_masks_are_consistent_between_passes_and_have_the_righ
         for j in range(i + 1, 4):
             assert not torch.equal(masks[i], masks[j])
     assert _lib.device_status() == 0
+
+
+@pytest.mark.parametrize("shape", [(1, 1, 256), (3, 17, 512), (2, 50, 768), (5, 130, 1024), (40, 33, 768)])
+@pytest.mark.parametrize("missing", ["none", "x", "scale", "shift"])
+@pytest.mark.parametrize("exact", [False, True])
+def test_ln_modulate_bf16_pair_kernels_match_the_single_ones(shape, missing, exact):
+    """The one-pass bf16 kernels against the kernels that take primal and tangent one at a time: y, ty and dtx are rounded
+    once in either form (so at most neighbouring bf16 values, 2^-7 relative), dx twice by the single kernels (2^-7 of its two
+    parts), the fp32 column sums differ in their order only."""
+    B, S, C = shape
+    x, t, sh, sc, tsh, tsc, norm, cots = _ln_inputs(B, S, C, torch.bfloat16, seed=C + S, tx=missing != "x")
+    tsh, tsc = None if missing == "shift" else tsh, None if missing == "scale" else tsc
+    w, b = norm.weight.detach().float(), norm.bias.detach().float()
+    g, gt = (c.to(torch.bfloat16) for c in cots)
+    new = lambda: torch.full_like(x, float("nan"))
+    stat = lambda: torch.full((B * S,), float("nan"), device="cuda")
+    y, ty, mean, rstd = new(), new(), stat(), stat()
+    dual_ops._ln_dual_launch(0, x, t, w, b, sh, sc, tsh, tsc, mean, rstd, y, ty, None, None, None, None, None, norm.eps, exact)
+    y1, ty1, mean1, rstd1 = new(), new(), stat(), stat()
+    tz = torch.zeros_like(x) if t is None else t
+    dual_ops._ln_launch(0, x, None, w, b, sh, sc, None, None, mean1, rstd1, y1, None, None, None, None, norm.eps, exact)
+    dual_ops._ln_launch(1, x, tz, w, b, None, sc, tsh, tsc, mean1, rstd1, ty1, None, None, None, None, norm.eps, exact)
+    _close(mean, mean1, "mean", 1e-5, 1e-6)
+    _close(rstd, rstd1, "rstd", 1e-5, 1e-6)
+    _close(y, y1, "y", 2 ** -7, 1e-5)
+    _close(ty, ty1, "ty", 2 ** -7, 1e-4)
+    sums, sums1 = (torch.zeros(5, B, C, device="cuda") for _ in range(2))
+    dx, dtx, dx1, dtx1 = new(), new(), new(), new()
+    dual_ops._ln_dual_launch(1, x, t, w, None, None, sc, None, tsc, mean, rstd, None, None, g, gt, dx, dtx, sums, norm.eps, exact)
+    dual_ops._ln_launch(2, x, None, w, None, None, sc, None, None, mean, rstd, None, g, dx1, None, sums1[:2], norm.eps, exact)
+    first = dx1.float().abs()
+    dual_ops._ln_launch(3, x, tz, w, None, None, sc, None, tsc, mean, rstd, None, gt, dx1, dtx1, sums1[2:], norm.eps, int(exact) | 2)
+    _close(dtx, dtx1, "dtx", 2 ** -7, 1e-4)
+    err = (dx.float() - dx1.float()).abs()
+    assert bool((err <= 2 ** -7 * (first + dx1.float().abs()) + 1e-4).all()), err.max()
+    sums1[0] += sums1[4]  # the pair kernel keeps sum(g n) + sum(gt nd) together
+    scale = sums1[:4].abs().max()
+    assert float((sums[:4] - sums1[:4]).abs().max()) <= 1e-5 * float(scale) * S ** 0.5 and not sums[4].any()
