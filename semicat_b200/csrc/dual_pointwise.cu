@@ -70,6 +70,19 @@ __device__ __forceinline__ void store8<__nv_bfloat16>(__nv_bfloat16 *p, const fl
   *reinterpret_cast<uint4 *>(p) = u;
 }
 
+// Adds 8 adjacent sums to global memory as two 16-byte reductions.  Element by element, the lanes of each instruction are 32
+// bytes apart: 32 sectors per request.  128 x 128 rows of 768: LayerNorm backward 60 -> 49 us, gated residual
+// backward 61 -> 51 us.
+__device__ __forceinline__ void add8(float *dst, const float (&f)[8]) {
+  if (reinterpret_cast<uintptr_t>(dst) % 16 == 0) {
+    atomicAdd(reinterpret_cast<float4 *>(dst), make_float4(f[0], f[1], f[2], f[3]));
+    atomicAdd(reinterpret_cast<float4 *>(dst) + 1, make_float4(f[4], f[5], f[6], f[7]));
+  } else {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) atomicAdd(dst + i, f[i]);
+  }
+}
+
 __device__ __forceinline__ float warp_sum(float x) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
@@ -441,7 +454,7 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) ln_modulate_bwd_tangent_ker
 // four column sums and the next row's four operands then fit the registers with room for several CTAs per SM (a warp per
 // row took all 255 at C = 768 and spilled; fp32 rows would not fit here either and keep the kernels above), the per-sample factors are loaded once, and the column sums need no pass through
 // shared memory.  The price is a block-wide reduction of the row's sums: one barrier per row (its buffer alternates).
-// 128 x 128 rows of 768: 99 us in two kernels, 60 us so.
+// 128 x 128 rows of 768: 99 us in two kernels, 60 us so, 49 us with the column sums added 16 bytes at a time.
 template <typename T, int NV>
 __global__ void __launch_bounds__(NV * 32, 16 / NV) ln_modulate_dual_bwd_kernel(LnArgs a, int rows_per_cta) {
   constexpr int C = NV * 256;
@@ -539,11 +552,7 @@ __global__ void __launch_bounds__(NV * 32, 16 / NV) ln_modulate_dual_bwd_kernel(
     store8<T>(static_cast<T *>(a.dtx) + e, o2);
   }
 #pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    float *dst = a.sums + ((int64_t)q * a.B + b) * C + c0;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) atomicAdd(dst + i, part[q][i]);
-  }
+  for (int q = 0; q < 4; ++q) add8(a.sums + ((int64_t)q * a.B + b) * C + c0, part[q]);
 }
 
 // ---- dropout keep mask computed in the kernel instead of read from memory.  Philox-4x32-10 (Salmon et al., "Parallel
@@ -754,11 +763,8 @@ __global__ void __launch_bounds__(128) gated_dual_bwd_kernel(GateDualArgs a, int
     if (a.d_ty) store8<T>(static_cast<T *>(a.d_ty) + e, o2);
   }
   float *dg = a.sums + (int64_t)b * a.C + c0, *dtg = a.sums + ((int64_t)a.B + b) * a.C + c0;
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    atomicAdd(dg + i, sg[i]);
-    if (a.gtz) atomicAdd(dtg + i, stg[i]);
-  }
+  add8(dg, sg);
+  if (a.gtz) add8(dtg, stg);
 }
 
 // ------------------------------------------------------------------------------------------------ GELU (tanh form)
