@@ -59,21 +59,28 @@ __host__ __device__ constexpr int bwd_parts(int tile) { return tile >= 64 ? JVPA
 // 48 cycles for 32 cycles of arithmetic and N = 32 takes 40 for 16, while N = 128 ([S | Sd], [A | C] of a 64-row tile)
 // reads as long as it multiplies.  Forward and backward of 128 heads at length 2048: 5.42 ms with 32-row tiles, 4.30 ms so.
 __host__ __device__ constexpr bool bwd_pair_ring(int D) { return D == 128; }
-__host__ __device__ constexpr bool bwd_two_issuers(int D, bool kv) { return !kv && !bwd_pair_ring(D); }
+// Without tangents two of the four tensors on either side, one of the two score products per region and the tangent
+// accumulators are absent.  At head_dim 64 two CTAs then share an SM, one's products beside the other's score algebra
+// (192 x 12 heads of length 128: key owner 55 -> 41 us, query owner 42 -> 35 us).
+__host__ __device__ constexpr bool bwd_compact(int D, bool has_t) { return D == 64 && !has_t; }
+__host__ __device__ constexpr bool bwd_two_issuers(int D, bool kv, bool has_t) { return !kv && !bwd_pair_ring(D) && !bwd_compact(D, has_t); }
 
-template <int D, int TILE, bool kKV, bool kDoK>
+template <int D, int TILE, bool kKV, bool kDoK, bool kHasT>
 struct BwdSmem {
   static constexpr int kBoxes = D / 64;
   static constexpr int kXBuf = D == 64 ? 2 : 1;  // owned-row tiles are double buffered where shared memory allows
   static constexpr int kStages = 2;
   static constexpr bool kRing = bwd_pair_ring(D);
   static constexpr int kStages2 = kRing && kDoK ? 1 : 2;  // stages of (Y2, Y3)
-  static constexpr int kXTensors = kDoK ? 4 : 2;          // the dV / dVd pass reads X0 and X1 only
+  static constexpr bool kCompact = bwd_compact(D, kHasT);  // tensor 0 and the one of 2 and 3 that is there, in slots 0 and 1
+  static constexpr int kXTensors = kDoK && !kCompact ? 4 : 2;  // the dV / dVd pass reads X0 and X1 only
+  static constexpr int kPer = kRing || kCompact ? 2 : 4;       // streamed tensors of a stage
+  static __host__ __device__ constexpr int slot(int t) { return kCompact ? t >> 1 : t; }
   alignas(1024) uint16_t x[kXBuf][kXTensors][kBoxes][kRows * 64];
   // Streamed tiles.  Within a stage the 64-channel box is outermost and the four tensors of a box (kRing: the two of a pair)
   // are adjacent, so that [Y0 ; Y1] and [Y2 ; Y3] are each one K-major B operand of 2 TILE rows (merged score products) at
   // any head dimension.  kRing: the stages of (Y0, Y1), then those of (Y2, Y3).
-  alignas(1024) uint16_t y[(kRing ? 2 * (kStages + kStages2) : 4 * kStages) * kBoxes][TILE * 64];
+  alignas(1024) uint16_t y[(kStages + (kRing ? kStages2 : 0)) * kPer * kBoxes][TILE * 64];
   float4 stats[kKV ? 2 : 1][kKV ? TILE : 1];  // key owner only: per query column {lse*log2e, mu, delta, dsum} (double buffered)
   // Query owner: the owned rows' statistics {lse, mu, delta, dsum} as four float arrays, brought in by bulk copies
   // that complete on the same barrier as the rows.  Its compute warps then issue no global loads at all: a load in
@@ -167,11 +174,11 @@ __global__ void __launch_bounds__(256) row_dots_kernel(BwdArgs a, float *delta, 
 }
 
 template <int D, int TILE, bool kKV, bool kDoK, bool kDoV, typename T, bool kPair, bool kHasT>
-__global__ void __launch_bounds__(bwd_threads(bwd_parts(TILE), bwd_two_issuers(D, kKV)), 1) sm100_bwd_kernel(const __grid_constant__ BwdMaps maps, BwdKernelArgs a) {
+__global__ void __launch_bounds__(bwd_threads(bwd_parts(TILE), bwd_two_issuers(D, kKV, kHasT)), bwd_compact(D, kHasT) ? 2 : 1) sm100_bwd_kernel(const __grid_constant__ BwdMaps maps, BwdKernelArgs a) {
   constexpr int kParts = bwd_parts(TILE);
   constexpr int kComputeThreads = 128 * kParts;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
-  using Smem = BwdSmem<D, TILE, kKV, kDoK>;
+  using Smem = BwdSmem<D, TILE, kKV, kDoK, kHasT>;
   Smem &s = *reinterpret_cast<Smem *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   if constexpr (Smem::kRing && kDoK) {  // no room was left to round up: the base must have been aligned
     if (reinterpret_cast<uintptr_t>(smem_raw) % 1024 != 0) {
@@ -183,17 +190,18 @@ __global__ void __launch_bounds__(bwd_threads(bwd_parts(TILE), bwd_two_issuers(D
   constexpr int kStages = Smem::kStages;
   constexpr bool kRing = Smem::kRing;
   constexpr int kStages2 = Smem::kStages2;
-  constexpr int kAcc = (kDoK ? 2 : 0) + (kDoV ? 2 : 0);
+  constexpr int kPairs = kHasT ? 2 : 1;  // a gradient and its tangent's
+  constexpr int kAcc = (kDoK ? kPairs : 0) + (kDoV ? kPairs : 0);
   // accumulators; the tangent-gradient tile sits below its partner so that one N = 2D instruction can update both
-  constexpr uint32_t kColKd = 0, kColK = D;                          // dX1, dX0
-  constexpr uint32_t kColVd = kDoK ? 2 * D : 0, kColV = kColVd + D;  // dVd, dV
+  constexpr uint32_t kColKd = 0, kColK = kHasT ? D : 0;                                   // dX1, dX0
+  constexpr uint32_t kColVd = kDoK ? kPairs * D : 0, kColV = kColVd + (kHasT ? D : 0);  // dVd, dV
   // two score regions that are in different phases of the pipeline: (S | Sd) and (A | C)
-  constexpr uint32_t kColS = kAcc * D, kColA = kColS + 2 * TILE, kColC = kColS + 3 * TILE;
+  constexpr uint32_t kColS = kAcc * D, kColA = kColS + kPairs * TILE, kColC = kColS + (2 * kPairs - 1) * TILE;
   // Query owner: its two accumulators leave room for a separate, double-buffered home of the W1 / W2 operands
   // (TILE / 2 packed columns each), so that the (A | C) region is free again as soon as the score algebra has read it
   // instead of when the output products have consumed the operands written over it.
   // (Not at head_dim 128: accumulators and score regions of 64 columns fill tensor memory.)
-  constexpr bool kSplit = bwd_two_issuers(D, kKV);
+  constexpr bool kSplit = bwd_two_issuers(D, kKV, kHasT);
   // The dV / dVd pass at head_dim 128 has no (A | C): (S | Sd) takes both regions in turn, so that the tensor core forms the next
   // tile's scores while the compute warps work on this one's.
   // Scores and score algebra then run up to two tiles ahead of each other's waits, which a parity wait on one barrier would
@@ -202,7 +210,7 @@ __global__ void __launch_bounds__(bwd_threads(bwd_parts(TILE), bwd_two_issuers(D
   constexpr bool kAlternate = kRing && !kDoK;
   auto alt = [](int g) { return kAlternate ? g & 1 : 0; };
   auto alt_parity = [](int g) { return (kAlternate ? g >> 1 : g) & 1; };
-  constexpr uint32_t kColW = kAcc * D + 4 * TILE;
+  constexpr uint32_t kColW = kAcc * D + 2 * kPairs * TILE;
   constexpr uint32_t kWBuf = kPair ? 2 * TILE : TILE;  // columns of one buffer: W1, W2, each with its low parts where kPair
   constexpr uint32_t kUsed = kColW + (kSplit ? 2 * kWBuf : 0);
   static_assert(kUsed <= 512, "TMEM budget");
@@ -298,9 +306,9 @@ __global__ void __launch_bounds__(bwd_threads(bwd_parts(TILE), bwd_two_issuers(D
           return false;
         }
         mbar_expect_tx(&s.x_full[xb], __popc(a.xmask) * kRows * D * 2 + (kKV ? 0 : (has_t ? 4 : 3) * kRows * 4));
-        for (int t = 0; t < Smem::kXTensors; ++t)
+        for (int t = 0; t < (kDoK ? 4 : 2); ++t)
           if (a.xmask >> t & 1)
-            for (int x = 0; x < kBoxes; ++x) tma_load_4d(s.x[xb][t][x], &maps.x[t], &s.x_full[xb], 64 * x, x0, h, b);
+            for (int x = 0; x < kBoxes; ++x) tma_load_4d(s.x[xb][Smem::slot(t)][x], &maps.x[t], &s.x_full[xb], 64 * x, x0, h, b);
         if (!kKV) {
           if (n_ == 0) griddep_wait();  // delta / dsum are the row-dot kernel's output
           const size_t si = ((size_t)b * a.H + h) * a.stat_len + x0;  // stat_len is a multiple of 128: always in bounds
@@ -347,12 +355,12 @@ __global__ void __launch_bounds__(bwd_threads(bwd_parts(TILE), bwd_two_issuers(D
             ok = false;
             break;
           }
-          constexpr int kPer = kRing ? 2 : 4;  // tensors that complete on one barrier
-          mbar_expect_tx(&s.y_full[st], __popc(a.ymask & ((1 << kPer) - 1)) * kTileBytes);
-          for (int t = 0; t < kPer; ++t)
+          constexpr int kOne = kRing ? 2 : 4;  // tensors that complete on one barrier
+          mbar_expect_tx(&s.y_full[st], __popc(a.ymask & ((1 << kOne) - 1)) * kTileBytes);
+          for (int t = 0; t < kOne; ++t)
             if (a.ymask >> t & 1)
               for (int x = 0; x < kBoxes; ++x)
-                tma_load_4d(s.y[(st * kBoxes + x) * kPer + t], &maps.y[t], &s.y_full[st], 64 * x, j * TILE, h, b);
+                tma_load_4d(s.y[(st * kBoxes + x) * Smem::kPer + Smem::slot(t)], &maps.y[t], &s.y_full[st], 64 * x, j * TILE, h, b);
           if constexpr (kRing) {
             const int st2 = g % kStages2;
             if (!mbar_wait_for(a.wait_cycles, &s.y2_empty[st2], ((g / kStages2) & 1) ^ 1)) {
@@ -398,16 +406,16 @@ __global__ void __launch_bounds__(bwd_threads(bwd_parts(TILE), bwd_two_issuers(D
       // that issuing an MMA costs a handful of instructions (the issue rate of this one thread bounds the kernel).
       const uint32_t base16 = smem_u32(&s) >> 4;
       constexpr uint32_t kXTile = kRows * 128, kYTile = TILE * 128;  // bytes of one 64-channel box
-      constexpr int kPer = kRing ? 2 : 4;  // adjacent tensors of a box
+      constexpr int kPer = Smem::kPer;  // adjacent tensors of a box
       auto xbase = [&](int xb) { return base16 + (uint32_t)((offsetof(Smem, x) + (size_t)xb * Smem::kXTensors * kBoxes * kXTile) >> 4); };
       auto ybase = [&](int st) { return base16 + (uint32_t)((offsetof(Smem, y) + (size_t)st * kPer * kBoxes * kYTile) >> 4); };
       // base for tensors 2 and 3 of tile g (their place follows from their index as in a stage of four)
       auto ybase2 = [&](int g) { return kRing ? ybase(kStages + g % kStages2) - (2 * kYTile >> 4) : ybase(g % kStages); };
       auto xd = [&](uint32_t xlo, int t, int kk) {
-        return xlo + (uint32_t)(((t * kBoxes + (kk >> 2)) * kXTile + (kk & 3) * 32) >> 4) + kDescLoKMajor;
+        return xlo + (uint32_t)(((Smem::slot(t) * kBoxes + (kk >> 2)) * kXTile + (kk & 3) * 32) >> 4) + kDescLoKMajor;
       };
       auto yd = [&](uint32_t ylo, int t, int kk) {
-        return ylo + (uint32_t)((((kk >> 2) * kPer + t) * kYTile + (kk & 3) * 32) >> 4) + kDescLoKMajor;
+        return ylo + (uint32_t)((((kk >> 2) * kPer + Smem::slot(t)) * kYTile + (kk & 3) * 32) >> 4) + kDescLoKMajor;
       };
       // one accumulator at a time, 16 channels per instruction.  g = tile counter (stage / parity), xb = X buffer,
       // last = this is the item's last tile (its X tiles are released once no later score MMA needs them)
@@ -416,7 +424,7 @@ __global__ void __launch_bounds__(bwd_threads(bwd_parts(TILE), bwd_two_issuers(D
         if (!mbar_wait_for(a.wait_cycles, &s.y_full[st], (g / kStages) & 1)) return false;
         tc_fence_after();
         const uint32_t xlo = xbase(xb), ylo = ybase(st);
-        const uint32_t sc = kColS + (kAlternate ? (uint32_t)(g & 1) * 2 * TILE : 0);
+        const uint32_t sc = kColS + (kAlternate ? (uint32_t)(g & 1) * kPairs * TILE : 0);
         if (kMergeS && has_t) {
           // [S | Sd] = X0 [Y0 ; Y1]^T in one N = 2 TILE instruction per step, then Sd += X1 Y0^T
 #pragma unroll
@@ -477,7 +485,7 @@ __global__ void __launch_bounds__(bwd_threads(bwd_parts(TILE), bwd_two_issuers(D
       // one tensor (d = 128: kPer tiles apart) or, for the merged d = 64 products, two adjacent tensors
       constexpr uint32_t lbo = (kBoxes == 1 ? 1 : kPer) * TILE * 128;
       auto yb = [&](uint32_t ylo, int t, int kk) {
-        return ylo + (uint32_t)((t * kYTile + kk * 2048) >> 4) + desc_lo_mn_major(lbo);
+        return ylo + (uint32_t)((Smem::slot(t) * kYTile + kk * 2048) >> 4) + desc_lo_mn_major(lbo);
       };
       // the thread that owned score columns [16 kk, 16 kk + 16) left its 8 packed operand columns at the start
       // of its own column range (see the score-algebra warps)
@@ -661,7 +669,7 @@ __global__ void __launch_bounds__(bwd_threads(bwd_parts(TILE), bwd_two_issuers(D
         }
         tc_fence_after();
         const uint32_t ylo_out = ybase(st), ylo_v = ybase2(g);
-        const uint32_t sp_ = tmem + kColS + (kAlternate ? (uint32_t)(g & 1) * 2 * TILE : 0), spn_ = sp_ + TILE;
+        const uint32_t sp_ = tmem + kColS + (kAlternate ? (uint32_t)(g & 1) * kPairs * TILE : 0), spn_ = sp_ + TILE;
         // (the common case, both cotangents present, is issued as straight-line code: a run-time condition between
         //  two instructions of a group costs this thread tens of cycles per instruction)
         if constexpr (kPair) {
@@ -861,7 +869,7 @@ __global__ void __launch_bounds__(bwd_threads(bwd_parts(TILE), bwd_two_issuers(D
       tc_fence_after();
       const float4 *st = s.stats[g & 1];
       const int nvalid = a.Ly - j * TILE;  // streamed rows in this tile (masking for the query owner)
-      const uint32_t tS = tlane + kColS + (kAlternate ? (uint32_t)(g & 1) * 2 * TILE : 0), tSd = tS + TILE;
+      const uint32_t tS = tlane + kColS + (kAlternate ? (uint32_t)(g & 1) * kPairs * TILE : 0), tSd = tS + TILE;
       // ---- first half: P = exp2(s*scale*log2e - lse*log2e), N = scale*sd - mu
       float2 sp[CH / 2], nn[CH / 2];  // scale * P and N, carried into the second half
 #pragma unroll
@@ -1036,7 +1044,7 @@ __global__ void __launch_bounds__(bwd_threads(bwd_parts(TILE), bwd_two_issuers(D
           tmem_ld16(tlane + col + cbase, *reinterpret_cast<uint32_t(*)[16]>(&r[0]));
         }
         tc_wait_ld();
-        unsigned char *tile = reinterpret_cast<unsigned char *>(s.x[xb][which][0]);
+        unsigned char *tile = reinterpret_cast<unsigned char *>(s.x[xb][Smem::slot(which)][0]);
 #pragma unroll
         for (int i = 0; i < kChan / 8; ++i) {
           uint4 v;
@@ -1076,9 +1084,9 @@ __global__ void __launch_bounds__(bwd_threads(bwd_parts(TILE), bwd_two_issuers(D
         if (ctid == 0) {
           if (ok) {
             if (w0) tma_store_4d(&maps.out[0], s.x[xb][0][0], 0, x0, h, b);
-            if (w1) tma_store_4d(&maps.out[1], s.x[xb][1][0], 0, x0, h, b);
-            if (w2) tma_store_4d(&maps.out[2], s.x[xb][2][0], 0, x0, h, b);
-            if (w3) tma_store_4d(&maps.out[3], s.x[xb][3][0], 0, x0, h, b);
+            if (w1) tma_store_4d(&maps.out[1], s.x[xb][Smem::slot(1)][0], 0, x0, h, b);
+            if (w2) tma_store_4d(&maps.out[2], s.x[xb][Smem::slot(2)][0], 0, x0, h, b);
+            if (w3) tma_store_4d(&maps.out[3], s.x[xb][Smem::slot(3)][0], 0, x0, h, b);
             tma_store_commit();
           }
           pending_xb = xb;
@@ -1151,17 +1159,18 @@ cudaError_t launch_side(const BwdArgs &a, const float *delta, const float *dsum,
   ka.B = a.B; ka.H = a.H; ka.Lx = Lx; ka.Ly = Ly; ka.Lq = a.Lq; ka.stat_len = a.stat_len;
   ka.has_o = has_o; ka.scale = a.scale;
   auto kernel = sm100_bwd_kernel<D, TILE, kKV, kDoK, kDoV, T, kPair, kHasT>;
-  using Smem = BwdSmem<D, TILE, kKV, kDoK>;
+  using Smem = BwdSmem<D, TILE, kKV, kDoK, kHasT>;
   // room to round the base up to 1 KB, as far as the SM has it (the kernel checks that it fits)
   const size_t smem = std::min<size_t>(sizeof(Smem) + 1024, 227 * 1024);
   static_assert(sizeof(Smem) <= 227 * 1024, "shared memory of one SM");
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   const int64_t items = (int64_t)a.B * a.H * ((Lx + kRows - 1) / kRows);
-  dim3 grid((unsigned)std::min<int64_t>(items, sm_count()));  // persistent: one CTA per SM walks the items
+  // persistent: one CTA (two where they fit) per SM walks the items
+  dim3 grid((unsigned)std::min<int64_t>(items, sm_count() * (Smem::kCompact ? 2 : 1)));
   {
     LaunchScope scope(kKV ? kIdBwdKeyTc : kIdBwdQueryTc, stream);
-    e = launch_overlapped(kernel, grid, dim3(bwd_threads(bwd_parts(TILE), bwd_two_issuers(D, kKV))), smem, stream, maps, ka);
+    e = launch_overlapped(kernel, grid, dim3(bwd_threads(bwd_parts(TILE), bwd_two_issuers(D, kKV, kHasT))), smem, stream, maps, ka);
   }
   return e != cudaSuccess ? e : cudaGetLastError();
 }
@@ -1183,7 +1192,7 @@ cudaError_t launch_bwd(const BwdArgs &a, cudaStream_t stream) {
   cudaError_t e = cudaSuccess;
   if constexpr (D == 64) {
     // (query owner with operand pairs: two accumulators, a 64-column score tile and both W buffers would take 640 columns)
-    e = launch_side<D, kPair ? 32 : 64, false, true, false, T, kPair, kHasT>(a, delta, dsum, stream);
+    e = launch_side<D, kPair && kHasT ? 32 : 64, false, true, false, T, kPair, kHasT>(a, delta, dsum, stream);
     if (e != cudaSuccess) return e;
     return launch_side<D, 64, true, true, true, T, kPair, kHasT>(a, delta, dsum, stream);
   } else {

@@ -43,18 +43,24 @@ constexpr int kThreads = 192;
 template <typename T> struct RescaleThreshold { static constexpr float value = 8.0f; };
 template <> struct RescaleThreshold<__half> { static constexpr float value = 0.0f; };
 
-template <int D>
+template <int D, bool kHasT>
 struct FwdSmem {
   static constexpr int kBoxes = D / 64;
+  static constexpr int kPer = kHasT ? 2 : 1;  // tensors of a pair
   alignas(1024) uint16_t q[kBoxes][kBM * 64];
-  alignas(1024) uint16_t tq[kBoxes][kBM * 64];
+  alignas(1024) uint16_t tq[kHasT ? kBoxes : 1][kHasT ? kBM * 64 : 8];
   // Per stage the pairs (K, Kd) and (V, Vd), each with barriers of its own: the score products are done with K long before
   // the value products with V.  [K ; Kd] is one K-major operand of 128 rows (64-channel box outermost), [V | Vd] one MN-major
   // operand of 2 D columns (tensor outermost).
-  alignas(1024) uint16_t kv[kStages][2][2 * kBoxes][kBN * 64];
+  alignas(1024) uint16_t kv[kStages][2][kPer * kBoxes][kBN * 64];
   uint64_t q_full, k_full[kStages], k_empty[kStages], v_full[kStages], v_empty[kStages], s_full[2], p_full[2], o_done;
   uint32_t tmem_base;
 };
+
+// CTAs that share an SM.  Without tangents a CTA needs half the tensor memory and shared memory, so that twice as many could
+// work on short sequences, where a CTA is a chain of waits (load, scores, softmax, product, store): three at head_dim 64 (96
+// registers a thread; 192 x 12 heads of length 128: 44 -> 35 us), two at 128.
+__host__ __device__ constexpr int fwd_ctas_per_sm(int D, bool has_t) { return D == 64 ? (has_t ? 2 : 3) : (has_t ? 1 : 2); }
 
 struct FwdMaps {
   CUtensorMap q, tq, k, tk, v, tv;
@@ -62,19 +68,23 @@ struct FwdMaps {
 };
 
 template <int D, typename T, bool kHasT, bool kPair>
-__global__ void __launch_bounds__(kThreads, D == 64 ? 2 : 1) sm100_fwd_kernel(const __grid_constant__ FwdMaps maps, FwdArgs a) {
+__global__ void __launch_bounds__(kThreads, fwd_ctas_per_sm(D, kHasT)) sm100_fwd_kernel(const __grid_constant__ FwdMaps maps, FwdArgs a) {
   extern __shared__ unsigned char smem_raw[];
-  using Smem = FwdSmem<D>;
+  using Smem = FwdSmem<D, kHasT>;
   Smem &s = *reinterpret_cast<Smem *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   constexpr int kBoxes = D / 64;
-  constexpr uint32_t kTmemCols = (2 * D + 128) <= 256 ? 256 : 512;
-  constexpr uint32_t kColO = 0, kColOd = D, kColS = 2 * D;  // Sd / U 64 columns behind S / P
+  constexpr uint32_t kColO = 0, kColOd = D, kColS = (kHasT ? 2 : 1) * D;  // Sd / U 64 columns behind S / P
+  constexpr uint32_t kRegion = kHasT ? 128 : 64;                          // columns of (S | Sd)
   // D = 128 leaves one CTA per SM, with nothing to run beside its softmax: (S | Sd) alternates between two regions and the
   // scores of tile j + 1 are issued ahead of the value products of tile j.  Scores and softmax then run up to two tiles ahead of
   // each other's waits, which a parity wait on one barrier would mistake for none: their barriers alternate too.
   // 128 heads at length 2048: 934 -> 614 us.
   constexpr bool kAlternate = D == 128;
-  static_assert(2 * D + (kAlternate ? 256 : 128) <= kTmemCols, "TMEM budget");
+  constexpr uint32_t kUsed = kColS + (kAlternate ? 2 : 1) * kRegion;
+  constexpr uint32_t kTmemCols = kUsed <= 128 ? 128 : kUsed <= 256 ? 256 : 512;
+  static_assert(kUsed <= 512 && fwd_ctas_per_sm(D, kHasT) * kTmemCols <= 512, "TMEM budget");
+  // three CTAs per SM: 96 registers, so the scores are read again after the maximum instead of held
+  constexpr bool kReload = fwd_ctas_per_sm(D, kHasT) == 3;
   auto alt = [](int j) { return kAlternate ? j & 1 : 0; };
   auto alt_parity = [](int j) { return (kAlternate ? j >> 1 : j) & 1; };
   constexpr bool kBf16 = IsBf16<T>::value;
@@ -88,8 +98,8 @@ __global__ void __launch_bounds__(kThreads, D == 64 ? 2 : 1) sm100_fwd_kernel(co
     const int st = j % kStages;
     mbar_expect_tx(&s.k_full[st], kPairBytes + extra);
     for (int x = 0; x < kBoxes; ++x) {
-      tma_load_4d(s.kv[st][0][2 * x], &maps.k, &s.k_full[st], 64 * x, j * kBN, h, b);
-      if (kHasT) tma_load_4d(s.kv[st][0][2 * x + 1], &maps.tk, &s.k_full[st], 64 * x, j * kBN, h, b);
+      tma_load_4d(s.kv[st][0][Smem::kPer * x], &maps.k, &s.k_full[st], 64 * x, j * kBN, h, b);
+      if (kHasT) tma_load_4d(s.kv[st][0][Smem::kPer * x + 1], &maps.tk, &s.k_full[st], 64 * x, j * kBN, h, b);
     }
   };
   auto load_v = [&](int j) {
@@ -171,7 +181,7 @@ __global__ void __launch_bounds__(kThreads, D == 64 ? 2 : 1) sm100_fwd_kernel(co
       // Descriptors are one runtime base word plus compile-time offsets: this one thread issues every MMA of the CTA, so
       // instructions per MMA bound the tensor throughput.
       auto pair_base = [&](int st, int pair) {
-        return base16 + (uint32_t)((offsetof(Smem, kv) + (size_t)(st * 2 + pair) * 2 * kBoxes * kKvTile) >> 4);
+        return base16 + (uint32_t)((offsetof(Smem, kv) + (size_t)(st * 2 + pair) * Smem::kPer * kBoxes * kKvTile) >> 4);
       };
       // S = Q K^T ; Sd = Qd K^T + Q Kd^T      (K-major operands, 16 channels per instruction)
       auto scores = [&](int j) -> bool {
@@ -181,11 +191,11 @@ __global__ void __launch_bounds__(kThreads, D == 64 ? 2 : 1) sm100_fwd_kernel(co
           return false;
         }
         tc_fence_after();
-        const uint32_t klo = pair_base(st, 0), sc = tmem + kColS + alt(j) * 128;
+        const uint32_t klo = pair_base(st, 0), sc = tmem + kColS + alt(j) * kRegion;
         auto qd = [&](size_t member, int kk) {
           return base16 + (uint32_t)((member + (kk >> 2) * kQTile + (kk & 3) * 32) >> 4) + kDescLoKMajor;
         };
-        auto kd = [&](int kk) { return klo + (uint32_t)(((kk >> 2) * 2 * kKvTile + (kk & 3) * 32) >> 4) + kDescLoKMajor; };
+        auto kd = [&](int kk) { return klo + (uint32_t)(((kk >> 2) * Smem::kPer * kKvTile + (kk & 3) * 32) >> 4) + kDescLoKMajor; };
         // [S | Sd] = Q [K ; Kd]^T in one N = 128 instruction per step, then Sd += Qd K^T
 #pragma unroll
         for (int kk = 0; kk < D / 16; ++kk) mma_ss_lo(sc, qd(offsetof(Smem, q), kk), kd(kk), kHasT ? idesc_s2 : idesc_s, kk > 0);
@@ -210,7 +220,7 @@ __global__ void __launch_bounds__(kThreads, D == 64 ? 2 : 1) sm100_fwd_kernel(co
           break;
         }
         tc_fence_after();
-        const uint32_t vlo = pair_base(st, 1), pcol = tmem + kColS + alt(j) * 128, ucol = pcol + 64;
+        const uint32_t vlo = pair_base(st, 1), pcol = tmem + kColS + alt(j) * kRegion, ucol = pcol + 64;
         // O += P V ; Od' += U V + P Vd          (A from TMEM, B = value tile read MN-major, 16 keys per instruction)
 #pragma unroll
         for (int kk = 0; kk < kBN / 16; ++kk) {
@@ -252,7 +262,7 @@ __global__ void __launch_bounds__(kThreads, D == 64 ? 2 : 1) sm100_fwd_kernel(co
         break;
       }
       tc_fence_after();
-      const uint32_t tS = tlane + kColS + alt(j) * 128, tSd = tS + 64;
+      const uint32_t tS = tlane + kColS + alt(j) * kRegion, tSd = tS + 64;
       // the 64 scores of this row and the first half of Sd in flight at once, one wait
       uint32_t sv[64], sd[32];
       {
@@ -264,11 +274,15 @@ __global__ void __launch_bounds__(kThreads, D == 64 ? 2 : 1) sm100_fwd_kernel(co
         tc_wait_ld();
       }
       const int nvalid = a.Lk - j * kBN;  // >= 1; < 64 only on the last tile
-      if (nvalid < 64) {
+      auto mask32 = [&](uint32_t *v, int c0) {
+        if (nvalid < 64) {
 #pragma unroll
-        for (int c = 0; c < 64; ++c)
-          if (c >= nvalid) sv[c] = __float_as_uint(-INFINITY);
-      }
+          for (int c = 0; c < 32; ++c)
+            if (c0 + c >= nvalid) v[c] = __float_as_uint(-INFINITY);
+        }
+      };
+      mask32(&sv[0], 0);
+      mask32(&sv[32], 32);
       // row max of the raw scores on four independent chains (scale > 0 commutes with the max)
       float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
@@ -315,9 +329,17 @@ __global__ void __launch_bounds__(kThreads, D == 64 ? 2 : 1) sm100_fwd_kernel(co
           tmem_ld32(tSd + c0, sd);
           tc_wait_ld();
         }
+        uint32_t *sc = &sv[c0];
+        uint32_t again[kReload ? 32 : 1];
+        if constexpr (kReload) {
+          tmem_ld32(tS + c0, again);
+          tc_wait_ld();
+          mask32(again, c0);
+          sc = again;
+        }
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
-          const float2 t = __ffma2_rn(make_float2(__uint_as_float(sv[c0 + 2 * i]), __uint_as_float(sv[c0 + 2 * i + 1])), sl2x2, negm);
+          const float2 t = __ffma2_rn(make_float2(__uint_as_float(sc[2 * i]), __uint_as_float(sc[2 * i + 1])), sl2x2, negm);
           const float2 p = make_float2(fast_exp2(t.x), fast_exp2(t.y));
           psum[i & 1] = __fadd2_rn(psum[i & 1], p);
           pk[i] = pack2<T>(p.x, p.y);
@@ -375,7 +397,7 @@ __global__ void __launch_bounds__(kThreads, D == 64 ? 2 : 1) sm100_fwd_kernel(co
         if (kHasT) tmem_ld32(tlane + kColOd + c, rd);
         tc_wait_ld();
         unsigned char *otile = reinterpret_cast<unsigned char *>(s.q[c / 64]);
-        unsigned char *dtile = reinterpret_cast<unsigned char *>(s.tq[c / 64]);
+        unsigned char *dtile = reinterpret_cast<unsigned char *>(s.tq[kHasT ? c / 64 : 0]);
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           uint32_t po[4], pd[4];
@@ -429,7 +451,7 @@ cudaError_t launch_fwd(const FwdArgs &a, cudaStream_t stream) {
       return cudaErrorInvalidValue;
   }
   auto kernel = sm100_fwd_kernel<D, T, kHasT, kPair>;
-  const size_t smem = sizeof(FwdSmem<D>) + 1024;
+  const size_t smem = sizeof(FwdSmem<D, kHasT>) + 1024;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   dim3 grid((a.Lq + kBM - 1) / kBM, a.H, a.B);
