@@ -30,6 +30,8 @@ import torch.autograd.forward_ad as fwAD
 import torch.nn.functional as F
 
 from . import _lib
+from ._nodes import apply, node
+from .ops import _on_device
 
 _CODES = {torch.bfloat16: 0, torch.float32: 2}
 
@@ -86,7 +88,7 @@ def _ln_launch(which, x, tx, gamma, beta, shift, scale, tshift, tscale, mean, rs
     B, S, C = x.shape
     (sh, sc, sc_stride), (tsh, tsc, tstride) = _modulation_rows(shift, scale, tshift, tscale, B, C)
     lib = _lib.load()
-    with torch.cuda.device(x.device):
+    with _on_device(x.device):
         rc = lib.jvpattn_ln_modulate(which, _ptr(x), _ptr(tx), _ptr(gamma), _ptr(beta), _ptr(sh), _ptr(sc), _ptr(tsh), _ptr(tsc),
                                      sc_stride, tstride, _ptr(mean), _ptr(rstd), _ptr(out), _ptr(g), _ptr(dx), _ptr(dtx), _ptr(sums),
                                      B, S, C, float(eps), int(exact), _CODES[x.dtype], _stream(x))
@@ -98,7 +100,7 @@ def _ln_dual_launch(which, x, tx, gamma, beta, shift, scale, tshift, tscale, mea
     B, S, C = x.shape
     (sh, sc, sc_stride), (tsh, tsc, tstride) = _modulation_rows(shift, scale, tshift, tscale, B, C)
     lib = _lib.load()
-    with torch.cuda.device(x.device):
+    with _on_device(x.device):
         rc = lib.jvpattn_ln_modulate_dual(which, _ptr(x), _ptr(tx), _ptr(gamma), _ptr(beta), _ptr(sh), _ptr(sc), _ptr(tsh), _ptr(tsc),
                                           sc_stride, tstride, _ptr(mean), _ptr(rstd), _ptr(y), _ptr(ty), _ptr(g), _ptr(gt), _ptr(dx),
                                           _ptr(dtx), _ptr(sums), B, S, C, float(eps), int(exact), _CODES[x.dtype], _stream(x))
@@ -119,7 +121,7 @@ def _ln_finalize(sums_y, sums_ty, gamma, beta, scale, tscale, want_tangent_grads
     d_gamma = param_grads[0]
     d_beta = param_grads[1] if beta is not None else None
     lib = _lib.load()
-    with torch.cuda.device(dev):
+    with _on_device(dev):
         rc = lib.jvpattn_ln_finalize(_ptr(sums_y), _ptr(sums_ty), _ptr(gamma), _ptr(beta), _ptr(sc), _ptr(tsc), sc_stride, tsc_stride,
                                      _ptr(d_shift), _ptr(d_scale), _ptr(d_tshift), _ptr(d_tscale), _ptr(d_gamma), _ptr(d_beta),
                                      B, C, _CODES[dt], _stream(scale))
@@ -127,6 +129,7 @@ def _ln_finalize(sums_y, sums_ty, gamma, beta, scale, tscale, want_tangent_grads
     return d_shift, d_scale, d_tshift, d_tscale, d_gamma, d_beta
 
 
+@node
 class _LnModulateDual(torch.autograd.Function):
     """(x, gamma, beta, shift, scale, tx, tshift, tscale) -> (y, ty) as one autograd node: a reverse pass brings the
     cotangents of both outputs at once (bf16: to one backward kernel; fp32: to one each, which leave their sum in dx), and
@@ -189,6 +192,7 @@ class _LnModulateDual(torch.autograd.Function):
                 shaped(d_tshift, tshift), shaped(d_tscale, tscale), None, None)
 
 
+@node
 class _LnModulate(torch.autograd.Function):
     @staticmethod
     def forward(x, gamma, beta, shift, scale, eps, exact):
@@ -229,7 +233,7 @@ def ln_modulate(x: torch.Tensor, norm: torch.nn.LayerNorm, shift: torch.Tensor, 
     beta = norm.bias.float() if norm.bias is not None else None
     (xp, tx), (shp, tsh), (scp, tsc) = (fwAD.unpack_dual(t) for t in (x, shift, scale))
     if tx is None and tsh is None and tsc is None:
-        y, _, _ = _LnModulate.apply(x.contiguous(), norm.weight.float(), beta, shift, scale, norm.eps, exact)
+        y, _, _ = apply(_LnModulate, x.contiguous(), norm.weight.float(), beta, shift, scale, norm.eps, exact)
         return y
     # forward-mode AD is active: one node maps primals and tangents to (y, ty); the LayerNorm weight and bias are
     # parameters and carry no tangent where this is used
@@ -271,7 +275,7 @@ def _gate_launch(x, y, gate, mask, z, drop=None):
     B, S, C = y.shape
     gt, gt_stride = _rows(gate, B, C)
     lib = _lib.load()
-    with torch.cuda.device(y.device):
+    with _on_device(y.device):
         rc = lib.jvpattn_gated_residual(_ptr(x), _ptr(y), _ptr(gt), _ptr(mask), gt_stride, _ptr(z), B, S, C, _CODES[y.dtype],
                                         _drop_struct(drop), _stream(y))
     _lib.check(rc, "jvpattn_gated_residual")
@@ -282,13 +286,14 @@ def _gate_dual_launch(which, x, tx, y, ty, gate, tgate, mask, z, tz, gz, gtz, d_
     gt, gt_stride = _rows(gate, B, C)
     tg, tg_stride = _rows(tgate, B, C)
     lib = _lib.load()
-    with torch.cuda.device(y.device):
+    with _on_device(y.device):
         rc = lib.jvpattn_gated_residual_dual(which, _ptr(x), _ptr(tx), _ptr(y), _ptr(ty), _ptr(gt), _ptr(tg), _ptr(mask), gt_stride,
                                              tg_stride, _ptr(z), _ptr(tz), _ptr(gz), _ptr(gtz), _ptr(d_y), _ptr(d_ty), _ptr(sums),
                                              B, S, C, _CODES[y.dtype], _drop_struct(drop), _stream(y))
     _lib.check(rc, "jvpattn_gated_residual_dual")
 
 
+@node
 class _GatedResidualDual(torch.autograd.Function):
     """(x, y, gate, mask, tx, ty, tgate) -> (z, tz) = (x + m gate y, tx + m (gate ty + tgate y)) as one autograd node:
     one kernel forward, one kernel for the cotangents of both outputs.  Any of tx, ty, tgate may be absent (zero)."""
@@ -325,6 +330,7 @@ class _GatedResidualDual(torch.autograd.Function):
         return (gz, d_y, d_gate, None, gtz if ctx.has_tx else None, d_ty if ty is not None else None, d_tgate, None)
 
 
+@node
 class _GatedResidual(torch.autograd.Function):
     @staticmethod
     def forward(x, y, gate, mask, drop):
@@ -365,12 +371,13 @@ def gated_residual(skip: torch.Tensor, branch: torch.Tensor, gate: torch.Tensor,
         else:
             mask = torch.empty_like(yp).bernoulli_(1.0 - p).div_(1.0 - p)
     if tx is None and ty is None and tg is None:
-        return _GatedResidual.apply(skip.contiguous(), branch.contiguous(), gate, mask, drop)
+        return apply(_GatedResidual, skip.contiguous(), branch.contiguous(), gate, mask, drop)
     z, tz = _GatedResidualDual.apply(xp.contiguous(), yp.contiguous(), gp, mask, tx, ty, tg, drop)
     return fwAD.make_dual(z, tz)
 
 
 # ----------------------------------------------------------------------------------------------- linear layer
+@node
 class _DualLinear(torch.autograd.Function):
     """(x, tx, w, b) -> (x w^T + b, tx w^T) as one autograd node: two GEMMs forward; backward two GEMMs for dx / dtx, two
     for dw (the second accumulating into the first through the GEMM's own epilogue) and one reduction for db - no
@@ -425,11 +432,12 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None = No
 # ----------------------------------------------------------------------------------------------- GELU (tanh form)
 def _gelu_launch(mode, h, v, w, u, out, out2):
     lib = _lib.load()
-    with torch.cuda.device(h.device):
+    with _on_device(h.device):
         rc = lib.jvpattn_gelu_dual(mode, _ptr(h), _ptr(v), _ptr(w), _ptr(u), _ptr(out), _ptr(out2), h.numel(), _CODES[h.dtype], _stream(h))
     _lib.check(rc, "jvpattn_gelu_dual")
 
 
+@node
 class _GeluDual(torch.autograd.Function):
     """(h, th) -> (gelu(h), gelu'(h) th) as one autograd node; backward: d_h = gelu'(h) gy + gelu''(h) th gty,
     d_th = gelu'(h) gty, one kernel for whichever cotangents arrive."""
@@ -463,6 +471,7 @@ class _GeluDual(torch.autograd.Function):
         return d_h, d_th
 
 
+@node
 class _Gelu(torch.autograd.Function):
     @staticmethod
     def forward(h):
@@ -490,7 +499,7 @@ def gelu_tanh(h: torch.Tensor) -> torch.Tensor:
         return F.gelu(h, approximate="tanh")
     hp, th = fwAD.unpack_dual(h)
     if th is None:
-        return _Gelu.apply(h)
+        return apply(_Gelu, h)
     y, ty = _GeluDual.apply(hp, th)
     return fwAD.make_dual(y, ty)
 
@@ -510,12 +519,13 @@ def _head_launch(which, logits, tlogits, x, dt, ddt, lse, out, g, dl, dtl):
     if tlogits is not None:
         tlogits, ldt = _rows3(tlogits)
     lib = _lib.load()
-    with torch.cuda.device(logits.device):
+    with _on_device(logits.device):
         rc = lib.jvpattn_flow_map_head(which, _ptr(logits), _ptr(tlogits), ld, ldt, _ptr(x), _ptr(dt), _ptr(ddt), _ptr(lse), _ptr(out),
                                        _ptr(g), _ptr(dl), _ptr(dtl), B, L, V, _CODES[logits.dtype], _stream(logits))
     _lib.check(rc, "jvpattn_flow_map_head")
 
 
+@node
 class _FlowHeadTangent(torch.autograd.Function):
     """dv = ddt (p - x) + dt p o (tlogits - sum(p tlogits)); backward = VJP of a cotangent on dv w.r.t. both logits."""
 
@@ -539,6 +549,7 @@ class _FlowHeadTangent(torch.autograd.Function):
         return dl, dtl, None, None, None, None
 
 
+@node
 class _FlowHead(torch.autograd.Function):
     @staticmethod
     def forward(logits, x, dt):
@@ -585,5 +596,5 @@ def flow_map_head(logits: torch.Tensor, x: torch.Tensor, dt: torch.Tensor) -> to
               and x.shape == logits.shape and logits.shape[-1] * (4 if logits.dtype == torch.bfloat16 else 8) <= 200 * 1024 - 64)
     if not usable:
         return x + dt.view(-1, 1, 1) * (logits.softmax(dim=-1) - x)
-    xst, _ = _FlowHead.apply(logits, x, dt.float().contiguous())
+    xst, _ = apply(_FlowHead, logits, x, dt.float().contiguous())
     return xst

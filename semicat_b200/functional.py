@@ -36,6 +36,7 @@ import torch.autograd.forward_ad as fwAD
 from torch.autograd.function import once_differentiable
 
 from . import ops
+from ._nodes import node, unrecorded
 
 __all__ = ["sdpa_jvp", "safe_sdpa_jvp", "set_kernel_family"]
 
@@ -55,6 +56,7 @@ def _like_input(x: torch.Tensor) -> torch.Tensor:
     return out if out.stride(-1) == 1 else torch.empty(x.shape, dtype=x.dtype, device=x.device)
 
 
+@node
 class _AttentionDual(torch.autograd.Function):
     """The fused kernel as ONE autograd node: (q, k, v, tq, tk, tv) -> (y, ty).
 
@@ -102,17 +104,22 @@ class _AttentionDual(torch.autograd.Function):
         return tuple(grads)
 
 
+def _primal_forward(q, k, v):
+    B, H, S, _ = q.shape
+    fix = lambda t: t if t.stride(-1) == 1 else t.contiguous()
+    q, k, v = fix(q), fix(k), fix(v)
+    y = torch.empty((B, S, H, v.shape[-1]), dtype=q.dtype, device=q.device).transpose(1, 2)
+    lse = torch.empty((B, H, ops.stat_len(S)), dtype=torch.float32, device=q.device)
+    ops.jvp_attention_fwd(q, k, v, None, None, None, y, None, lse, None, kernels=_kernels)
+    return q, k, v, y, lse
+
+
 class _PrimalAttention(torch.autograd.Function):
     """Plain attention through the primal-only kernel instance; used when no input carries a tangent."""
 
     @staticmethod
     def forward(ctx, q, k, v):
-        B, H, S, _ = q.shape
-        fix = lambda t: t if t.stride(-1) == 1 else t.contiguous()
-        q, k, v = fix(q), fix(k), fix(v)
-        y = torch.empty((B, S, H, v.shape[-1]), dtype=q.dtype, device=q.device).transpose(1, 2)
-        lse = torch.empty((B, H, ops.stat_len(S)), dtype=torch.float32, device=q.device)
-        ops.jvp_attention_fwd(q, k, v, None, None, None, y, None, lse, None, kernels=_kernels)
+        q, k, v, y, lse = _primal_forward(q, k, v)
         ctx.save_for_backward(q, k, v, y, lse)
         return y
 
@@ -154,7 +161,7 @@ def sdpa_jvp(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor) -> torch.Tensor:
     _validate(q, k, v)
     (qp, tq), (kp, tk), (vp, tv) = (fwAD.unpack_dual(t) for t in (q, k, v))
     if tq is None and tk is None and tv is None:
-        return _PrimalAttention.apply(q, k, v)
+        return _primal_forward(q, k, v)[3] if unrecorded() else _PrimalAttention.apply(q, k, v)
     # an input without a tangent has tangent zero
     tq = torch.zeros_like(qp) if tq is None else tq
     tk = torch.zeros_like(kp) if tk is None else tk

@@ -17,6 +17,8 @@ import torch
 import torch.autograd.forward_ad as fwAD
 
 from . import _lib
+from ._nodes import apply, node
+from .ops import _on_device
 
 _CODES = {torch.bfloat16: 0, torch.float16: 1, torch.float32: 2}
 
@@ -35,7 +37,7 @@ def _launch(x: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, out_dtype: to
     sin = sin.to(device=x.device, dtype=torch.float32).contiguous()
     y = torch.empty((B, S, H, D), dtype=out_dtype, device=x.device)
     lib = _lib.load()
-    with torch.cuda.device(x.device):
+    with _on_device(x.device):
         rc = lib.jvpattn_rotary_cast(x.data_ptr(), x.stride(0), x.stride(1), x.stride(2), _CODES[x.dtype], y.data_ptr(),
                                      _CODES[out_dtype], cos.data_ptr(), sin.data_ptr(), B, S, H, D, int(transpose),
                                      torch.cuda.current_stream(x.device).cuda_stream)
@@ -43,6 +45,7 @@ def _launch(x: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, out_dtype: to
     return y
 
 
+@node
 class _RotaryCast(torch.autograd.Function):
     """y = R x (rounded to ``out_dtype``); jvp: R x_t through the same function, so that the tangent output is itself
     differentiable; backward: R^T g in the dtype of x."""
@@ -69,7 +72,7 @@ def apply_rotary_cast(x: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, out
     """Rotate the halves of the last axis of ``x`` (B, S, H, D) by the angles whose cosines / sines are ``cos``,
     ``sin`` (S, D/2), in fp32, and return the result as a contiguous (B, S, H, D) tensor of ``out_dtype``.
     Equal, bit for bit, to ``torch.cat((x1*cos - x2*sin, x1*sin + x2*cos), -1).to(out_dtype)`` evaluated in fp32."""
-    return _RotaryCast.apply(x, cos.detach(), sin.detach(), out_dtype, False)
+    return apply(_RotaryCast, x, cos.detach(), sin.detach(), out_dtype, False)
 
 
 # ------------------------------------------------------------------------------------------------ q, k, v in one launch
@@ -84,7 +87,7 @@ def _launch_qkv(ins, outs, cos, sin, transpose: bool):
     B, S, H, D = ins[0].shape
     P3, S9 = ctypes.c_void_p * 3, ctypes.c_int64 * 9
     lib = _lib.load()
-    with torch.cuda.device(ins[0].device):
+    with _on_device(ins[0].device):
         rc = lib.jvpattn_rotary_qkv(ctypes.byref(P3(*[t.data_ptr() for t in ins])), ctypes.byref(S9(*sum((_strides3(t) for t in ins), []))),
                                     _QKV_CODES[ins[0].dtype], ctypes.byref(P3(*[t.data_ptr() for t in outs])),
                                     ctypes.byref(S9(*sum((_strides3(t) for t in outs), []))), _QKV_CODES[outs[0].dtype],
@@ -113,6 +116,7 @@ def _split_backward(grads, shape, like, cos, sin):
     return d
 
 
+@node
 class _RotaryQkv(torch.autograd.Function):
     @staticmethod
     def forward(qkv, cos, sin, out_dtype):
@@ -132,6 +136,7 @@ class _RotaryQkv(torch.autograd.Function):
         return _split_backward((gq, gk, gv), ctx.shape, ctx.like, ctx.cos, ctx.sin), None, None, None
 
 
+@node
 class _RotaryQkvDual(torch.autograd.Function):
     """(qkv, its tangent) -> (q, k, v, tq, tk, tv): the map is linear, so primal and tangent go through the same kernel,
     and one node receives all six cotangents."""
@@ -170,6 +175,6 @@ def rotary_qkv(qkv: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, out_dtyp
     cos = cos.detach().to(device=p.device, dtype=torch.float32).contiguous()
     sin = sin.detach().to(device=p.device, dtype=torch.float32).contiguous()
     if t is None:
-        return _RotaryQkv.apply(qkv, cos, sin, out_dtype)
+        return apply(_RotaryQkv, qkv, cos, sin, out_dtype)
     q, k, v, tq, tk, tv = _RotaryQkvDual.apply(p, t, cos, sin, out_dtype)
     return fwAD.make_dual(q, tq), fwAD.make_dual(k, tk), fwAD.make_dual(v, tv)

@@ -72,6 +72,29 @@ def test_cross_entropy_padded(V, eps):
         assert float(g[..., V:].abs().max()) == 0.0
 
 
+@pytest.mark.parametrize("V", [1, 7, 8, 9, 2047, 2048, 2056, 4095, 4104])
+@pytest.mark.parametrize("dtype,eps", [(torch.bfloat16, 0.0), (torch.bfloat16, 0.1), (torch.float32, 0.1)])
+def test_chunk_edges(V, dtype, eps):
+    """Vocabularies around the 8-column chunks and the 256-thread rounds, rows of one thread and ids at either end: forward
+    values to fp32 rounding, gradients and the flow map to one rounding of their type."""
+    x0, ids, s, t, l, *_ = _case(V, dtype=dtype, seed=V)
+    ids[0, 0], ids[-1, -1] = 0, V - 1
+    lp = l.clone().requires_grad_(True)
+    loss = vocab_ops.cross_entropy_padded(lp, ids, V, eps)
+    (g,) = torch.autograd.grad(loss, lp)
+    lf = l[..., :V].double().requires_grad_(True)
+    want = F.cross_entropy(lf.reshape(-1, V), ids.reshape(-1), label_smoothing=eps)
+    (gw,) = torch.autograd.grad(want, lf)
+    tol = 2 ** -7 if dtype == torch.bfloat16 else 1e-5
+    assert abs(loss.item() - want.item()) <= 1e-5 * abs(want.item()) + 1e-6
+    assert torch.allclose(g[..., :V].double(), gw, rtol=tol, atol=1e-7) and not g[..., V:].any()
+    xst, lse = vocab_ops.flow_map_input(l, x0, ids, s, t)
+    xs = _onehot_mix(x0, ids, s)
+    dt = ((t - s) / (1.0 - s + 1e-8)).view(-1, 1, 1)
+    assert torch.allclose(xst[..., :V].float(), (xs + dt * (lf.detach().softmax(-1) - xs)).float(), rtol=tol, atol=1e-5)
+    assert torch.allclose(lse.view(l.shape[:2]).double(), lf.detach().logsumexp(-1), rtol=1e-5, atol=1e-5) and not xst[..., V:].any()
+
+
 def _sd_loss_reference(l, tl, lt, x0, ids, s, t):
     """The reference's expressions: flow map, its t-derivative by the product rule, squared error (fp32)."""
     p = l.softmax(-1)

@@ -1,0 +1,62 @@
+"""When the library's autograd nodes may be left out: only where nothing could be recorded."""
+import inspect
+
+import torch
+import torch.autograd.forward_ad as fwAD
+
+from semicat_b200 import _nodes, dual_ops, functional, rotary
+
+
+def test_unrecorded_only_without_gradients_transforms_and_forward_mode():
+    assert not _nodes.unrecorded()
+    with torch.no_grad():
+        assert _nodes.unrecorded()
+        with fwAD.dual_level():
+            assert not _nodes.unrecorded()
+        seen = []
+        probe = lambda x: (seen.append(_nodes.unrecorded()), x * 2)[1]
+        torch.func.jvp(probe, (torch.ones(2),), (torch.ones(2),))
+        torch.func.vmap(probe)(torch.ones(2, 2))
+        torch.func.grad(lambda x: probe(x).sum())(torch.ones(2))
+        assert seen == [False] * 3
+        with torch.enable_grad():
+            assert not _nodes.unrecorded()
+    with torch.inference_mode():
+        assert _nodes.unrecorded()
+
+
+def test_node_signatures_are_those_of_forward():
+    nodes = [functional._AttentionDual, *(v for m in (dual_ops, rotary) for v in vars(m).values()
+                                          if inspect.isclass(v) and issubclass(v, torch.autograd.Function))]
+    assert len(nodes) > 8
+    for cls in nodes:
+        kept = cls.forward.__signature__
+        del cls.forward.__signature__
+        try:
+            assert kept == inspect.signature(cls.forward)
+        finally:
+            cls.forward.__signature__ = kept
+
+
+def test_apply_records_where_gradients_are_on():
+    class Twice(torch.autograd.Function):
+        @staticmethod
+        def forward(x):
+            return x * 2
+
+        @staticmethod
+        def setup_context(ctx, inputs, output):
+            pass
+
+        @staticmethod
+        def backward(ctx, g):
+            return g * 2
+
+    _nodes.node(Twice)
+    x = torch.ones(3, requires_grad=True)
+    y = _nodes.apply(Twice, x)
+    y.sum().backward()
+    assert torch.equal(x.grad, torch.full((3,), 2.0))
+    with torch.no_grad():
+        z = _nodes.apply(Twice, x)
+    assert torch.equal(z, y) and not z.requires_grad
