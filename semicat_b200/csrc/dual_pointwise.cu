@@ -35,6 +35,10 @@ __device__ __forceinline__ void load8<float>(const float *p, float (&f)[8]) {
 }
 // 8 elements as loaded
 template <typename T> struct alignas(16) Raw8 { uint32_t w[2 * sizeof(T)]; };
+__device__ __forceinline__ void unpack8(const Raw8<float> &u, float (&f)[8]) {
+#pragma unroll
+  for (int i = 0; i < 8; ++i) f[i] = __uint_as_float(u.w[i]);
+}
 __device__ __forceinline__ void unpack8(const Raw8<__nv_bfloat16> &u, float (&f)[8]) {
   const __nv_bfloat162 *h = reinterpret_cast<const __nv_bfloat162 *>(&u);
 #pragma unroll
@@ -299,56 +303,6 @@ __device__ __forceinline__ void flush_column_sums(float *smem, const float (&par
     }
 }
 
-// ---- backward of y.  u = G gamma (1 + scale);  dx = rstd P_n(u);  sums[0] += G n, sums[1] += G   (per sample)
-template <typename T, int NV>
-__global__ void __launch_bounds__(kWarpsPerCta * 32) ln_modulate_bwd_kernel(LnArgs a, int rows_per_cta) {
-  extern __shared__ float smem_raw[];
-  constexpr int C = NV * 256;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int ctas_per_sample = (a.S + rows_per_cta - 1) / rows_per_cta;
-  const int b = blockIdx.x / ctas_per_sample;
-  const int s0 = (blockIdx.x % ctas_per_sample) * rows_per_cta;
-  const T *sc = static_cast<const T *>(a.scale) + (int64_t)b * a.mod_stride;
-  float part[2][NV][8] = {};
-  for (int r = warp; r < rows_per_cta && s0 + r < a.S; r += kWarpsPerCta) {
-    const int64_t row = (int64_t)b * a.S + s0 + r;
-    const T *x = static_cast<const T *>(a.x) + row * C;
-    const T *g = static_cast<const T *>(a.g) + row * C;
-    const float mean = a.mean[row], rstd = a.rstd[row];
-    float n[NV][8], u[NV][8];
-    float su = 0.f, sun = 0.f;
-#pragma unroll
-    for (int v = 0; v < NV; ++v) {
-      const int c0 = chan(v, lane);
-      float xv[8], gv[8], gam[8], scv[8];
-      load8<T>(x + c0, xv);
-      load8<T>(g + c0, gv);
-      load8<float>(a.gamma + c0, gam);
-      load8<T>(sc + c0, scv);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        n[v][i] = (xv[i] - mean) * rstd;
-        u[v][i] = gv[i] * gam[i] * (1.f + scv[i]);
-        su += u[v][i];
-        sun += u[v][i] * n[v][i];
-        part[0][v][i] += gv[i] * n[v][i];
-        part[1][v][i] += gv[i];
-      }
-    }
-    const float mu_ = warp_sum(su) / C, mun = warp_sum(sun) / C;
-    T *dx = static_cast<T *>(a.dx) + row * C;
-#pragma unroll
-    for (int v = 0; v < NV; ++v) {
-      float out[8];
-#pragma unroll
-      for (int i = 0; i < 8; ++i) out[i] = rstd * (u[v][i] - mu_ - n[v][i] * mun);
-      store8<T>(dx + chan(v, lane), out);
-    }
-  }
-  float *const dst[2] = {a.sums + (int64_t)b * C, a.sums + ((int64_t)a.B + b) * C};
-  flush_column_sums<2, NV>(smem_raw, part, lane, dst);
-}
-
 // ---- backward of ty.  u = G gamma (1 + scale), w = G gamma tscale, nd = rstd P_n(tx):
 //   dtx = rstd P_n(u)
 //   exact:        dx = rstd P_n(w + gn) - rstd n mean(u nd),   gn = -rstd (u mean(n tx) + tx mean(u n))
@@ -446,8 +400,9 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) ln_modulate_bwd_tangent_ker
   flush_column_sums<3, NV>(smem_raw, part, lane, dst);
 }
 
-// Both backward kernels in one pass, for the cotangents g on y and gt on ty: x is read once and dx written once, 6 row-sized
-// transfers instead of 9, and dx is rounded once.  With u1 = g gamma (1 + scale) and w, u of the kernel above, dx follows
+// ---- backward of y (kTan = false).  w = G gamma (1 + scale);  dx = rstd P_n(w);  sums[0] += G n, sums[1] += G   (per sample)
+// kTan = true: with the kernel above in the same pass, for the cotangents g on y and gt on ty: x is read once and dx
+// written once, 6 row-sized transfers instead of 9, and dx is rounded once.  With u1 = g gamma (1 + scale) and w, u of the kernel above, dx follows
 // from u1 + w in the place of w.  gamma (1 + scale) multiplies sum(g n) and sum(gt nd) alike, so those share one column
 // sum: sums[0] += g n + gt nd, sums[1] += g, sums[2] += gt n, sums[3] += gt.
 // Bound by memory.  A thread owns 8 channels of every row of its CTA (C / 8 threads), not a lane 8 NV of one row in four: the
@@ -455,8 +410,8 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) ln_modulate_bwd_tangent_ker
 // row took all 255 at C = 768 and spilled; fp32 rows would not fit here either and keep the kernels above), the per-sample factors are loaded once, and the column sums need no pass through
 // shared memory.  The price is a block-wide reduction of the row's sums: one barrier per row (its buffer alternates).
 // 128 x 128 rows of 768: 99 us in two kernels, 60 us so, 49 us with the column sums added 16 bytes at a time.
-template <typename T, int NV>
-__global__ void __launch_bounds__(NV * 32, 16 / NV) ln_modulate_dual_bwd_kernel(LnArgs a, int rows_per_cta) {
+template <typename T, int NV, bool kTan>
+__global__ void __launch_bounds__(NV * 32, (sizeof(T) == 2 ? 16 : 12) / NV) ln_modulate_bwd_kernel(LnArgs a, int rows_per_cta) {
   constexpr int C = NV * 256;
   __shared__ float scratch[2][8][NV];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, c0 = threadIdx.x * 8;
@@ -477,15 +432,15 @@ __global__ void __launch_bounds__(NV * 32, 16 / NV) ln_modulate_dual_bwd_kernel(
     }
   }
   struct Row {
-    Raw8<T> x, t, g, gt;
+    Raw8<T> x, g, t, gt;  // (t, gt: kTan)
     float mean, rstd;
   };
   auto load_row = [&](int s, Row &r) {
     const int64_t row = (int64_t)b * a.S + s, e = row * C + c0;
     r.x = *reinterpret_cast<const Raw8<T> *>(static_cast<const T *>(a.x) + e);
-    r.t = a.tx ? *reinterpret_cast<const Raw8<T> *>(static_cast<const T *>(a.tx) + e) : Raw8<T>{};
+    if (kTan) r.t = a.tx ? *reinterpret_cast<const Raw8<T> *>(static_cast<const T *>(a.tx) + e) : Raw8<T>{};
     r.g = *reinterpret_cast<const Raw8<T> *>(static_cast<const T *>(a.g) + e);
-    r.gt = *reinterpret_cast<const Raw8<T> *>(static_cast<const T *>(a.gt) + e);
+    if (kTan) r.gt = *reinterpret_cast<const Raw8<T> *>(static_cast<const T *>(a.gt) + e);
     r.mean = a.mean[row];
     r.rstd = a.rstd[row];
   };
@@ -494,25 +449,29 @@ __global__ void __launch_bounds__(NV * 32, 16 / NV) ln_modulate_dual_bwd_kernel(
   load_row(s0, cur);
   for (int s = s0; s < s1; ++s) {
     const float mean = cur.mean, rstd = cur.rstd;
-    float n[8], t[8], g[8], gt[8];
-    unpack8(cur.x, n), unpack8(cur.t, t), unpack8(cur.g, g), unpack8(cur.gt, gt);
+    float n[8], g[8], t[8] = {}, gt[8] = {};
+    unpack8(cur.x, n), unpack8(cur.g, g);
+    if (kTan) unpack8(cur.t, t), unpack8(cur.gt, gt);
     if (s + 1 < s1) load_row(s + 1, cur);  // in flight across the barrier below
-    float v[7] = {};  // t, n t, u, u n, w, w n, u t
+    float v[7] = {};  // w, w n, and with kTan t, n t, u, u n, u t
+    const int nsum = !kTan ? 2 : exact ? 7 : 6;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       n[i] = (n[i] - mean) * rstd;
-      const float u = gt[i] * gs[i], w = g[i] * gs[i] + gt[i] * gw[i];
-      v[0] += t[i];
-      v[1] += n[i] * t[i];
-      v[2] += u;
-      v[3] += u * n[i];
-      v[4] += w;
-      v[5] += w * n[i];
-      v[6] += u * t[i];
+      const float u = gt[i] * gs[i], w = g[i] * gs[i] + (kTan ? gt[i] * gw[i] : 0.f);
+      v[0] += w;
+      v[1] += w * n[i];
+      if (kTan) {
+        v[2] += t[i];
+        v[3] += n[i] * t[i];
+        v[4] += u;
+        v[5] += u * n[i];
+        v[6] += u * t[i];
+      }
     }
 #pragma unroll
     for (int q = 0; q < 7; ++q) {
-      if (q == 6 && !exact) break;
+      if (q >= nsum) break;
       v[q] = warp_sum(v[q]);
       if (NV > 1 && lane == 0) scratch[s & 1][q][warp] = v[q];
     }
@@ -520,20 +479,26 @@ __global__ void __launch_bounds__(NV * 32, 16 / NV) ln_modulate_dual_bwd_kernel(
       __syncthreads();
 #pragma unroll
       for (int q = 0; q < 7; ++q) {
-        if (q == 6 && !exact) break;
+        if (q >= nsum) break;
         v[q] = scratch[s & 1][q][0];
 #pragma unroll
         for (int k = 1; k < NV; ++k) v[q] += scratch[s & 1][q][k];
       }
     }
     constexpr float inv = 1.f / C;
-    const float m_t = v[0] * inv, m_nt = v[1] * inv, m_u = v[2] * inv, m_un = v[3] * inv, m_w = v[4] * inv, m_wn = v[5] * inv;
+    const float m_w = v[0] * inv, m_wn = v[1] * inv, m_t = v[2] * inv, m_nt = v[3] * inv, m_u = v[4] * inv, m_un = v[5] * inv;
     const float m_und = exact ? rstd * (v[6] * inv - m_u * m_t - m_un * m_nt) : 0.f;
     const float m_gn = -rstd * (m_u * m_nt + m_t * m_un), m_gnn = -2.f * rstd * m_un * m_nt;
     float o1[8], o2[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-      const float u = gt[i] * gs[i], w = g[i] * gs[i] + gt[i] * gw[i];
+      const float u = gt[i] * gs[i], w = g[i] * gs[i] + (kTan ? gt[i] * gw[i] : 0.f);
+      if (!kTan) {
+        o1[i] = rstd * (w - m_w - n[i] * m_wn);
+        part[0][i] += g[i] * n[i];
+        part[1][i] += g[i];
+        continue;
+      }
       const float nd = rstd * (t[i] - m_t - n[i] * m_nt);
       o2[i] = rstd * (u - m_u - n[i] * m_un);
       if (exact) {
@@ -549,10 +514,10 @@ __global__ void __launch_bounds__(NV * 32, 16 / NV) ln_modulate_dual_bwd_kernel(
     }
     const int64_t e = ((int64_t)b * a.S + s) * C + c0;
     store8<T>(static_cast<T *>(a.dx) + e, o1);
-    store8<T>(static_cast<T *>(a.dtx) + e, o2);
+    if (kTan) store8<T>(static_cast<T *>(a.dtx) + e, o2);
   }
 #pragma unroll
-  for (int q = 0; q < 4; ++q) add8(a.sums + ((int64_t)q * a.B + b) * C + c0, part[q]);
+  for (int q = 0; q < (kTan ? 4 : 2); ++q) add8(a.sums + ((int64_t)q * a.B + b) * C + c0, part[q]);
 }
 
 // ---- dropout keep mask computed in the kernel instead of read from memory.  Philox-4x32-10 (Salmon et al., "Parallel
@@ -600,14 +565,20 @@ struct GateArgs {
   DropArgs drop;             // used when mask is null and drop.seed is not
 };
 
+// Index type of the forward kernels, which take a linear chunk index apart into (sample, row, channels): 32 bits wherever they
+// hold the index and a grid stride, since two 64-bit divisions per chunk of 8 elements cost more than the chunk's arithmetic
+// (128 x 128 rows of 768, pair: 36.5 -> 33.7 us).
+inline bool index32(int64_t chunks) { return chunks < (int64_t(1) << 31); }
+
 // z = x + m g y without a tangent (the passes that run outside forward-mode AD)
-template <typename T>
+template <typename T, typename I>
 __global__ void __launch_bounds__(256) gated_residual_fwd_kernel(GateArgs a) {
-  const int64_t total = (int64_t)a.B * a.S * a.C / 8;
-  for (int64_t i8 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i8 < total; i8 += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t e = i8 * 8;
-    const int c0 = (int)(e % a.C);
-    const int b = (int)(e / ((int64_t)a.S * a.C));
+  const I total = (I)((int64_t)a.B * a.S * a.C / 8), per_row = (I)(a.C / 8);
+  for (I i8 = (I)blockIdx.x * blockDim.x + threadIdx.x; i8 < total; i8 += (I)gridDim.x * blockDim.x) {
+    const int64_t e = (int64_t)i8 * 8;
+    const I row = i8 / per_row;
+    const int c0 = (int)(i8 - row * per_row) * 8;
+    const int b = (int)(row / (I)a.S);
     float xv[8], yv[8], gv[8], mv[8], out[8];
     load8<T>(static_cast<const T *>(a.x) + e, xv);
     load8<T>(static_cast<const T *>(a.y) + e, yv);
@@ -697,13 +668,14 @@ struct GateDualArgs {
   DropArgs drop;
 };
 
-template <typename T>
+template <typename T, typename I>
 __global__ void __launch_bounds__(256) gated_dual_fwd_kernel(GateDualArgs a) {
-  const int64_t total = (int64_t)a.B * a.S * a.C / 8;
-  for (int64_t i8 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i8 < total; i8 += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t e = i8 * 8;
-    const int c0 = (int)(e % a.C);
-    const int b = (int)(e / ((int64_t)a.S * a.C));
+  const I total = (I)((int64_t)a.B * a.S * a.C / 8), per_row = (I)(a.C / 8);
+  for (I i8 = (I)blockIdx.x * blockDim.x + threadIdx.x; i8 < total; i8 += (I)gridDim.x * blockDim.x) {
+    const int64_t e = (int64_t)i8 * 8;
+    const I row = i8 / per_row;
+    const int c0 = (int)(i8 - row * per_row) * 8;
+    const int b = (int)(row / (I)a.S);
     float xv[8], txv[8], yv[8], tyv[8], gv[8], tgv[8], mv[8], o[8], to[8];
     load8<T>(static_cast<const T *>(a.x) + e, xv);
     load8<T>(static_cast<const T *>(a.y) + e, yv);
@@ -728,7 +700,8 @@ __global__ void __launch_bounds__(256) gated_dual_fwd_kernel(GateDualArgs a) {
 }
 
 // One thread owns 8 adjacent channels of `rows_per_cta` rows of one sample: the column sums stay in registers and leave
-// with one atomic per channel and CTA; adjacent threads read adjacent 16-byte pieces of a row.
+// with one atomic per channel and CTA; adjacent threads read adjacent 16-byte pieces of a row.  (The compiler cannot move the
+// next row's loads above this row's stores by itself: 51 -> 36 us at 128 x 128 rows of 768.)
 template <typename T>
 __global__ void __launch_bounds__(128) gated_dual_bwd_kernel(GateDualArgs a, int rows_per_cta) {
   const int c0 = threadIdx.x * 8;
@@ -740,16 +713,25 @@ __global__ void __launch_bounds__(128) gated_dual_bwd_kernel(GateDualArgs a, int
   load8<T>(static_cast<const T *>(a.gate) + (int64_t)b * a.gate_stride + c0, gt);
   if (a.tgate) load8<T>(static_cast<const T *>(a.tgate) + (int64_t)b * a.tgate_stride + c0, tgt);
   const int s1 = min(a.S, s0 + rows_per_cta);
-#pragma unroll 2
+  struct Row {
+    Raw8<T> y, ty, g1, g2, m;
+  };
+  auto load_row = [&](int s, Row &r) {
+    const int64_t e = ((int64_t)b * a.S + s) * a.C + c0;
+    r.y = *reinterpret_cast<const Raw8<T> *>(static_cast<const T *>(a.y) + e);
+    if (a.gz) r.g1 = *reinterpret_cast<const Raw8<T> *>(static_cast<const T *>(a.gz) + e);
+    if (a.gtz) r.g2 = *reinterpret_cast<const Raw8<T> *>(static_cast<const T *>(a.gtz) + e);
+    if (a.ty && a.gtz) r.ty = *reinterpret_cast<const Raw8<T> *>(static_cast<const T *>(a.ty) + e);
+    if (a.mask) r.m = *reinterpret_cast<const Raw8<T> *>(static_cast<const T *>(a.mask) + e);
+  };
+  Row cur{};
+  load_row(s0, cur);
   for (int s = s0; s < s1; ++s) {
     const int64_t e = ((int64_t)b * a.S + s) * a.C + c0;
     float yv[8], tyv[8], mv[8], g1[8], g2[8], o1[8], o2[8];
-    load8<T>(static_cast<const T *>(a.y) + e, yv);
-    if (a.gz) load8<T>(static_cast<const T *>(a.gz) + e, g1);
-    if (a.gtz) load8<T>(static_cast<const T *>(a.gtz) + e, g2);
-    if (a.ty && a.gtz) load8<T>(static_cast<const T *>(a.ty) + e, tyv);
-    if (a.mask) load8<T>(static_cast<const T *>(a.mask) + e, mv);
-    else if (a.drop.seed) dropout8(a.drop, e / 8, mv);
+    unpack8(cur.y, yv), unpack8(cur.ty, tyv), unpack8(cur.g1, g1), unpack8(cur.g2, g2), unpack8(cur.m, mv);
+    if (s + 1 < s1) load_row(s + 1, cur);  // in flight across this row's arithmetic and stores
+    if (!a.mask && a.drop.seed) dropout8(a.drop, e / 8, mv);
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       const float m = (a.mask || a.drop.seed) ? mv[i] : 1.f;
@@ -868,7 +850,7 @@ cudaError_t ln_modulate(int which, const void *x, const void *tx, const float *g
       const int rows_cta = rows_per_cta(B, S, 16);
       const unsigned grid = (unsigned)(B * ((S + rows_cta - 1) / rows_cta));
       if (which == 2) {
-        ln_modulate_bwd_kernel<T, NV><<<grid, kWarpsPerCta * 32, kWarpsPerCta * 2 * NV * 256 * 4, stream>>>(a, rows_cta);
+        ln_modulate_bwd_kernel<T, NV, false><<<grid, NV * 32, 0, stream>>>(a, rows_cta);
       } else {
         auto k = ln_modulate_bwd_tangent_kernel<T, NV>;
         constexpr int smem = kWarpsPerCta * 3 * NV * 256 * 4;
@@ -898,7 +880,7 @@ cudaError_t ln_modulate_dual(int which, const void *x, const void *tx, const flo
       ln_modulate_dual_fwd_kernel<T, NV><<<(unsigned)((rows + kWarpsPerCta - 1) / kWarpsPerCta), kWarpsPerCta * 32, 0, stream>>>(a);
     } else {
       const int rows_cta = rows_per_cta(B, S, 16);
-      ln_modulate_dual_bwd_kernel<T, NV><<<(unsigned)(B * ((S + rows_cta - 1) / rows_cta)), NV * 32, 0, stream>>>(a, rows_cta);
+      ln_modulate_bwd_kernel<T, NV, true><<<(unsigned)(B * ((S + rows_cta - 1) / rows_cta)), NV * 32, 0, stream>>>(a, rows_cta);
     }
     return cudaGetLastError();
   });
@@ -913,10 +895,15 @@ cudaError_t gated_residual(const void *x, const void *y, const void *gate, const
   GateArgs a{x, y, gate, mask, gate_stride, z, B, S, C, {drop_seed, drop_call, drop_p}};
   LaunchScope scope(kIdDual, stream);
   const unsigned grid = (unsigned)std::min<int64_t>((total + 255) / 256, 148 * 8);
-  if (dtype == JVPATTN_BF16) gated_residual_fwd_kernel<__nv_bfloat16><<<grid, 256, 0, stream>>>(a);
-  else if (dtype == JVPATTN_FP32) gated_residual_fwd_kernel<float><<<grid, 256, 0, stream>>>(a);
-  else return cudaErrorInvalidValue;
-  return cudaGetLastError();
+  auto launch = [&](auto tag) -> cudaError_t {
+    using T = decltype(tag);
+    if (index32(total)) gated_residual_fwd_kernel<T, uint32_t><<<grid, 256, 0, stream>>>(a);
+    else gated_residual_fwd_kernel<T, int64_t><<<grid, 256, 0, stream>>>(a);
+    return cudaGetLastError();
+  };
+  if (dtype == JVPATTN_BF16) return launch(__nv_bfloat16{});
+  if (dtype == JVPATTN_FP32) return launch(float{});
+  return cudaErrorInvalidValue;
 }
 
 cudaError_t ln_finalize(const float *p, const float *t, const float *gamma, const float *beta, const void *scale,
@@ -946,10 +933,12 @@ cudaError_t gated_residual_dual(int which, const void *x, const void *tx, const 
     using T = decltype(tag);
     if (which == 0) {
       const int64_t n8 = (int64_t)B * S * C / 8;
-      gated_dual_fwd_kernel<T><<<(unsigned)std::min<int64_t>((n8 + 255) / 256, 148 * 16), 256, 0, stream>>>(a);
+      const unsigned grid = (unsigned)std::min<int64_t>((n8 + 255) / 256, 148 * 16);
+      if (index32(n8)) gated_dual_fwd_kernel<T, uint32_t><<<grid, 256, 0, stream>>>(a);
+      else gated_dual_fwd_kernel<T, int64_t><<<grid, 256, 0, stream>>>(a);
     } else {
-      const int rows_cta = rows_per_cta(B, S, 8);
-      gated_dual_bwd_kernel<T><<<(unsigned)(B * ((S + rows_cta - 1) / rows_cta)), 128, 0, stream>>>(a, rows_cta);
+      const int rows_cta = rows_per_cta(B, S, 16);
+      gated_dual_bwd_kernel<T><<<(unsigned)(B * ((S + rows_cta - 1) / rows_cta)), (C / 8 + 31) / 32 * 32, 0, stream>>>(a, rows_cta);
     }
     return cudaGetLastError();
   };

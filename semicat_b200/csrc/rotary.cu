@@ -146,19 +146,22 @@ struct QkvArgs {
   int B, S, H, D, transpose;
 };
 
-template <typename TI, typename TO>
+// I: type of the linear thread index, which is taken apart into (tensor, sample, position, head, channels): 32 bits wherever it
+// fits.  The kernel is bound by memory, but five 64-bit divisions per 16 elements were most of its
+// instructions (128 x 128 positions of 3 x 768 channels in bf16: 35.6 -> 30.3 us).
+template <typename TI, typename TO, typename I>
 __global__ void __launch_bounds__(256) rotary_qkv_kernel(QkvArgs a) {
-  const int half = a.D / 2, per_row = half / 8;
-  const int64_t rows = (int64_t)a.B * a.S * a.H;
-  const int64_t gid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t rr = gid / per_row;
+  const int half = a.D / 2;
+  const I per_row = (I)(half / 8), rows = (I)((int64_t)a.B * a.S * a.H);
+  const I gid = (I)blockIdx.x * 256 + threadIdx.x;
+  const I rr = gid / per_row;
   if (rr >= 3 * rows) return;
   const int t = (int)(rr / rows);
-  const int64_t r = rr % rows;
-  const int c0 = (int)(gid % per_row) * 8;
-  const int h = (int)(r % a.H);
-  const int s = (int)((r / a.H) % a.S);
-  const int b = (int)(r / ((int64_t)a.H * a.S));
+  const I r = rr - t * rows, bs = r / (I)a.H;
+  const int c0 = (int)(gid - rr * per_row) * 8;
+  const int h = (int)(r - bs * (I)a.H);
+  const int b = (int)(bs / (I)a.S);
+  const int s = (int)(bs - (I)b * (I)a.S);
   const TI *xr = static_cast<const TI *>(a.in[t]) + b * a.isb[t] + s * a.iss[t] + h * a.ish[t];
   TO *yr = static_cast<TO *>(a.out[t]) + b * a.osb[t] + s * a.oss[t] + h * a.osh[t];
   float x1[8], x2[8], y1[8], y2[8];
@@ -191,7 +194,9 @@ cudaError_t launch_qkv(const QkvArgs &a, cudaStream_t stream) {
   const int64_t threads = (int64_t)3 * a.B * a.S * a.H * (a.D / 16);
   if (threads == 0) return cudaSuccess;
   LaunchScope scope(kIdRotary, stream);
-  rotary_qkv_kernel<TI, TO><<<(unsigned)((threads + 255) / 256), 256, 0, stream>>>(a);
+  const unsigned grid = (unsigned)((threads + 255) / 256);
+  if (threads < (int64_t(1) << 31)) rotary_qkv_kernel<TI, TO, uint32_t><<<grid, 256, 0, stream>>>(a);
+  else rotary_qkv_kernel<TI, TO, int64_t><<<grid, 256, 0, stream>>>(a);
   return cudaGetLastError();
 }
 
