@@ -113,11 +113,80 @@ struct LnArgs {
                                  // bit 1 = add to what dx holds instead of overwriting it
 };
 
-// ---- forward.  kTangent = false: y = (n gamma + beta)(1 + scale) + shift, saves mean / rstd.
-//               kTangent = true:  ty = nd gamma (1 + scale) + (n gamma + beta) tscale + tshift,  nd = rstd P_n(tx),
-//               where P_n(z) = z - mean(z) - n mean(n z)
-template <typename T, int NV, bool kTangent>
-__global__ void __launch_bounds__(kWarpsPerCta * 32) ln_modulate_fwd_kernel(LnArgs a) {
+// ---- forward of y = (n gamma + beta)(1 + scale) + shift; saves mean / rstd.  A warp walks rows of one sample with the two
+// per-channel factors of n in registers (gamma (1 + scale), beta (1 + scale) + shift) and the next row in flight: read per row, the
+// four parameter vectors were six times the row itself on its way through L1.  Bound by memory (8 x 128 rows of 768, a launch
+// among others: 3.8 -> 3.5 us).
+template <typename T, int NV>
+__global__ void __launch_bounds__(kWarpsPerCta * 32) ln_modulate_fwd_kernel(LnArgs a, int rows_per_cta) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  constexpr int C = NV * 256;
+  const int ctas_per_sample = (a.S + rows_per_cta - 1) / rows_per_cta;
+  const int b = blockIdx.x / ctas_per_sample;
+  const int s0 = (blockIdx.x % ctas_per_sample) * rows_per_cta + warp;
+  const int s1 = min(a.S, (int)(blockIdx.x % ctas_per_sample + 1) * rows_per_cta);
+  if (s0 >= s1) return;
+  Raw8<T> cur[NV];
+  auto load_row = [&](int s) {
+    const T *x = static_cast<const T *>(a.x) + ((int64_t)b * a.S + s) * C;
+#pragma unroll
+    for (int v = 0; v < NV; ++v) cur[v] = *reinterpret_cast<const Raw8<T> *>(x + chan(v, lane));
+  };
+  load_row(s0);
+  float ga[NV][8], be[NV][8];
+#pragma unroll
+  for (int v = 0; v < NV; ++v) {
+    const int c0 = chan(v, lane);
+    float scv[8], shv[8];
+    load8<float>(a.gamma + c0, ga[v]);
+    if (a.beta) load8<float>(a.beta + c0, be[v]);
+    load8<T>(static_cast<const T *>(a.scale) + (int64_t)b * a.mod_stride + c0, scv);
+    load8<T>(static_cast<const T *>(a.shift) + (int64_t)b * a.mod_stride + c0, shv);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      ga[v][i] *= 1.f + scv[i];
+      be[v][i] = (a.beta ? be[v][i] * (1.f + scv[i]) : 0.f) + shv[i];
+    }
+  }
+  for (int s = s0; s < s1; s += kWarpsPerCta) {
+    const int64_t row = (int64_t)b * a.S + s;
+    float xv[NV][8], t = 0.f;
+#pragma unroll
+    for (int v = 0; v < NV; ++v) {
+      unpack8(cur[v], xv[v]);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) t += xv[v][i];
+    }
+    if (s + kWarpsPerCta < s1) load_row(s + kWarpsPerCta);
+    const float mean = warp_sum(t) / C;
+    float q = 0.f;
+#pragma unroll
+    for (int v = 0; v < NV; ++v)
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        xv[v][i] -= mean;
+        q += xv[v][i] * xv[v][i];
+      }
+    const float rstd = rsqrtf(warp_sum(q) / C + a.eps);
+    if (lane == 0) {
+      a.mean[row] = mean;
+      a.rstd[row] = rstd;
+    }
+    T *y = static_cast<T *>(a.y) + row * C;
+#pragma unroll
+    for (int v = 0; v < NV; ++v) {
+      float out[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) out[i] = xv[v][i] * rstd * ga[v][i] + be[v][i];
+      store8<T>(y + chan(v, lane), out);
+    }
+  }
+}
+
+// ---- forward of the tangent alone:  ty = nd gamma (1 + scale) + (n gamma + beta) tscale + tshift,  nd = rstd P_n(tx),
+//      where P_n(z) = z - mean(z) - n mean(n z)
+template <typename T, int NV>
+__global__ void __launch_bounds__(kWarpsPerCta * 32) ln_modulate_fwd_tangent_kernel(LnArgs a) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t row = (int64_t)blockIdx.x * kWarpsPerCta + warp;
   if (row >= (int64_t)a.B * a.S) return;
@@ -125,89 +194,45 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) ln_modulate_fwd_kernel(LnAr
   constexpr int C = NV * 256;
   const T *x = static_cast<const T *>(a.x) + row * C;
   float xv[NV][8];
-  float s = 0.f;
 #pragma unroll
-  for (int v = 0; v < NV; ++v) {
-    load8<T>(x + chan(v, lane), xv[v]);
-#pragma unroll
-    for (int i = 0; i < 8; ++i) s += xv[v][i];
-  }
-  float mean, rstd;
-  if (!kTangent) {
-    mean = warp_sum(s) / C;
-    float q = 0.f;
-#pragma unroll
-    for (int v = 0; v < NV; ++v) {
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const float d = xv[v][i] - mean;
-        q += d * d;
-      }
-    }
-    rstd = rsqrtf(warp_sum(q) / C + a.eps);
-    if (lane == 0) {
-      a.mean[row] = mean;
-      a.rstd[row] = rstd;
-    }
-  } else {
-    mean = a.mean[row];
-    rstd = a.rstd[row];
-  }
+  for (int v = 0; v < NV; ++v) load8<T>(x + chan(v, lane), xv[v]);
+  const float mean = a.mean[row], rstd = a.rstd[row];
   const T *sc = static_cast<const T *>(a.scale) + (int64_t)b * a.mod_stride;
   T *y = static_cast<T *>(a.y) + row * C;
-  if (!kTangent) {
-    const T *sh = static_cast<const T *>(a.shift) + (int64_t)b * a.mod_stride;
+  const T *tx = static_cast<const T *>(a.tx) + row * C;
+  float tv[NV][8];
+  float s1 = 0.f, s2 = 0.f;
 #pragma unroll
-    for (int v = 0; v < NV; ++v) {
-      const int c0 = chan(v, lane);
-      float g[8], be[8], scv[8], shv[8], out[8];
-      load8<float>(a.gamma + c0, g);
-      if (a.beta) load8<float>(a.beta + c0, be);
-      load8<T>(sc + c0, scv);
-      load8<T>(sh + c0, shv);
+  for (int v = 0; v < NV; ++v) {
+    load8<T>(tx + chan(v, lane), tv[v]);
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const float ln = (xv[v][i] - mean) * rstd * g[i] + (a.beta ? be[i] : 0.f);
-        out[i] = ln * (1.f + scv[i]) + shv[i];
-      }
-      store8<T>(y + c0, out);
+    for (int i = 0; i < 8; ++i) {
+      s1 += tv[v][i];
+      s2 += (xv[v][i] - mean) * rstd * tv[v][i];
     }
-  } else {
-    const T *tx = static_cast<const T *>(a.tx) + row * C;
-    float tv[NV][8];
-    float s1 = 0.f, s2 = 0.f;
+  }
+  const float m1 = warp_sum(s1) / C, m2 = warp_sum(s2) / C;
+  const T *tsc = a.tscale ? static_cast<const T *>(a.tscale) + (int64_t)b * a.tmod_stride : nullptr;
+  const T *tsh = a.tshift ? static_cast<const T *>(a.tshift) + (int64_t)b * a.tmod_stride : nullptr;
 #pragma unroll
-    for (int v = 0; v < NV; ++v) {
-      load8<T>(tx + chan(v, lane), tv[v]);
+  for (int v = 0; v < NV; ++v) {
+    const int c0 = chan(v, lane);
+    float g[8], be[8], scv[8], tscv[8], tshv[8], out[8];
+    load8<float>(a.gamma + c0, g);
+    if (a.beta) load8<float>(a.beta + c0, be);
+    load8<T>(sc + c0, scv);
+    if (tsc) load8<T>(tsc + c0, tscv);
+    if (tsh) load8<T>(tsh + c0, tshv);
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        s1 += tv[v][i];
-        s2 += (xv[v][i] - mean) * rstd * tv[v][i];
-      }
+    for (int i = 0; i < 8; ++i) {
+      const float n = (xv[v][i] - mean) * rstd;
+      const float nd = rstd * (tv[v][i] - m1 - n * m2);
+      float o = nd * g[i] * (1.f + scv[i]);
+      if (tsc) o += (n * g[i] + (a.beta ? be[i] : 0.f)) * tscv[i];
+      if (tsh) o += tshv[i];
+      out[i] = o;
     }
-    const float m1 = warp_sum(s1) / C, m2 = warp_sum(s2) / C;
-    const T *tsc = a.tscale ? static_cast<const T *>(a.tscale) + (int64_t)b * a.tmod_stride : nullptr;
-    const T *tsh = a.tshift ? static_cast<const T *>(a.tshift) + (int64_t)b * a.tmod_stride : nullptr;
-#pragma unroll
-    for (int v = 0; v < NV; ++v) {
-      const int c0 = chan(v, lane);
-      float g[8], be[8], scv[8], tscv[8], tshv[8], out[8];
-      load8<float>(a.gamma + c0, g);
-      if (a.beta) load8<float>(a.beta + c0, be);
-      load8<T>(sc + c0, scv);
-      if (tsc) load8<T>(tsc + c0, tscv);
-      if (tsh) load8<T>(tsh + c0, tshv);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const float n = (xv[v][i] - mean) * rstd;
-        const float nd = rstd * (tv[v][i] - m1 - n * m2);
-        float o = nd * g[i] * (1.f + scv[i]);
-        if (tsc) o += (n * g[i] + (a.beta ? be[i] : 0.f)) * tscv[i];
-        if (tsh) o += tshv[i];
-        out[i] = o;
-      }
-      store8<T>(y + c0, out);
-    }
+    store8<T>(y + c0, out);
   }
 }
 
@@ -595,10 +620,10 @@ __global__ void __launch_bounds__(256) gated_residual_fwd_kernel(GateArgs a) {
 // Rows of one sample that a CTA of the backward kernels walks before it adds its column sums to global memory.  Every CTA
 // costs one atomic per column and sum, and at a few hundred samples those atomics (millions per launch, a dozen
 // contenders per address) took longer than the rows themselves; so the count grows with the problem as long as
-// eight CTAs per SM remain.
-inline int rows_per_cta(int B, int S, int base) {
+// eight CTAs per SM remain (four where there are no sums and the point is what a CTA loads once).
+inline int rows_per_cta(int B, int S, int base, int ctas_per_sm = 8) {
   int rows = base;
-  while (rows < 64 && (int64_t)B * ((S + 2 * rows - 1) / (2 * rows)) >= 148 * 8) rows *= 2;
+  while (rows < 64 && (int64_t)B * ((S + 2 * rows - 1) / (2 * rows)) >= 148 * ctas_per_sm) rows *= 2;
   return rows;
 }
 
@@ -844,8 +869,12 @@ cudaError_t ln_modulate(int which, const void *x, const void *tx, const float *g
     constexpr int NV = decltype(nv)::value;
     if (which == 0 || which == 1) {
       const unsigned grid = (unsigned)((rows + kWarpsPerCta - 1) / kWarpsPerCta);
-      if (which == 0) ln_modulate_fwd_kernel<T, NV, false><<<grid, kWarpsPerCta * 32, 0, stream>>>(a);
-      else ln_modulate_fwd_kernel<T, NV, true><<<grid, kWarpsPerCta * 32, 0, stream>>>(a);
+      if (which == 0) {
+        const int rows_cta = rows_per_cta(B, S, kWarpsPerCta, 4);  // (four blocks fit an SM; small batches: a row per warp)
+        ln_modulate_fwd_kernel<T, NV><<<(unsigned)(B * ((S + rows_cta - 1) / rows_cta)), kWarpsPerCta * 32, 0, stream>>>(a, rows_cta);
+      } else {
+        ln_modulate_fwd_tangent_kernel<T, NV><<<grid, kWarpsPerCta * 32, 0, stream>>>(a);
+      }
     } else {
       const int rows_cta = rows_per_cta(B, S, 16);
       const unsigned grid = (unsigned)(B * ((S + rows_cta - 1) / rows_cta));
