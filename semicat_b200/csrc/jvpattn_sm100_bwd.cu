@@ -58,20 +58,23 @@ __host__ __device__ constexpr int bwd_parts(int tile) { return tile >= 64 ? JVPA
 // whose A operand comes from shared memory re-reads all of A for every N: at 128 B / clk a 16-channel step of N = 64 takes
 // 48 cycles for 32 cycles of arithmetic and N = 32 takes 40 for 16, while N = 128 ([S | Sd], [A | C] of a 64-row tile)
 // reads as long as it multiplies.  Forward and backward of 128 heads at length 2048: 5.42 ms with 32-row tiles, 4.30 ms so.
-__host__ __device__ constexpr bool bwd_pair_ring(int D) { return D == 128; }
+// The query owner of head_dim 64 (with tangents) streams pairs for another reason: two whole stages fit, but (Y0, Y1) of a tile are
+// released by its last products and were wanted again right after them, so every second tile waited 1400 cycles for its load.
+// It has three stages of (Y0, Y1) and two of (Y2, Y3): 564 -> 510 us for 128 heads at length 2048.
+__host__ __device__ constexpr bool bwd_pair_ring(int D, bool kv, bool has_t) { return D == 128 || (!kv && has_t); }
 // Without tangents two of the four tensors on either side, one of the two score products per region and the tangent
 // accumulators are absent.  At head_dim 64 two CTAs then share an SM, one's products beside the other's score algebra
 // (192 x 12 heads of length 128: key owner 55 -> 41 us, query owner 42 -> 35 us).
 __host__ __device__ constexpr bool bwd_compact(int D, bool has_t) { return D == 64 && !has_t; }
-__host__ __device__ constexpr bool bwd_two_issuers(int D, bool kv, bool has_t) { return !kv && !bwd_pair_ring(D) && !bwd_compact(D, has_t); }
+__host__ __device__ constexpr bool bwd_two_issuers(int D, bool kv, bool has_t) { return D == 64 && !kv && !bwd_compact(D, has_t); }
 
 template <int D, int TILE, bool kKV, bool kDoK, bool kHasT>
 struct BwdSmem {
   static constexpr int kBoxes = D / 64;
   static constexpr int kXBuf = D == 64 ? 2 : 1;  // owned-row tiles are double buffered where shared memory allows
-  static constexpr int kStages = 2;
-  static constexpr bool kRing = bwd_pair_ring(D);
-  static constexpr int kStages2 = kRing && kDoK ? 1 : 2;  // stages of (Y2, Y3)
+  static constexpr bool kRing = bwd_pair_ring(D, kKV, kHasT);
+  static constexpr int kStages = kRing && D == 64 ? 3 : 2;           // stages (kRing: of (Y0, Y1))
+  static constexpr int kStages2 = kRing && D == 128 && kDoK ? 1 : 2;  // stages of (Y2, Y3)
   static constexpr bool kCompact = bwd_compact(D, kHasT);  // tensor 0 and the one of 2 and 3 that is there, in slots 0 and 1
   static constexpr int kXTensors = kDoK && !kCompact ? 4 : 2;  // the dV / dVd pass reads X0 and X1 only
   static constexpr int kPer = kRing || kCompact ? 2 : 4;       // streamed tensors of a stage
@@ -180,7 +183,7 @@ __global__ void __launch_bounds__(bwd_threads(bwd_parts(TILE), bwd_two_issuers(D
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   using Smem = BwdSmem<D, TILE, kKV, kDoK, kHasT>;
   Smem &s = *reinterpret_cast<Smem *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  if constexpr (Smem::kRing && kDoK) {  // no room was left to round up: the base must have been aligned
+  if constexpr (D == 128 && kDoK) {  // no room was left to round up: the base must have been aligned
     if (reinterpret_cast<uintptr_t>(smem_raw) % 1024 != 0) {
       if (threadIdx.x == 0) atomicCAS(a.status, 0u, 220u);
       return;
@@ -502,8 +505,8 @@ __global__ void __launch_bounds__(bwd_threads(bwd_parts(TILE), bwd_two_issuers(D
         //                         read (A | C) - neither waits for an output product;
         //   issuer B (last warp): outK(j) once compute2(j) has written W1 / W2; its commits (stage free, item done)
         //                         drain only its own queue.
-        // Hazards: W[g & 1] is rewritten by compute2(g + 2), which needs scores2(g + 2), which needs the streamed
-        // stage of tile g reloaded, which needs outK(g) complete (y_empty): outK(g) has long read it.
+        // Hazards: W[g & 1] is rewritten by compute2(g + 2), which therefore waits for outK(g) (y_empty of its stage; that barrier
+        // cannot complete again before outK(g + 3), so the parity is unambiguous).
         int it = blockIdx.x, j = 0, n = 0, g = 0;
         bool ok = it < items;
         if (warp == 1) {
@@ -554,8 +557,8 @@ __global__ void __launch_bounds__(bwd_threads(bwd_parts(TILE), bwd_two_issuers(D
             // Two barriers, by tile parity.  Nothing that this thread issues gates the second half of the score algebra,
             // so the compute warps can complete two tiles (g and g + 1) while this thread is still held up behind the
             // other issuer's MMAs, and a parity wait on a single barrier would then take the incomplete phase g + 2
-            // for phase g and never return.  Tile g + 2 cannot complete before outK(g) (its streamed stage is reloaded
-            // only then), so with one barrier per parity the wait is unambiguous.
+            // for phase g and never return.  Tile g + 2 cannot complete before outK(g) (the score algebra waits for it
+            // before it overwrites W), so with one barrier per parity the wait is unambiguous.
             if (!mbar_wait_for(a.wait_cycles, &s.c2_done[g & 1], (g >> 1) & 1)) {  // W1 / W2 of tile g are in place
               atomicCAS(a.status, 0u, 216u);
               break;
@@ -945,6 +948,13 @@ __global__ void __launch_bounds__(bwd_threads(bwd_parts(TILE), bwd_two_issuers(D
       // ---- second half: W1 = scale P (A - delta), W2 = scale P ((A - delta) N + C - dsum)
       if (!__all_sync(0xffffffffu, mbar_wait_for(a.wait_cycles, &s.s2_full, g & 1))) {
         atomicCAS(a.status, 0u, 208u);
+        ok = false;
+        continue;
+      }
+      // W1 / W2 of tile g go where those of tile g - 2 were: its output products must have read them
+      if (kSplit && g >= 2 &&
+          !__all_sync(0xffffffffu, mbar_wait_for(a.wait_cycles, &s.y_empty[(g - 2) % kStages], ((g - 2) / kStages) & 1))) {
+        atomicCAS(a.status, 0u, 221u);
         ok = false;
         continue;
       }
