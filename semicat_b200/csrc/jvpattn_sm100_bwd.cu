@@ -60,7 +60,7 @@ __host__ __device__ constexpr int bwd_parts(int tile) { return tile >= 64 ? JVPA
 // reads as long as it multiplies.  Forward and backward of 128 heads at length 2048: 5.42 ms with 32-row tiles, 4.30 ms so.
 // The query owner of head_dim 64 (with tangents) streams pairs for another reason: two whole stages fit, but (Y0, Y1) of a tile are
 // released by its last products and were wanted again right after them, so every second tile waited 1400 cycles for its load.
-// It has three stages of (Y0, Y1) and two of (Y2, Y3): 564 -> 510 us for 128 heads at length 2048.
+// It has three stages of (Y0, Y1) and two of (Y2, Y3): 564 -> 507 us for 128 heads at length 2048.
 __host__ __device__ constexpr bool bwd_pair_ring(int D, bool kv, bool has_t) { return D == 128 || (!kv && has_t); }
 // Without tangents two of the four tensors on either side, one of the two score products per region and the tangent
 // accumulators are absent.  At head_dim 64 two CTAs then share an SM, one's products beside the other's score algebra
