@@ -253,7 +253,9 @@ __global__ void __launch_bounds__(bwd_threads(bwd_parts(TILE), bwd_two_issuers(D
   if (threadIdx.x == 0) {
     for (int i = 0; i < kXBuf; ++i) {
       mbar_init(&s.x_full[i], 1);
-      mbar_init(&s.x_empty[i], kBoxes == 1 ? 2 : 1);  // MMA issuer, plus the thread whose output stores read the buffer
+      // MMA issuer, plus the thread whose output stores read the buffer; single row buffer of the query owner: plus
+      // each compute warp once it has its rows' statistics (see there)
+      mbar_init(&s.x_empty[i], kBoxes == 1 ? 2 : kKV ? 1 : 1 + kComputeThreads / 32);
     }
     mbar_init(&s.acc_free, kComputeThreads);
     for (int i = 0; i < kStages; ++i) {
@@ -855,6 +857,13 @@ __global__ void __launch_bounds__(bwd_threads(bwd_parts(TILE), bwd_two_issuers(D
       if (ok && x0 + row < a.Lx)
         rstat = make_float4(s.xstat[xb_][0][row] * kLog2e - lscale, has_t ? s.xstat[xb_][1][row] : 0.f, s.xstat[xb_][2][row],
                             s.xstat[xb_][3][row]);
+      if (kXBuf == 1) {
+        // The issuer's release does not cover these reads: with one streamed tile per item its last score products are
+        // queued while these warps are still in the epilogue of the item before, and the rows of the item after next
+        // could land here first.  (Two buffers: the release behind the output stores comes after every warp's reads.)
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&s.x_empty[xb_]);
+      }
     }
     for (int j = 0; j < ntiles; ++j, ++g) {
       if (kKV) {
