@@ -53,7 +53,7 @@ struct FwdSmem {
   // the value products with V.  [K ; Kd] is one K-major operand of 128 rows (64-channel box outermost), [V | Vd] one MN-major
   // operand of 2 D columns (tensor outermost).
   alignas(1024) uint16_t kv[kStages][2][kPer * kBoxes][kBN * 64];
-  uint64_t q_full, k_full[kStages], k_empty[kStages], v_full[kStages], v_empty[kStages], s_full[2], p_full[2], o_done;
+  uint64_t q_full, k_full[kStages], k_empty[kStages], v_full[kStages], v_empty[kStages], s_full[2], p_full[2], o_done[2];
   uint32_t tmem_base;
 };
 
@@ -76,8 +76,8 @@ __global__ void __launch_bounds__(kThreads, fwd_ctas_per_sm(D, kHasT)) sm100_fwd
   constexpr uint32_t kColO = 0, kColOd = D, kColS = (kHasT ? 2 : 1) * D;  // Sd / U 64 columns behind S / P
   constexpr uint32_t kRegion = kHasT ? 128 : 64;                          // columns of (S | Sd)
   // D = 128 leaves one CTA per SM, with nothing to run beside its softmax: (S | Sd) alternates between two regions and the
-  // scores of tile j + 1 are issued ahead of the value products of tile j.  Scores and softmax then run up to two tiles ahead of
-  // each other's waits, which a parity wait on one barrier would mistake for none: their barriers alternate too.
+  // scores of tile j + 1 are issued ahead of the value products of tile j.  Scores, softmax and value products then run up to two
+  // tiles ahead of each other's waits, which a parity wait on one barrier would mistake for none: their barriers alternate too.
   // 128 heads at length 2048: 934 -> 614 us.
   constexpr bool kAlternate = D == 128;
   constexpr uint32_t kUsed = kColS + (kAlternate ? 2 : 1) * kRegion;
@@ -122,8 +122,8 @@ __global__ void __launch_bounds__(kThreads, fwd_ctas_per_sm(D, kHasT)) sm100_fwd
     for (int i = 0; i < 2; ++i) {
       mbar_init(&s.s_full[i], 1);
       mbar_init(&s.p_full[i], 128);
+      mbar_init(&s.o_done[i], 1);
     }
-    mbar_init(&s.o_done, 1);
     fence_barrier_init();
     // The barriers this thread just initialised are all the first requests need: the query rows and the first
     // key tiles are on their way while the other warps allocate tensor memory and meet at the barrier below.
@@ -243,7 +243,7 @@ __global__ void __launch_bounds__(kThreads, fwd_ctas_per_sm(D, kHasT)) sm100_fwd
           }
         }
         tc_commit(&s.v_empty[st]);
-        tc_commit(&s.o_done);
+        tc_commit(&s.o_done[alt(j)]);
       }
     }
   } else {
@@ -299,7 +299,7 @@ __global__ void __launch_bounds__(kThreads, fwd_ctas_per_sm(D, kHasT)) sm100_fwd
         // S of this tile is complete, so every earlier O / Od' update has retired (kAlternate: all but the last one, which
         // was issued behind S of this tile): safe to rescale in place.
         if (kAlternate) {
-          if (!__all_sync(0xffffffffu, mbar_wait_for(a.wait_cycles, &s.o_done, (j - 1) & 1))) {
+          if (!__all_sync(0xffffffffu, mbar_wait_for(a.wait_cycles, &s.o_done[alt(j - 1)], alt_parity(j - 1)))) {
             atomicCAS(a.status, 0u, 107u);
             ok = false;
             break;
@@ -376,9 +376,11 @@ __global__ void __launch_bounds__(kThreads, fwd_ctas_per_sm(D, kHasT)) sm100_fwd
       mbar_arrive(&s.p_full[alt(j)]);
     }
     // ---- epilogue: O = acc / l ; Od = Od'/l - (mu/l) O ; statistics
-    // (kAlternate: the last two value products may both be outstanding, and a parity wait tells adjacent phases apart only)
-    if (ok && ((kAlternate && ntiles > 1 && !__all_sync(0xffffffffu, mbar_wait_for(a.wait_cycles, &s.o_done, ntiles & 1))) ||
-               !__all_sync(0xffffffffu, mbar_wait_for(a.wait_cycles, &s.o_done, (ntiles - 1) & 1)))) {
+    // (kAlternate: the last two value products may both be outstanding here, or neither.  With one barrier a wait for the last
+    // could take the phase before it for its own, and a wait for that one first could find both over and never return.
+    // With two, the phase before the last tile's on its barrier is that of two tiles earlier, complete before the scores of
+    // the last tile, and none follows it: one wait, and it covers every product issued before.)
+    if (ok && !__all_sync(0xffffffffu, mbar_wait_for(a.wait_cycles, &s.o_done[alt(ntiles - 1)], alt_parity(ntiles - 1)))) {
       atomicCAS(a.status, 0u, 106u);
       ok = false;
     }

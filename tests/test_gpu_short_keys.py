@@ -46,3 +46,29 @@ def test_many_items_with_one_key_tile(D, Lk, mode):
     for n in got:
         G.assert_close(got[n][:, heads].float().cpu().numpy(), want[n], f"{n} D={D} Lk={Lk} {mode}")
     assert _lib.device_status() == 0
+
+
+@pytest.mark.parametrize("tangents", [True, False])
+@pytest.mark.parametrize("ntiles", [1, 2, 3, 5])
+@pytest.mark.parametrize("D", [72, 128])
+def test_forward_at_few_key_tiles(D, ntiles, tangents):
+    """Heads wider than 64 channels alternate between two score regions; the last value products may be over before a warp
+    asks for them.  Many CTAs, several times: every call complete, equal and close to the oracle on sampled heads."""
+    ins = G.rounded(G.synth(B, H, LQ, 64 * ntiles - 5, D, seed=D + ntiles), torch.bfloat16)
+    t = {n: G.place(ins[n], torch.bfloat16, "bshd") for n in G.IN_NAMES}
+    first = None
+    for _ in range(4):
+        o, to = torch.full_like(t["q"], G.CANARY), torch.full_like(t["q"], G.CANARY) if tangents else None
+        lse = torch.full((B, H, ops.stat_len(LQ)), G.CANARY, device="cuda")
+        mu = torch.full_like(lse, G.CANARY) if tangents else None
+        tang = [t[n] if tangents else None for n in ("tq", "tk", "tv")]
+        ops.jvp_attention_fwd(t["q"], t["k"], t["v"], *tang, o, to, lse, mu)
+        out = [x for x in (o, to, lse, mu) if x is not None]
+        first = first or out
+        assert all(torch.equal(x, y) for x, y in zip(out, first))
+    heads = slice(3, None, 41)
+    want = G.oracle({n: x[:, heads] for n, x in ins.items()}, None)
+    G.assert_close(first[0][:, heads].float().cpu().numpy(), want["o"], "o")
+    if tangents:
+        G.assert_close(first[1][:, heads].float().cpu().numpy(), want["to"], "to")
+    assert _lib.device_status() == 0
