@@ -17,9 +17,11 @@ def node(cls):
 
 def unrecorded() -> bool:
     """Nothing can come of a node: gradients are off, no forward-mode level is open, no function transform is active and
-    nothing is being traced.  A node's ``forward`` may then be called directly (a sampling pass: 10.1 -> 6.4 ms with both)."""
+    nothing is being traced (``torch.jit.trace`` records a node as one operation; of a bare ``forward`` it would see the
+    allocations only, and the traced function would return them unwritten).  A node's ``forward`` may then be called
+    directly (a sampling pass: 10.1 -> 6.4 ms with both)."""
     return (not torch.is_grad_enabled() and fwAD._current_level < 0 and not torch._C._are_functorch_transforms_active()
-            and not torch.compiler.is_compiling())
+            and not torch.compiler.is_compiling() and not torch.jit.is_tracing())
 
 
 def apply(cls, *args):

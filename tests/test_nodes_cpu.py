@@ -60,3 +60,30 @@ def test_apply_records_where_gradients_are_on():
     with torch.no_grad():
         z = _nodes.apply(Twice, x)
     assert torch.equal(z, y) and not z.requires_grad
+
+
+class _Outside(torch.autograd.Function):
+    """Doubles its input as a kernel does, where a tracer sees nothing of it but the allocation."""
+
+    @staticmethod
+    def forward(x):
+        y = torch.empty_like(x)
+        y.numpy()[...] = 2 * x.numpy()
+        return y
+
+    @staticmethod
+    def setup_context(ctx, inputs, output):
+        pass
+
+    @staticmethod
+    def backward(ctx, g):
+        return g * 2
+
+
+def test_a_trace_records_the_node():
+    with torch.no_grad():
+        traced = torch.jit.trace(lambda x: _nodes.apply(_Outside, x) + 1, (torch.ones(3),), check_trace=False)
+        assert torch.equal(traced(torch.full((3,), 5.0)), torch.full((3,), 11.0))
+        seen = []
+        torch.jit.trace(lambda x: (seen.append(_nodes.unrecorded()), x + 1)[1], (torch.ones(3),), check_trace=False)
+        assert seen == [False]
