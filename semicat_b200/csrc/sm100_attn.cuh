@@ -31,12 +31,13 @@ __device__ __forceinline__ uint32_t pack2<__half>(float a, float b) {
 }
 
 // What the pair (a, b) is above its 16-bit rounding `hi` = pack2(a, b), rounded to 16 bits itself: hi + rest carries 16
-// significant bits where bf16 carries 8.
+// significant bits where bf16 carries 8.  Nothing above an infinite value (inf - inf would make it NaN).
 template <typename T>
 __device__ __forceinline__ uint32_t pack2_rest(float a, float b, uint32_t hi);
 template <>
 __device__ __forceinline__ uint32_t pack2_rest<__nv_bfloat16>(float a, float b, uint32_t hi) {
-  return pack2<__nv_bfloat16>(a - __uint_as_float(hi << 16), b - __uint_as_float(hi & 0xffff0000u));
+  const float ha = __uint_as_float(hi << 16), hb = __uint_as_float(hi & 0xffff0000u);
+  return pack2<__nv_bfloat16>(fabsf(ha) < INFINITY ? a - ha : 0.f, fabsf(hb) < INFINITY ? b - hb : 0.f);
 }
 
 template <typename T> struct IsBf16 { static constexpr bool value = false; };

@@ -58,3 +58,17 @@ def test_forced_family_keeps_its_head_dimensions():
     # widths whose rows are not 16-byte aligned and fp16 heads stay on the portable kernels
     assert ops.selected_kernels(1, 1, 64, 64, 20) == ops.KERNELS_SIMT
     assert ops.selected_kernels(1, 1, 64, 64, 32, dtype=torch.float16) == ops.KERNELS_SIMT
+
+
+@pytest.mark.parametrize("D", [16, 32, 56, 72, 96, 120])
+def test_infinite_tangents_come_out_as_from_the_portable_kernels(D):
+    """One infinite element of the keys' tangent: scores' tangents, and with them U, are infinite in that column.  The low
+    part of an infinite operand is zero, not inf - inf, so infinities and NaN appear where the portable kernels have them."""
+    ins = G.rounded(G.synth(2, 2, 70, 90, D, seed=D), torch.bfloat16)
+    ins["tk"][:, :, 37, 3] = np.inf
+    with np.errstate(invalid="ignore"):
+        got, simt = (G.run(ins, mode=None, kernels=k)["to"] for k in (ops.KERNELS_AUTO, ops.KERNELS_SIMT))
+    assert np.isinf(simt).any() and np.isnan(simt).any()
+    assert np.array_equal(np.isnan(got), np.isnan(simt))
+    bad = ~np.isfinite(simt) & ~np.isnan(simt)
+    assert np.array_equal(got[bad], simt[bad]) and np.isfinite(got[np.isfinite(simt)]).all()
