@@ -49,8 +49,8 @@ enum { JVPATTN_BF16 = 0, JVPATTN_FP16 = 1 };
 
 /* Selects the kernel family.  AUTO picks the tcgen05/TMA kernels whenever the shape allows and the
  * portable SIMT kernels otherwise; the other two force one family (the forced tcgen05 choice returns
- * JVPATTN_EINVAL for a shape it cannot run and for every head_dim but 64 and 128; AUTO also takes bf16
- * heads of other widths there).  Used by the parity tests to check one family against the other on the device. */
+ * JVPATTN_EINVAL for a shape it cannot run; it runs what jvpattn_selected_kernels reports).  Used by the parity
+ * tests to check one family against the other on the device. */
 enum { JVPATTN_KERNELS_AUTO = 0, JVPATTN_KERNELS_SIMT = 1, JVPATTN_KERNELS_TCGEN05 = 2 };
 
 /* A 4-D tensor indexed (batch, head, position, channel) with element strides; stride[3] must be 1.
@@ -282,7 +282,7 @@ int jvpattn_profile_end(double *total_ms, uint64_t *launches);
 const char *jvpattn_kernel_name(int id);
 
 /* Synchronises the current device and returns the device-side status word: 0 if no bounded wait has
- * run out since the last call, else a code identifying the wait that gave up (101..107 forward, 201..216
+ * run out since the last call, else a code identifying the wait that gave up (101..107 forward, 201..221
  * backward).  Clears the word.  Every wait inside the kernels is bounded (about two seconds): a kernel whose
  * wait runs out stops computing, leaves through its normal teardown and leaves its outputs unwritten or partial;
  * the context stays usable. */

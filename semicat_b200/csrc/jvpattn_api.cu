@@ -8,7 +8,6 @@
 #include <vector>
 
 #include "jvpattn_common.cuh"
-#include "sm100_attn.cuh"
 #include "sm100_ptx.cuh"
 
 namespace jvpattn {
@@ -529,7 +528,7 @@ int jvpattn_fwd(const jvpattn_problem *p, const jvpattn_tensor *q, const jvpattn
   a.status = d->status;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   bool fast = p->kernels != JVPATTN_KERNELS_SIMT && sm100_fwd_supported(a);
-  if (p->kernels == JVPATTN_KERNELS_TCGEN05 && (!fast || !sm100_native_head_dim(a.D))) return JVPATTN_EINVAL;
+  if (p->kernels == JVPATTN_KERNELS_TCGEN05 && !fast) return JVPATTN_EINVAL;
   if (fast) a.inject = g_inject_fwd.exchange(0);  // one-shot test hook
   return note_cuda(fast ? sm100_fwd(a, s) : simt_fwd(a, s));
 }
@@ -559,7 +558,7 @@ int jvpattn_bwd(const jvpattn_problem *p, const jvpattn_tensor *q, const jvpattn
   a.status = d->status;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   bool fast = p->kernels != JVPATTN_KERNELS_SIMT && sm100_bwd_supported(a);
-  if (p->kernels == JVPATTN_KERNELS_TCGEN05 && (!fast || !sm100_native_head_dim(a.D))) return JVPATTN_EINVAL;
+  if (p->kernels == JVPATTN_KERNELS_TCGEN05 && !fast) return JVPATTN_EINVAL;
   return note_cuda(fast ? sm100_bwd(a, s) : simt_bwd(a, s));
 }
 

@@ -50,14 +50,22 @@ def test_without_tangents(D):
     G.assert_close(lse[..., :L].cpu().numpy(), want["lse"], "lse")
 
 
-def test_forced_family_keeps_its_head_dimensions():
-    ins = G.rounded(G.synth(1, 1, 64, 64, 32, seed=1), torch.bfloat16)
+@pytest.mark.parametrize("D", [16, 40, 64, 96, 128])
+def test_forcing_the_selected_family_gives_what_auto_gives(D):
+    ins = G.rounded(G.synth(1, 2, 70, 90, D, seed=1), torch.bfloat16)
+    assert ops.selected_kernels(1, 2, 70, 90, D) == ops.KERNELS_TCGEN05
+    auto, forced = (G.run(ins, kernels=k) for k in (ops.KERNELS_AUTO, ops.KERNELS_TCGEN05))
+    assert auto.keys() == forced.keys() and all(np.array_equal(auto[n], forced[n]) for n in auto)
+
+
+@pytest.mark.parametrize("D,dtype", [(20, torch.bfloat16), (32, torch.float16), (121, torch.bfloat16)])
+def test_widths_that_stay_on_the_portable_kernels_cannot_be_forced(D, dtype):
+    """Rows that are not 16-byte aligned, and fp16 heads of other widths (their parts lack the exponent range)."""
+    assert ops.selected_kernels(1, 1, 64, 64, D, dtype=dtype) == ops.KERNELS_SIMT
+    ins = G.rounded(G.synth(1, 1, 64, 64, D, seed=1), dtype)
     with pytest.raises(_lib.JvpAttnError) as e:
-        G.run(ins, kernels=ops.KERNELS_TCGEN05, mode=None)
+        G.run(ins, dtype=dtype, kernels=ops.KERNELS_TCGEN05, mode=None)
     assert e.value.code == -1
-    # widths whose rows are not 16-byte aligned and fp16 heads stay on the portable kernels
-    assert ops.selected_kernels(1, 1, 64, 64, 20) == ops.KERNELS_SIMT
-    assert ops.selected_kernels(1, 1, 64, 64, 32, dtype=torch.float16) == ops.KERNELS_SIMT
 
 
 @pytest.mark.parametrize("D", [16, 32, 56, 72, 96, 120])
