@@ -107,6 +107,47 @@ def test_ln_modulate_bf16_and_missing_tangent_on_x():
             _close(a, r, f"{name} (tx={tx})", 3e-2, 3e-2 * float(r.float().abs().max()))
 
 
+@pytest.mark.parametrize("cotangents", ["both", "tangent", "primal"])
+@pytest.mark.parametrize("exact", [False, True])
+@pytest.mark.parametrize("tx", [True, False])
+def test_ln_modulate_bf16_launches_and_gradients(tx, exact, cotangents):
+    """The bf16 pair through the public entry point: one kernel forward, one for whichever cotangents arrive, one finalize, and
+    every gradient against fp64.  bf16 results to one rounding (2^-8; 2^-7 where values that were rounded themselves
+    enter), fp32 parameter gradients to the order of their sums."""
+    B, S, C = 3, 50, 768
+    x, t, sh, sc, tsh, tsc, norm, cots = _ln_inputs(B, S, C, torch.bfloat16, seed=11, tx=tx)
+    cots = [c.to(torch.bfloat16) for c in cots]
+    names = ["x", "shift", "scale"] + ["tx"] * tx + ["tshift", "tscale", "gamma", "beta"]
+
+    def run(leaf, layer_norm):
+        prim = [leaf(v) for v in (x, sh, sc)]
+        tang = [leaf(v) for v in (t, tsh, tsc) if v is not None]
+        w, b = (v.detach().clone().to(torch.float32 if leaf is same else torch.float64).requires_grad_(True) for v in (norm.weight, norm.bias))
+        duals, rest = (prim, []) if tx else (prim[1:], prim[:1])
+        y, ty = torch.func.jvp(lambda *d: layer_norm(*rest, *d, w, b), tuple(duals), tuple(tang))
+        outs, gs = {"both": ([y, ty], cots), "tangent": ([ty], cots[1:]), "primal": ([y], cots[:1])}[cotangents]
+        grads = torch.autograd.grad(outs, [*prim, *tang, w, b], [g.to(y.dtype) for g in gs], allow_unused=True)
+        return y, ty, dict(zip(names, grads))
+
+    same = lambda v: v.detach().clone().requires_grad_(True)
+    double = lambda v: v.detach().double().requires_grad_(True)
+    ours = lambda x_, sh_, sc_, w, b: dual_ops.ln_modulate(
+        x_, types.SimpleNamespace(weight=w, bias=b, eps=norm.eps, normalized_shape=(C,)), sh_, sc_, exact=exact)
+    ref_ln = (lambda v, w, b: _manual_ln(v, w, b, norm.eps)) if exact else (lambda v, w, b: F.layer_norm(v, (C,), w, b, norm.eps))
+    before = _lib.launch_count()
+    y, ty, got = run(same, ours)
+    assert _lib.launch_count() - before == 3
+    y_ref, ty_ref, want = run(double, lambda x_, sh_, sc_, w, b: ref_ln(x_, w, b) * (1 + sc_) + sh_)
+    _close(y, y_ref, "y", 2 ** -8, 1e-4)
+    _close(ty, ty_ref, "ty", 2 ** -8, 1e-4)
+    for n in names:
+        if want[n] is None:
+            assert got[n] is None or not got[n].any(), n
+            continue
+        peak = float(want[n].abs().max())
+        _close(got[n], want[n], f"{n} (tx={tx}, exact={exact}, {cotangents})", 2 ** -7 if n not in ("gamma", "beta") else 1e-5, 1e-4 * peak)
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_gated_residual_matches_pytorch(dtype):
     B, S, C = 3, 50, 768
