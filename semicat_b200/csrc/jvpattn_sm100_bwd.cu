@@ -553,7 +553,7 @@ __global__ void __launch_bounds__(bwd_threads(bwd_parts(TILE), bwd_two_issuers(D
             it = it2; j = j2; n = n2; ++g;
           }
         } else {
-          const bool acc_merge = kMerge && has_t;
+          static_assert(kMerge && kHasT, "[dX1 | dX0] are one accumulator");
           for (; ok; ) {
             const int st = g % kStages;
             // Two barriers, by tile parity.  Nothing that this thread issues gates the second half of the score algebra,
@@ -574,40 +574,21 @@ __global__ void __launch_bounds__(bwd_threads(bwd_parts(TILE), bwd_two_issuers(D
             const uint32_t w1 = tmem + kColW + (uint32_t)(g & 1) * kWBuf, w2 = w1 + kWBuf / 2;
             if constexpr (kPair) {
               constexpr uint32_t kLow = TILE / 2;  // low parts behind the high parts
-              bool init0 = j > 0;
+              const bool acc = j > 0;
 #pragma unroll
               for (int kk = 0; kk < TILE / 16; ++kk) {
 #pragma unroll
                 for (uint32_t part = 0; part <= kLow; part += kLow) {
-                  if (acc_merge) {
-                    mma_ts_lo(tmem + kColKd, w1 + part + 8 * kk, yb(ylo_out, 0, kk), idesc_o2, init0);
-                    init0 = true;
-                  } else if (has_t) {
-                    mma_ts_lo(tmem + kColKd, w1 + part + 8 * kk, yb(ylo_out, 0, kk), idesc_o, init0);
-                    mma_ts_lo(tmem + kColK, w1 + part + 8 * kk, yb(ylo_out, 1, kk), idesc_o, init0);
-                    init0 = true;
-                  }
-                  mma_ts_lo(tmem + kColK, w2 + part + 8 * kk, yb(ylo_out, 0, kk), idesc_o, init0);
-                  init0 = true;
+                  mma_ts_lo(tmem + kColKd, w1 + part + 8 * kk, yb(ylo_out, 0, kk), idesc_o2, acc || kk > 0 || part > 0);
+                  mma_ts_lo(tmem + kColK, w2 + part + 8 * kk, yb(ylo_out, 0, kk), idesc_o, true);
                 }
               }
-            } else if (acc_merge) {
+            } else {
               const bool acc = j > 0;
 #pragma unroll
               for (int kk = 0; kk < TILE / 16; ++kk) {
                 mma_ts_lo(tmem + kColKd, w1 + 8 * kk, yb(ylo_out, 0, kk), idesc_o2, acc || kk > 0);  // [dX1 | dX0] += W1 [Y0 | Y1]
                 mma_ts_lo(tmem + kColK, w2 + 8 * kk, yb(ylo_out, 0, kk), idesc_o, true);          // dX0 += W2 Y0
-              }
-            } else {
-#pragma unroll
-              for (int kk = 0; kk < TILE / 16; ++kk) {
-                bool init0 = j > 0 || kk > 0;
-                if (has_t) {
-                  mma_ts_lo(tmem + kColKd, w1 + 8 * kk, yb(ylo_out, 0, kk), idesc_o, init0);   // dX1 += W1 Y0
-                  mma_ts_lo(tmem + kColK, w1 + 8 * kk, yb(ylo_out, 1, kk), idesc_o, init0);    // dX0 += W1 Y1
-                  init0 = true;
-                }
-                mma_ts_lo(tmem + kColK, w2 + 8 * kk, yb(ylo_out, 0, kk), idesc_o, init0);      // dX0 += W2 Y0
               }
             }
             tc_commit(&s.y_empty[st]);
@@ -713,20 +694,14 @@ __global__ void __launch_bounds__(bwd_threads(bwd_parts(TILE), bwd_two_issuers(D
         } else if (kDoV) {
 #pragma unroll
           for (int kk = 0; kk < TILE / 16; ++kk) {
-            if (kMerge && has_t && has_o) {
-              mma_ts_lo(tmem + kColVd, sp_ + oa(kk), yb(ylo_v, 2, kk), idesc_o2, initvd);  // [dVd | dV] += P [G | gO]
-              mma_ts_lo(tmem + kColV, spn_ + oa(kk), yb(ylo_v, 2, kk), idesc_o, true);     // dV += (P o N) G
+            if (has_t) {
+              mma_ts_lo(tmem + kColVd, sp_ + oa(kk), yb(ylo_v, 2, kk), idesc_o, initvd);  // dVd += P G
+              mma_ts_lo(tmem + kColV, spn_ + oa(kk), yb(ylo_v, 2, kk), idesc_o, initv);   // dV  += (P o N) G
               initv = initvd = true;
-            } else {
-              if (has_t) {
-                mma_ts_lo(tmem + kColVd, sp_ + oa(kk), yb(ylo_v, 2, kk), idesc_o, initvd);  // dVd += P G
-                mma_ts_lo(tmem + kColV, spn_ + oa(kk), yb(ylo_v, 2, kk), idesc_o, initv);   // dV  += (P o N) G
-                initv = initvd = true;
-              }
-              if (has_o) {
-                mma_ts_lo(tmem + kColV, sp_ + oa(kk), yb(ylo_v, 3, kk), idesc_o, initv);    // dV  += P gO
-                initv = true;
-              }
+            }
+            if (has_o) {
+              mma_ts_lo(tmem + kColV, sp_ + oa(kk), yb(ylo_v, 3, kk), idesc_o, initv);    // dV  += P gO
+              initv = true;
             }
           }
         }
@@ -764,19 +739,17 @@ __global__ void __launch_bounds__(bwd_threads(bwd_parts(TILE), bwd_two_issuers(D
               mma_ts_lo(tmem + kColK, tmem + kColC + oa(kk), yb(ylo_out, 0, kk), idesc_o, true);          // dX0 += W2 Y0
             }
             init0 = init1 = true;
-          } else
+          } else {
 #pragma unroll
-          for (int kk = 0; kk < TILE / 16; ++kk) {
-            if (kMerge && has_t) {
-              mma_ts_lo(tmem + kColKd, tmem + kColA + oa(kk), yb(ylo_out, 0, kk), idesc_o2, init1);  // [dX1 | dX0] += W1 [Y0 | Y1]
-              init0 = init1 = true;
-            } else if (has_t) {
-              mma_ts_lo(tmem + kColKd, tmem + kColA + oa(kk), yb(ylo_out, 0, kk), idesc_o, init1);   // dX1 += W1 Y0
-              mma_ts_lo(tmem + kColK, tmem + kColA + oa(kk), yb(ylo_out, 1, kk), idesc_o, init0);    // dX0 += W1 Y1
-              init0 = init1 = true;
+            for (int kk = 0; kk < TILE / 16; ++kk) {
+              if (has_t) {
+                mma_ts_lo(tmem + kColKd, tmem + kColA + oa(kk), yb(ylo_out, 0, kk), idesc_o, init1);  // dX1 += W1 Y0
+                mma_ts_lo(tmem + kColK, tmem + kColA + oa(kk), yb(ylo_out, 1, kk), idesc_o, init0);   // dX0 += W1 Y1
+                init0 = init1 = true;
+              }
+              mma_ts_lo(tmem + kColK, tmem + kColC + oa(kk), yb(ylo_out, 0, kk), idesc_o, init0);     // dX0 += W2 Y0
+              init0 = true;
             }
-            mma_ts_lo(tmem + kColK, tmem + kColC + oa(kk), yb(ylo_out, 0, kk), idesc_o, init0);      // dX0 += W2 Y0
-            init0 = true;
           }
         }
         tc_commit(kAlternate ? &s.y2_empty[g % kStages2] : &s.y_empty[st]);
