@@ -23,7 +23,7 @@
 // The 16-bit operands P, PoN, W1, W2 are written over the fp32 score columns in TMEM and fed back to the
 // tensor core as the A operand; the Y tiles are read MN-major as the B operand.
 //
-//   warp 0      TMA producer (X once, Y through a 2-stage ring)
+//   warp 0      TMA producer (X once per item, Y through rings of one to three stages, see BwdSmem)
 //   warp 1      MMA issuer (query owner: the score products)
 //   last warp   query owner only: second MMA issuer (the output products)
 //   warps 2..   kParts threads per owned row (each on 1/kParts of the tile's columns): score algebra, operand
@@ -891,7 +891,7 @@ __global__ void __launch_bounds__(bwd_threads(bwd_parts(TILE), bwd_two_issuers(D
           nn[c / 2 + i] = n;
           if (kDoV) {
             kp[i] = pack2<T>(p.x, p.y);
-            if constexpr (kPair) kpl[i] = pack2_rest<T>(p.x, p.y, kp[i]);
+            if constexpr (kPair) kpl[i] = pack2_rest<T, true>(p.x, p.y, kp[i]);
             if (has_t) {
               const float2 pn = __fmul2_rn(p, n);
               kpn[i] = pack2<T>(pn.x, pn.y);

@@ -343,7 +343,7 @@ __global__ void __launch_bounds__(kThreads, fwd_ctas_per_sm(D, kHasT)) sm100_fwd
           const float2 p = make_float2(fast_exp2(t.x), fast_exp2(t.y));
           psum[i & 1] = __fadd2_rn(psum[i & 1], p);
           pk[i] = pack2<T>(p.x, p.y);
-          if constexpr (kPair) pl[i] = pack2_rest<T>(p.x, p.y, pk[i]);
+          if constexpr (kPair) pl[i] = pack2_rest<T, true>(p.x, p.y, pk[i]);
           if (kHasT) {
             const float2 u = __fmul2_rn(__fmul2_rn(p, scx2),
                                         make_float2(__uint_as_float(sd[2 * i]), __uint_as_float(sd[2 * i + 1])));
