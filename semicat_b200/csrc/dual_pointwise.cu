@@ -33,14 +33,25 @@ __device__ __forceinline__ void load8<float>(const float *p, float (&f)[8]) {
   const float4 a = reinterpret_cast<const float4 *>(p)[0], b = reinterpret_cast<const float4 *>(p)[1];
   f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w; f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
 }
-// 8 elements as loaded
-template <typename T> struct alignas(16) Raw8 { uint32_t w[2 * sizeof(T)]; };
+// 8 elements as loaded.  Copied as a whole before anything looks into it: bf16 pairs read through a reference to global memory
+// are loads of 4 bytes each (LayerNorm forward of 32 x 128 rows of 768: 6.2 us so, 5.0 us with one load of 16 bytes).
+template <typename T> struct Raw8 { uint4 q[sizeof(T) / 2]; };
+template <typename T>
+__device__ __forceinline__ Raw8<T> load_raw8(const T *p) {
+  Raw8<T> u;
+#pragma unroll
+  for (int i = 0; i < (int)(sizeof(T) / 2); ++i) u.q[i] = reinterpret_cast<const uint4 *>(p)[i];
+  return u;
+}
 __device__ __forceinline__ void unpack8(const Raw8<float> &u, float (&f)[8]) {
 #pragma unroll
-  for (int i = 0; i < 8; ++i) f[i] = __uint_as_float(u.w[i]);
+  for (int i = 0; i < 2; ++i) {
+    f[4 * i] = __uint_as_float(u.q[i].x), f[4 * i + 1] = __uint_as_float(u.q[i].y);
+    f[4 * i + 2] = __uint_as_float(u.q[i].z), f[4 * i + 3] = __uint_as_float(u.q[i].w);
+  }
 }
 __device__ __forceinline__ void unpack8(const Raw8<__nv_bfloat16> &u, float (&f)[8]) {
-  const __nv_bfloat162 *h = reinterpret_cast<const __nv_bfloat162 *>(&u);
+  const __nv_bfloat162 *h = reinterpret_cast<const __nv_bfloat162 *>(&u.q[0]);
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const float2 v = __bfloat1622float2(h[i]);
@@ -50,7 +61,7 @@ __device__ __forceinline__ void unpack8(const Raw8<__nv_bfloat16> &u, float (&f)
 }
 template <>
 __device__ __forceinline__ void load8<__nv_bfloat16>(const __nv_bfloat16 *p, float (&f)[8]) {
-  unpack8(*reinterpret_cast<const Raw8<__nv_bfloat16> *>(p), f);
+  unpack8(load_raw8(p), f);
 }
 template <typename T> __device__ __forceinline__ float ldf(const T *p);
 template <> __device__ __forceinline__ float ldf<float>(const float *p) { return *p; }
@@ -130,7 +141,7 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) ln_modulate_fwd_kernel(LnAr
   auto load_row = [&](int s) {
     const T *x = static_cast<const T *>(a.x) + ((int64_t)b * a.S + s) * C;
 #pragma unroll
-    for (int v = 0; v < NV; ++v) cur[v] = *reinterpret_cast<const Raw8<T> *>(x + chan(v, lane));
+    for (int v = 0; v < NV; ++v) cur[v] = load_raw8(x + chan(v, lane));
   };
   load_row(s0);
   float ga[NV][8], be[NV][8];
@@ -462,10 +473,10 @@ __global__ void __launch_bounds__(NV * 32, (sizeof(T) == 2 ? 16 : 12) / NV) ln_m
   };
   auto load_row = [&](int s, Row &r) {
     const int64_t row = (int64_t)b * a.S + s, e = row * C + c0;
-    r.x = *reinterpret_cast<const Raw8<T> *>(static_cast<const T *>(a.x) + e);
-    if (kTan) r.t = a.tx ? *reinterpret_cast<const Raw8<T> *>(static_cast<const T *>(a.tx) + e) : Raw8<T>{};
-    r.g = *reinterpret_cast<const Raw8<T> *>(static_cast<const T *>(a.g) + e);
-    if (kTan) r.gt = *reinterpret_cast<const Raw8<T> *>(static_cast<const T *>(a.gt) + e);
+    r.x = load_raw8(static_cast<const T *>(a.x) + e);
+    if (kTan) r.t = a.tx ? load_raw8(static_cast<const T *>(a.tx) + e) : Raw8<T>{};
+    r.g = load_raw8(static_cast<const T *>(a.g) + e);
+    if (kTan) r.gt = load_raw8(static_cast<const T *>(a.gt) + e);
     r.mean = a.mean[row];
     r.rstd = a.rstd[row];
   };
@@ -592,7 +603,7 @@ struct GateArgs {
 
 // Index type of the forward kernels, which take a linear chunk index apart into (sample, row, channels): 32 bits wherever they
 // hold the index and a grid stride, since two 64-bit divisions per chunk of 8 elements cost more than the chunk's arithmetic
-// (128 x 128 rows of 768, pair: 36.5 -> 33.7 us).
+// (128 x 128 rows of 768, pair: 30.6 -> 26.8 us).
 inline bool index32(int64_t chunks) { return chunks < (int64_t(1) << 31); }
 
 // z = x + m g y without a tangent (the passes that run outside forward-mode AD)
@@ -743,11 +754,11 @@ __global__ void __launch_bounds__(128) gated_dual_bwd_kernel(GateDualArgs a, int
   };
   auto load_row = [&](int s, Row &r) {
     const int64_t e = ((int64_t)b * a.S + s) * a.C + c0;
-    r.y = *reinterpret_cast<const Raw8<T> *>(static_cast<const T *>(a.y) + e);
-    if (a.gz) r.g1 = *reinterpret_cast<const Raw8<T> *>(static_cast<const T *>(a.gz) + e);
-    if (a.gtz) r.g2 = *reinterpret_cast<const Raw8<T> *>(static_cast<const T *>(a.gtz) + e);
-    if (a.ty && a.gtz) r.ty = *reinterpret_cast<const Raw8<T> *>(static_cast<const T *>(a.ty) + e);
-    if (a.mask) r.m = *reinterpret_cast<const Raw8<T> *>(static_cast<const T *>(a.mask) + e);
+    r.y = load_raw8(static_cast<const T *>(a.y) + e);
+    if (a.gz) r.g1 = load_raw8(static_cast<const T *>(a.gz) + e);
+    if (a.gtz) r.g2 = load_raw8(static_cast<const T *>(a.gtz) + e);
+    if (a.ty && a.gtz) r.ty = load_raw8(static_cast<const T *>(a.ty) + e);
+    if (a.mask) r.m = load_raw8(static_cast<const T *>(a.mask) + e);
   };
   Row cur{};
   load_row(s0, cur);
