@@ -194,6 +194,58 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) ln_modulate_fwd_kernel(LnAr
   }
 }
 
+// The same with a row per warp and the parameter vectors read per row: half the registers, so twice the warps per SM, and no
+// warp idle where a sample has fewer rows than a CTA has warps.
+template <typename T, int NV>
+__global__ void __launch_bounds__(kWarpsPerCta * 32) ln_modulate_fwd_row_kernel(LnArgs a) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int64_t row = (int64_t)blockIdx.x * kWarpsPerCta + warp;
+  if (row >= (int64_t)a.B * a.S) return;
+  const int b = (int)(row / a.S);
+  constexpr int C = NV * 256;
+  const T *x = static_cast<const T *>(a.x) + row * C;
+  float xv[NV][8];
+  float s = 0.f;
+#pragma unroll
+  for (int v = 0; v < NV; ++v) {
+    load8<T>(x + chan(v, lane), xv[v]);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) s += xv[v][i];
+  }
+  const float mean = warp_sum(s) / C;
+  float q = 0.f;
+#pragma unroll
+  for (int v = 0; v < NV; ++v)
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const float d = xv[v][i] - mean;
+      q += d * d;
+    }
+  const float rstd = rsqrtf(warp_sum(q) / C + a.eps);
+  if (lane == 0) {
+    a.mean[row] = mean;
+    a.rstd[row] = rstd;
+  }
+  const T *sc = static_cast<const T *>(a.scale) + (int64_t)b * a.mod_stride;
+  const T *sh = static_cast<const T *>(a.shift) + (int64_t)b * a.mod_stride;
+  T *y = static_cast<T *>(a.y) + row * C;
+#pragma unroll
+  for (int v = 0; v < NV; ++v) {
+    const int c0 = chan(v, lane);
+    float g[8], be[8], scv[8], shv[8], out[8];
+    load8<float>(a.gamma + c0, g);
+    if (a.beta) load8<float>(a.beta + c0, be);
+    load8<T>(sc + c0, scv);
+    load8<T>(sh + c0, shv);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const float ln = (xv[v][i] - mean) * rstd * g[i] + (a.beta ? be[i] : 0.f);
+      out[i] = ln * (1.f + scv[i]) + shv[i];
+    }
+    store8<T>(y + c0, out);
+  }
+}
+
 // ---- forward of the tangent alone:  ty = nd gamma (1 + scale) + (n gamma + beta) tscale + tshift,  nd = rstd P_n(tx),
 //      where P_n(z) = z - mean(z) - n mean(n z)
 template <typename T, int NV>
@@ -881,8 +933,11 @@ cudaError_t ln_modulate(int which, const void *x, const void *tx, const float *g
     if (which == 0 || which == 1) {
       const unsigned grid = (unsigned)((rows + kWarpsPerCta - 1) / kWarpsPerCta);
       if (which == 0) {
-        const int rows_cta = rows_per_cta(B, S, kWarpsPerCta, 4);  // (four blocks fit an SM; small batches: a row per warp)
-        ln_modulate_fwd_kernel<T, NV><<<(unsigned)(B * ((S + rows_cta - 1) / rows_cta)), kWarpsPerCta * 32, 0, stream>>>(a, rows_cta);
+        const int rows_cta = rows_per_cta(B, S, kWarpsPerCta, 4);  // (four blocks fit an SM)
+        if (std::min(S, rows_cta) >= (NV == 4 ? 16 : 8))
+          ln_modulate_fwd_kernel<T, NV><<<(unsigned)(B * ((S + rows_cta - 1) / rows_cta)), kWarpsPerCta * 32, 0, stream>>>(a, rows_cta);
+        else
+          ln_modulate_fwd_row_kernel<T, NV><<<grid, kWarpsPerCta * 32, 0, stream>>>(a);
       } else {
         ln_modulate_fwd_tangent_kernel<T, NV><<<grid, kWarpsPerCta * 32, 0, stream>>>(a);
       }

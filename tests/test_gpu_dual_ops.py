@@ -302,3 +302,33 @@ def test_ln_modulate_bf16_pair_kernels_match_the_single_ones(shape, missing, exa
     sums1[0] += sums1[4]  # the pair kernel keeps sum(g n) + sum(gt nd) together
     scale = sums1[:4].abs().max()
     assert float((sums[:4] - sums1[:4]).abs().max()) <= 1e-5 * float(scale) * S ** 0.5 and not sums[4].any()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("shape", [(1, 1, 256), (1100, 3, 768), (9, 50, 512), (2, 128, 1024), (600, 8, 768), (1200, 9, 256),
+                                   (300, 50, 1024), (75, 128, 768), (148, 129, 512)])
+def test_primal_ln_and_gate_over_the_ways_rows_are_split(shape, dtype):
+    """Without tangents a row per warp or several, a few rows per CTA or many, by the number of samples and rows: results and
+    gradients against fp64.  bf16 results to one rounding (2^-8), fp32 ones and the column sums to the order of the sums."""
+    B, S, C = shape
+    x, y, sh, ga, _, _, norm, (gh, gz) = _ln_inputs(B, S, C, dtype, seed=B + S)
+    sc = ga * 0.5
+    gh, gz = gh.to(dtype), gz.to(dtype)
+    leaves = [v.detach().clone().requires_grad_(True) for v in (x, y, sh, sc, ga)]
+    w, b = norm.weight, norm.bias
+    h = dual_ops.ln_modulate(leaves[0], norm, leaves[2], leaves[3])
+    z = dual_ops.gated_residual(leaves[0], leaves[1], leaves[4], p=0.0, training=True)
+    got = torch.autograd.grad([h, z], [*leaves[1:], w, b], [gh, gz], retain_graph=True)
+    dx_h, = torch.autograd.grad(h, leaves[0], gh)
+    ref = [v.detach().double().requires_grad_(True) for v in (x, y, sh, sc, ga, w, b)]
+    hr = F.layer_norm(ref[0], (C,), ref[5], ref[6], norm.eps) * (1 + ref[3]) + ref[2]
+    zr = ref[0] + ref[4] * ref[1]
+    want = torch.autograd.grad([hr, zr], ref[1:], [gh.double(), gz.double()], retain_graph=True)
+    dxr_h, = torch.autograd.grad(hr, ref[0], gh.double())
+    tol = 2 ** -8 if dtype == torch.bfloat16 else 1e-5
+    _close(h, hr, "h", tol, 1e-4 if dtype == torch.bfloat16 else 1e-5)
+    _close(z, zr, "z", tol, 1e-5)
+    _close(dx_h, dxr_h, "dx", tol, 1e-4 * float(dxr_h.abs().max()))
+    for n, a, r in zip(("dy", "dshift", "dscale", "dgate", "dgamma", "dbeta"), got, want):
+        _close(a, r, n, tol if n not in ("dgamma", "dbeta") else 1e-5, 1e-4 * float(r.abs().max()))
+    assert _lib.device_status() == 0
