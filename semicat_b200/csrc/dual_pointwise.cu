@@ -683,10 +683,16 @@ __global__ void __launch_bounds__(256) gated_residual_fwd_kernel(GateArgs a) {
 // Rows of one sample that a CTA of the backward kernels walks before it adds its column sums to global memory.  Every CTA
 // costs one atomic per column and sum, and at a few hundred samples those atomics (millions per launch, a dozen
 // contenders per address) took longer than the rows themselves; so the count grows with the problem as long as
-// eight CTAs per SM remain (four where there are no sums and the point is what a CTA loads once).
-inline int rows_per_cta(int B, int S, int base, int ctas_per_sm = 8) {
+// eight CTAs per SM remain (four where there are no sums and the point is what a CTA loads once).  Kernels that walk their rows
+// one after another (`resident` = CTAs of theirs that an SM holds) take fewer than `base` where the GPU would otherwise not be
+// full: a row is then latency only (8 x 128 rows of 768, pair of LayerNorm cotangents 15.0 -> 7.4 us, gated residual 6.2 -> 5.2; 2 x 50
+// rows of 256 17.1 -> 5.6).  Not fewer than four: the column sums of two-row CTAs contend (8 x 128 rows of 256, primal: 4.5 us, 3.4
+// with four rows).
+inline int rows_per_cta(int B, int S, int base, int ctas_per_sm = 8, int resident = 0) {
+  auto ctas = [&](int rows) { return (int64_t)B * ((S + rows - 1) / rows); };
   int rows = base;
-  while (rows < 64 && (int64_t)B * ((S + 2 * rows - 1) / (2 * rows)) >= 148 * ctas_per_sm) rows *= 2;
+  while (rows < 64 && ctas(2 * rows) >= 148 * ctas_per_sm) rows *= 2;
+  while (rows > 4 && 2 * ctas(rows) <= 148 * resident) rows /= 2;
   return rows;
 }
 
@@ -942,7 +948,7 @@ cudaError_t ln_modulate(int which, const void *x, const void *tx, const float *g
         ln_modulate_fwd_tangent_kernel<T, NV><<<grid, kWarpsPerCta * 32, 0, stream>>>(a);
       }
     } else {
-      const int rows_cta = rows_per_cta(B, S, 16);
+      const int rows_cta = rows_per_cta(B, S, 16, 8, which == 2 ? std::min(8, (sizeof(T) == 2 ? 16 : 12) / NV) : 0);
       const unsigned grid = (unsigned)(B * ((S + rows_cta - 1) / rows_cta));
       if (which == 2) {
         ln_modulate_bwd_kernel<T, NV, false><<<grid, NV * 32, 0, stream>>>(a, rows_cta);
@@ -974,7 +980,7 @@ cudaError_t ln_modulate_dual(int which, const void *x, const void *tx, const flo
     } else if (which == 0) {
       ln_modulate_dual_fwd_kernel<T, NV><<<(unsigned)((rows + kWarpsPerCta - 1) / kWarpsPerCta), kWarpsPerCta * 32, 0, stream>>>(a);
     } else {
-      const int rows_cta = rows_per_cta(B, S, 16);
+      const int rows_cta = rows_per_cta(B, S, 16, 8, 16 / NV);
       ln_modulate_bwd_kernel<T, NV, true><<<(unsigned)(B * ((S + rows_cta - 1) / rows_cta)), NV * 32, 0, stream>>>(a, rows_cta);
     }
     return cudaGetLastError();
@@ -1035,8 +1041,9 @@ cudaError_t gated_residual_dual(int which, const void *x, const void *tx, const 
       if (index32(n8)) gated_dual_fwd_kernel<T, uint32_t><<<grid, 256, 0, stream>>>(a);
       else gated_dual_fwd_kernel<T, int64_t><<<grid, 256, 0, stream>>>(a);
     } else {
-      const int rows_cta = rows_per_cta(B, S, 16);
-      gated_dual_bwd_kernel<T><<<(unsigned)(B * ((S + rows_cta - 1) / rows_cta)), (C / 8 + 31) / 32 * 32, 0, stream>>>(a, rows_cta);
+      const int threads = (C / 8 + 31) / 32 * 32;
+      const int rows_cta = rows_per_cta(B, S, 16, 8, 512 / threads);
+      gated_dual_bwd_kernel<T><<<(unsigned)(B * ((S + rows_cta - 1) / rows_cta)), threads, 0, stream>>>(a, rows_cta);
     }
     return cudaGetLastError();
   };
