@@ -335,9 +335,10 @@ struct SdRow {
 };
 
 // (five CTAs per SM: 48 registers.  Fewer rows at a time, so that the second pass finds them in L2, is slower: 2048 rows of
-// 30522 take 172 us, 186 at four CTAs by registers, 208 / 211 / 245 at four / three / two by shared memory.)
+// 30522 take 172 us, 186 at four CTAs by registers, 208 / 211 / 245 at four / three / two by shared memory.  Noise off
+// the 16-byte pitch needs 64 registers: held to 48 they spill, 512 rows of 30522 59 us, 53 at four CTAs; fp32 logits 77, 71.)
 template <typename T, bool kVec>
-__global__ void __launch_bounds__(kThreads, 5) sd_fwd_kernel(VocabArgs a) {
+__global__ void __launch_bounds__(kThreads, kVec ? 5 : 4) sd_fwd_kernel(VocabArgs a) {
   __shared__ float scratch[24];
   const int64_t row = blockIdx.x;
   const int b = (int)(row / a.rows_per_sample), V = a.V;
