@@ -101,14 +101,16 @@ __device__ __forceinline__ float2 exp2x(float a, float b, float c) {
 }
 
 // Calls f(first column, whole) for this thread's chunks of 8 columns.  Only the row's last chunk can reach past V: `whole` is a
-// compile-time constant that takes the bounds checks out of all others.  With them and scalar exponents the passes over 16-bit
+// compile-time constant that takes the per-element checks of the arithmetic out of all others (what remains is one test per
+// chunk in load_logits, and load_x0's own for noise off the 16-byte pitch).  With them and scalar exponents the passes over 16-bit
 // logits were bound by instructions: 6144 rows of 30522, cross-entropy forward 112 -> 72 us (57 us at the memory rate),
-// backward 148 -> 124 us (115 us), 2048 rows of the flow map 112 -> 102 us (77 us).
+// backward 148 -> 124 us (115 us), 2048 rows of the flow map 112 -> 102 us (77 us).  The last chunk goes to another warp than the
+// one before it, beside which it runs (256 rows of 27: self-distillation forward 6.2 -> 5.8 us).
 template <typename F>
 __device__ __forceinline__ void for_chunks(int V, F &&f) {
   const int nfull = V / 8;
   for (int c = threadIdx.x; c < nfull; c += kThreads) f(c * 8, std::true_type{});
-  if (V % 8 && threadIdx.x == nfull % kThreads) f(nfull * 8, std::false_type{});
+  if (V % 8 && threadIdx.x == (nfull + 32) % kThreads) f(nfull * 8, std::false_type{});
 }
 
 // Running (max, sum of exp) of one thread's elements, then across the block: returns the row's log-sum-exp.
@@ -261,8 +263,9 @@ __global__ void __launch_bounds__(kThreads) xst_kernel(VocabArgs a) {
 }
 
 // ------------------------------------------------------------------------------------------------ cross-entropy
+// (eight CTAs per SM: fp32 logits otherwise take 37 registers and six; 2048 rows of 30522 with smoothing 49 -> 43.5 us)
 template <typename T>
-__global__ void __launch_bounds__(kThreads) ce_fwd_kernel(VocabArgs a) {
+__global__ void __launch_bounds__(kThreads, 8) ce_fwd_kernel(VocabArgs a) {
   __shared__ float scratch[16];
   const int64_t row = blockIdx.x;
   const int id = (int)a.ids[row], V = a.V;
