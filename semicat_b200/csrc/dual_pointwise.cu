@@ -685,7 +685,7 @@ __global__ void __launch_bounds__(256) gated_residual_fwd_kernel(GateArgs a) {
 // contenders per address) took longer than the rows themselves; so the count grows with the problem as long as
 // eight CTAs per SM remain (four where there are no sums and the point is what a CTA loads once).  Kernels that walk their rows
 // one after another (`resident` = CTAs of theirs that an SM holds) take fewer than `base` where the GPU would otherwise not be
-// full: a row is then latency only (8 x 128 rows of 768, pair of LayerNorm cotangents 15.0 -> 7.4 us, gated residual 6.2 -> 5.2; 2 x 50
+// full: a row is then latency only (8 x 128 rows of 768, pair of LayerNorm cotangents 15.0 -> 7.4 us, gated residual 6.2 -> 4.1; 2 x 50
 // rows of 256 17.1 -> 5.6).  Not fewer than four: the column sums of two-row CTAs contend (8 x 128 rows of 256, primal: 4.5 us, 3.4
 // with four rows).
 inline int rows_per_cta(int B, int S, int base, int ctas_per_sm = 8, int resident = 0) {
