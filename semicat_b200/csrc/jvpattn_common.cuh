@@ -46,6 +46,8 @@ struct BwdArgs {
   float scale;
 };
 
+int sm_count();  // SMs of the current device
+
 // launchers (each returns a cudaError_t from the launch; they never synchronise)
 cudaError_t simt_fwd(const FwdArgs &a, cudaStream_t stream);
 cudaError_t simt_bwd(const BwdArgs &a, cudaStream_t stream);

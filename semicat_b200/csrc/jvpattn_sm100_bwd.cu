@@ -96,19 +96,6 @@ struct BwdSmem {
 };
 
 
-// Number of SMs of the current device (cached per device id).
-int sm_count() {
-  static int cached[64] = {0};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
-  if (cached[dev] == 0) {
-    int n = 0;
-    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
-    cached[dev] = n;
-  }
-  return cached[dev];
-}
-
 struct BwdMaps {
   CUtensorMap x[4], y[4];
   CUtensorMap out[4];  // dX0, dX1, dV, dVd as 128-row x 64-channel store boxes (D = 64 only)
@@ -1199,6 +1186,19 @@ cudaError_t launch_bwd(const BwdArgs &a, cudaStream_t stream) {
 }
 
 }  // namespace
+
+// Number of SMs of the current device (cached per device id).
+int sm_count() {
+  static int cached[64] = {0};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
+  if (cached[dev] == 0) {
+    int n = 0;
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
+    cached[dev] = n;
+  }
+  return cached[dev];
+}
 
 size_t sm100_bwd_workspace_bytes(int B, int H, int Lq, int Lk, int D, int stat_len) {
   (void)Lq; (void)Lk; (void)D;

@@ -126,6 +126,35 @@ def test_sd_lag_loss_value_and_gradients(V, dtype):
     assert _lib.device_status() == 0
 
 
+@pytest.mark.parametrize("V,B,L", [(1, 3, 5), (6144, 3, 5), (6145, 3, 5), (12289, 3, 5), (18432, 3, 5), (18433, 3, 5), (20001, 7, 64),
+                                   (24577, 2, 5), (36864, 2, 3), (36865, 2, 3)])
+def test_rows_held_between_passes(V, B, L):
+    """Vocabularies at the edges of the kernels that hold a row in shared memory, more rows than CTAs in one case, and times s on
+    both sides of where the noise enters the residual, against the formulas in 64 bits.  Gradients and the flow map carry one
+    bf16 rounding (2^-9) and fp32 sums of V terms; noise off the 16-byte pitch in the odd widths."""
+    x0, ids, s, t, l, tl, lt = _case(V, B, L, seed=V, padded_noise=V % 2 == 0)
+    s = torch.tensor([0.2, 0.9, 1 - 1e-6, 0.8322, 0.0, 0.5, 0.99], device="cuda")[:B].contiguous()
+    t = s + (1 - s) * t
+    ids[0, 0], ids[-1, -1] = 0, V - 1
+    lp, tlp = l.clone().requires_grad_(True), tl.clone().requires_grad_(True)
+    xst, lse = vocab_ops.flow_map_input(lp, x0, ids, s, t)
+    loss = vocab_ops.sd_lag_loss(lp, tlp, lt, x0, ids, s, t, lse)
+    g_l, g_tl = torch.autograd.grad(loss, [lp, tlp])
+    ld, tld = l[..., :V].double().requires_grad_(True), tl[..., :V].double().requires_grad_(True)
+    s, t = s.double(), t.double()
+    want = _sd_loss_reference(ld, tld, lt[..., :V].double(), x0.double(), ids, s, t)
+    w_l, w_tl = torch.autograd.grad(want, [ld, tld])
+    xs = (1 - s.view(-1, 1, 1)) * x0.double() + s.view(-1, 1, 1) * F.one_hot(ids, V)
+    w_x = xs + ((t - s) / (1 - s + 1e-8)).view(-1, 1, 1) * (ld.detach().softmax(-1) - xs)
+    assert torch.allclose(xst[..., :V].double(), w_x, rtol=2 ** -8, atol=1e-5) and not xst[..., V:].any()
+    assert torch.allclose(lse.view(B, L).double(), ld.detach().logsumexp(-1), rtol=1e-5, atol=1e-5)
+    assert abs(loss.item() - want.item()) <= 1e-5 * abs(want.item()) + 1e-9
+    for got, ref in ((g_l, w_l), (g_tl, w_tl)):
+        assert torch.allclose(got[..., :V].double(), ref, rtol=2 ** -7, atol=1e-4 * float(ref.abs().max()) + 1e-12)
+        assert not got[..., V:].any()
+    assert _lib.device_status() == 0
+
+
 def test_sd_lag_loss_agrees_with_jvp_of_the_flow_map():
     """The kernel's dv is the forward-mode derivative of the flow map: check against torch.func.jvp of the reference's
     expression with logits that depend on t."""
