@@ -15,6 +15,7 @@ import threading
 _PKG_DIR = os.path.dirname(os.path.abspath(__file__))
 _CSRC = os.path.join(_PKG_DIR, "csrc")
 LIB_PATH = os.path.join(_PKG_DIR, "libjvpattn.so")
+NATIVE_PATH = os.path.join(_PKG_DIR, "_native.so")  # the autograd nodes, see csrc/torch_nodes.cpp
 SOURCES = ["jvpattn_api.cu", "jvpattn_simt.cu", "jvpattn_sm100_fwd.cu", "jvpattn_sm100_bwd.cu",
            "sm100_tensormap.cu", "rotary.cu", "dual_pointwise.cu", "vocab_head.cu", "vocab_loss.cu"]
 NVCC_FLAGS = [
@@ -69,7 +70,7 @@ def _sources_newer_than_lib() -> bool:
     if not os.path.exists(LIB_PATH):
         return True
     t = os.path.getmtime(LIB_PATH)
-    deps = [os.path.join(_CSRC, f) for f in os.listdir(_CSRC)] + [
+    deps = [os.path.join(_CSRC, f) for f in os.listdir(_CSRC) if not f.endswith(".cpp")] + [
         os.path.join(os.path.dirname(_PKG_DIR), "include", "jvpattn.h")]
     return any(os.path.getmtime(d) > t for d in deps if os.path.isfile(d))
 
@@ -91,6 +92,35 @@ def build(force: bool = False, verbose: bool = False) -> str:
     if verbose:
         print(proc.stderr)
     return LIB_PATH
+
+
+def native_built() -> bool:
+    return os.path.exists(NATIVE_PATH)
+
+
+def build_native(force: bool = False) -> str:
+    """Compile ``_native.so`` against the installed torch and ``libjvpattn.so`` (host code only)."""
+    import sysconfig
+
+    import torch
+    from torch.utils import cpp_extension
+
+    src = os.path.join(_CSRC, "torch_nodes.cpp")
+    deps = [src, os.path.join(os.path.dirname(_PKG_DIR), "include", "jvpattn.h")]
+    if not force and native_built() and all(os.path.getmtime(d) <= os.path.getmtime(NATIVE_PATH) for d in deps):
+        return NATIVE_PATH
+    build()
+    cuda = os.path.dirname(os.path.dirname(shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"))
+    includes = [*cpp_extension.include_paths(), os.path.join(cuda, "include"), sysconfig.get_paths()["include"]]
+    cmd = [shutil.which("g++") or "g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-DTORCH_EXTENSION_NAME=_native",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *[f"-I{d}" for d in includes],
+           "-o", NATIVE_PATH + ".tmp", src, *[f"-L{d}" for d in cpp_extension.library_paths()], f"-L{_PKG_DIR}",
+           "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python", "-lc10", "-lc10_cuda", "-l:libjvpattn.so", "-Wl,-rpath,$ORIGIN"]
+    proc = subprocess.run(cmd, capture_output=True, text=True)
+    if proc.returncode != 0:
+        raise RuntimeError("g++ failed:\n" + proc.stdout + proc.stderr)
+    os.replace(NATIVE_PATH + ".tmp", NATIVE_PATH)
+    return NATIVE_PATH
 
 
 _lib = None

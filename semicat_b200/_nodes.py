@@ -3,6 +3,7 @@ host: a node with ``setup_context`` has its ``forward`` inspected on every call 
 130 us, measured in a sampling pass of the twelve-block denoiser, which makes 73 such calls)."""
 from __future__ import annotations
 
+import importlib
 import inspect
 
 import torch
@@ -27,3 +28,39 @@ def unrecorded() -> bool:
 def apply(cls, *args):
     """``cls.apply(*args)`` for a node whose ``forward`` takes no context, without the node where none can be recorded."""
     return cls.forward(*args) if unrecorded() else cls.apply(*args)
+
+
+_module = None
+
+
+def _load():
+    global _module
+    from . import _lib, functional
+
+    _lib.load()  # says how to build what is missing
+    if not _lib.native_built():
+        raise RuntimeError(f"{_lib.NATIVE_PATH} is missing: build it with `python -c 'import __graft_entry__ as g; g.build()'`")
+    mod = importlib.import_module("semicat_b200._native")
+    mod.set_kernels(functional._kernels)
+    _module = mod
+    return mod
+
+
+def set_kernels(kind: int) -> None:
+    if _module is not None:
+        _module.set_kernels(kind)
+
+
+def native(name: str, first: torch.Tensor, *args):
+    """Op ``name`` of ``csrc/torch_nodes.cpp`` on these arguments, or ``None`` where the situation or the inputs are none of
+    its own: outside all function transforms, or inside one ``torch.func.jvp`` and nothing else, on plain CUDA tensors.
+    (One attention call under ``torch.func.jvp`` with its gradients: 780-850 us through the classes here, 230-260 us so; a sampling pass of the
+    twelve-block denoiser 6.7 -> 3.7 ms.)"""
+    if not first.is_cuda or torch.compiler.is_compiling():
+        return None
+    jvp = torch._C._are_functorch_transforms_active()
+    if jvp:
+        levels = torch._C._functorch.get_interpreter_stack()
+        if len(levels) != 1 or levels[0].key() != torch._C._functorch.TransformType.Jvp:
+            return None
+    return getattr(_module or _load(), name)(jvp, first, *args)

@@ -30,7 +30,7 @@ import torch.autograd.forward_ad as fwAD
 import torch.nn.functional as F
 
 from . import _lib
-from ._nodes import apply, node
+from ._nodes import apply, native, node
 from .ops import _on_device
 
 _CODES = {torch.bfloat16: 0, torch.float32: 2}
@@ -228,6 +228,10 @@ def ln_modulate(x: torch.Tensor, norm: torch.nn.LayerNorm, shift: torch.Tensor, 
     """``norm(x) * (1 + scale) + shift`` for ``x`` (B, S, C) and per-sample ``shift`` / ``scale`` ((B, 1, C) or (B, C)).
     The result has the dtype of ``x`` (under autocast the reference computes it in fp32 and the next linear layer rounds
     it to bf16: the same values)."""
+    if norm.weight is not None and norm.normalized_shape == x.shape[-1:]:
+        y = native("ln_modulate", x, norm.weight, norm.bias, shift, scale, norm.eps, exact)
+        if y is not None:
+            return y
     if norm.weight is None or not _usable(x, shift, scale) or tuple(norm.normalized_shape) != (x.shape[-1],):
         return norm(x) * (1.0 + scale) + shift
     beta = norm.bias.float() if norm.bias is not None else None
@@ -360,6 +364,12 @@ def gated_residual(skip: torch.Tensor, branch: torch.Tensor, gate: torch.Tensor,
     """``dropout(branch * gate, p) + skip`` with ``gate`` (B, 1, C) or (B, C).  The dropout keep mask (scaled by
     1 / (1 - p)) is shared by primal, tangent and both backward passes: a tensor drawn here, or, inside
     :func:`dropout_seed`, regenerated by each kernel from the step's seed."""
+    dropped = training and p > 0.0
+    if not dropped or (_Drop.seed is not None and _Drop.seed.device == skip.device):
+        z = native("gated_residual", skip, branch, gate, _Drop.seed if dropped else None, _Drop.calls, float(p))
+        if z is not None:
+            _Drop.calls += dropped
+            return z
     if not _usable(branch, skip, gate) or skip.shape != branch.shape:
         return F.dropout(branch * gate, p, training) + skip
     (xp, tx), (yp, ty), (gp, tg) = (fwAD.unpack_dual(t) for t in (skip, branch, gate))
@@ -422,6 +432,9 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None = No
     """``F.linear`` that keeps primal and tangent in one autograd node under forward-mode AD (weight and bias are
     parameters and carry no tangent where this is used).  Falls back to ``F.linear`` when no tangent is attached or the
     operands' dtypes differ (autocast then does its own casting)."""
+    y = native("linear", x, weight, bias)
+    if y is not None:
+        return y
     xp, tx = fwAD.unpack_dual(x)
     if tx is None or not x.is_cuda or xp.dtype != weight.dtype or (bias is not None and bias.dtype != weight.dtype):
         return F.linear(x, weight, bias)
@@ -495,6 +508,9 @@ class _Gelu(torch.autograd.Function):
 def gelu_tanh(h: torch.Tensor) -> torch.Tensor:
     """``F.gelu(h, approximate="tanh")`` (the MLP of semicat/net/duo.py:118-123) as one kernel for the primal, one for the
     tangent and one per cotangent; fp32 arithmetic, one rounding per output."""
+    y = native("gelu", h)
+    if y is not None:
+        return y
     if not (h.is_cuda and h.dtype in _CODES and h.is_contiguous() and h.numel() % 8 == 0 and (h.storage_offset() * h.element_size()) % 16 == 0):
         return F.gelu(h, approximate="tanh")
     hp, th = fwAD.unpack_dual(h)

@@ -36,7 +36,8 @@ import torch.autograd.forward_ad as fwAD
 from torch.autograd.function import once_differentiable
 
 from . import ops
-from ._nodes import node, unrecorded
+from . import _nodes
+from ._nodes import native, node, unrecorded
 
 __all__ = ["sdpa_jvp", "safe_sdpa_jvp", "set_kernel_family"]
 
@@ -47,6 +48,7 @@ def set_kernel_family(kind: int) -> int:
     """Force a kernel family for subsequent calls (``ops.KERNELS_*``); returns the previous setting."""
     global _kernels
     prev, _kernels = _kernels, int(kind)
+    _nodes.set_kernels(_kernels)
     return prev
 
 
@@ -158,6 +160,9 @@ def sdpa_jvp(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor) -> torch.Tensor:
     plain attention through the primal-only kernels, differentiable in reverse mode (the reference returns an
     uninitialised buffer in that case, functional.py:286-287).
     """
+    y = native("attention", q, k, v, False)
+    if y is not None:
+        return y
     _validate(q, k, v)
     (qp, tq), (kp, tk), (vp, tv) = (fwAD.unpack_dual(t) for t in (q, k, v))
     if tq is None and tk is None and tv is None:
@@ -173,6 +178,9 @@ def sdpa_jvp(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor) -> torch.Tensor:
 def safe_sdpa_jvp(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor) -> torch.Tensor:
     """(B, S, H, D) wrapper around :func:`sdpa_jvp` that casts non-half inputs to bfloat16 and the result
     back to the caller's dtype (keyed on ``q.dtype`` alone, like the reference)."""
+    y = native("attention", q, k, v, True)
+    if y is not None:
+        return y
     orig = q.dtype
     if orig not in (torch.bfloat16, torch.float16):
         q, k, v = q.to(torch.bfloat16), k.to(torch.bfloat16), v.to(torch.bfloat16)

@@ -17,7 +17,7 @@ import torch
 import torch.autograd.forward_ad as fwAD
 
 from . import _lib
-from ._nodes import apply, node
+from ._nodes import apply, native, node
 from .ops import _on_device
 
 _CODES = {torch.bfloat16: 0, torch.float16: 1, torch.float32: 2}
@@ -164,6 +164,10 @@ def rotary_qkv(qkv: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, out_dtyp
     as by :func:`apply_rotary_cast`, in one launch; the backward writes the projection's gradient in place in one launch
     (instead of three tensors that are concatenated afterwards).  Works under forward-mode AD.  Inputs the kernel does not
     take (fp16, unaligned views) go through :func:`apply_rotary_cast` per tensor."""
+    if out_dtype in _QKV_CODES:
+        out = native("rotary_qkv", qkv, cos, sin, out_dtype == torch.bfloat16)
+        if out is not None:
+            return out
     p, t = fwAD.unpack_dual(qkv)
     ok = (p.is_cuda and p.dim() == 5 and p.shape[2] == 3 and p.dtype in _QKV_CODES and out_dtype in _QKV_CODES and p.shape[-1] % 16 == 0
           and p.stride(4) == 1 and all(st % 8 == 0 for st in p.stride()[:4]) and (p.storage_offset() * p.element_size()) % 16 == 0)
