@@ -691,6 +691,7 @@ def main():
             "row_dots_kernel": (4 * T + 2 * stat, 0),
             "sm100_bwd_kernel<query owner>": (10 * T + 4 * stat, 9),
             "sm100_bwd_kernel<key owner>": (12 * T + 4 * stat, 12),
+            "sm100_bwd_short_kernel": (14 * T + 2 * stat, 15),
         }
         with sampler:
             prof = run_profile(sets, max(8, min(args.steps, 40)))

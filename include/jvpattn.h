@@ -276,7 +276,7 @@ uint64_t jvpattn_launch_count(void);
  * triton.testing.do_bench around whole calls, ryu_triton.py:958-1007).  Between _begin and _end every
  * launch is bracketed by CUDA events on its stream; _end synchronises the device and returns, per kernel
  * id in [0, JVPATTN_NUM_KERNELS), the summed device time in milliseconds and the launch count. */
-#define JVPATTN_NUM_KERNELS 9
+#define JVPATTN_NUM_KERNELS 10
 int jvpattn_profile_begin(void);
 int jvpattn_profile_end(double *total_ms, uint64_t *launches);
 const char *jvpattn_kernel_name(int id);

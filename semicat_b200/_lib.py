@@ -17,7 +17,8 @@ _CSRC = os.path.join(_PKG_DIR, "csrc")
 LIB_PATH = os.path.join(_PKG_DIR, "libjvpattn.so")
 NATIVE_PATH = os.path.join(_PKG_DIR, "_native.so")  # the autograd nodes, see csrc/torch_nodes.cpp
 SOURCES = ["jvpattn_api.cu", "jvpattn_simt.cu", "jvpattn_sm100_fwd.cu", "jvpattn_sm100_bwd.cu",
-           "sm100_tensormap.cu", "rotary.cu", "dual_pointwise.cu", "vocab_head.cu", "vocab_loss.cu"]
+           "jvpattn_sm100_bwd_short.cu", "sm100_tensormap.cu", "rotary.cu", "dual_pointwise.cu", "vocab_head.cu",
+           "vocab_loss.cu"]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
     "-Xcompiler", "-fPIC", "-shared",
@@ -36,7 +37,7 @@ EXPORTS = (
 )
 DEBUG_WAIT_CYCLES, DEBUG_STALL_NEXT_FWD = 0, 1
 STATIC_SCRATCH_ROWS = 262144
-NUM_KERNELS = 9
+NUM_KERNELS = 10
 
 
 class Dropout(ctypes.Structure):

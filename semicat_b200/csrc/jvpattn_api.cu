@@ -453,6 +453,7 @@ const char *jvpattn_kernel_name(int id) {
     case kIdBwdKeySimt: return "simt_bwd_kv_kernel";
     case kIdRotary: return "rotary_cast_kernel";
     case kIdDual: return "dual_pointwise_kernels";
+    case kIdBwdShortTc: return "sm100_bwd_short_kernel";
     default: return "?";
   }
 }

@@ -1233,6 +1233,7 @@ cudaError_t dispatch_bwd(const BwdArgs &a, cudaStream_t stream) {
 }
 
 cudaError_t sm100_bwd(const BwdArgs &a, cudaStream_t stream) {
+  if (sm100_bwd_short_ok(a)) return sm100_bwd_short(a, stream);
   return a.g_to.ptr ? dispatch_bwd<true>(a, stream) : dispatch_bwd<false>(a, stream);
 }
 
