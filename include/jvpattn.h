@@ -219,6 +219,17 @@ int jvpattn_gated_residual_dual(int which, const void *x, const void *tx, const 
                                 const void *gz, const void *gtz, void *d_y, void *d_ty, float *sums, int batch, int len,
                                 int channels, int dtype, const jvpattn_dropout *drop, void *stream);
 
+/* 16-bit copies of fp32 matrices (rows, cols), contiguous, in one launch per 64 of them: dst (rows_out, cols_out) = scale * src,
+ * zero beyond rows and cols.  dtype: JVPATTN_BF16 or JVPATTN_FP16.  dst 16-byte aligned; where rows_out or cols_out differ from
+ * rows and cols, they must not be smaller and cols_out must be a multiple of 8 (else JVPATTN_EINVAL). */
+typedef struct jvpattn_cast {
+  const float *src;
+  void *dst;
+  int32_t rows, cols, rows_out, cols_out;
+  float scale;
+} jvpattn_cast;
+int jvpattn_cast_params(const jvpattn_cast *entries, int n, int dtype, void *stream);
+
 /* Turns the column sums that jvpattn_ln_modulate's backward kernels leave (sums_y: which = 2, (2, batch, channels);
  * sums_ty: which = 3, (3, batch, channels); either may be NULL) into the gradients of shift, scale, their tangents
  * ((batch, channels) contiguous in `dtype`; NULL = not wanted) and of the LayerNorm weight and bias (fp32 (channels),

@@ -51,6 +51,11 @@ def set_kernels(kind: int) -> None:
         _module.set_kernels(kind)
 
 
+def module():
+    """The compiled module (loaded on first use; CUDA only)."""
+    return _module or _load()
+
+
 def native(name: str, first: torch.Tensor, *args):
     """Op ``name`` of ``csrc/torch_nodes.cpp`` on these arguments, or ``None`` where the situation or the inputs are none of
     its own: outside all function transforms, or inside one ``torch.func.jvp`` and nothing else, on plain CUDA tensors.

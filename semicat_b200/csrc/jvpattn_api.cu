@@ -336,6 +336,21 @@ int jvpattn_gelu_dual(int mode, const void *h, const void *v, const void *w, con
   return note_cuda(gelu_dual(mode, h, v, w, u, out, out2, n, dtype, static_cast<cudaStream_t>(stream)));
 }
 
+int jvpattn_cast_params(const jvpattn_cast *entries, int n, int dtype, void *stream) {
+  if (n < 0 || (n > 0 && !entries) || (dtype != JVPATTN_BF16 && dtype != JVPATTN_FP16)) return JVPATTN_EINVAL;
+  for (int i = 0; i < n; ++i) {
+    const jvpattn_cast &e = entries[i];
+    if (e.rows < 0 || e.cols < 0 || e.rows_out < e.rows || e.cols_out < e.cols) return JVPATTN_EINVAL;
+    if ((e.rows_out != e.rows || e.cols_out != e.cols) && e.cols_out % 8) return JVPATTN_EINVAL;
+    if ((int64_t)e.rows_out * e.cols_out == 0) continue;
+    if (!e.dst || (!e.src && (int64_t)e.rows * e.cols > 0)) return JVPATTN_EINVAL;
+    if (reinterpret_cast<uintptr_t>(e.dst) % 16 || reinterpret_cast<uintptr_t>(e.src) % 4) return JVPATTN_EALIGN;
+  }
+  DeviceInfo *d = nullptr;
+  if (int rc = current_device(&d)) return rc;
+  return note_cuda(cast_params(entries, n, dtype, static_cast<cudaStream_t>(stream)));
+}
+
 int jvpattn_ln_finalize(const float *sums_y, const float *sums_ty, const float *gamma, const float *beta, const void *scale,
                         const void *tscale, int64_t mod_stride, int64_t tmod_stride, void *d_shift, void *d_scale, void *d_tshift,
                         void *d_tscale, float *d_gamma, float *d_beta, int batch, int channels, int dtype, void *stream) {

@@ -90,6 +90,9 @@ cudaError_t gated_residual_dual(int which, const void *x, const void *tx, const 
 cudaError_t gelu_dual(int mode, const void *h, const void *v, const void *w, const void *u, void *out, void *out2, int64_t n,
                       int dtype, cudaStream_t stream);
 
+// cast_params.cu: 16-bit copies of parameters
+cudaError_t cast_params(const jvpattn_cast *entries, int n, int dtype, cudaStream_t stream);
+
 // vocab_loss.cu: interpolation, flow map, cross-entropy and self-distillation loss over the vocabulary axis
 cudaError_t vocab_loss(int op, const void *l, const void *tl, const void *lt, int64_t ld, const float *x0, int64_t ldx,
                        const int64_t *ids, const float *s, const float *t, float *lse, float *stats, float *loss, const float *g,

@@ -940,6 +940,38 @@ py::object rotary_py(bool jvp, py::handle qkv_, py::handle cos_, py::handle sin_
   return py::make_tuple(out[0], out[1], out[2]);
 }
 
+// 16-bit copies of contiguous fp32 CUDA parameters, side by side in one buffer (each from 16 bytes on): of a matrix as it is, or
+// (`align`) with rows and columns padded to multiples of 8; times `scale`.  None where they are not all of that kind.
+py::object cast_params(const std::vector<Tensor> &params, const std::vector<double> &scale, const std::vector<bool> &align, bool bf16) {
+  if (params.empty() || scale.size() != params.size() || align.size() != params.size()) return py::none();
+  const Tensor &p0 = params[0];
+  std::vector<jvpattn_cast> e(params.size());
+  std::vector<int64_t> offset(params.size());
+  int64_t total = 0;
+  for (size_t i = 0; i < params.size(); ++i) {
+    const Tensor &p = params[i];
+    if (!p.is_cuda() || p.device() != p0.device() || p.layout() != at::kStrided || p.scalar_type() != at::kFloat || p.dim() < 1 || p.dim() > 2 ||
+        !p.is_contiguous() || p.key_set().has(c10::DispatchKey::Python) || p.size(0) > INT32_MAX - 8 || p.size(-1) > INT32_MAX - 8)
+      return py::none();
+    const int64_t rows = p.dim() == 2 ? p.size(0) : 1, cols = p.size(-1);
+    const auto up = [&](int64_t n) { return align[i] ? (n + 7) / 8 * 8 : n; };
+    e[i] = {p.data_ptr<float>(), nullptr, (int32_t)rows, (int32_t)cols, (int32_t)(p.dim() == 2 ? up(rows) : 1), (int32_t)up(cols), (float)scale[i]};
+    offset[i] = total;
+    total += ((int64_t)e[i].rows_out * e[i].cols_out + 7) / 8 * 8;
+  }
+  c10::cuda::CUDAGuard guard(p0.device());
+  at::AutoDispatchBelowADInplaceOrView below;
+  const Tensor flat = at::empty({total}, p0.options().dtype(bf16 ? at::kBFloat16 : at::kHalf));
+  std::vector<Tensor> out(params.size());
+  for (size_t i = 0; i < params.size(); ++i) {
+    e[i].dst = static_cast<char *>(flat.data_ptr()) + 2 * offset[i];
+    out[i] = params[i].dim() == 2 ? flat.as_strided({e[i].rows_out, e[i].cols_out}, {e[i].cols_out, 1}, offset[i])
+                                  : flat.as_strided({e[i].cols_out}, {1}, offset[i]);
+  }
+  check(jvpattn_cast_params(e.data(), (int)e.size(), bf16 ? JVPATTN_BF16 : JVPATTN_FP16, stream_of(p0)), "jvpattn_cast_params");
+  return py::cast(out);
+}
+
 }  // namespace
 
 PYBIND11_MODULE(_native, m) {
@@ -951,6 +983,7 @@ PYBIND11_MODULE(_native, m) {
     }
   });
   m.def("set_kernels", [](int kind) { g_kernels.store(kind); });
+  m.def("cast_params", cast_params);
   m.def("attention", attention_py);
   m.def("ln_modulate", ln_py);
   m.def("gated_residual", gate_py);

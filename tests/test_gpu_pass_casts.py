@@ -1,0 +1,60 @@
+"""16-bit copies of a model's parameters in one launch: bit for bit what ``Tensor.to`` and zero padding give, over vectors and
+matrices whose sizes are no multiple of anything, and the denoiser's pass that uses them against the one that does not."""
+import pytest
+import torch
+
+from semicat_b200 import _lib, _nodes, train_step, vocab_ops
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_copies(dtype):
+    g = torch.Generator(device="cuda").manual_seed(0)
+    base = torch.randn(4099, device="cuda", generator=g)
+    shapes = [(1,), (7,), (8,), (4608,), (1, 1), (3, 5), (9, 16), (768, 1003), (30, 30522), (33, 8200), (0,), (5, 0)] + [(17, 24)] * 60
+    params = [torch.randn(s, device="cuda", generator=g) * 3 for s in shapes] + [base[3:4000], base[2:4098]]  # and off the 16-byte grid
+    for align in (False, True):
+        flags, scale = [align] * len(params), [1.0 + 0.37 * (i % 3) for i in range(len(params))]
+        out = _nodes.module().cast_params(params, scale, flags, dtype == torch.bfloat16)
+        for p, s, o in zip(params, scale, out):
+            want = (p * s).to(dtype)
+            pad = [(-n) % 8 if align else 0 for n in (p.shape if p.dim() == 2 else (1, *p.shape))]
+            want = torch.nn.functional.pad(want, (0, pad[1], 0, pad[0]) if p.dim() == 2 else (0, pad[1]))
+            assert o.shape == want.shape and o.dtype == dtype and o.data_ptr() % 16 == 0 and torch.equal(o, want)
+    assert _nodes.module().cast_params([base.half()], [1.0], [False], True) is None
+    assert _nodes.module().cast_params([torch.ones(4, 4, device="cuda").t()[:2]], [1.0], [False], True) is None
+    assert _lib.device_status() == 0
+
+
+@pytest.mark.parametrize("V,B,L,dtype", [(1003, 3, 40, torch.bfloat16), (1024, 2, 64, torch.bfloat16), (27, 2, 33, torch.bfloat16), (1003, 2, 40, torch.float16)])
+@pytest.mark.parametrize("attention", ["lib", "sdpa"])
+def test_pass(monkeypatch, V, B, L, dtype, attention):
+    torch.manual_seed(0)
+    with torch.device("cuda"):
+        net = train_step.DiT(V, 256, 64, 3, 4, dropout=0.0, length=L, embed_type="rms" if V < 512 else "naive")
+    train_step.randomise_zero_init(net)
+    net.eval()
+    x1 = torch.randint(0, V, (B, L), device="cuda")
+    noise = train_step.draw_noise(x1, V)
+    s, t = noise["u_sd"] * noise["t_sd"], noise["t_sd"]
+    plain = train_step.interpolate(noise["x0"], x1, s.view(-1, 1, 1))
+    inputs = [plain] if V < 512 or dtype == torch.float16 else [plain, vocab_ops.interpolate_cast(noise["x0"], x1, s)]
+    used = []
+    of = train_step._PassCasts.of
+    for x in inputs:
+        out = []
+        for way in (lambda *a: (used.append(of(*a)), used[-1])[1], lambda *a: None):
+            monkeypatch.setattr(train_step._PassCasts, "of", staticmethod(way))
+            with torch.no_grad(), torch.autocast("cuda", dtype=dtype):
+                out.append(net(x, s, t, attention=attention, padded_logits=True))
+        # the modulation comes from another GEMM (16-bit results, 64 terms): half a unit of 2^-8 now and then, through three blocks
+        assert out[0].shape == out[1].shape and out[0].dtype == out[1].dtype
+        assert float((out[0] - out[1]).float().norm() / out[1].float().norm()) < 2 ** -8
+    assert all(u is not None for u in used)
+    with torch.autocast("cuda", dtype=dtype):  # gradients may be wanted: not for this pass
+        assert of(net, plain, attention) is None
+    with torch.no_grad():
+        assert of(net, plain, attention) is None
+        with torch.autocast("cuda", dtype=dtype):
+            assert of(net.half(), plain, attention) is None
