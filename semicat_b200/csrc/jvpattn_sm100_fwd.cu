@@ -203,17 +203,23 @@ __global__ void __launch_bounds__(kThreads, fwd_ctas_per_sm(D, kHasT)) sm100_fwd
 #pragma unroll
           for (int kk = 0; kk < D / 16; ++kk) mma_ss_lo(sc + 64, qd(offsetof(Smem, tq), kk), kd(kk), idesc_s, true);
         }
-        tc_commit(&s.s_full[alt(j)]);
-        tc_commit(&s.k_empty[st]);
         return true;
+      };
+      auto commit_scores = [&](int j) {
+        tc_commit(&s.s_full[alt(j)]);
+        tc_commit(&s.k_empty[j % kStages]);
       };
       bool ok = mbar_wait_for(a.wait_cycles, &s.q_full, 0);
       if (!ok) atomicCAS(a.status, 0u, 102u);
-      if (ok && kAlternate) ok = scores(0);
+      if (ok) ok = scores(0);
+      if (ok) commit_scores(0);
       for (int j = 0; ok && j < ntiles; ++j) {
         const int st = j % kStages;
-        // (the region of tile j + 1 was the operand of the value products of tile j - 1, which are ahead in the queue)
-        if (kAlternate ? (j + 1 < ntiles && !scores(j + 1)) : !scores(j)) break;
+        if (kAlternate && j + 1 < ntiles) {
+          // (the region of tile j + 1 was the operand of the value products of tile j - 1, which are ahead in the queue)
+          if (!scores(j + 1)) break;
+          commit_scores(j + 1);
+        }
         if (!mbar_wait_for(a.wait_cycles, &s.p_full[alt(j)], alt_parity(j)) ||
             !mbar_wait_for(a.wait_cycles, &s.v_full[st], (j / kStages) & 1)) {
           atomicCAS(a.status, 0u, 104u);
@@ -241,6 +247,14 @@ __global__ void __launch_bounds__(kThreads, fwd_ctas_per_sm(D, kHasT)) sm100_fwd
             mma_ts_lo(tmem + kColO, pcol + 8 * kk, dv, idesc_p, acc);              // [O | Od'] += P [V | Vd]
             if (kHasT) mma_ts_lo(tmem + kColOd, ucol + 8 * kk, dv, idesc_o, true);  // Od' += U V
           }
+        }
+        if (!kAlternate && j + 1 < ntiles) {
+          // Behind the value products, whose operands lie in the same region.  A commit holds this thread until what it has queued is
+          // over, so one drain serves both: 128 heads of 64 channels at length 2048 377 -> 364 us, 16 x 16 of length 512 73.6 -> 71.1.
+          // (At head_dim 128 the value products' stage would be released too late: 596 -> 816 us.  Starting the two CTAs of an
+          // SM half a tile apart, or two softmax threads per row at 96 registers, is slower here.)
+          if (!scores(j + 1)) break;
+          commit_scores(j + 1);
         }
         tc_commit(&s.v_empty[st]);
         tc_commit(&s.o_done[alt(j)]);
