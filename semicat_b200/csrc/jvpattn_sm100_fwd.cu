@@ -257,7 +257,7 @@ __global__ void __launch_bounds__(kThreads, fwd_ctas_per_sm(D, kHasT)) sm100_fwd
           commit_scores(j + 1);
         }
         tc_commit(&s.v_empty[st]);
-        tc_commit(&s.o_done[alt(j)]);
+        tc_commit(&s.o_done[j & 1]);
       }
     }
   } else {
@@ -313,7 +313,7 @@ __global__ void __launch_bounds__(kThreads, fwd_ctas_per_sm(D, kHasT)) sm100_fwd
         // S of this tile is complete, so every earlier O / Od' update has retired (kAlternate: all but the last one, which
         // was issued behind S of this tile): safe to rescale in place.
         if (kAlternate) {
-          if (!__all_sync(0xffffffffu, mbar_wait_for(a.wait_cycles, &s.o_done[alt(j - 1)], alt_parity(j - 1)))) {
+          if (!__all_sync(0xffffffffu, mbar_wait_for(a.wait_cycles, &s.o_done[(j - 1) & 1], ((j - 1) >> 1) & 1))) {
             atomicCAS(a.status, 0u, 107u);
             ok = false;
             break;
@@ -390,11 +390,12 @@ __global__ void __launch_bounds__(kThreads, fwd_ctas_per_sm(D, kHasT)) sm100_fwd
       mbar_arrive(&s.p_full[alt(j)]);
     }
     // ---- epilogue: O = acc / l ; Od = Od'/l - (mu/l) O ; statistics
-    // (kAlternate: the last two value products may both be outstanding here, or neither.  With one barrier a wait for the last
-    // could take the phase before it for its own, and a wait for that one first could find both over and never return.
-    // With two, the phase before the last tile's on its barrier is that of two tiles earlier, complete before the scores of
-    // the last tile, and none follows it: one wait, and it covers every product issued before.)
-    if (ok && !__all_sync(0xffffffffu, mbar_wait_for(a.wait_cycles, &s.o_done[alt(ntiles - 1)], alt_parity(ntiles - 1)))) {
+    // (The last two value products may both be outstanding here, or neither; where they are not, the arrivals of the first and of the
+    // scores behind it come in no order.  With one barrier a wait for the last could take the phase before it for its own, and
+    // a wait for that one first could find both over and never return.  With two, the phase before the last tile's on its
+    // barrier is that of two tiles earlier, complete before the scores of the last tile were issued, and none follows it: one wait,
+    // and it covers every product issued before.)
+    if (ok && !__all_sync(0xffffffffu, mbar_wait_for(a.wait_cycles, &s.o_done[(ntiles - 1) & 1], ((ntiles - 1) >> 1) & 1))) {
       atomicCAS(a.status, 0u, 106u);
       ok = false;
     }
