@@ -219,6 +219,13 @@ int jvpattn_gated_residual_dual(int which, const void *x, const void *tx, const 
                                 const void *gz, const void *gtz, void *d_y, void *d_ty, float *sums, int batch, int len,
                                 int channels, int dtype, const jvpattn_dropout *drop, void *stream);
 
+/* jvpattn_gated_residual without a mask and jvpattn_ln_modulate (which = 0) of its result in one launch: z = x + gate y,
+ * h = LayerNorm(z) (1 + scale) + shift, for passes without a backward (no statistics are kept).  Shapes and types as there;
+ * every pointer 16-byte aligned (else JVPATTN_EALIGN). */
+int jvpattn_gate_ln(const void *x, const void *y, const void *gate, int64_t gate_stride, const float *gamma, const float *beta,
+                    const void *shift, const void *scale, int64_t mod_stride, void *z, void *h, int batch, int len, int channels, float eps,
+                    int dtype, void *stream);
+
 /* 16-bit copies of fp32 matrices (rows, cols), contiguous, in one launch per 64 of them: dst (rows_out, cols_out) = scale * src,
  * zero beyond rows and cols.  dtype: JVPATTN_BF16 or JVPATTN_FP16.  dst 16-byte aligned; where rows_out or cols_out differ from
  * rows and cols, they must not be smaller and cols_out must be a multiple of 8 (else JVPATTN_EINVAL). */

@@ -33,7 +33,7 @@ EXPORTS = (
     "jvpattn_abi_version", "jvpattn_profile_begin", "jvpattn_profile_end", "jvpattn_kernel_name",
     "jvpattn_bwd_static", "jvpattn_rotary_cast", "jvpattn_stream_check", "jvpattn_debug_set",
     "jvpattn_ln_modulate", "jvpattn_ln_modulate_dual", "jvpattn_gated_residual", "jvpattn_flow_map_head", "jvpattn_gelu_dual", "jvpattn_vocab_op",
-    "jvpattn_gated_residual_dual", "jvpattn_ln_finalize", "jvpattn_rotary_qkv", "jvpattn_cast_params",
+    "jvpattn_gated_residual_dual", "jvpattn_ln_finalize", "jvpattn_rotary_qkv", "jvpattn_cast_params", "jvpattn_gate_ln",
 )
 DEBUG_WAIT_CYCLES, DEBUG_STALL_NEXT_FWD = 0, 1
 STATIC_SCRATCH_ROWS = 262144

@@ -680,6 +680,74 @@ __global__ void __launch_bounds__(256) gated_residual_fwd_kernel(GateArgs a) {
   }
 }
 
+// z = x + gate y and h = LN(z) (1 + scale) + shift in one pass, for passes in which nothing is recorded: the residual behind a branch
+// and the LayerNorm in front of the next, with z rounded to its type before the LayerNorm as between the two kernels.  A warp
+// per row; bound by launches where it is used (a sampling pass has few rows): one instead of two, and z is not read back.
+struct GateLnArgs {
+  const void *x, *y, *gate;
+  int64_t gate_stride;
+  const float *gamma, *beta;
+  const void *shift, *scale;
+  int64_t mod_stride;
+  void *z, *h;
+  int B, S;
+  float eps;
+};
+
+template <typename T, int NV>
+__global__ void __launch_bounds__(kWarpsPerCta * 32) gate_ln_fwd_kernel(GateLnArgs a) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int64_t row = (int64_t)blockIdx.x * kWarpsPerCta + warp;
+  if (row >= (int64_t)a.B * a.S) return;
+  const int64_t b = row / a.S;
+  constexpr int C = NV * 256;
+  Raw8<T> rx[NV], ry[NV], rg[NV];
+#pragma unroll
+  for (int v = 0; v < NV; ++v) {
+    rx[v] = load_raw8(static_cast<const T *>(a.x) + row * C + chan(v, lane));
+    ry[v] = load_raw8(static_cast<const T *>(a.y) + row * C + chan(v, lane));
+    rg[v] = load_raw8(static_cast<const T *>(a.gate) + b * a.gate_stride + chan(v, lane));
+  }
+  float z[NV][8], s = 0.f;
+#pragma unroll
+  for (int v = 0; v < NV; ++v) {
+    float y[8], g[8];
+    unpack8(rx[v], z[v]), unpack8(ry[v], y), unpack8(rg[v], g);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      z[v][i] += g[i] * y[i];
+      if constexpr (sizeof(T) == 2) z[v][i] = __bfloat162float(__float2bfloat16_rn(z[v][i]));
+      s += z[v][i];
+    }
+    store8<T>(static_cast<T *>(a.z) + row * C + chan(v, lane), z[v]);
+  }
+  const float mean = warp_sum(s) / C;
+  float q = 0.f;
+#pragma unroll
+  for (int v = 0; v < NV; ++v)
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const float d = z[v][i] - mean;
+      q += d * d;
+    }
+  const float rstd = rsqrtf(warp_sum(q) / C + a.eps);
+#pragma unroll
+  for (int v = 0; v < NV; ++v) {
+    const int c0 = chan(v, lane);
+    float g[8], be[8], scv[8], shv[8], out[8];
+    load8<float>(a.gamma + c0, g);
+    if (a.beta) load8<float>(a.beta + c0, be);
+    load8<T>(static_cast<const T *>(a.scale) + b * a.mod_stride + c0, scv);
+    load8<T>(static_cast<const T *>(a.shift) + b * a.mod_stride + c0, shv);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const float ln = (z[v][i] - mean) * rstd * g[i] + (a.beta ? be[i] : 0.f);
+      out[i] = ln * (1.f + scv[i]) + shv[i];
+    }
+    store8<T>(static_cast<T *>(a.h) + row * C + c0, out);
+  }
+}
+
 // Rows of one sample that a CTA of the backward kernels walks before it adds its column sums to global memory.  Every CTA
 // costs one atomic per column and sum, and at a few hundred samples those atomics (millions per launch, a dozen
 // contenders per address) took longer than the rows themselves; so the count grows with the problem as long as
@@ -1008,6 +1076,18 @@ cudaError_t gated_residual(const void *x, const void *y, const void *gate, const
   if (dtype == JVPATTN_BF16) return launch(__nv_bfloat16{});
   if (dtype == JVPATTN_FP32) return launch(float{});
   return cudaErrorInvalidValue;
+}
+
+cudaError_t gate_ln(const void *x, const void *y, const void *gate, int64_t gate_stride, const float *gamma, const float *beta, const void *shift,
+                    const void *scale, int64_t mod_stride, void *z, void *h, int B, int S, int C, float eps, int dtype, cudaStream_t stream) {
+  const int64_t rows = (int64_t)B * S;
+  if (rows == 0) return cudaSuccess;
+  const GateLnArgs a{x, y, gate, gate_stride, gamma, beta, shift, scale, mod_stride, z, h, B, S, eps};
+  LaunchScope scope(kIdDual, stream);
+  return dispatch(dtype, C, [&](auto t, auto nv) -> cudaError_t {
+    gate_ln_fwd_kernel<decltype(t), decltype(nv)::value><<<(unsigned)((rows + kWarpsPerCta - 1) / kWarpsPerCta), kWarpsPerCta * 32, 0, stream>>>(a);
+    return cudaGetLastError();
+  });
 }
 
 cudaError_t ln_finalize(const float *p, const float *t, const float *gamma, const float *beta, const void *scale,

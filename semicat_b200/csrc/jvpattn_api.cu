@@ -336,6 +336,21 @@ int jvpattn_gelu_dual(int mode, const void *h, const void *v, const void *w, con
   return note_cuda(gelu_dual(mode, h, v, w, u, out, out2, n, dtype, static_cast<cudaStream_t>(stream)));
 }
 
+int jvpattn_gate_ln(const void *x, const void *y, const void *gate, int64_t gate_stride, const float *gamma, const float *beta,
+                    const void *shift, const void *scale, int64_t mod_stride, void *z, void *h, int batch, int len, int channels, float eps,
+                    int dtype, void *stream) {
+  if (!dual_shape_ok(batch, len, channels) || (dtype != JVPATTN_BF16 && dtype != JVPATTN_FP32)) return JVPATTN_EINVAL;
+  DeviceInfo *d = nullptr;
+  if (int rc = current_device(&d)) return rc;
+  if ((int64_t)batch * len == 0) return JVPATTN_OK;
+  if (!x || !y || !gate || !gamma || !shift || !scale || !z || !h) return JVPATTN_EINVAL;
+  for (const void *p : {x, y, gate, (const void *)gamma, (const void *)beta, shift, scale, (const void *)z, (const void *)h})
+    if (p && reinterpret_cast<uintptr_t>(p) % 16) return JVPATTN_EALIGN;
+  if (gate_stride % 8 || mod_stride % 8) return JVPATTN_EALIGN;
+  return note_cuda(gate_ln(x, y, gate, gate_stride, gamma, beta, shift, scale, mod_stride, z, h, batch, len, channels, eps, dtype,
+                           static_cast<cudaStream_t>(stream)));
+}
+
 int jvpattn_cast_params(const jvpattn_cast *entries, int n, int dtype, void *stream) {
   if (n < 0 || (n > 0 && !entries) || (dtype != JVPATTN_BF16 && dtype != JVPATTN_FP16)) return JVPATTN_EINVAL;
   for (int i = 0; i < n; ++i) {

@@ -80,6 +80,8 @@ cudaError_t ln_modulate_dual(int which, const void *x, const void *tx, const flo
 cudaError_t gated_residual(const void *x, const void *y, const void *gate, const void *mask, int64_t gate_stride, void *z, int B,
                            int S, int C, int dtype, const unsigned long long *drop_seed, unsigned drop_call, float drop_p,
                            cudaStream_t stream);
+cudaError_t gate_ln(const void *x, const void *y, const void *gate, int64_t gate_stride, const float *gamma, const float *beta, const void *shift,
+                    const void *scale, int64_t mod_stride, void *z, void *h, int B, int S, int C, float eps, int dtype, cudaStream_t stream);
 cudaError_t ln_finalize(const float *p, const float *t, const float *gamma, const float *beta, const void *scale,
                         const void *tscale, int64_t mod_stride, int64_t tmod_stride, void *d_shift, void *d_scale, void *d_tshift,
                         void *d_tscale, float *d_gamma, float *d_beta, int B, int C, int dtype, cudaStream_t stream);

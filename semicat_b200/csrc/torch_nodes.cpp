@@ -876,13 +876,14 @@ bool rows_ok(const Tensor &x) {
   return C == 256 || C == 512 || C == 768 || C == 1024;
 }
 
+bool param_ok(const Tensor &p, const Tensor &x) {
+  return p.scalar_type() == at::kFloat && p.dim() == 1 && p.size(0) == x.size(2) && p.is_contiguous() && p.device() == x.device();
+}
+
 py::object ln_py(bool jvp, py::handle x_, py::handle w_, py::handle b_, py::handle shift_, py::handle scale_, double eps, bool exact) {
   const Arg x(x_), w(w_), b(b_), shift(shift_), scale(scale_);
   if (!fits(jvp, {&x, &w, &b, &shift, &scale}) || !rows_ok(x.t) || !modulation_ok(shift.t, x.t) || !modulation_ok(scale.t, x.t)) return py::none();
-  auto param_ok = [&](const Tensor &p) {
-    return p.scalar_type() == at::kFloat && p.dim() == 1 && p.size(0) == x.t.size(2) && p.is_contiguous() && p.device() == x.t.device();
-  };
-  if (!w.t.defined() || !param_ok(w.t) || (b.t.defined() && !param_ok(b.t))) return py::none();
+  if (!w.t.defined() || !param_ok(w.t, x.t) || (b.t.defined() && !param_ok(b.t, x.t))) return py::none();
   if (jvp)
     return py::cast(handle<decltype(ln_jvp)>("jvpattn::ln").call(x.t, w.t, opt(b.t), shift.t, scale.t, eps, exact));
   return py::cast(ln_primal_autograd(x.t, w.t, opt(b.t), shift.t, scale.t, eps, exact));
@@ -895,6 +896,26 @@ py::object gate_py(bool jvp, py::handle x_, py::handle y_, py::handle gate_, py:
     return py::none();
   if (jvp) return py::cast(handle<decltype(gate_jvp)>("jvpattn::gate").call(x.t, y.t, gate.t, opt(seed.t), call, p));
   return py::cast(gate_primal_autograd(x.t, y.t, gate.t, opt(seed.t), call, p));
+}
+
+// gated_residual and ln_modulate of its result, where nothing is recorded: (z, h).
+py::object gate_ln_py(py::handle x_, py::handle y_, py::handle gate_, py::handle w_, py::handle b_, py::handle shift_, py::handle scale_,
+                      double eps) {
+  const Arg x(x_), y(y_), gate(gate_), w(w_), b(b_), shift(shift_), scale(scale_);
+  if (!fits(false, {&x, &y, &gate, &w, &b, &shift, &scale}) || !rows_ok(y.t) || !x.t.defined() || x.t.sizes() != y.t.sizes() ||
+      x.t.scalar_type() != y.t.scalar_type() || x.t.device() != y.t.device() || !modulation_ok(gate.t, y.t) || !modulation_ok(shift.t, y.t) ||
+      !modulation_ok(scale.t, y.t) || !w.t.defined() || !param_ok(w.t, y.t) || (b.t.defined() && !param_ok(b.t, y.t)))
+    return py::none();
+  at::AutoDispatchBelowADInplaceOrView below;
+  c10::cuda::CUDAGuard guard(y.t.device());
+  const Tensor xc = dense(x.t), yc = dense(y.t), g = mod_rows(gate.t);
+  Tensor sh = mod_rows(shift.t), sc = mod_rows(scale.t);
+  equal_pitch(sh, sc);
+  Tensor z = at::empty_like(yc), h = at::empty_like(yc);
+  check(jvpattn_gate_ln(ptr(xc), ptr(yc), ptr(g), pitch(g, {}), fptr(w.t), fptr(b.t), ptr(sh), ptr(sc), pitch(sc, {}), ptr(z), ptr(h),
+                        (int)yc.size(0), (int)yc.size(1), (int)yc.size(2), (float)eps, code(yc), stream_of(yc)),
+        "jvpattn_gate_ln");
+  return py::make_tuple(z, h);
 }
 
 py::object gelu_py(bool jvp, py::handle h_) {
@@ -987,6 +1008,7 @@ PYBIND11_MODULE(_native, m) {
   m.def("attention", attention_py);
   m.def("ln_modulate", ln_py);
   m.def("gated_residual", gate_py);
+  m.def("gate_ln", gate_ln_py);
   m.def("gelu", gelu_py);
   m.def("linear", linear_py);
   m.def("rotary_qkv", rotary_py);

@@ -30,7 +30,7 @@ import torch.autograd.forward_ad as fwAD
 import torch.nn.functional as F
 
 from . import _lib
-from ._nodes import apply, native, node
+from ._nodes import apply, module, native, node, unrecorded
 from .ops import _on_device
 
 _CODES = {torch.bfloat16: 0, torch.float32: 2}
@@ -384,6 +384,17 @@ def gated_residual(skip: torch.Tensor, branch: torch.Tensor, gate: torch.Tensor,
         return apply(_GatedResidual, skip.contiguous(), branch.contiguous(), gate, mask, drop)
     z, tz = _GatedResidualDual.apply(xp.contiguous(), yp.contiguous(), gp, mask, tx, ty, tg, drop)
     return fwAD.make_dual(z, tz)
+
+
+def gated_residual_ln(skip, branch, gate, norm: torch.nn.LayerNorm, shift, scale):
+    """``z = gated_residual(skip, branch, gate)`` and ``ln_modulate(z, norm, shift, scale)``, in one launch where nothing is
+    recorded and the kernel takes the shapes."""
+    if unrecorded() and skip.is_cuda and norm.weight is not None and norm.normalized_shape == skip.shape[-1:]:
+        out = module().gate_ln(skip, branch, gate, norm.weight, norm.bias, shift, scale, norm.eps)
+        if out is not None:
+            return out
+    z = gated_residual(skip, branch, gate)
+    return z, ln_modulate(z, norm, shift, scale)
 
 
 # ----------------------------------------------------------------------------------------------- linear layer

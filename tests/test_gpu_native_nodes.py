@@ -136,6 +136,28 @@ def test_pointwise_chain(monkeypatch, B, S, C, dtype, missing):
     assert _lib.device_status() == 0
 
 
+@pytest.mark.parametrize("B,S,C,dtype", [(3, 5, 256, torch.bfloat16), (2, 50, 768, torch.bfloat16), (2, 9, 512, torch.float32), (1, 1, 1024, torch.bfloat16)])
+@pytest.mark.parametrize("bias", [True, False])
+def test_gated_residual_and_layer_norm_in_one(B, S, C, dtype, bias):
+    """Against the two kernels: z bit for bit, the LayerNorm up to the order of its factors (one rounding of the result)."""
+    norm = torch.nn.LayerNorm(C, device="cuda", bias=bias)
+    with torch.no_grad():
+        norm.weight.normal_()
+    mod = _rand(5, B, 3 * C, dtype=dtype)
+    gate, shift, scale = mod[:, :C], mod[:, C:2 * C], mod[:, 2 * C:]
+    x, y = _rand(1, B, S, C, dtype=dtype), _rand(2, S, B, C, dtype=dtype).transpose(0, 1)
+    with torch.no_grad():
+        before = _lib.launch_count()
+        z, h = dual_ops.gated_residual_ln(x, y, gate, norm, shift, scale)
+        assert _lib.launch_count() - before == 1
+    z2 = dual_ops.gated_residual(x, y, gate)
+    h2 = dual_ops.ln_modulate(z2, norm, shift, scale)
+    assert torch.equal(z, z2) and torch.allclose(h.float(), h2.float(), rtol=2 ** -7 if dtype == torch.bfloat16 else 1e-5, atol=1e-5)
+    a = dual_ops.gated_residual_ln(x.requires_grad_(True), y, gate, norm, shift, scale)  # recorded: the two nodes
+    assert a[0].requires_grad and torch.equal(a[0], z2) and torch.equal(a[1], h2)
+    assert _lib.device_status() == 0
+
+
 def _leaves(seed=0, D=64):
     return [_rand(seed + i, 2, 3, 64, D, scale=0.5).requires_grad_(True) for i in range(6)]
 

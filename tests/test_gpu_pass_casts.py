@@ -41,17 +41,30 @@ def test_pass(monkeypatch, V, B, L, dtype, attention):
     plain = train_step.interpolate(noise["x0"], x1, s.view(-1, 1, 1))
     inputs = [plain] if V < 512 or dtype == torch.float16 else [plain, vocab_ops.interpolate_cast(noise["x0"], x1, s)]
     used = []
-    of = train_step._PassCasts.of
+    of, chained = train_step._PassCasts.of, train_step._PassCasts.chained
     for x in inputs:
         out = []
-        for way in (lambda *a: (used.append(of(*a)), used[-1])[1], lambda *a: None):
+        for way, chain in ((lambda *a: (used.append(of(*a)), used[-1])[1], True), (of, False), (lambda *a: None, False)):
             monkeypatch.setattr(train_step._PassCasts, "of", staticmethod(way))
+            if not chain:
+                monkeypatch.setattr(train_step._PassCasts, "chained", staticmethod(lambda n: False))
             with torch.no_grad(), torch.autocast("cuda", dtype=dtype):
                 out.append(net(x, s, t, attention=attention, padded_logits=True))
+            monkeypatch.setattr(train_step._PassCasts, "chained", staticmethod(chained))
+        assert float((out[0] - out[2]).float().norm() / out[2].float().norm()) < 2 ** -8
         # the modulation comes from another GEMM (16-bit results, 64 terms): half a unit of 2^-8 now and then, through three blocks
         assert out[0].shape == out[1].shape and out[0].dtype == out[1].dtype
         assert float((out[0] - out[1]).float().norm() / out[1].float().norm()) < 2 ** -8
     assert all(u is not None for u in used)
+    # (the blocks as one chain, or one by one where somebody listens or drops out)
+    assert chained(net)
+    handle = net.blocks[1].register_forward_hook(lambda *a: None)
+    assert not chained(net)
+    handle.remove()
+    net.blocks[0].drop.p = 0.5
+    assert chained(net) and not chained(net.train())
+    net.blocks[0].drop.p = 0.0
+    net.eval()
     with torch.autocast("cuda", dtype=dtype):  # gradients may be wanted: not for this pass
         assert of(net, plain, attention) is None
     with torch.no_grad():
