@@ -149,54 +149,66 @@ struct QkvArgs {
 // I: type of the linear thread index, which is taken apart into (tensor, sample, position, head, channels): 32 bits wherever it
 // fits.  The kernel is bound by memory, but five 64-bit divisions per 16 elements were most of its
 // instructions (128 x 128 positions of 3 x 768 channels in bf16: 35.6 -> 30.3 us).
-template <typename TI, typename TO, typename I>
+// A thread takes its channels of q, k and v, which share their place and the angles (24.9 against 30.2 us), or (kSpread) those of
+// the tensor blockIdx.y, where there are too few for that (8 x 128 positions: 3.8 against 4.2 us).
+template <typename TI, typename TO, typename I, bool kSpread>
 __global__ void __launch_bounds__(256) rotary_qkv_kernel(QkvArgs a) {
   const int half = a.D / 2;
   const I per_row = (I)(half / 8), rows = (I)((int64_t)a.B * a.S * a.H);
   const I gid = (I)blockIdx.x * 256 + threadIdx.x;
-  const I rr = gid / per_row;
-  if (rr >= 3 * rows) return;
-  const int t = (int)(rr / rows);
-  const I r = rr - t * rows, bs = r / (I)a.H;
-  const int c0 = (int)(gid - rr * per_row) * 8;
+  const I r = gid / per_row;
+  if (r >= rows) return;
+  const I bs = r / (I)a.H;
+  const int c0 = (int)(gid - r * per_row) * 8;
   const int h = (int)(r - bs * (I)a.H);
   const int b = (int)(bs / (I)a.S);
   const int s = (int)(bs - (I)b * (I)a.S);
-  const TI *xr = static_cast<const TI *>(a.in[t]) + b * a.isb[t] + s * a.iss[t] + h * a.ish[t];
-  TO *yr = static_cast<TO *>(a.out[t]) + b * a.osb[t] + s * a.oss[t] + h * a.osh[t];
-  float x1[8], x2[8], y1[8], y2[8];
-  Vec8<TI>::load(xr + c0, x1);
-  Vec8<TI>::load(xr + half + c0, x2);
-  if (t < 2) {
-    float c[8], sn[8];
+  constexpr int kTensors = kSpread ? 1 : 3;
+  const int t0 = kSpread ? (int)blockIdx.y : 0;
+  float x1[kTensors][8], x2[kTensors][8], c[8], sn[8];
+#pragma unroll
+  for (int k = 0; k < kTensors; ++k) {
+    const int t = t0 + k;
+    const TI *xr = static_cast<const TI *>(a.in[t]) + b * a.isb[t] + s * a.iss[t] + h * a.ish[t];
+    Vec8<TI>::load(xr + c0, x1[k]);
+    Vec8<TI>::load(xr + half + c0, x2[k]);
+  }
+  if (!kSpread || t0 < 2) {
     Vec8<float>::load(a.cosv + (int64_t)s * half + c0, c);
     Vec8<float>::load(a.sinv + (int64_t)s * half + c0, sn);
+  }
+#pragma unroll
+  for (int k = 0; k < kTensors; ++k) {
+    const int t = t0 + k;
+    float y1[8], y2[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-      if (a.transpose) {
-        y1[i] = __fadd_rn(__fmul_rn(x1[i], c[i]), __fmul_rn(x2[i], sn[i]));
-        y2[i] = __fsub_rn(__fmul_rn(x2[i], c[i]), __fmul_rn(x1[i], sn[i]));
+      if (t == 2) {
+        y1[i] = x1[k][i], y2[i] = x2[k][i];
+      } else if (a.transpose) {
+        y1[i] = __fadd_rn(__fmul_rn(x1[k][i], c[i]), __fmul_rn(x2[k][i], sn[i]));
+        y2[i] = __fsub_rn(__fmul_rn(x2[k][i], c[i]), __fmul_rn(x1[k][i], sn[i]));
       } else {
-        y1[i] = __fsub_rn(__fmul_rn(x1[i], c[i]), __fmul_rn(x2[i], sn[i]));
-        y2[i] = __fadd_rn(__fmul_rn(x1[i], sn[i]), __fmul_rn(x2[i], c[i]));
+        y1[i] = __fsub_rn(__fmul_rn(x1[k][i], c[i]), __fmul_rn(x2[k][i], sn[i]));
+        y2[i] = __fadd_rn(__fmul_rn(x1[k][i], sn[i]), __fmul_rn(x2[k][i], c[i]));
       }
     }
-  } else {
-#pragma unroll
-    for (int i = 0; i < 8; ++i) y1[i] = x1[i], y2[i] = x2[i];
+    TO *yr = static_cast<TO *>(a.out[t]) + b * a.osb[t] + s * a.oss[t] + h * a.osh[t];
+    Vec8<TO>::store(yr + c0, y1);
+    Vec8<TO>::store(yr + half + c0, y2);
   }
-  Vec8<TO>::store(yr + c0, y1);
-  Vec8<TO>::store(yr + half + c0, y2);
 }
 
 template <typename TI, typename TO>
 cudaError_t launch_qkv(const QkvArgs &a, cudaStream_t stream) {
-  const int64_t threads = (int64_t)3 * a.B * a.S * a.H * (a.D / 16);
+  const int64_t threads = (int64_t)a.B * a.S * a.H * (a.D / 16);
   if (threads == 0) return cudaSuccess;
   LaunchScope scope(kIdRotary, stream);
   const unsigned grid = (unsigned)((threads + 255) / 256);
-  if (threads < (int64_t(1) << 31)) rotary_qkv_kernel<TI, TO, uint32_t><<<grid, 256, 0, stream>>>(a);
-  else rotary_qkv_kernel<TI, TO, int64_t><<<grid, 256, 0, stream>>>(a);
+  const bool wide = threads >= (int64_t(1) << 31), spread = threads < 148 * 1024;
+  if (spread) rotary_qkv_kernel<TI, TO, uint32_t, true><<<dim3(grid, 3), 256, 0, stream>>>(a);
+  else if (wide) rotary_qkv_kernel<TI, TO, int64_t, false><<<grid, 256, 0, stream>>>(a);
+  else rotary_qkv_kernel<TI, TO, uint32_t, false><<<grid, 256, 0, stream>>>(a);
   return cudaGetLastError();
 }
 

@@ -304,6 +304,13 @@ def test_ln_modulate_bf16_pair_kernels_match_the_single_ones(shape, missing, exa
     assert float((sums[:4] - sums1[:4]).abs().max()) <= 1e-5 * float(scale) * S ** 0.5 and not sums[4].any()
 
 
+@pytest.mark.parametrize("shape", [(600, 9, 768), (128, 50, 256), (37, 130, 1024), (1500, 4, 512), (1500, 3, 512)])
+@pytest.mark.parametrize("missing", ["none", "x", "scale", "shift"])
+def test_ln_modulate_bf16_pair_kernels_with_rows_walked(shape, missing):
+    """The same where a warp walks several rows of a sample, some fewer than others, and on both sides of the fewest rows for that."""
+    test_ln_modulate_bf16_pair_kernels_match_the_single_ones(shape, missing, False)
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("shape", [(1, 1, 256), (1100, 3, 768), (9, 50, 512), (2, 128, 1024), (600, 8, 768), (1200, 9, 256),
                                    (300, 50, 1024), (75, 128, 768), (148, 129, 512)])

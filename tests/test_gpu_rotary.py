@@ -130,3 +130,22 @@ def test_rotary_qkv_equals_the_per_tensor_path_under_forward_and_reverse_mode(le
     xl2 = qkv.clone().requires_grad_(True)
     (want,) = torch.autograd.grad(list(per_tensor(xl2)), [xl2], cots[:3])
     assert torch.equal(dx, want)
+
+
+@pytest.mark.parametrize("shape", [(148, 64, 1, 256), (37, 131, 9, 64), (1, 8192, 37, 16)])
+def test_rotary_qkv_with_one_thread_for_all_three(shape):
+    """Enough positions that a thread takes q, k and v: bit-equal to apply_rotary_cast per tensor, and the transpose to its
+    gradient."""
+    from semicat_b200.rotary import rotary_qkv
+    B, S, H, D = shape
+    g = torch.Generator(device="cuda").manual_seed(S)
+    qkv = torch.randn(B, S, 3, H, D, device="cuda", generator=g).bfloat16()
+    cots = [torch.randn(B, S, H, D, device="cuda", generator=g).bfloat16() for _ in range(3)]
+    cos, sin = _tables(S, D, "cuda")
+    xl, xr = (qkv.clone().requires_grad_(True) for _ in range(2))
+    outs = rotary_qkv(xl, cos, sin, torch.bfloat16)
+    q, k, v = xr.unbind(2)
+    want = (apply_rotary_cast(q, cos, sin, torch.bfloat16), apply_rotary_cast(k, cos, sin, torch.bfloat16), v)
+    for a, b in zip(outs, want):
+        assert torch.equal(a, b)
+    assert torch.equal(torch.autograd.grad(outs, [xl], cots)[0], torch.autograd.grad(want, [xr], cots)[0])

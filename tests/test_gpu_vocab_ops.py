@@ -197,6 +197,31 @@ def test_gelu_tanh_dual(dtype):
         assert torch.allclose(got.double(), ref, rtol=tol, atol=tol), name
 
 
+def test_gelu_tanh_over_all_bf16_values():
+    """Every bf16 value whose h^5 fp32 can hold, and both infinities, in a last chunk that is not full: value and both derivatives
+    against fp64.  One rounding (2^-8 relative) and, where a derivative passes through zero, the error of its terms in fp32: they
+    are below 2^2, the exponent of 2^u is good to 2^-24 of |u| < 2^4 where they have not died out, so 2^-18 and twice that for
+    the other roundings."""
+    bits = torch.arange(-2 ** 15, 2 ** 15, device="cuda", dtype=torch.int32).to(torch.int16)
+    h = bits.view(torch.bfloat16)
+    h = h[h.float().abs() < 1.2e8]
+    h = h[: h.numel() // 8 * 8 - 8 * 3]
+    one = torch.ones_like(h)
+    y, d1, d1b, d2 = (torch.full_like(h, float("nan")) for _ in range(4))
+    dual_ops._gelu_launch(3, h, one, None, None, y, d1)
+    dual_ops._gelu_launch(2, h, one, one, None, d1b, d2)
+    hd = h.double().requires_grad_(True)
+    ref = F.gelu(hd, approximate="tanh")
+    (r1,) = torch.autograd.grad(ref, hd, torch.ones_like(hd), create_graph=True)
+    (r2,) = torch.autograd.grad(r1, hd, torch.ones_like(hd))
+    for got, want, name in ((y, ref, "g"), (d1, r1, "g'"), (d1b, r1, "g' (backward)"), (d2, r2, "g''")):
+        assert torch.allclose(got.double(), want.detach(), rtol=2 ** -8, atol=2 ** -17), name
+    ends = torch.tensor([float("inf"), float("-inf"), 3e38, -3e38] * 2, device="cuda", dtype=torch.bfloat16)
+    out = torch.empty_like(ends)
+    dual_ops._gelu_launch(0, ends, None, None, None, out, None)
+    assert torch.equal(out[[0, 2]], ends[[0, 2]]) and out[1].isnan() and out[3] == 0
+
+
 @pytest.mark.parametrize("autocast", [None, torch.bfloat16])
 def test_training_step_with_fused_vocabulary_side_matches_plain_path(autocast):
     """Model level: vocabulary large enough for the fused kernels (and not a multiple of 8), against the plain-formula path."""
