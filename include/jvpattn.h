@@ -237,6 +237,13 @@ typedef struct jvpattn_cast {
 } jvpattn_cast;
 int jvpattn_cast_params(const jvpattn_cast *entries, int n, int dtype, void *stream);
 
+/* out[c] = sum of x[r * ld + c] over the rows, accumulated in fp32 and rounded once.  JVPATTN_BF16 only; x, out and workspace
+ * 16-byte aligned (else JVPATTN_EALIGN), cols and ld multiples of 8, workspace at least jvpattn_column_sum_workspace_bytes (else
+ * JVPATTN_EINVAL). */
+int64_t jvpattn_column_sum_workspace_bytes(int64_t rows, int cols);
+int jvpattn_column_sum(const void *x, int64_t rows, int cols, int64_t ld, void *out, int dtype, void *workspace, int64_t workspace_bytes,
+                       void *stream);
+
 /* Turns the column sums that jvpattn_ln_modulate's backward kernels leave (sums_y: which = 2, (2, batch, channels);
  * sums_ty: which = 3, (3, batch, channels); either may be NULL) into the gradients of shift, scale, their tangents
  * ((batch, channels) contiguous in `dtype`; NULL = not wanted) and of the LayerNorm weight and bias (fp32 (channels),

@@ -18,7 +18,7 @@ LIB_PATH = os.path.join(_PKG_DIR, "libjvpattn.so")
 NATIVE_PATH = os.path.join(_PKG_DIR, "_native.so")  # the autograd nodes, see csrc/torch_nodes.cpp
 SOURCES = ["jvpattn_api.cu", "jvpattn_simt.cu", "jvpattn_sm100_fwd.cu", "jvpattn_sm100_bwd.cu",
            "jvpattn_sm100_bwd_short.cu", "sm100_tensormap.cu", "rotary.cu", "dual_pointwise.cu", "vocab_head.cu",
-           "vocab_loss.cu", "cast_params.cu"]
+           "vocab_loss.cu", "cast_params.cu", "column_sum.cu"]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
     "-Xcompiler", "-fPIC", "-shared",
@@ -34,6 +34,7 @@ EXPORTS = (
     "jvpattn_bwd_static", "jvpattn_rotary_cast", "jvpattn_stream_check", "jvpattn_debug_set",
     "jvpattn_ln_modulate", "jvpattn_ln_modulate_dual", "jvpattn_gated_residual", "jvpattn_flow_map_head", "jvpattn_gelu_dual", "jvpattn_vocab_op",
     "jvpattn_gated_residual_dual", "jvpattn_ln_finalize", "jvpattn_rotary_qkv", "jvpattn_cast_params", "jvpattn_gate_ln",
+    "jvpattn_column_sum", "jvpattn_column_sum_workspace_bytes",
 )
 DEBUG_WAIT_CYCLES, DEBUG_STALL_NEXT_FWD = 0, 1
 STATIC_SCRATCH_ROWS = 262144

@@ -366,6 +366,20 @@ int jvpattn_cast_params(const jvpattn_cast *entries, int n, int dtype, void *str
   return note_cuda(cast_params(entries, n, dtype, static_cast<cudaStream_t>(stream)));
 }
 
+int64_t jvpattn_column_sum_workspace_bytes(int64_t rows, int cols) { return rows < 0 || cols < 0 ? 0 : column_sum_workspace(rows, cols); }
+
+int jvpattn_column_sum(const void *x, int64_t rows, int cols, int64_t ld, void *out, int dtype, void *workspace, int64_t workspace_bytes,
+                       void *stream) {
+  if (dtype != JVPATTN_BF16 || rows < 0 || cols < 0 || cols % 8 || ld % 8 || ld < cols || !out || (!x && rows > 0) || !workspace ||
+      workspace_bytes < column_sum_workspace(rows, cols))
+    return JVPATTN_EINVAL;
+  for (const void *p : {x, static_cast<const void *>(out), static_cast<const void *>(workspace)})
+    if (reinterpret_cast<uintptr_t>(p) % 16) return JVPATTN_EALIGN;
+  DeviceInfo *d = nullptr;
+  if (int rc = current_device(&d)) return rc;
+  return note_cuda(column_sum(x, rows, cols, ld, out, static_cast<float *>(workspace), static_cast<cudaStream_t>(stream)));
+}
+
 int jvpattn_ln_finalize(const float *sums_y, const float *sums_ty, const float *gamma, const float *beta, const void *scale,
                         const void *tscale, int64_t mod_stride, int64_t tmod_stride, void *d_shift, void *d_scale, void *d_tshift,
                         void *d_tscale, float *d_gamma, float *d_beta, int batch, int channels, int dtype, void *stream) {

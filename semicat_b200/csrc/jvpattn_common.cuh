@@ -92,6 +92,10 @@ cudaError_t gated_residual_dual(int which, const void *x, const void *tx, const 
 cudaError_t gelu_dual(int mode, const void *h, const void *v, const void *w, const void *u, void *out, void *out2, int64_t n,
                       int dtype, cudaStream_t stream);
 
+// column_sum.cu: sums over the rows of a bf16 matrix
+int64_t column_sum_workspace(int64_t rows, int cols);
+cudaError_t column_sum(const void *x, int64_t rows, int cols, int64_t ld, void *out, float *workspace, cudaStream_t stream);
+
 // cast_params.cu: 16-bit copies of parameters
 cudaError_t cast_params(const jvpattn_cast *entries, int n, int dtype, cudaStream_t stream);
 

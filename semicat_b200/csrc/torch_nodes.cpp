@@ -573,6 +573,43 @@ std::tuple<Tensor, Tensor> linear_pair(const Tensor &x, const Tensor &tx, const 
   return {at::linear(x, w, b), at::linear(tx, w)};
 }
 
+// The sum of a matrix over its rows: by the library's kernel for plain bf16 values, by torch's reduction for whatever else a backward
+// pass may be given (batched, dual or recorded cotangents, other types).
+Tensor column_sum(const Tensor &g) {
+  const auto keys = g.key_set();
+  if (g.scalar_type() != at::kBFloat16 || !g.is_cuda() || g.layout() != at::kStrided || keys.has(c10::DispatchKey::Python) ||
+      keys.has(c10::DispatchKey::Functionalize) || keys.has(c10::DispatchKey::FuncTorchBatched) || keys.has(c10::DispatchKey::Batched) ||
+      keys.has(c10::DispatchKey::FuncTorchGradWrapper) || !g.has_storage() || g.is_neg() || c10::impl::TorchDispatchModeTLS::any_modes_set() ||
+      (at::GradMode::is_enabled() && g.requires_grad()) || g._fw_grad(0).defined() || g.size(1) % 8 || g.numel() == 0 || g.stride(1) != 1 ||
+      g.stride(0) % 8 || g.stride(0) < g.size(1) || (g.storage_offset() * 2) % 16)
+    return g.sum(0);
+  at::AutoDispatchBelowADInplaceOrView below;
+  c10::cuda::CUDAGuard guard(g.device());
+  Tensor out = at::empty({g.size(1)}, g.options());
+  const int64_t bytes = jvpattn_column_sum_workspace_bytes(g.size(0), (int)g.size(1));
+  const Tensor workspace = at::empty({bytes}, g.options().dtype(at::kByte));
+  check(jvpattn_column_sum(ptr(g), g.size(0), (int)g.size(1), g.stride(0), ptr(out), JVPATTN_BF16, ptr(workspace), bytes, stream_of(g)), "jvpattn_column_sum");
+  return out;
+}
+
+// Without a tangent: torch's own layer, but for the gradient of the bias.  (Differentiable again, as torch's is.)
+struct LinearPrimal : Function<LinearPrimal> {
+  static Tensor forward(AutogradContext *ctx, const Tensor &x, const Tensor &w, const Tensor &b) {
+    at::AutoDispatchBelowADInplaceOrView below;
+    ctx->save_for_backward({x, w});
+    return at::linear(x, w, b);
+  }
+  static variable_list backward(AutogradContext *ctx, const variable_list &g) {
+    const auto s = ctx->get_saved_variables();
+    const Tensor x = s[0], w = s[1], g2 = g[0].reshape({-1, w.size(0)});
+    variable_list d(3);
+    if (ctx->needs_input_grad(0)) d[0] = at::mm(g2, w).view(x.sizes());
+    if (ctx->needs_input_grad(1)) d[1] = at::mm(g2.t(), x.reshape({-1, w.size(1)}));
+    if (ctx->needs_input_grad(2)) d[2] = column_sum(g2);
+    return d;
+  }
+};
+
 // Two GEMMs forward; backward two for dx / dtx, two for dw (the second adds to the first in its epilogue), one reduction for db.
 struct LinearPair : Function<LinearPair> {
   static variable_list forward(AutogradContext *ctx, const Tensor &x, const Tensor &tx_, const Tensor &w, const Opt &b) {
@@ -596,7 +633,7 @@ struct LinearPair : Function<LinearPair> {
         const Tensor g2 = g[0].reshape({-1, N});
         if (ctx->needs_input_grad(0)) d[0] = at::mm(g2, w).view(x.sizes());
         if (ctx->needs_input_grad(2)) d[2] = at::mm(g2.t(), x.reshape({-1, K}));
-        if (ctx->saved_data["bias"].toBool() && ctx->needs_input_grad(3)) d[3] = g2.sum(0);
+        if (ctx->saved_data["bias"].toBool() && ctx->needs_input_grad(3)) d[3] = column_sum(g2);
       }
       if (g[1].defined()) {
         const Tensor t2 = g[1].reshape({-1, N});
@@ -927,14 +964,20 @@ py::object gelu_py(bool jvp, py::handle h_) {
   return py::cast(gelu_primal_autograd(h.t));
 }
 
-// Only where x carries a tangent: without one the layer is torch's own.
+// Without a tangent on x the layer is torch's own, but where a bf16 bias wants its gradient.
 py::object linear_py(bool jvp, py::handle x_, py::handle w_, py::handle b_) {
   const Arg x(x_), w(w_), b(b_);
-  if (!jvp || !fits(jvp, {&x, &w, &b}) || !x.t.defined() || !w.t.defined() || !x.t._fw_grad(0).defined()) return py::none();
+  if (!fits(jvp, {&x, &w, &b}) || !x.t.defined() || !w.t.defined() || (jvp && !x.t._fw_grad(0).defined())) return py::none();
   const auto dt = x.t.scalar_type();
   if (w.t.scalar_type() != dt || w.t.dim() != 2 || (b.t.defined() && b.t.scalar_type() != dt) ||
       (at::autocast::is_autocast_enabled(at::kCUDA) && at::autocast::get_autocast_dtype(at::kCUDA) != dt))
     return py::none();
+  if (!jvp) {
+    if (dt != at::kBFloat16 || !b.t.defined() || !any_grad({&b.t}) || b.t.dim() != 1 || x.t.dim() < 2 || x.t.numel() == 0 || x.t.size(-1) != w.t.size(1) ||
+        b.t.size(0) != w.t.size(0) || w.t.size(0) % 8 || w.t.device() != x.t.device() || b.t.device() != x.t.device())
+      return py::none();
+    return py::cast(LinearPrimal::apply(x.t, w.t, b.t));
+  }
   return py::cast(handle<decltype(linear_jvp)>("jvpattn::linear").call(x.t, w.t, opt(b.t)));
 }
 

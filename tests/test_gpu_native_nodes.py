@@ -219,3 +219,30 @@ def test_errors_are_those_of_the_library():
         sdpa_jvp(half[0], half[1][:1], half[2])
     with pytest.raises(TypeError):
         sdpa_jvp(*(t.float() for t in x[:3]))
+
+
+@pytest.mark.parametrize("rows,cols", [(1, 8), (7, 24), (257, 40), (513, 264), (4096, 768), (16385, 3072), (2049, 2368), (100, 4608)])
+def test_bias_gradient(rows, cols):
+    """The sum over rows, also of a matrix with a row pitch of its own, against fp64: one rounding (2^-8) and the order of an fp32
+    sum (2^-24 of the sum of magnitudes per level of adding; under 2^7 of them).  What is no plain bf16 value is summed by torch."""
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    r = lambda *s: torch.randn(*s, device="cuda", generator=g).bfloat16()
+    x, w, b = r(rows, 16).requires_grad_(True), r(cols, 16).requires_grad_(True), r(cols).requires_grad_(True)
+    plain = torch.nn.functional.linear
+    for gy in (r(rows, cols), r(rows, cols + 8)[:, :cols], r(rows, cols + 1)[:, 1:], r(cols, rows).t()):
+        y = dual_ops.linear(x, w, b)
+        assert torch.equal(y, plain(x, w, b))
+        got, want = torch.autograd.grad(y, [x, w, b], gy), torch.autograd.grad(plain(x, w, b), [x, w, b], gy)
+        assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1]) and got[1].stride() == want[1].stride()
+        ref, size = gy.double().sum(0), gy.double().abs().sum(0)
+        assert bool(((got[2].double() - ref).abs() <= 2 ** -8 * ref.abs() + 2 ** -17 * size).all())
+    gy = r(rows, cols).requires_grad_(True)
+
+    def twice(linear):  # recorded cotangents: the second derivatives are torch's own
+        once = torch.autograd.grad(linear(x, w, b), [x, w, b], gy, create_graph=True)
+        return torch.autograd.grad([t.float().pow(2).sum() for t in once], [x, w, gy])
+
+    for a, c in zip(twice(dual_ops.linear), twice(plain)):
+        assert torch.equal(a, c)
+    batched, = torch.autograd.grad(dual_ops.linear(x, w, b), [b], r(2, rows, cols), is_grads_batched=True)
+    assert batched.shape == (2, cols)
