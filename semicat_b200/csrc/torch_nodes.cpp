@@ -742,9 +742,10 @@ std::vector<Tensor> rotary_pair_autograd(const Tensor &qkv, const Opt &tqkv, con
 }
 
 // ------------------------------------------------------------------------------------------------ under torch.func.jvp
-template <typename F>
+// (Of the op that F implements: one per function, since several have the same signature.)
+template <auto *F>
 const auto &handle(const char *name) {
-  static const auto op = c10::Dispatcher::singleton().findSchemaOrThrow(name, "").typed<F>();
+  static const auto op = c10::Dispatcher::singleton().findSchemaOrThrow(name, "").typed<std::remove_pointer_t<decltype(F)>>();
   return op;
 }
 Opt tangent(const Tensor &t) { return opt(t._fw_grad(/*level=*/0)); }
@@ -758,8 +759,8 @@ Tensor attention_jvp(const Tensor &q, const Tensor &k, const Tensor &v, bool bsh
   std::tuple<Tensor, Tensor> out;
   {
     at::AutoDispatchBelowADInplaceOrView below;  // the op leaves the transform's level here
-    if (!tq && !tk && !tv) return handle<decltype(attention_primal)>("jvpattn::attention_primal").call(q, k, v, bshd);
-    out = handle<decltype(attention_pair)>("jvpattn::attention_pair").call(q, k, v, tq, tk, tv, bshd);
+    if (!tq && !tk && !tv) return handle<attention_primal>("jvpattn::attention_primal").call(q, k, v, bshd);
+    out = handle<attention_pair>("jvpattn::attention_pair").call(q, k, v, tq, tk, tv, bshd);
   }
   return dual(std::get<0>(out), std::get<1>(out));
 }
@@ -768,8 +769,8 @@ Tensor ln_jvp(const Tensor &x, const Tensor &gamma, const Opt &beta, const Tenso
   std::tuple<Tensor, Tensor> out;
   {
     at::AutoDispatchBelowADInplaceOrView below;
-    if (!tx && !tsh && !tsc) return handle<decltype(ln_primal)>("jvpattn::ln_primal").call(x, gamma, beta, shift, scale, eps, exact);
-    out = handle<decltype(ln_pair)>("jvpattn::ln_pair").call(x, gamma, beta, shift, scale, tx, tsh, tsc, eps, exact);
+    if (!tx && !tsh && !tsc) return handle<ln_primal>("jvpattn::ln_primal").call(x, gamma, beta, shift, scale, eps, exact);
+    out = handle<ln_pair>("jvpattn::ln_pair").call(x, gamma, beta, shift, scale, tx, tsh, tsc, eps, exact);
   }
   return dual(std::get<0>(out), std::get<1>(out));
 }
@@ -778,8 +779,8 @@ Tensor gate_jvp(const Tensor &x, const Tensor &y, const Tensor &gate, const Opt 
   std::tuple<Tensor, Tensor> out;
   {
     at::AutoDispatchBelowADInplaceOrView below;
-    if (!tx && !ty && !tg) return handle<decltype(gate_primal)>("jvpattn::gate_primal").call(x, y, gate, seed, call, p);
-    out = handle<decltype(gate_pair)>("jvpattn::gate_pair").call(x, y, gate, seed, tx, ty, tg, call, p);
+    if (!tx && !ty && !tg) return handle<gate_primal>("jvpattn::gate_primal").call(x, y, gate, seed, call, p);
+    out = handle<gate_pair>("jvpattn::gate_pair").call(x, y, gate, seed, tx, ty, tg, call, p);
   }
   return dual(std::get<0>(out), std::get<1>(out));
 }
@@ -788,8 +789,8 @@ Tensor gelu_jvp(const Tensor &h) {
   std::tuple<Tensor, Tensor> out;
   {
     at::AutoDispatchBelowADInplaceOrView below;
-    if (!th) return handle<decltype(gelu_primal)>("jvpattn::gelu_primal").call(h);
-    out = handle<decltype(gelu_pair)>("jvpattn::gelu_pair").call(h, *th);
+    if (!th) return handle<gelu_primal>("jvpattn::gelu_primal").call(h);
+    out = handle<gelu_pair>("jvpattn::gelu_pair").call(h, *th);
   }
   return dual(std::get<0>(out), std::get<1>(out));
 }
@@ -798,7 +799,7 @@ Tensor linear_jvp(const Tensor &x, const Tensor &w, const Opt &b) {
   std::tuple<Tensor, Tensor> out;
   {
     at::AutoDispatchBelowADInplaceOrView below;
-    out = handle<decltype(linear_pair)>("jvpattn::linear_pair").call(x, *tx, w, b);
+    out = handle<linear_pair>("jvpattn::linear_pair").call(x, *tx, w, b);
   }
   return dual(std::get<0>(out), std::get<1>(out));
 }
@@ -807,7 +808,7 @@ std::vector<Tensor> rotary_jvp(const Tensor &qkv, const Tensor &cos, const Tenso
   std::vector<Tensor> out;
   {
     at::AutoDispatchBelowADInplaceOrView below;
-    out = handle<decltype(rotary_pair)>("jvpattn::rotary_pair").call(qkv, t, cos, sin, dtype);
+    out = handle<rotary_pair>("jvpattn::rotary_pair").call(qkv, t, cos, sin, dtype);
   }
   if (!t) return out;
   return {dual(out[0], out[3]), dual(out[1], out[4]), dual(out[2], out[5])};
@@ -898,7 +899,7 @@ py::object attention_py(bool jvp, py::handle q_, py::handle k_, py::handle v_, b
       (dt != at::kBFloat16 && dt != at::kHalf) || k.t.scalar_type() != dt || v.t.scalar_type() != dt || k.t.device() != q.t.device() ||
       v.t.device() != q.t.device())
     return py::none();
-  if (jvp) return py::cast(handle<decltype(attention_jvp)>("jvpattn::attention").call(q.t, k.t, v.t, bshd));
+  if (jvp) return py::cast(handle<attention_jvp>("jvpattn::attention").call(q.t, k.t, v.t, bshd));
   return py::cast(attention_primal_autograd(q.t, k.t, v.t, bshd));
 }
 
@@ -922,7 +923,7 @@ py::object ln_py(bool jvp, py::handle x_, py::handle w_, py::handle b_, py::hand
   if (!fits(jvp, {&x, &w, &b, &shift, &scale}) || !rows_ok(x.t) || !modulation_ok(shift.t, x.t) || !modulation_ok(scale.t, x.t)) return py::none();
   if (!w.t.defined() || !param_ok(w.t, x.t) || (b.t.defined() && !param_ok(b.t, x.t))) return py::none();
   if (jvp)
-    return py::cast(handle<decltype(ln_jvp)>("jvpattn::ln").call(x.t, w.t, opt(b.t), shift.t, scale.t, eps, exact));
+    return py::cast(handle<ln_jvp>("jvpattn::ln").call(x.t, w.t, opt(b.t), shift.t, scale.t, eps, exact));
   return py::cast(ln_primal_autograd(x.t, w.t, opt(b.t), shift.t, scale.t, eps, exact));
 }
 
@@ -931,7 +932,7 @@ py::object gate_py(bool jvp, py::handle x_, py::handle y_, py::handle gate_, py:
   if (!fits(jvp, {&x, &y, &gate, &seed}) || !rows_ok(y.t) || !x.t.defined() || x.t.sizes() != y.t.sizes() || x.t.scalar_type() != y.t.scalar_type() ||
       x.t.device() != y.t.device() || !modulation_ok(gate.t, y.t))
     return py::none();
-  if (jvp) return py::cast(handle<decltype(gate_jvp)>("jvpattn::gate").call(x.t, y.t, gate.t, opt(seed.t), call, p));
+  if (jvp) return py::cast(handle<gate_jvp>("jvpattn::gate").call(x.t, y.t, gate.t, opt(seed.t), call, p));
   return py::cast(gate_primal_autograd(x.t, y.t, gate.t, opt(seed.t), call, p));
 }
 
@@ -960,7 +961,7 @@ py::object gelu_py(bool jvp, py::handle h_) {
   if (!fits(jvp, {&h}) || !h.t.defined() || (h.t.scalar_type() != at::kBFloat16 && h.t.scalar_type() != at::kFloat) || !h.t.is_contiguous() ||
       h.t.numel() % 8 || (h.t.storage_offset() * h.t.element_size()) % 16)
     return py::none();
-  if (jvp) return py::cast(handle<decltype(gelu_jvp)>("jvpattn::gelu").call(h.t));
+  if (jvp) return py::cast(handle<gelu_jvp>("jvpattn::gelu").call(h.t));
   return py::cast(gelu_primal_autograd(h.t));
 }
 
@@ -978,7 +979,7 @@ py::object linear_py(bool jvp, py::handle x_, py::handle w_, py::handle b_) {
       return py::none();
     return py::cast(LinearPrimal::apply(x.t, w.t, b.t));
   }
-  return py::cast(handle<decltype(linear_jvp)>("jvpattn::linear").call(x.t, w.t, opt(b.t)));
+  return py::cast(handle<linear_jvp>("jvpattn::linear").call(x.t, w.t, opt(b.t)));
 }
 
 py::object rotary_py(bool jvp, py::handle qkv_, py::handle cos_, py::handle sin_, bool bf16) {
@@ -999,7 +1000,7 @@ py::object rotary_py(bool jvp, py::handle qkv_, py::handle cos_, py::handle sin_
   const Tensor &t = x._fw_grad(0);
   if (t.defined() && (t.scalar_type() != x.scalar_type() || t.strides() != x.strides() || !layout_ok(t))) return py::none();
   const int64_t dtype = (int64_t)(bf16 ? at::kBFloat16 : at::kFloat);
-  const std::vector<Tensor> out = jvp ? handle<decltype(rotary_jvp)>("jvpattn::rotary").call(x, cos.t, sin.t, dtype)
+  const std::vector<Tensor> out = jvp ? handle<rotary_jvp>("jvpattn::rotary").call(x, cos.t, sin.t, dtype)
                                                    : rotary_pair_autograd(x, Opt(), cos.t, sin.t, dtype);
   return py::make_tuple(out[0], out[1], out[2]);
 }

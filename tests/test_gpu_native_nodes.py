@@ -246,3 +246,29 @@ def test_bias_gradient(rows, cols):
         assert torch.equal(a, c)
     batched, = torch.autograd.grad(dual_ops.linear(x, w, b), [b], r(2, rows, cols), is_grads_batched=True)
     assert batched.shape == (2, cols)
+
+
+@pytest.mark.parametrize("form", ["detached", "plain", "recorded"])
+def test_inside_a_jvp_without_a_tangent(form):
+    """Under a transform whose tangents do not reach the op: its value and its gradients are those of a call outside."""
+    B, S, H, C = 2, 5, 4, 256
+    norm = torch.nn.LayerNorm(C, device="cuda")
+    lin = torch.nn.Linear(C, 24, device="cuda").bfloat16()
+    cos, sin = _rand(1, S, 32, dtype=torch.float32), _rand(2, S, 32, dtype=torch.float32)
+    heads = [_rand(10 + i, B, S, H, 64) for i in range(3)]
+    rows = [_rand(20 + i, B, S, C) for i in range(2)]
+    mods = [_rand(30 + i, B, C) for i in range(3)]
+    for args, op in ((heads, safe_sdpa_jvp), ([t.transpose(1, 2) for t in heads], sdpa_jvp),
+                     (rows[:1] + mods[:2], lambda x, sh, sc: dual_ops.ln_modulate(x, norm, sh, sc)), (rows + mods[:1], dual_ops.gated_residual),
+                     (rows[:1], dual_ops.gelu_tanh), (rows[:1], lambda x: dual_ops.linear(x, lin.weight, lin.bias)),
+                     ([_rand(40, B, S, 3, H, 64)], lambda x: torch.stack(rotary.rotary_qkv(x, cos, sin)))):
+        args = [t.detach().requires_grad_(form == "recorded") for t in args]
+        one = torch.ones((), device="cuda")
+        inside = lambda a, *x: (op(*(t.detach() for t in x)) if form == "detached" else op(*args)) * 1.0 + 0.0 * a
+        x = tuple(t.detach() for t in args)
+        y, _ = torch.func.jvp(inside, (one, *x), (one, *x))
+        want = op(*args)
+        assert torch.equal(y.detach(), want.detach())
+        if form == "recorded":
+            g = _rand(50, *want.shape, dtype=want.dtype)
+            _equal(torch.autograd.grad(y, args, g.to(y.dtype)), torch.autograd.grad(want, args, g))
