@@ -914,8 +914,9 @@ bool rows_ok(const Tensor &x) {
   return C == 256 || C == 512 || C == 768 || C == 1024;
 }
 
+// (A parameter with a tangent of its own is refused by the classes: the terms it would add are not formed here.)
 bool param_ok(const Tensor &p, const Tensor &x) {
-  return p.scalar_type() == at::kFloat && p.dim() == 1 && p.size(0) == x.size(2) && p.is_contiguous() && p.device() == x.device();
+  return !p._fw_grad(0).defined() && p.scalar_type() == at::kFloat && p.dim() == 1 && p.size(0) == x.size(2) && p.is_contiguous() && p.device() == x.device();
 }
 
 py::object ln_py(bool jvp, py::handle x_, py::handle w_, py::handle b_, py::handle shift_, py::handle scale_, double eps, bool exact) {
@@ -965,10 +966,13 @@ py::object gelu_py(bool jvp, py::handle h_) {
   return py::cast(gelu_primal_autograd(h.t));
 }
 
-// Without a tangent on x the layer is torch's own, but where a bf16 bias wants its gradient.
+// Without a tangent on x the layer is torch's own, but where a bf16 bias wants its gradient; with one on a parameter it is refused
+// by the class.
 py::object linear_py(bool jvp, py::handle x_, py::handle w_, py::handle b_) {
   const Arg x(x_), w(w_), b(b_);
-  if (!fits(jvp, {&x, &w, &b}) || !x.t.defined() || !w.t.defined() || (jvp && !x.t._fw_grad(0).defined())) return py::none();
+  if (!fits(jvp, {&x, &w, &b}) || !x.t.defined() || !w.t.defined() ||
+      (jvp && (!x.t._fw_grad(0).defined() || w.t._fw_grad(0).defined() || (b.t.defined() && b.t._fw_grad(0).defined()))))
+    return py::none();
   const auto dt = x.t.scalar_type();
   if (w.t.scalar_type() != dt || w.t.dim() != 2 || (b.t.defined() && b.t.scalar_type() != dt) ||
       (at::autocast::is_autocast_enabled(at::kCUDA) && at::autocast::get_autocast_dtype(at::kCUDA) != dt))

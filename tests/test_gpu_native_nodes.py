@@ -272,3 +272,43 @@ def test_inside_a_jvp_without_a_tangent(form):
         if form == "recorded":
             g = _rand(50, *want.shape, dtype=want.dtype)
             _equal(torch.autograd.grad(y, args, g.to(y.dtype)), torch.autograd.grad(want, args, g))
+
+
+def _jvp_or_refusal(f, prim, tang):
+    try:
+        return [t.detach() for t in torch.func.jvp(f, prim, tang)]
+    except NotImplementedError:
+        return None
+
+
+@pytest.mark.parametrize("with_x", [False, True])
+@pytest.mark.parametrize("which", [("weight",), ("bias",), ("weight", "bias")])
+@pytest.mark.parametrize("grad", [False, True])
+def test_tangents_of_parameters(which, with_x, grad):
+    """A tangent on a weight or a bias either is in the result or the call is refused: never left out."""
+    C = 256
+    x, tx, shift, scale = (_rand(i, 2, 3, C, dtype=torch.float32) for i in range(4))
+    x.requires_grad_(grad)
+    for make, call, plain in (
+            (lambda: torch.nn.Linear(C, 24), lambda m, a: dual_ops.linear(a, m.weight, m.bias), lambda m, a: m(a)),
+            (lambda: torch.nn.LayerNorm(C), lambda m, a: dual_ops.ln_modulate(a, m, shift[:, 0], scale[:, 0]),
+             lambda m, a: m(a) * (1 + scale[:, :1]) + shift[:, :1])):
+        class Layer(torch.nn.Module):
+            def __init__(self):
+                super().__init__()
+                self.inner, self.call = make().cuda(), call
+
+            def forward(self, a):
+                return self.call(self.inner, a)
+
+        layer = Layer()
+        p = dict(layer.named_parameters())
+        names = [f"inner.{n}" for n in which]
+        prim = tuple(p[n].detach() for n in names) + ((x,) if with_x else ())
+        tang = tuple(_rand(20 + i, *t.shape, dtype=torch.float32) for i, t in enumerate(prim[:len(names)])) + ((tx,) if with_x else ())
+        f = lambda *a: torch.func.functional_call(layer, dict(zip(names, a)), (a[-1] if with_x else x,))
+        got = _jvp_or_refusal(f, prim, tang)
+        layer.call = plain
+        want = torch.func.jvp(f, prim, tang)
+        if got is not None:
+            assert float((got[1] - want[1]).norm()) <= 1e-5 * float(want[1].norm())
