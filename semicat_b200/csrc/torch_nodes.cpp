@@ -871,6 +871,15 @@ struct Arg {
   }
 };
 
+// A tangent may be of another type or on another device than its primal (torch.func.jvp hands it on as given): the kernels read
+// it with the primal's, so it must be a plain tensor of the same kind.
+bool tangent_fits(const Tensor &t, const Tensor &p) {
+  const auto keys = t.key_set();
+  return t.scalar_type() == p.scalar_type() && t.device() == p.device() && t.layout() == at::kStrided && t.sizes() == p.sizes() &&
+         !keys.has(c10::DispatchKey::Python) && !keys.has(c10::DispatchKey::Functionalize) && !keys.has(c10::DispatchKey::FuncTorchBatched) &&
+         !t.is_conj() && !t.is_neg();
+}
+
 // `jvp`: one torch.func.jvp is open and no other transform; else none is.
 bool fits(bool jvp, std::initializer_list<const Arg *> args) {
   if (c10::impl::TorchDispatchModeTLS::any_modes_set() || at::impl::torch_function_mode_enabled() || torch::jit::tracer::isTracing()) return false;
@@ -881,9 +890,11 @@ bool fits(bool jvp, std::initializer_list<const Arg *> args) {
     if (!a->t.is_cuda() || a->t.layout() != at::kStrided || keys.has(c10::DispatchKey::Python) || keys.has(c10::DispatchKey::Functionalize) ||
         keys.has(c10::DispatchKey::FuncTorchBatched) || a->t.is_conj() || a->t.is_neg())
       return false;
+    const Tensor &t = a->t._fw_grad(/*level=*/0);
     if (keys.has(c10::DispatchKey::FuncTorchGradWrapper)) {
       if (!jvp || a->t.requires_grad()) return false;  // (reverse mode inside the transform)
-    } else if (a->t._fw_grad(0).defined()) {
+      if (t.defined() && !tangent_fits(t, a->t)) return false;
+    } else if (t.defined()) {
       return false;  // a dual of a plain forward_ad level
     }
   }
@@ -1002,7 +1013,7 @@ py::object rotary_py(bool jvp, py::handle qkv_, py::handle cos_, py::handle sin_
   if ((x.scalar_type() != at::kBFloat16 && x.scalar_type() != at::kFloat) || x.size(4) % 16 || !layout_ok(x) || !table_ok(cos.t) || !table_ok(sin.t))
     return py::none();
   const Tensor &t = x._fw_grad(0);
-  if (t.defined() && (t.scalar_type() != x.scalar_type() || t.strides() != x.strides() || !layout_ok(t))) return py::none();
+  if (t.defined() && (t.strides() != x.strides() || !layout_ok(t))) return py::none();
   const int64_t dtype = (int64_t)(bf16 ? at::kBFloat16 : at::kFloat);
   const std::vector<Tensor> out = jvp ? handle<rotary_jvp>("jvpattn::rotary").call(x, cos.t, sin.t, dtype)
                                                    : rotary_pair_autograd(x, Opt(), cos.t, sin.t, dtype);

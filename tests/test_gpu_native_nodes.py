@@ -312,3 +312,26 @@ def test_tangents_of_parameters(which, with_x, grad):
         want = torch.func.jvp(f, prim, tang)
         if got is not None:
             assert float((got[1] - want[1]).norm()) <= 1e-5 * float(want[1].norm())
+
+
+def test_tangents_of_another_kind():
+    """A tangent in another type or on another device than its primal: the attention refuses it, a linear layer casts it, the rotary
+    embedding goes through the operation per tensor."""
+    x = [t.detach() for t in _leaves()]
+    for entry in (sdpa_jvp, safe_sdpa_jvp):
+        for i in range(3):
+            for other, error in ((x[3 + i].float(), TypeError), (x[3 + i].half(), TypeError), (x[3 + i].cpu(), ValueError)):
+                with pytest.raises(error):
+                    torch.func.jvp(entry, tuple(x[:3]), tuple(other if j == i else x[3 + j] for j in range(3)))
+    for grad in (False, True):
+        h, w, b = (t.requires_grad_(grad) for t in (_rand(0, 2, 5, 32), _rand(1, 24, 32), _rand(2, 24)))
+        th = _rand(3, 2, 5, 32, dtype=torch.float32)
+        layer = lambda a: dual_ops.linear(a, w, b)
+        _equal([t.detach() for t in torch.func.jvp(layer, (h,), (th,))], [t.detach() for t in torch.func.jvp(layer, (h,), (th.bfloat16(),))])
+        with pytest.raises(RuntimeError):
+            torch.func.jvp(layer, (h,), (th.bfloat16().cpu(),))
+    qkv, tqkv, (cos, sin) = _rand(5, 2, 6, 3, 4, 64), _rand(6, 2, 6, 3, 4, 64, dtype=torch.float32), (_rand(7 + i, 6, 32, dtype=torch.float32) for i in range(2))
+    q, k, v = zip(*torch.func.jvp(lambda t: rotary.rotary_qkv(t, cos, sin), (qkv,), (tqkv,)))
+    for got, i in ((q, 0), (k, 1)):
+        _equal(got, [rotary.apply_rotary_cast(t[:, :, i], cos, sin) for t in (qkv, tqkv)])
+    _equal([t.contiguous() for t in v], [t[:, :, 2].contiguous() for t in (qkv, tqkv)])  # (Tensor.to leaves what has the type already)
