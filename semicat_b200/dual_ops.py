@@ -60,6 +60,19 @@ def _nz(t):
     return t
 
 
+def _tangent(t, p):
+    """A tangent in the type of its primal ``p``, as the kernels read it (torch.func.jvp hands it on as given)."""
+    if t is None:
+        return None
+    if t.device != p.device:
+        raise ValueError(f"a tangent is on {t.device}, its primal on {p.device}")
+    return t if t.dtype == p.dtype else t.to(p.dtype)
+
+
+def _unpack(*duals):
+    return tuple((p, _tangent(t, p)) for p, t in map(fwAD.unpack_dual, duals))
+
+
 def _ptr(t):
     return t.data_ptr() if t is not None else None
 
@@ -235,7 +248,7 @@ def ln_modulate(x: torch.Tensor, norm: torch.nn.LayerNorm, shift: torch.Tensor, 
     if norm.weight is None or not _usable(x, shift, scale) or tuple(norm.normalized_shape) != (x.shape[-1],):
         return norm(x) * (1.0 + scale) + shift
     beta = norm.bias.float() if norm.bias is not None else None
-    (xp, tx), (shp, tsh), (scp, tsc) = (fwAD.unpack_dual(t) for t in (x, shift, scale))
+    (xp, tx), (shp, tsh), (scp, tsc) = _unpack(x, shift, scale)
     if tx is None and tsh is None and tsc is None:
         y, _, _ = apply(_LnModulate, x.contiguous(), norm.weight.float(), beta, shift, scale, norm.eps, exact)
         return y
@@ -372,7 +385,7 @@ def gated_residual(skip: torch.Tensor, branch: torch.Tensor, gate: torch.Tensor,
             return z
     if not _usable(branch, skip, gate) or skip.shape != branch.shape:
         return F.dropout(branch * gate, p, training) + skip
-    (xp, tx), (yp, ty), (gp, tg) = (fwAD.unpack_dual(t) for t in (skip, branch, gate))
+    (xp, tx), (yp, ty), (gp, tg) = _unpack(skip, branch, gate)
     mask = drop = None
     if training and p > 0.0:
         if _Drop.seed is not None and _Drop.seed.device == yp.device:
@@ -524,7 +537,7 @@ def gelu_tanh(h: torch.Tensor) -> torch.Tensor:
         return y
     if not (h.is_cuda and h.dtype in _CODES and h.is_contiguous() and h.numel() % 8 == 0 and (h.storage_offset() * h.element_size()) % 16 == 0):
         return F.gelu(h, approximate="tanh")
-    hp, th = fwAD.unpack_dual(h)
+    ((hp, th),) = _unpack(h)
     if th is None:
         return apply(_Gelu, h)
     y, ty = _GeluDual.apply(hp, th)
@@ -600,8 +613,7 @@ class _FlowHead(torch.autograd.Function):
         logits, x, dt, lse = ctx.saved_for_forward
         if tdt is None:
             tdt = torch.zeros_like(dt)
-        if tlogits is None:
-            tlogits = torch.zeros_like(logits)
+        tlogits = torch.zeros_like(logits) if tlogits is None else _tangent(tlogits, logits)
         return _FlowHeadTangent.apply(logits, tlogits, x, dt, tdt.float().contiguous(), lse), None
 
     @staticmethod

@@ -172,7 +172,7 @@ def rotary_qkv(qkv: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, out_dtyp
     ok = (p.is_cuda and p.dim() == 5 and p.shape[2] == 3 and p.dtype in _QKV_CODES and out_dtype in _QKV_CODES and p.shape[-1] % 16 == 0
           and p.stride(4) == 1 and all(st % 8 == 0 for st in p.stride()[:4]) and (p.storage_offset() * p.element_size()) % 16 == 0)
     if t is not None:
-        ok = ok and t.dtype == p.dtype and t.stride() == p.stride() and (t.storage_offset() * t.element_size()) % 16 == 0
+        ok = ok and t.dtype == p.dtype and t.device == p.device and t.stride() == p.stride() and (t.storage_offset() * t.element_size()) % 16 == 0
     if not ok:
         q, k, v = qkv.unbind(2)
         return apply_rotary_cast(q, cos, sin, out_dtype), apply_rotary_cast(k, cos, sin, out_dtype), v.to(out_dtype)

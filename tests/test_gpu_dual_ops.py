@@ -339,3 +339,32 @@ def test_primal_ln_and_gate_over_the_ways_rows_are_split(shape, dtype):
     for n, a, r in zip(("dy", "dshift", "dscale", "dgate", "dgamma", "dbeta"), got, want):
         _close(a, r, n, tol if n not in ("dgamma", "dbeta") else 1e-5, 1e-4 * float(r.abs().max()))
     assert _lib.device_status() == 0
+
+
+@pytest.mark.parametrize("dtype,other", [(torch.float32, torch.bfloat16), (torch.bfloat16, torch.float32), (torch.float32, torch.float16)])
+@pytest.mark.parametrize("grad", [False, True])
+def test_tangents_of_another_type(dtype, other, grad):
+    """A tangent in another type than its primal counts as that value in the primal's type; one on another device is refused."""
+    g = torch.Generator(device="cuda").manual_seed(0)
+    mk = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    B, S, C, V = 2, 5, 256, 40
+    norm = torch.nn.LayerNorm(C, device="cuda")
+    dt = torch.rand(B, device="cuda", generator=g)
+    data = mk(B, S, V)
+    for op, shapes in ((lambda x, sh, sc: dual_ops.ln_modulate(x, norm, sh, sc), [(B, S, C), (B, 1, C), (B, 1, C)]),
+                       (dual_ops.gated_residual, [(B, S, C), (B, S, C), (B, C)]), (dual_ops.gelu_tanh, [(B, S, C)]),
+                       (lambda l: dual_ops.flow_map_head(l, data, dt), [(B, S, V)])):
+        prim = tuple(mk(*s).to(dtype).requires_grad_(grad) for s in shapes)
+        tang = tuple(mk(*s).to(other) for s in shapes)
+        y, ty = torch.func.jvp(op, prim, tang)
+        want = torch.func.jvp(op, prim, tuple(t.to(dtype) for t in tang))
+        assert ty.dtype == want[1].dtype and torch.equal(y, want[0]) and torch.equal(ty, want[1])
+        if grad:
+            cots = [mk(*y.shape).to(y.dtype) for _ in range(2)]
+            for a, b in zip(torch.autograd.grad([y, ty], prim, cots), torch.autograd.grad(want, prim, cots)):
+                # (column sums are added by atomics in any order, and rounded once)
+                assert torch.allclose(a.float(), b.float(), rtol=2 ** -7, atol=1e-5)
+        for i in range(len(prim)):
+            with pytest.raises((ValueError, RuntimeError)):
+                torch.func.jvp(op, prim, tuple(t.to(dtype).cpu() if j == i else t.to(dtype) for j, t in enumerate(tang)))
+    assert _lib.device_status() == 0
