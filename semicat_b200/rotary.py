@@ -163,14 +163,15 @@ def rotary_qkv(qkv: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, out_dtyp
     """Split a (B, S, 3, H, D) projection into q, k, v (each contiguous (B, S, H, D) of ``out_dtype``) with q and k rotated
     as by :func:`apply_rotary_cast`, in one launch; the backward writes the projection's gradient in place in one launch
     (instead of three tensors that are concatenated afterwards).  Works under forward-mode AD.  Inputs the kernel does not
-    take (fp16, unaligned views) go through :func:`apply_rotary_cast` per tensor."""
+    take (fp16, unaligned views) go through :func:`apply_rotary_cast` per tensor; tables of fewer than (S, D / 2) entries are refused there."""
     if out_dtype in _QKV_CODES:
         out = native("rotary_qkv", qkv, cos, sin, out_dtype == torch.bfloat16)
         if out is not None:
             return out
     p, t = fwAD.unpack_dual(qkv)
     ok = (p.is_cuda and p.dim() == 5 and p.shape[2] == 3 and p.dtype in _QKV_CODES and out_dtype in _QKV_CODES and p.shape[-1] % 16 == 0
-          and p.stride(4) == 1 and all(st % 8 == 0 for st in p.stride()[:4]) and (p.storage_offset() * p.element_size()) % 16 == 0)
+          and p.stride(4) == 1 and all(st % 8 == 0 for st in p.stride()[:4]) and (p.storage_offset() * p.element_size()) % 16 == 0
+          and min(cos.numel(), sin.numel()) >= p.shape[1] * (p.shape[-1] // 2))
     if t is not None:
         ok = ok and t.dtype == p.dtype and t.device == p.device and t.stride() == p.stride() and (t.storage_offset() * t.element_size()) % 16 == 0
     if not ok:

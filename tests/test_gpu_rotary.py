@@ -149,3 +149,29 @@ def test_rotary_qkv_with_one_thread_for_all_three(shape):
     for a, b in zip(outs, want):
         assert torch.equal(a, b)
     assert torch.equal(torch.autograd.grad(outs, [xl], cots)[0], torch.autograd.grad(want, [xr], cots)[0])
+
+
+@pytest.mark.parametrize("cos,sin", [((7, 32), (8, 32)), ((8, 32), (8, 16)), ((8, 16), (8, 16)), ((255,), (256,))])
+def test_rotary_qkv_refuses_tables_that_are_too_small(cos, sin):
+    """The kernel reads S rows of D / 2 entries of either table."""
+    from semicat_b200.rotary import rotary_qkv
+
+    qkv = torch.randn(2, 8, 3, 4, 64, device="cuda").bfloat16()
+    cos, sin = torch.zeros(cos, device="cuda"), torch.zeros(sin, device="cuda")
+    with pytest.raises(ValueError):
+        rotary_qkv(qkv, cos, sin)
+    with pytest.raises(ValueError):
+        torch.func.jvp(lambda t: rotary_qkv(t, cos, sin), (qkv,), (qkv,))
+    with pytest.raises(ValueError):
+        rotary_qkv(qkv.clone().requires_grad_(True), cos, sin)
+
+
+@pytest.mark.parametrize("shape", [(9, 32), (1, 8, 32), (256,)])
+def test_rotary_qkv_takes_tables_in_other_shapes(shape):
+    from semicat_b200.rotary import rotary_qkv
+
+    qkv = torch.randn(2, 8, 3, 4, 64, device="cuda").bfloat16()
+    cos, sin = torch.randn(shape, device="cuda"), torch.randn(shape, device="cuda")
+    rows = lambda t: t.flatten()[:256].view(8, 32)
+    for a, b in zip(rotary_qkv(qkv, cos, sin), rotary_qkv(qkv, rows(cos), rows(sin))):
+        assert torch.equal(a, b)
