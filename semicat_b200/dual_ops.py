@@ -34,10 +34,11 @@ from ._nodes import apply, module, native, node, unrecorded
 from .ops import _on_device
 
 _CODES = {torch.bfloat16: 0, torch.float32: 2}
+CHANNELS = (256, 512, 768, 1024)  # that the LayerNorm and gate kernels take
 
 
 def _usable(x: torch.Tensor, *others) -> bool:
-    if not x.is_cuda or x.dim() != 3 or x.dtype not in _CODES or x.shape[-1] not in (256, 512, 768, 1024):
+    if not x.is_cuda or x.dim() != 3 or x.dtype not in _CODES or x.shape[-1] not in CHANNELS:
         return False
     return all(o is None or (o.dtype == x.dtype and o.is_cuda) for o in others)
 

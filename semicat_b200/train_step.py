@@ -26,7 +26,7 @@ import torch.nn as nn
 import torch.nn.functional as F
 
 from . import _nodes, vocab_ops
-from .dual_ops import dropout_seed, flow_map_head, gated_residual, gated_residual_ln, gelu_tanh, ln_modulate
+from .dual_ops import CHANNELS, dropout_seed, flow_map_head, gated_residual, gated_residual_ln, gelu_tanh, ln_modulate
 from .dual_ops import linear as dual_linear
 from .functional import safe_sdpa_jvp
 from .rotary import apply_rotary_cast, rotary_qkv
@@ -237,7 +237,10 @@ class _PassCasts:
 
     @staticmethod
     def chained(net):
-        """Whether the blocks may be run as one chain of operations: plain blocks that nobody listens to, no dropout."""
+        """Whether the blocks may be run as one chain of operations: plain blocks that nobody listens to, no dropout, and a width
+        that the LayerNorm and gate kernels take (for others it is autocast that makes torch's LayerNorm accept 16-bit rows)."""
+        if net.ada_out.weight.shape[0] not in [2 * c for c in CHANNELS]:
+            return False
         hooks = torch.nn.modules.module
         if hooks._global_forward_hooks or hooks._global_forward_pre_hooks:
             return False

@@ -71,3 +71,30 @@ def test_pass(monkeypatch, V, B, L, dtype, attention):
         assert of(net, plain, attention) is None
         with torch.autocast("cuda", dtype=dtype):
             assert of(net.half(), plain, attention) is None
+
+
+def _small(width=256, blocks=2, V=1003, L=32, **kw):
+    torch.manual_seed(0)
+    with torch.device("cuda"):
+        net = train_step.DiT(V, width, 64, blocks, width // 64, dropout=0.0, length=L, **kw)
+    train_step.randomise_zero_init(net)
+    x1 = torch.randint(0, V, (2, L), device="cuda")
+    noise = train_step.draw_noise(x1, V)
+    s, t = noise["u_sd"] * noise["t_sd"], noise["t_sd"]
+    return net.eval(), train_step.interpolate(noise["x0"], x1, s.view(-1, 1, 1)), s, t
+
+
+def _pass(net, x, s, t, **kw):
+    with torch.no_grad(), torch.autocast("cuda", dtype=torch.bfloat16):
+        return net(x, s, t, attention="lib", **kw)
+
+
+@pytest.mark.parametrize("width", [64, 128, 384])
+def test_pass_of_widths_without_a_kernel(monkeypatch, width):
+    """Widths that the LayerNorm and gate kernels do not take: the pass is that of autocast."""
+    net, *inputs = _small(width)
+    out = _pass(net, *inputs)
+    monkeypatch.setattr(train_step._PassCasts, "of", staticmethod(lambda *a: None))
+    want = _pass(net, *inputs)
+    assert out.shape == want.shape and out.dtype == want.dtype
+    assert float((out - want).float().norm() / want.float().norm()) < 2 ** -8  # as in test_pass
