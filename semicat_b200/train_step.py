@@ -192,8 +192,8 @@ class _PassCasts:
     at batch 8, length 128 and twelve blocks: 286 -> 143 launches, 3.7 -> 2.1 ms, of which :meth:`run` 24 and 0.4)."""
 
     def __init__(self, casts, ada, naive, biased):
-        n, self.sizes = len(ada), [m.out_features for m in ada]
-        rows, k = sum(self.sizes), ada[0].in_features
+        n, self.sizes = len(ada), [m.weight.shape[0] for m in ada]
+        rows, k = sum(self.sizes), ada[0].weight.shape[1]
         self.ada_weight = casts[0].as_strided((rows, k), (k, 1))
         self.ada_bias = casts[n].as_strided((rows,), (1,))
         rest = iter(casts[2 * n:])
@@ -204,19 +204,21 @@ class _PassCasts:
 
     @staticmethod
     def of(net, x, attention):
-        """For this pass of ``net``, or ``None`` where autocast is off, something may be recorded or a parameter is not
-        contiguous fp32."""
+        """For this pass of ``net``, or ``None`` where autocast is off, something may be recorded, a part of the model is not as
+        it was built or a parameter is not contiguous fp32."""
         if attention == "math" or not x.is_cuda or not torch.is_autocast_enabled("cuda") or not _nodes.unrecorded():
+            return None
+        if not all(_PassCasts._plain(b, Block) and b.ada.bias is not None for b in net.blocks) or net.ada_out.bias is None or net.head.bias is None:
             return None
         dtype = torch.get_autocast_dtype("cuda")
         ada = [blk.ada for blk in net.blocks] + [net.ada_out]
         if dtype not in (torch.bfloat16, torch.float16) or ada[0].weight.dtype != torch.float32 or getattr(net.head, "_prepared", None) is not None:
             return None
-        if any(m.weight.numel() % 8 or m.out_features % 8 or m.in_features != ada[0].in_features for m in ada):
+        if any(m.weight.shape[0] % 8 or m.weight.shape[1:] != ada[0].weight.shape[1:] for m in ada):
             return None  # they would not lie side by side
         params = [m.weight for m in ada] + [m.bias for m in ada] + [net.head.weight, net.head.bias]
         scale, align = [1.0] * len(params), [False] * (len(params) - 2) + [True] * 2
-        naive = isinstance(net.embed, NaiveEmbed)
+        naive = _PassCasts._plain(net.embed, NaiveEmbed) and net.embed.seq.bias is not None
         if naive:
             params += [net.embed.seq.weight, net.embed.seq.bias]
             scale += [1.0 / net.embed.coeff, 1.0]
@@ -236,22 +238,26 @@ class _PassCasts:
         return F.linear(cond, self.ada_weight, self.ada_bias).split(self.sizes, dim=1)
 
     @staticmethod
-    def chained(net):
-        """Whether the blocks may be run as one chain of operations: plain blocks that nobody listens to, no dropout, and a width
-        that the LayerNorm and gate kernels take (for others it is autocast that makes torch's LayerNorm accept 16-bit rows)."""
-        if net.ada_out.weight.shape[0] not in [2 * c for c in CHANNELS]:
-            return False
+    def _plain(module, cls):
+        """Whether calling ``module`` is ``cls.forward`` and nothing else: no subclass, wrapper, replaced method or hook, any of
+        which may look at the arguments or change them."""
         hooks = torch.nn.modules.module
-        if hooks._global_forward_hooks or hooks._global_forward_pre_hooks:
-            return False
-        return all(type(b) is Block and "forward" not in b.__dict__ and not (b._forward_hooks or b._forward_pre_hooks)
-                   and not (b.training and b.drop.p > 0.0) for b in net.blocks)
+        return (type(module) is cls and "forward" not in module.__dict__ and not (module._forward_hooks or module._forward_pre_hooks)
+                and not (hooks._global_forward_hooks or hooks._global_forward_pre_hooks))
+
+    @staticmethod
+    def chained(net):
+        """Whether the blocks may be run as one chain of operations: plain blocks, no dropout, and LayerNorms that the kernels take
+        (for others it is autocast that makes torch's LayerNorm accept 16-bit rows, and keeps its result in fp32)."""
+        norms = [n for b in net.blocks for n in (b.norm1, b.norm2)] + [net.norm_out]
+        return (len(net.blocks) > 0 and all(_PassCasts._plain(b, Block) and not (b.training and b.drop.p > 0.0) for b in net.blocks)
+                and all(isinstance(n, nn.LayerNorm) and n.weight is not None and n.weight.dtype == torch.float32
+                        and n.weight.numel() in CHANNELS for n in norms))
 
     def run(self, net, h, mods, attention):
         """``net``'s blocks and output normalisation: each gated residual goes with the LayerNorm behind it, also across blocks.
         Everything is in 16 bits, so autocast has nothing left to do."""
         B, S, C = h.shape
-        heads = net.blocks[0].heads
         rot = h.dtype if h.dtype in (torch.bfloat16, torch.float16) else torch.bfloat16
         parts = [m.unflatten(1, (-1, C)).unbind(1) for m in mods]
         norms = [b.norm1 for b in net.blocks] + [net.norm_out]
@@ -260,7 +266,7 @@ class _PassCasts:
             for i, blk in enumerate(net.blocks):
                 _, _, g1, sh2, sc2, g2 = parts[i]
                 qkv, out, up, down = self.blocks[i]
-                q, k, v = rotary_qkv(F.linear(n, *qkv).view(B, S, 3, heads, C // heads), net.cos, net.sin, rot)
+                q, k, v = rotary_qkv(F.linear(n, *qkv).view(B, S, 3, blk.heads, C // blk.heads), net.cos, net.sin, rot)
                 if attention in ("jvp", "lib"):
                     a = safe_sdpa_jvp(q, k, v)
                 else:

@@ -98,3 +98,63 @@ def test_pass_of_widths_without_a_kernel(monkeypatch, width):
     want = _pass(net, *inputs)
     assert out.shape == want.shape and out.dtype == want.dtype
     assert float((out - want).float().norm() / want.float().norm()) < 2 ** -8  # as in test_pass
+
+
+class _Wrapped(torch.nn.Module):
+    def __init__(self, inner):
+        super().__init__()
+        self.inner = inner
+
+    def forward(self, x, cos, sin, c, attention):
+        return self.inner(x, cos, sin, c, attention)
+
+
+class _FiveArguments(train_step.Block):
+    def forward(self, x, cos, sin, c, attention):
+        return super().forward(x, cos, sin, c, attention)
+
+
+def _changes(net, what):
+    blk = net.blocks[0]
+    if what == "wrapper":
+        net.blocks[0] = _Wrapped(blk)
+    elif what == "subclass":
+        blk.__class__ = _FiveArguments
+    elif what == "pre-hook":
+        blk.register_forward_pre_hook(lambda m, a: (*a[:3], a[3] * 2.0, *a[4:]))
+    elif what == "hook with arguments":
+        blk.register_forward_hook(lambda m, a, out: out * float(len(a)))
+    elif what == "own forward":
+        blk.forward = lambda x, cos, sin, c, attention: x
+    elif what == "ada without bias":
+        blk.ada.bias = None
+    elif what == "head without bias":
+        net.head.bias = None
+    elif what == "embedding hook":
+        net.embed.register_forward_pre_hook(lambda m, a: tuple(a) if len(a) == 3 else 1 / 0)
+    elif what == "embedding subclass":
+        class Embed(train_step.NaiveEmbed):
+            def forward(self, x, t, cond):
+                return super().forward(x, t, cond)
+        net.embed.__class__ = Embed
+    elif what == "norm without weight":
+        blk.norm1 = torch.nn.LayerNorm(256, elementwise_affine=False)
+    elif what == "norm in bf16":
+        blk.norm2.bfloat16()
+    elif what == "no blocks":
+        net.blocks = torch.nn.ModuleList()
+
+
+@pytest.mark.parametrize("what", ["wrapper", "subclass", "pre-hook", "hook with arguments", "own forward", "ada without bias", "head without bias",
+                                  "embedding hook", "embedding subclass", "norm without weight", "norm in bf16", "no blocks"])
+def test_pass_of_changed_models(monkeypatch, what):
+    """What a program has made of the model's parts is what runs."""
+    net, *inputs = _small()
+    plain = _pass(net, *inputs)
+    _changes(net, what)
+    out = _pass(net, *inputs)
+    monkeypatch.setattr(train_step._PassCasts, "of", staticmethod(lambda *a: None))
+    want = _pass(net, *inputs)
+    assert float((out - want).float().norm() / want.float().norm()) < 2 ** -8  # as in test_pass
+    if what in ("pre-hook", "hook with arguments", "own forward", "no blocks"):
+        assert float((plain - want).float().norm() / want.float().norm()) > 2 ** -5
