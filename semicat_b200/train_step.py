@@ -108,8 +108,7 @@ class Block(nn.Module):
         nn.init.zeros_(self.ada.bias)
 
     def linears(self):
-        up, _, down = self.mlp
-        return self.attn_qkv, self.attn_out, up, down
+        return self.attn_qkv, self.attn_out, self.mlp[0], self.mlp[2]
 
     def forward(self, x, cos, sin, c, attention, mod=None, cast=None):
         """``mod``, ``cast``: the adaLN projection of ``c`` and the (weight, bias) of :meth:`linears` in 16 bits, where the caller has

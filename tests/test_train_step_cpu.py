@@ -139,3 +139,11 @@ def test_noise_release_is_reported_once_and_buffers_refill_in_place(sd_prop):
     again = train_step.draw_noise(x1, VOCAB, out=noise)
     assert again is noise and noise["x0"].data_ptr() == ptr and not torch.equal(noise["x0"], before)
     assert noise["x0"].shape == before.shape and float(noise["t_vfm"].min()) >= 0.0 and float(noise["t_vfm"].max()) <= 1.0
+
+
+def test_an_mlp_of_more_modules_is_read_by_index():
+    blk = train_step.Block(32, 2, 8, 0.0)
+    blk.mlp.append(torch.nn.Identity())
+    assert blk.linears() == (blk.attn_qkv, blk.attn_out, blk.mlp[0], blk.mlp[2])
+    ang = torch.zeros(4, 8)
+    assert blk(torch.randn(1, 4, 32), ang.cos(), ang.sin(), torch.randn(1, 8), "math").shape == (1, 4, 32)
