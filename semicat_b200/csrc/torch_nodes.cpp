@@ -880,9 +880,13 @@ bool tangent_fits(const Tensor &t, const Tensor &p) {
          !t.is_conj() && !t.is_neg();
 }
 
+bool watched() {
+  return c10::impl::TorchDispatchModeTLS::any_modes_set() || at::impl::torch_function_mode_enabled() || torch::jit::tracer::isTracing();
+}
+
 // `jvp`: one torch.func.jvp is open and no other transform; else none is.
 bool fits(bool jvp, std::initializer_list<const Arg *> args) {
-  if (c10::impl::TorchDispatchModeTLS::any_modes_set() || at::impl::torch_function_mode_enabled() || torch::jit::tracer::isTracing()) return false;
+  if (watched()) return false;
   for (const Arg *a : args) {
     if (!a->ok) return false;
     if (!a->t.defined()) continue;
@@ -1021,9 +1025,10 @@ py::object rotary_py(bool jvp, py::handle qkv_, py::handle cos_, py::handle sin_
 }
 
 // 16-bit copies of contiguous fp32 CUDA parameters, side by side in one buffer (each from 16 bytes on): of a matrix as it is, or
-// (`align`) with rows and columns padded to multiples of 8; times `scale`.  None where they are not all of that kind.
+// (`align`) with rows and columns padded to multiples of 8; times `scale`.  None where they are not all of that kind, and under a
+// dispatch or function mode or a trace, which would not see the kernel's writes.
 py::object cast_params(const std::vector<Tensor> &params, const std::vector<double> &scale, const std::vector<bool> &align, bool bf16) {
-  if (params.empty() || scale.size() != params.size() || align.size() != params.size()) return py::none();
+  if (params.empty() || scale.size() != params.size() || align.size() != params.size() || watched()) return py::none();
   const Tensor &p0 = params[0];
   std::vector<jvpattn_cast> e(params.size());
   std::vector<int64_t> offset(params.size());

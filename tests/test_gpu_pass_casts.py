@@ -158,3 +158,23 @@ def test_pass_of_changed_models(monkeypatch, what):
     assert float((out - want).float().norm() / want.float().norm()) < 2 ** -8  # as in test_pass
     if what in ("pre-hook", "hook with arguments", "own forward", "no blocks"):
         assert float((plain - want).float().norm() / want.float().norm()) > 2 ** -5
+
+
+def test_modes_see_the_copies():
+    """Under a dispatch mode the pass makes its copies with torch's own operations, which the mode sees."""
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    class Casts(TorchDispatchMode):
+        seen = 0
+
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            self.seen += "_to_copy" in str(func)
+            return func(*args, **(kwargs or {}))
+
+    net, *inputs = _small()
+    with torch.no_grad():
+        want = [m.weight.bfloat16() for m in net.modules() if isinstance(m, torch.nn.Linear)]
+        with Casts() as mode:
+            assert _nodes.module().cast_params([net.head.weight], [1.0], [False], True) is None
+            _pass(net, *inputs)
+    assert mode.seen >= len(want)
