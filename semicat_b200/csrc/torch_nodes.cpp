@@ -596,15 +596,18 @@ Tensor column_sum(const Tensor &g) {
 struct LinearPrimal : Function<LinearPrimal> {
   static Tensor forward(AutogradContext *ctx, const Tensor &x, const Tensor &w, const Tensor &b) {
     at::AutoDispatchBelowADInplaceOrView below;
-    ctx->save_for_backward({x, w});
+    // (only what the backward reads: the rest may be freed, or written to)
+    ctx->save_for_backward({w.requires_grad() ? x : Tensor(), x.requires_grad() ? w : Tensor()});
+    ctx->saved_data["x"] = x.sizes().vec();
     return at::linear(x, w, b);
   }
   static variable_list backward(AutogradContext *ctx, const variable_list &g) {
     const auto s = ctx->get_saved_variables();
-    const Tensor x = s[0], w = s[1], g2 = g[0].reshape({-1, w.size(0)});
+    const std::vector<int64_t> shape = ctx->saved_data["x"].toIntVector();
+    const Tensor x = s[0], w = s[1], g2 = g[0].reshape({-1, g[0].size(-1)});
     variable_list d(3);
-    if (ctx->needs_input_grad(0)) d[0] = at::mm(g2, w).view(x.sizes());
-    if (ctx->needs_input_grad(1)) d[1] = at::mm(g2.t(), x.reshape({-1, w.size(1)}));
+    if (ctx->needs_input_grad(0)) d[0] = at::mm(g2, w).view(shape);
+    if (ctx->needs_input_grad(1)) d[1] = at::mm(g2.t(), x.reshape({-1, shape.back()}));
     if (ctx->needs_input_grad(2)) d[2] = column_sum(g2);
     return d;
   }

@@ -335,3 +335,17 @@ def test_tangents_of_another_kind():
     for got, i in ((q, 0), (k, 1)):
         _equal(got, [rotary.apply_rotary_cast(t[:, :, i], cos, sin) for t in (qkv, tqkv)])
     _equal([t.contiguous() for t in v], [t[:, :, 2].contiguous() for t in (qkv, tqkv)])  # (Tensor.to leaves what has the type already)
+
+
+def test_a_bias_alone_keeps_no_input():
+    """Where only the bias wants a gradient nothing of the input or the weight is needed again, and either may be written to."""
+    x, w, b = _rand(0, 4, 32), _rand(1, 24, 32), _rand(2, 24).requires_grad_(True)
+    y = dual_ops.linear(x, w, b)
+    x.zero_(), w.zero_()
+    (db,) = torch.autograd.grad(y, [b], torch.ones_like(y))
+    assert torch.equal(db, torch.full_like(db, 4.0))
+    x = _rand(0, 4, 32).requires_grad_(True)
+    w = _rand(1, 24, 32)
+    y = dual_ops.linear(x * 1.0, w, b)
+    dx, db = torch.autograd.grad(y, [x, b], torch.ones_like(y))
+    assert torch.equal(dx, torch.ones_like(y) @ w) and torch.equal(db, torch.full_like(db, 4.0))
