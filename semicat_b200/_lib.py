@@ -16,6 +16,7 @@ _PKG_DIR = os.path.dirname(os.path.abspath(__file__))
 _CSRC = os.path.join(_PKG_DIR, "csrc")
 LIB_PATH = os.path.join(_PKG_DIR, "libjvpattn.so")
 NATIVE_PATH = os.path.join(_PKG_DIR, "_native.so")  # the autograd nodes, see csrc/torch_nodes.cpp
+NATIVE_TORCH_PATH = NATIVE_PATH + ".torch"  # the torch version they were compiled against
 SOURCES = ["jvpattn_api.cu", "jvpattn_simt.cu", "jvpattn_sm100_fwd.cu", "jvpattn_sm100_bwd.cu",
            "jvpattn_sm100_bwd_short.cu", "sm100_tensormap.cu", "rotary.cu", "dual_pointwise.cu", "vocab_head.cu",
            "vocab_loss.cu", "cast_params.cu", "column_sum.cu"]
@@ -96,8 +97,20 @@ def build(force: bool = False, verbose: bool = False) -> str:
     return LIB_PATH
 
 
+def _native_torch() -> str | None:
+    """The torch version that ``_native.so`` was compiled against, where that was written down beside it."""
+    try:
+        with open(NATIVE_TORCH_PATH) as f:
+            return f.read().strip()
+    except FileNotFoundError:
+        return None
+
+
 def native_built() -> bool:
-    return os.path.exists(NATIVE_PATH)
+    """Whether ``_native.so`` is there and not known to be of another torch than the one installed."""
+    import torch
+
+    return os.path.exists(NATIVE_PATH) and _native_torch() in (None, torch.__version__)
 
 
 def build_native(force: bool = False) -> str:
@@ -109,7 +122,7 @@ def build_native(force: bool = False) -> str:
 
     src = os.path.join(_CSRC, "torch_nodes.cpp")
     deps = [src, os.path.join(os.path.dirname(_PKG_DIR), "include", "jvpattn.h")]
-    if not force and native_built() and all(os.path.getmtime(d) <= os.path.getmtime(NATIVE_PATH) for d in deps):
+    if not force and native_built() and _native_torch() and all(os.path.getmtime(d) <= os.path.getmtime(NATIVE_PATH) for d in deps):
         return NATIVE_PATH
     build()
     cuda = os.path.dirname(os.path.dirname(shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"))
@@ -122,6 +135,8 @@ def build_native(force: bool = False) -> str:
     if proc.returncode != 0:
         raise RuntimeError("g++ failed:\n" + proc.stdout + proc.stderr)
     os.replace(NATIVE_PATH + ".tmp", NATIVE_PATH)
+    with open(NATIVE_TORCH_PATH, "w") as f:
+        f.write(torch.__version__ + "\n")
     return NATIVE_PATH
 
 
@@ -140,7 +155,7 @@ def load() -> ctypes.CDLL:
         if not os.path.exists(LIB_PATH):
             raise RuntimeError(
                 f"{LIB_PATH} is missing: build it with `python -c 'import __graft_entry__ as g; g.build()'` "
-                "(or semicat_b200._lib.build()).  There is no CPU or PyTorch fallback for these kernels.")
+                "(or semicat_b200._lib.build(), and build_native() for the autograd nodes).  There is no CPU or PyTorch fallback for these kernels.")
         lib = ctypes.CDLL(LIB_PATH)
         T = ctypes.POINTER(Tensor4)
         P = ctypes.POINTER(Problem)

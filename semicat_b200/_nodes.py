@@ -5,6 +5,7 @@ from __future__ import annotations
 
 import importlib
 import inspect
+import warnings
 
 import torch
 import torch.autograd.forward_ad as fwAD
@@ -30,7 +31,7 @@ def apply(cls, *args):
     return cls.forward(*args) if unrecorded() else cls.apply(*args)
 
 
-_module = None
+_module = None  # the compiled module; False where there is none for this torch
 
 
 def _load():
@@ -39,7 +40,11 @@ def _load():
 
     _lib.load()  # says how to build what is missing
     if not _lib.native_built():
-        raise RuntimeError(f"{_lib.NATIVE_PATH} is missing: build it with `python -c 'import __graft_entry__ as g; g.build()'`")
+        warnings.warn(f"{_lib.NATIVE_PATH} is missing or was compiled against another torch than {torch.__version__}: the ops run through "
+                      "their classes in Python, whose calls take three times as long on the host.  Build it with "
+                      "`python -c 'import __graft_entry__ as g; g.build()'` (or semicat_b200._lib.build_native()).", RuntimeWarning, stacklevel=3)
+        _module = False
+        return False
     mod = importlib.import_module("semicat_b200._native")
     mod.set_kernels(functional._kernels)
     _module = mod
@@ -47,18 +52,19 @@ def _load():
 
 
 def set_kernels(kind: int) -> None:
-    if _module is not None:
+    if _module:
         _module.set_kernels(kind)
 
 
 def module():
-    """The compiled module (loaded on first use; CUDA only)."""
-    return _module or _load()
+    """The compiled module (loaded on first use; CUDA only), or ``False``."""
+    return _load() if _module is None else _module
 
 
 def native(name: str, first: torch.Tensor, *args):
     """Op ``name`` of ``csrc/torch_nodes.cpp`` on these arguments, or ``None`` where the situation or the inputs are none of
-    its own: outside all function transforms, or inside one ``torch.func.jvp`` and nothing else, on plain CUDA tensors.
+    its own: outside all function transforms, or inside one ``torch.func.jvp`` and nothing else, on plain CUDA tensors, with the
+    module built.
     (One attention call under ``torch.func.jvp`` with its gradients: 780-850 us through the classes here, 230-260 us so; a sampling pass of the
     twelve-block denoiser 6.7 -> 3.7 ms.)"""
     if not first.is_cuda or torch.compiler.is_compiling():
@@ -68,4 +74,5 @@ def native(name: str, first: torch.Tensor, *args):
         levels = torch._C._functorch.get_interpreter_stack()
         if len(levels) != 1 or levels[0].key() != torch._C._functorch.TransformType.Jvp:
             return None
-    return getattr(_module or _load(), name)(jvp, first, *args)
+    mod = _load() if _module is None else _module
+    return getattr(mod, name)(jvp, first, *args) if mod else None

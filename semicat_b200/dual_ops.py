@@ -403,7 +403,7 @@ def gated_residual(skip: torch.Tensor, branch: torch.Tensor, gate: torch.Tensor,
 def gated_residual_ln(skip, branch, gate, norm: torch.nn.LayerNorm, shift, scale):
     """``z = gated_residual(skip, branch, gate)`` and ``ln_modulate(z, norm, shift, scale)``, in one launch where nothing is
     recorded and the kernel takes the shapes."""
-    if unrecorded() and skip.is_cuda and norm.weight is not None and norm.normalized_shape == skip.shape[-1:]:
+    if unrecorded() and skip.is_cuda and norm.weight is not None and norm.normalized_shape == skip.shape[-1:] and module():
         out = module().gate_ln(skip, branch, gate, norm.weight, norm.bias, shift, scale, norm.eps)
         if out is not None:
             return out

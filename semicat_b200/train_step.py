@@ -205,7 +205,7 @@ class _PassCasts:
     def of(net, x, attention):
         """For this pass of ``net``, or ``None`` where autocast is off, something may be recorded, a part of the model is not as
         it was built or a parameter is not contiguous fp32."""
-        if attention == "math" or not x.is_cuda or not torch.is_autocast_enabled("cuda") or not _nodes.unrecorded():
+        if attention == "math" or not x.is_cuda or not torch.is_autocast_enabled("cuda") or not _nodes.unrecorded() or not _nodes.module():
             return None
         if not all(_PassCasts._plain(b, Block) and b.ada.bias is not None for b in net.blocks) or net.ada_out.bias is None or net.head.bias is None:
             return None

@@ -1,10 +1,13 @@
 """When the library's autograd nodes may be left out: only where nothing could be recorded."""
 import inspect
+import types
+import warnings
 
+import pytest
 import torch
 import torch.autograd.forward_ad as fwAD
 
-from semicat_b200 import _nodes, dual_ops, functional, rotary
+from semicat_b200 import _lib, _nodes, dual_ops, functional, rotary
 
 
 def test_unrecorded_only_without_gradients_transforms_and_forward_mode():
@@ -87,3 +90,25 @@ def test_a_trace_records_the_node():
         seen = []
         torch.jit.trace(lambda x: (seen.append(_nodes.unrecorded()), x + 1)[1], (torch.ones(3),), check_trace=False)
         assert seen == [False]
+
+
+def test_without_the_compiled_module_the_classes_run(monkeypatch, tmp_path):
+    """Missing, or compiled against another torch: the native entries take no call, and say so once."""
+    _lib.build()
+    monkeypatch.setattr(_lib, "NATIVE_PATH", str(tmp_path / "_native.so"))
+    monkeypatch.setattr(_lib, "NATIVE_TORCH_PATH", str(tmp_path / "_native.so.torch"))
+    assert not _lib.native_built()
+    (tmp_path / "_native.so").write_bytes(b"")
+    assert _lib.native_built()
+    (tmp_path / "_native.so.torch").write_text("1.0\n")
+    assert not _lib.native_built()
+    monkeypatch.setattr(_nodes, "_module", None)
+    cuda = types.SimpleNamespace(is_cuda=True)
+    with pytest.warns(RuntimeWarning, match="compiled against another torch"):
+        assert _nodes.native("gelu", cuda) is None
+    with warnings.catch_warnings():
+        warnings.simplefilter("error")
+        assert _nodes.native("gelu", cuda) is None and not _nodes.module()
+        _nodes.set_kernels(0)
+    (tmp_path / "_native.so.torch").write_text(torch.__version__ + "\n")
+    assert _lib.native_built()
