@@ -882,12 +882,14 @@ constexpr int kFinalSamples = 4;  // samples per thread of the finalize kernel
 // channels 11.4 -> 3.1 us, 8 samples 10.1 -> 2.3.)
 template <typename T>
 __global__ void ln_finalize_kernel(LnFinalArgs a) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  // (one grid axis for channels and samples: the second holds no more than 65535)
+  const unsigned chunks = ((unsigned)a.C + blockDim.x - 1) / blockDim.x;
+  const int c = blockIdx.x % chunks * blockDim.x + threadIdx.x;
   if (c >= a.C) return;
   const float gam = a.gamma[c], bet = a.beta ? a.beta[c] : 0.f;
   float dg = 0.f, db = 0.f;
   const int64_t BC = (int64_t)a.B * a.C;
-  const int b0 = blockIdx.y * kFinalSamples;
+  const int b0 = blockIdx.x / chunks * kFinalSamples;
   float sc1[kFinalSamples], tsc[kFinalSamples], p[2][kFinalSamples], t[3][kFinalSamples];
 #pragma unroll
   for (int k = 0; k < kFinalSamples; ++k) {
@@ -1260,9 +1262,10 @@ cudaError_t ln_finalize(const float *p, const float *t, const float *gamma, cons
   LnFinalArgs a{p, t, gamma, beta, scale, tscale, mod_stride, tmod_stride, d_shift, d_scale, d_tshift, d_tscale, d_gamma, d_beta, B, C};
   LaunchScope scope(kIdDual, stream);
   if (B == 0) return cudaSuccess;
-  const dim3 grid((unsigned)((C + 127) / 128), (unsigned)((B + kFinalSamples - 1) / kFinalSamples));
-  if (dtype == JVPATTN_BF16) ln_finalize_kernel<__nv_bfloat16><<<grid, 128, 0, stream>>>(a);
-  else if (dtype == JVPATTN_FP32) ln_finalize_kernel<float><<<grid, 128, 0, stream>>>(a);
+  const int64_t grid = (int64_t)((C + 127) / 128) * (((int64_t)B + kFinalSamples - 1) / kFinalSamples);
+  if (grid > INT32_MAX) return cudaErrorInvalidValue;
+  if (dtype == JVPATTN_BF16) ln_finalize_kernel<__nv_bfloat16><<<(unsigned)grid, 128, 0, stream>>>(a);
+  else if (dtype == JVPATTN_FP32) ln_finalize_kernel<float><<<(unsigned)grid, 128, 0, stream>>>(a);
   else return cudaErrorInvalidValue;
   return cudaGetLastError();
 }

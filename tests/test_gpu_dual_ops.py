@@ -368,3 +368,20 @@ def test_tangents_of_another_type(dtype, other, grad):
             with pytest.raises((ValueError, RuntimeError)):
                 torch.func.jvp(op, prim, tuple(t.to(dtype).cpu() if j == i else t.to(dtype) for j, t in enumerate(tang)))
     assert _lib.device_status() == 0
+
+
+@pytest.mark.parametrize("B", [262139, 262141, 524289])
+def test_ln_modulate_gradients_of_many_samples(B):
+    """One row per sample: the gradient of shift is the cotangent itself, that of scale the cotangent times the normalised row
+    (one rounding to 16 bits, 2^-8, and fp32 sums below it)."""
+    C = 256
+    g = torch.Generator(device="cuda").manual_seed(0)
+    mk = lambda: torch.randn(B, 1, C, device="cuda", generator=g).bfloat16()
+    norm = torch.nn.LayerNorm(C, device="cuda")
+    x, gy, shift, scale = mk(), mk(), mk().requires_grad_(True), mk().requires_grad_(True)
+    y = dual_ops.ln_modulate(x, norm, shift, scale)
+    d_shift, d_scale = torch.autograd.grad(y, [shift, scale], gy)
+    assert torch.equal(d_shift, gy)
+    want = torch.nn.functional.layer_norm(x.float(), (C,)) * gy.float()
+    assert bool(((d_scale.float() - want).abs() <= 2 ** -7 * want.abs() + 1e-5).all())
+    assert _lib.device_status() == 0
