@@ -300,10 +300,14 @@ uint64_t jvpattn_launch_count(void);
 /* Optional per-kernel timing for measurement harnesses (no counterpart in the reference, which relies on
  * triton.testing.do_bench around whole calls, ryu_triton.py:958-1007).  Between _begin and _end every
  * launch is bracketed by CUDA events on its stream; _end synchronises the device and returns, per kernel
- * id in [0, JVPATTN_NUM_KERNELS), the summed device time in milliseconds and the launch count. */
-#define JVPATTN_NUM_KERNELS 10
+ * id, the summed device time in milliseconds and the launch count: _end_n of the ids in [0, n), whatever their
+ * number (zero beyond JVPATTN_KERNEL_IDS); _end of the JVPATTN_NUM_KERNELS ids that the first version of this
+ * interface had, for callers whose arrays hold no more. */
+#define JVPATTN_NUM_KERNELS 9
+#define JVPATTN_KERNEL_IDS 10
 int jvpattn_profile_begin(void);
 int jvpattn_profile_end(double *total_ms, uint64_t *launches);
+int jvpattn_profile_end_n(int n, double *total_ms, uint64_t *launches);
 const char *jvpattn_kernel_name(int id);
 
 /* Synchronises the current device and returns the device-side status word: 0 if no bounded wait has

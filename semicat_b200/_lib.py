@@ -31,7 +31,7 @@ KERNELS_AUTO, KERNELS_SIMT, KERNELS_TCGEN05 = 0, 1, 2
 EXPORTS = (
     "jvpattn_fwd", "jvpattn_bwd", "jvpattn_bwd_workspace_bytes", "jvpattn_selected_kernels",
     "jvpattn_launch_count", "jvpattn_device_status", "jvpattn_strerror", "jvpattn_last_cuda_error",
-    "jvpattn_abi_version", "jvpattn_profile_begin", "jvpattn_profile_end", "jvpattn_kernel_name",
+    "jvpattn_abi_version", "jvpattn_profile_begin", "jvpattn_profile_end", "jvpattn_profile_end_n", "jvpattn_kernel_name",
     "jvpattn_bwd_static", "jvpattn_rotary_cast", "jvpattn_stream_check", "jvpattn_debug_set",
     "jvpattn_ln_modulate", "jvpattn_ln_modulate_dual", "jvpattn_gated_residual", "jvpattn_flow_map_head", "jvpattn_gelu_dual", "jvpattn_vocab_op",
     "jvpattn_gated_residual_dual", "jvpattn_ln_finalize", "jvpattn_rotary_qkv", "jvpattn_cast_params", "jvpattn_gate_ln",
@@ -211,6 +211,8 @@ def load() -> ctypes.CDLL:
         lib.jvpattn_profile_begin.restype = ctypes.c_int
         lib.jvpattn_profile_end.argtypes = [ctypes.POINTER(ctypes.c_double), ctypes.POINTER(ctypes.c_uint64)]
         lib.jvpattn_profile_end.restype = ctypes.c_int
+        lib.jvpattn_profile_end_n.argtypes = [ctypes.c_int, *lib.jvpattn_profile_end.argtypes]
+        lib.jvpattn_profile_end_n.restype = ctypes.c_int
         lib.jvpattn_kernel_name.argtypes = [ctypes.c_int]
         lib.jvpattn_kernel_name.restype = ctypes.c_char_p
         if lib.jvpattn_abi_version() != 1:
@@ -257,5 +259,5 @@ def profile_end() -> dict:
     lib = load()
     ms = (ctypes.c_double * NUM_KERNELS)()
     n = (ctypes.c_uint64 * NUM_KERNELS)()
-    check(lib.jvpattn_profile_end(ms, n), "jvpattn_profile_end")
+    check(lib.jvpattn_profile_end_n(NUM_KERNELS, ms, n), "jvpattn_profile_end_n")
     return {lib.jvpattn_kernel_name(i).decode(): (float(ms[i]), int(n[i])) for i in range(NUM_KERNELS) if n[i]}

@@ -461,18 +461,21 @@ int jvpattn_profile_begin(void) {
   return JVPATTN_OK;
 }
 
-int jvpattn_profile_end(double *total_ms, uint64_t *launches) {
+int jvpattn_profile_end(double *total_ms, uint64_t *launches) { return jvpattn_profile_end_n(JVPATTN_NUM_KERNELS, total_ms, launches); }
+
+int jvpattn_profile_end_n(int n, double *total_ms, uint64_t *launches) {
+  if (n < 0) return JVPATTN_EINVAL;
   g_profiling.store(false);
   cudaError_t e = cudaDeviceSynchronize();
   std::lock_guard<std::mutex> lock(g_prof_mutex);
-  for (int i = 0; i < JVPATTN_NUM_KERNELS; ++i) {
+  for (int i = 0; i < n; ++i) {
     if (total_ms) total_ms[i] = 0.0;
     if (launches) launches[i] = 0;
   }
   for (ProfSlot *slot : g_prof_slots) {
     float ms = 0.f;
     if (e == cudaSuccess && cudaEventElapsedTime(&ms, slot->start, slot->stop) == cudaSuccess && slot->id >= 0 &&
-        slot->id < JVPATTN_NUM_KERNELS) {
+        slot->id < n) {
       if (total_ms) total_ms[slot->id] += ms;
       if (launches) launches[slot->id] += 1;
     }
@@ -486,7 +489,7 @@ int jvpattn_profile_end(double *total_ms, uint64_t *launches) {
 }
 
 const char *jvpattn_kernel_name(int id) {
-  static_assert(kNumKernelIds == JVPATTN_NUM_KERNELS, "kernel id table");
+  static_assert(kNumKernelIds == JVPATTN_KERNEL_IDS, "kernel id table");
   switch (id) {
     case kIdFwdTc: return "sm100_fwd_kernel";
     case kIdRowDots: return "row_dots_kernel";

@@ -87,3 +87,15 @@ def test_backward_scratch_is_two_row_vectors(lib, B, H, Lq):
         need = lib.jvpattn_bwd_workspace_bytes(ctypes.byref(p))
         assert need == (8 * B * H * stat + 255) // 256 * 256
     assert 8 * _lib.STATIC_SCRATCH_ROWS == 2 * 1024 * 1024
+
+
+def test_profile_end_writes_what_the_first_version_wrote(lib):
+    """Callers of ABI version 1 have arrays of nine entries; more are written only where the caller says how many there are."""
+    F, N = ctypes.c_double * 12, ctypes.c_uint64 * 12
+    for n in (9, 0, 10, 12):
+        ms, launches = F(*[7.0] * 12), N(*[7] * 12)
+        lib.jvpattn_profile_begin()
+        lib.jvpattn_profile_end(ms, launches) if n == 9 else lib.jvpattn_profile_end_n(n, ms, launches)
+        assert list(ms) == [0.0] * n + [7.0] * (12 - n) and list(launches) == [0] * n + [7] * (12 - n)
+    assert [lib.jvpattn_kernel_name(i) == b"?" for i in range(_lib.NUM_KERNELS + 1)] == [False] * _lib.NUM_KERNELS + [True]
+    assert lib.jvpattn_profile_end_n(-1, None, None) == -1
