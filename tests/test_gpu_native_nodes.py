@@ -19,8 +19,8 @@ def _both_ways(monkeypatch, f):
 
     def strict(*a):
         out = _nodes.native(*a)
-        if out is None and a[0] != "linear":  # (which is torch's own without a tangent)
-            refused.append(a[0])
+        if out is None and (a[0] != "linear" or torch.autograd.forward_ad.unpack_dual(a[1]).tangent is not None):
+            refused.append(a[0])  # (a linear layer without a tangent is torch's own)
         return out
 
     for way in (strict, lambda *a: None):

@@ -121,10 +121,11 @@ def test_forced_tcgen05_rejects_what_it_cannot_run():
         G.run(ins, kernels=ops.KERNELS_TCGEN05, mode=None)
     assert e.value.code == -1
 
-@pytest.mark.parametrize("shape", [(64, 12, 128, 64), (3, 5, 640, 64), (2, 3, 384, 128)])
+@pytest.mark.parametrize("shape", [(64, 12, 128, 64), (3, 5, 640, 64), (2, 3, 384, 128), (32, 12, 192, 64), (16, 12, 192, 128)])
 def test_backward_launch_overlap_is_ordered(shape):
     """The backward's three (d = 128: four) launches overlap: the query owner starts while the row-dot kernel
-    drains and the key owner runs beside the query owner.  Every call must still see complete row dots: the
+    drains and the key owner runs beside the query owner, here with fewer work items than SMs and with several per CTA.
+    (Length 128 at d = 64 is one launch without scratch.)  Every call must still see complete row dots: the
     scratch is poisoned with NaN before each of many back-to-back calls (no synchronisation between them), all
     results must be finite and bit-identical to the first call's, and the first call's must match the oracle."""
     B, H, L, D = shape
@@ -143,8 +144,10 @@ def test_backward_launch_overlap_is_ordered(shape):
     for r in range(rounds):
         if ws is not None:
             ws.view(torch.float32).fill_(float("nan"))
+        launches = _lib.launch_count()
         ws = ops.jvp_attention_bwd(t["q"], t["k"], t["v"], t["tq"], t["tk"], t["tv"], o, to, g_o, g_to, lse, mu,
                                    *grads[r], workspace=ws)
+        assert _lib.launch_count() - launches == (4 if D == 128 else 3 if L > 128 else 1)
         if r == 0:
             ws.view(torch.float32).fill_(float("nan"))  # the very first call ran on unpoisoned scratch: redo it
             ops.jvp_attention_bwd(t["q"], t["k"], t["v"], t["tq"], t["tk"], t["tv"], o, to, g_o, g_to, lse, mu,

@@ -1,5 +1,6 @@
 """GPU: many back-to-back forward + backward calls replayed from a CUDA graph, at the shape the training step gives the
-library (128 samples x 12 heads, length 128, head dimension 64), in the three cotangent modes.
+library (128 samples x 12 heads, length 128, head dimension 64; its backward is one kernel) and at a length whose backward is
+the chain of row dots, query owner and key owner, in the three cotangent modes.
 
 With several MMA-issuing threads per CTA the roles of a kernel run ahead of one another by whole tiles; a wait that is
 only correct while the waiter stays within one barrier phase of the signaller then fails rarely and only under
@@ -16,8 +17,9 @@ if torch.cuda.is_available():
 
 
 @pytest.mark.parametrize("mode", ["tan", "both", "pri"])
-def test_graph_replays_back_to_back(mode):
-    B, H, L, D = 128, 12, 128, 64
+@pytest.mark.parametrize("B,L", [(128, 128), (64, 192)])
+def test_graph_replays_back_to_back(B, L, mode):
+    H, D = 12, 64
     g = torch.Generator(device="cuda").manual_seed(1)
     mk = lambda: torch.randn(B, L, H, D, device="cuda", generator=g).bfloat16().transpose(1, 2)
     q, k, v, tq, tk, tv, go, gto = (mk() for _ in range(8))
@@ -36,7 +38,9 @@ def test_graph_replays_back_to_back(mode):
             ws[0] = ops.jvp_attention_bwd(q, k, v, tq, tk, tv, o, to, go if mode == "both" else None, gto, lse, mu, *grads,
                                           workspace=ws[0])
 
+    launches = _lib.launch_count()
     step()
+    assert _lib.launch_count() - launches == 1 + (1 if L <= 128 else 3)
     torch.cuda.synchronize()
     assert _lib.device_status() == 0
     first = [x.clone() for x in (o, to, *grads[:n_out])]
