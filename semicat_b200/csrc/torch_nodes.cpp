@@ -574,13 +574,14 @@ std::tuple<Tensor, Tensor> linear_pair(const Tensor &x, const Tensor &tx, const 
 }
 
 // The sum of a matrix over its rows: by the library's kernel for plain bf16 values, by torch's reduction for whatever else a backward
-// pass may be given (batched, dual or recorded cotangents, other types).
+// pass may be given (batched, dual or recorded cotangents, other types), and for a single row or 8 columns, where that is faster
+// (1 x 768 2.3 against 2.7 us; 262144 x 8 10.4 against 12.8, of 16 columns 14.5 against 13.1).
 Tensor column_sum(const Tensor &g) {
   const auto keys = g.key_set();
   if (g.scalar_type() != at::kBFloat16 || !g.is_cuda() || g.layout() != at::kStrided || keys.has(c10::DispatchKey::Python) ||
       keys.has(c10::DispatchKey::Functionalize) || keys.has(c10::DispatchKey::FuncTorchBatched) || keys.has(c10::DispatchKey::Batched) ||
       keys.has(c10::DispatchKey::FuncTorchGradWrapper) || !g.has_storage() || g.is_neg() || c10::impl::TorchDispatchModeTLS::any_modes_set() ||
-      (at::GradMode::is_enabled() && g.requires_grad()) || g._fw_grad(0).defined() || g.size(1) % 8 || g.numel() == 0 || g.stride(1) != 1 ||
+      (at::GradMode::is_enabled() && g.requires_grad()) || g._fw_grad(0).defined() || g.size(1) % 8 || g.size(0) < 2 || g.size(1) < 16 || g.stride(1) != 1 ||
       g.stride(0) % 8 || g.stride(0) < g.size(1) || (g.storage_offset() * 2) % 16)
     return g.sum(0);
   at::AutoDispatchBelowADInplaceOrView below;

@@ -349,3 +349,14 @@ def test_a_bias_alone_keeps_no_input():
     y = dual_ops.linear(x * 1.0, w, b)
     dx, db = torch.autograd.grad(y, [x, b], torch.ones_like(y))
     assert torch.equal(dx, torch.ones_like(y) @ w) and torch.equal(db, torch.full_like(db, 4.0))
+
+
+@pytest.mark.parametrize("rows,cols,launches", [(1, 768, 0), (2, 768, 2), (4096, 8, 0), (4096, 16, 2)])
+def test_bias_gradient_by_torch_where_that_is_faster(rows, cols, launches):
+    x, w, b = _rand(0, rows, 16), _rand(1, cols, 16), _rand(2, cols).requires_grad_(True)
+    y, g = dual_ops.linear(x, w, b), _rand(3, rows, cols)
+    before = _lib.launch_count()
+    (db,) = torch.autograd.grad(y, [b], g)
+    assert _lib.launch_count() - before == launches
+    ref, size = g.double().sum(0), g.double().abs().sum(0)  # (bound as in test_bias_gradient)
+    assert bool(((db.double() - ref).abs() <= 2 ** -8 * ref.abs() + 2 ** -17 * size).all())
