@@ -108,7 +108,8 @@ class Block(nn.Module):
         nn.init.zeros_(self.ada.bias)
 
     def linears(self):
-        return self.attn_qkv, self.attn_out, self.mlp[0], self.mlp[2]
+        layers = list(self.mlp)  # (indexing a Sequential takes 2 us each)
+        return self.attn_qkv, self.attn_out, layers[0], layers[2]
 
     def forward(self, x, cos, sin, c, attention, mod=None, cast=None):
         """``mod``, ``cast``: the adaLN projection of ``c`` and the (weight, bias) of :meth:`linears` in 16 bits, where the caller has
@@ -184,15 +185,20 @@ class NaiveEmbed(nn.Module):
         return _aligned_linear(x, self.seq, 1.0 / self.coeff, prepared=prepared)
 
 
+def _params(module):
+    """(weight, bias) of a module."""
+    own = module._parameters
+    return (own["weight"], own["bias"]) if "weight" in own and "bias" in own else (module.weight, module.bias)
+
+
 class _PassCasts:
     """The 16-bit copies of a model's ``nn.Linear`` parameters for one pass under autocast in which nothing is recorded.  Autocast
     itself makes one launch per parameter, and more for the padded vocabulary-sized ones; here two launches make all of
     them, the adaLN projections' side by side, so that one GEMM gives the modulation of every block (a sampling pass
     at batch 8, length 128 and twelve blocks: 286 -> 143 launches, 3.7 -> 2.1 ms, of which :meth:`run` 24 and 0.4)."""
 
-    def __init__(self, casts, ada, naive, biased):
-        n, self.sizes = len(ada), [m.weight.shape[0] for m in ada]
-        rows, k = sum(self.sizes), ada[0].weight.shape[1]
+    def __init__(self, casts, sizes, k, naive, biased):
+        n, rows, self.sizes = len(sizes), sum(sizes), sizes
         self.ada_weight = casts[0].as_strided((rows, k), (k, 1))
         self.ada_bias = casts[n].as_strided((rows,), (1,))
         rest = iter(casts[2 * n:])
@@ -207,31 +213,35 @@ class _PassCasts:
         it was built or a parameter is not contiguous fp32."""
         if attention == "math" or not x.is_cuda or not torch.is_autocast_enabled("cuda") or not _nodes.unrecorded() or not _nodes.module():
             return None
-        if not all(_PassCasts._plain(b, Block) and b.ada.bias is not None for b in net.blocks) or net.ada_out.bias is None or net.head.bias is None:
+        blocks = _PassCasts._plain_blocks(net)
+        if blocks is None:
             return None
         dtype = torch.get_autocast_dtype("cuda")
-        ada = [blk.ada for blk in net.blocks] + [net.ada_out]
-        if dtype not in (torch.bfloat16, torch.float16) or ada[0].weight.dtype != torch.float32 or getattr(net.head, "_prepared", None) is not None:
+        # (parameters are taken from the modules' own tables: a pass that is bound by the host asks some hundred attributes here)
+        ada = [_params(b._modules["ada"]) for b in blocks] + [_params(net.ada_out)]
+        head, embed, first = _params(net.head), net.embed, ada[0][0]
+        if dtype not in (torch.bfloat16, torch.float16) or first.dtype != torch.float32 or getattr(net.head, "_prepared", None) is not None:
             return None
-        if any(m.weight.shape[0] % 8 or m.weight.shape[1:] != ada[0].weight.shape[1:] for m in ada):
-            return None  # they would not lie side by side
-        params = [m.weight for m in ada] + [m.bias for m in ada] + [net.head.weight, net.head.bias]
+        k = first.shape[1:]
+        if head[1] is None or any(b is None or w.shape[1:] != k or w.shape[0] % 8 for w, b in ada):
+            return None  # (adaLN projections that would not lie side by side)
+        params = [w for w, _ in ada] + [b for _, b in ada] + [*head]
         scale, align = [1.0] * len(params), [False] * (len(params) - 2) + [True] * 2
-        naive = _PassCasts._plain(net.embed, NaiveEmbed) and net.embed.seq.bias is not None
+        naive = _PassCasts._plain(embed, NaiveEmbed) and embed.seq.bias is not None
         if naive:
-            params += [net.embed.seq.weight, net.embed.seq.bias]
-            scale += [1.0 / net.embed.coeff, 1.0]
+            params += _params(embed.seq)
+            scale += [1.0 / embed.coeff, 1.0]
             align += [True] * 2
         biased = []
-        for blk in net.blocks:
+        for blk in blocks:
             for m in blk.linears():
-                b = m.bias
+                w, b = _params(m)
                 biased.append(b is not None)
-                params += [m.weight] if b is None else [m.weight, b]
+                params += [w] if b is None else [w, b]
         scale += [1.0] * (len(params) - len(scale))
         align += [False] * (len(params) - len(align))
         casts = _nodes.module().cast_params(params, scale, align, dtype == torch.bfloat16)
-        return None if casts is None else _PassCasts(casts, ada, naive, biased)
+        return None if casts is None else _PassCasts(casts, [w.shape[0] for w, _ in ada], k[0], naive, biased)
 
     def modulation(self, cond):
         return F.linear(cond, self.ada_weight, self.ada_bias).split(self.sizes, dim=1)
@@ -240,18 +250,25 @@ class _PassCasts:
     def _plain(module, cls):
         """Whether calling ``module`` is ``cls.forward`` and nothing else: no subclass, wrapper, replaced method or hook, any of
         which may look at the arguments or change them."""
-        hooks = torch.nn.modules.module
-        return (type(module) is cls and "forward" not in module.__dict__ and not (module._forward_hooks or module._forward_pre_hooks)
+        own, hooks = module.__dict__, torch.nn.modules.module
+        return (type(module) is cls and "forward" not in own and not (own["_forward_hooks"] or own["_forward_pre_hooks"])
                 and not (hooks._global_forward_hooks or hooks._global_forward_pre_hooks))
+
+    @staticmethod
+    def _plain_blocks(net):
+        blocks = list(net.blocks)
+        return blocks if all([_PassCasts._plain(b, Block) for b in blocks]) else None
 
     @staticmethod
     def chained(net):
         """Whether the blocks may be run as one chain of operations: plain blocks, no dropout, and LayerNorms that the kernels take
         (for others it is autocast that makes torch's LayerNorm accept 16-bit rows, and keeps its result in fp32)."""
-        norms = [n for b in net.blocks for n in (b.norm1, b.norm2)] + [net.norm_out]
-        return (len(net.blocks) > 0 and all(_PassCasts._plain(b, Block) and not (b.training and b.drop.p > 0.0) for b in net.blocks)
-                and all(isinstance(n, nn.LayerNorm) and n.weight is not None and n.weight.dtype == torch.float32
-                        and n.weight.numel() in CHANNELS for n in norms))
+        blocks = _PassCasts._plain_blocks(net)
+        if not blocks or any([b.training and b.drop.p > 0.0 for b in blocks]):
+            return False
+        norms = [b._modules[n] for b in blocks for n in ("norm1", "norm2")] + [net.norm_out]
+        weights = [_params(n)[0] for n in norms if isinstance(n, nn.LayerNorm)]
+        return len(weights) == len(norms) and all([w is not None and w.dtype == torch.float32 and w.numel() in CHANNELS for w in weights])
 
     def run(self, net, h, mods, attention):
         """``net``'s blocks and output normalisation: each gated residual goes with the LayerNorm behind it, also across blocks.
