@@ -312,7 +312,7 @@ const char *jvpattn_kernel_name(int id);
 
 /* Synchronises the current device and returns the device-side status word: 0 if no bounded wait has
  * run out since the last call, else a code identifying the wait that gave up (101..107 forward, 201..221
- * backward).  Clears the word.  Every wait inside the kernels is bounded (about two seconds): a kernel whose
+ * backward, 300..328 the backward of sequences within one tile).  Clears the word.  Every wait inside the kernels is bounded (about two seconds): a kernel whose
  * wait runs out stops computing, leaves through its normal teardown and leaves its outputs unwritten or partial;
  * the context stays usable. */
 int jvpattn_device_status(void);

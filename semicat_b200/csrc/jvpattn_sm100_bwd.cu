@@ -789,7 +789,7 @@ __global__ void __launch_bounds__(bwd_threads(bwd_parts(TILE), bwd_two_issuers(D
     // per-column statistics of the key owner: the first TILE compute threads fetch one query column each,
     // one tile ahead (also across items), and publish it through shared memory
     // (bh: the item's (batch, head) row of the statistics.  Taking the item apart at every tile kept all warps in front of the barrier
-    // below: 2585 -> 2445 cycles per tile at head_dim 64.  Long calls run at the power limit, where the clock takes most of that back.)
+    // below: 4 x 16 heads of length 2048 at head_dim 64 573.9k -> 567.5k cycles.)
     auto fetch_stat = [&](int bh, int j_) -> float4 {
       const int col = j_ * TILE + ctid;
       if (ctid >= TILE || col >= a.Lq) return make_float4(INFINITY, 0.f, 0.f, 0.f);  // padded query: P = 0

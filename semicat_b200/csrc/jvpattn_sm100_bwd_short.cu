@@ -483,8 +483,11 @@ cudaError_t launch_short(const BwdArgs &a, cudaStream_t stream) {
 
 }  // namespace
 
-// Fewer than 16 pairs leave most of the GPU idle either way and their call is bound by the host (8 pairs of length 128: 10.7 us in
-// three kernels, 8.4 us here, 250 us the call); they keep the kernels that split a pair.
+// The line at 16 pairs is not where the kernels cross.  In a graph this one is faster from the first pair on: 1, 8 and 15 pairs of
+// length 128 8.2, 8.4, 8.4 us against 10.2, 10.4, 10.4 in three kernels, of length 32 6.3 against 8.3, without tangents 6.2 against
+// 8.4.  Fewer pairs keep the kernels that split a pair because the PyTorch call around either takes 250 us.  From 16 on it is the
+// faster one at every length (24 to 3072 pairs, queries x keys 1 x 1: 5.6-61 us against 8.1-120; 1 x 128 7.8-104 against 9.1-159;
+// 128 x 1 7.1-87 against 9.6-181; 100 x 100 8.2-122 against 10.8-222).
 bool sm100_bwd_short_ok(const BwdArgs &a) {
   return a.D == 64 && a.Lq <= kRows && a.Lk <= kRows && (int64_t)a.B * a.H >= 16 && (int64_t)a.B * a.H < (int64_t(1) << 30);
 }
