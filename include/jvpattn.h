@@ -150,7 +150,8 @@ int jvpattn_rotary_qkv(const void *const in[3], const int64_t in_strides[9], int
  * tangent with respect to x: 0 reproduces PyTorch,
  * whose forward-mode formula for native_layer_norm treats the saved mean / rstd as constants when it is differentiated
  * again; 1 includes their dependence on x.  Bit 1 (which = 3 only): add to what dx holds instead of overwriting it, so that
- * the two backward kernels of one (primal, tangent) pair leave their sum. */
+ * the two backward kernels of one (primal, tangent) pair leave their sum.  Every pointer but mean, rstd and sums 16-byte aligned
+ * (else JVPATTN_EALIGN). */
 int jvpattn_ln_modulate(int which, const void *x, const void *tx, const float *gamma, const float *beta, const void *shift,
                         const void *scale, const void *tshift, const void *tscale, int64_t mod_stride, int64_t tmod_stride,
                         float *mean, float *rstd, void *out, const void *g, void *dx, void *dtx, float *sums, int batch, int len,

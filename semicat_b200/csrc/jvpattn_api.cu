@@ -265,6 +265,9 @@ int jvpattn_ln_modulate(int which, const void *x, const void *tx, const float *g
   if ((which == 0 && (!shift || !out)) || (which == 1 && (!tx || !out)) || (which >= 2 && (!g || !dx || !sums)) ||
       (which == 3 && (!tx || !dtx)))
     return JVPATTN_EINVAL;
+  for (const void *p : {x, tx, (const void *)gamma, (const void *)beta, shift, scale, tshift, tscale, (const void *)out, g, (const void *)dx,
+                        (const void *)dtx})
+    if (p && reinterpret_cast<uintptr_t>(p) % 16) return JVPATTN_EALIGN;
   if (mod_stride % 8 || tmod_stride % 8) return JVPATTN_EALIGN;
   return note_cuda(ln_modulate(which, x, tx, gamma, beta, shift, scale, tshift, tscale, mod_stride, tmod_stride, mean, rstd, out, g,
                                dx, dtx, sums, batch, len, channels, eps, exact, dtype, static_cast<cudaStream_t>(stream)));

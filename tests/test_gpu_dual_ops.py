@@ -385,3 +385,32 @@ def test_ln_modulate_gradients_of_many_samples(B):
     want = torch.nn.functional.layer_norm(x.float(), (C,)) * gy.float()
     assert bool(((d_scale.float() - want).abs() <= 2 ** -7 * want.abs() + 1e-5).all())
     assert _lib.device_status() == 0
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("which", ["x", "shift", "weight", "bias", "cotangent"])
+def test_ln_modulate_refuses_rows_off_the_16_byte_grid(dtype, which):
+    """The kernels read 16 bytes at a time: contiguous tensors that start between two such places are refused, as by the other ops."""
+    B, S, C = 2, 5, 256
+    off = lambda t: torch.cat((t.flatten()[:1], t.flatten()))[1:].view(t.shape)
+    place = lambda name, t: off(t) if name == which else t
+    norm = torch.nn.LayerNorm(C, device="cuda")
+    norm.weight = torch.nn.Parameter(place("weight", torch.ones(C, device="cuda")))
+    norm.bias = torch.nn.Parameter(place("bias", torch.ones(C, device="cuda")))
+    x, shift, scale = place("x", torch.ones(B, S, C, device="cuda", dtype=dtype)), *(place(n, torch.ones(B, C, device="cuda", dtype=dtype)) for n in ("shift", "scale"))
+
+    def refused(f):
+        with pytest.raises(_lib.JvpAttnError) as e:
+            f()
+        assert e.value.code == -3
+
+    if which == "cotangent":
+        y = dual_ops.ln_modulate(x.requires_grad_(True), norm, shift, scale)
+        refused(lambda: torch.autograd.grad(y, [x], off(torch.ones_like(y))))
+    else:
+        call = lambda a: dual_ops.ln_modulate(a, norm, shift, scale)
+        with torch.no_grad():
+            refused(lambda: call(x))
+        refused(lambda: torch.func.jvp(call, (x,), (torch.ones_like(x),)))
+        refused(lambda: call(x.detach().requires_grad_(True)))
+    assert _lib.device_status() == 0
